@@ -19,6 +19,10 @@ struct dgc_ctx {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_begin = nullptr, ev_end = nullptr, ev_sync = nullptr;
   int32_t *status_dev = nullptr;  // device status word: kernels report failures here
+  // cells of launches whose blocks hand values on (chain.cuh): one set for the context stream, one for the side stream,
+  // so that a plan may run such a launch on both at once
+  unsigned long long *chain_dev[2] = {nullptr, nullptr};
+  uint64_t chain_cells[2] = {0, 0};
   unsigned int *ticket_dev = nullptr;  // last-block-done counter of the multi-block reductions (kept at 0)
   int64_t launches = 0;
   char err[512] = {0};
@@ -81,6 +85,8 @@ int32_t dgc_fail(dgc_ctx *ctx, int32_t code, const char *fmt, ...);
 int32_t dgc_check_launch(dgc_ctx *ctx, const char *what);
 // returns device pointer to at least n floats of context scratch (nullptr + error set on failure)
 float *dgc_ctx_scratch(dgc_ctx *ctx, uint64_t nfloats);
+// 1 + n zero-initialised 64-bit words for a launch on the current stream: the ticket word, then n cells (chain.cuh)
+unsigned long long *dgc_ctx_chain(dgc_ctx *ctx, uint64_t n);
 // [F][4] ints: frames whose floor control row is r are [a,b) and [c,d) (second run: after the clock wrap)
 const int *dgc_ctx_row_ranges(dgc_ctx *ctx, int F, int T);
 // [T] float2: x = bits of the floor control row (int), y = lerp fraction of sampleRow at the cached clock

@@ -46,6 +46,30 @@ float *dgc_ctx_scratch(dgc_ctx *ctx, uint64_t nfloats) {
   return p;
 }
 
+unsigned long long *dgc_ctx_chain(dgc_ctx *ctx, uint64_t n) {
+  const int side = ctx->aux_stream && ctx->stream == ctx->aux_stream;
+  if (n <= ctx->chain_cells[side]) return ctx->chain_dev[side];
+  if (ctx->chain_dev[side]) {
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(ctx->chain_dev[side]);
+    ctx->chain_dev[side] = nullptr;
+    ctx->chain_cells[side] = 0;
+    ctx->buffer_generation++;
+  }
+  const uint64_t want = n < 4096 ? 4096 : n;
+  unsigned long long *p = nullptr;
+  cudaError_t e = cudaMalloc(&p, (want + 1) * sizeof(*p));
+  if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, (want + 1) * sizeof(*p), ctx->stream);
+  if (e != cudaSuccess) {
+    if (p) cudaFree(p);
+    dgc_fail(ctx, DGC_ERR_OOM, "%llu chain cells: %s", (unsigned long long)want, cudaGetErrorString(e));
+    return nullptr;
+  }
+  ctx->chain_dev[side] = p;
+  ctx->chain_cells[side] = want;
+  return p;
+}
+
 template <typename T>
 static T *upload_table(dgc_ctx *ctx, const std::vector<T> &h) {
   T *d = nullptr;
@@ -195,6 +219,8 @@ DGC_EXPORT int32_t dgc_ctx_destroy(dgc_ctx *c) {
   if (c->fork_ev) cudaEventDestroy(c->fork_ev);
   if (c->join_ev) cudaEventDestroy(c->join_ev);
   if (c->aux_stream) cudaStreamDestroy(c->aux_stream);
+  for (auto &p : c->chain_dev)
+    if (p) cudaFree(p);
   if (c->wt_buf) cudaFree(c->wt_buf);
   if (c->dzt_buf) cudaFree(c->dzt_buf);
   if (c->status_dev) cudaFree(c->status_dev);

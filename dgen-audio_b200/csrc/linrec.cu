@@ -8,6 +8,9 @@
 // chunk-to-chunk carry is an affine map (a power of the 2x2 transition matrix) resolved by a short
 // scan, and a second sweep produces the output (forward) or the gradient sums (backward; by
 // linearity the sums are corrected for the carried adjoint state without re-reading the signals).
+#include <math.h>
+
+#include "chain.cuh"
 #include "common.cuh"
 
 namespace {
@@ -15,140 +18,206 @@ namespace {
 // ---------------------------------------------------------------------------------------------
 // one-pole  y[n] = x[n] + a*y[n-1]
 // ---------------------------------------------------------------------------------------------
-constexpr int OP_THREADS = 256, OP_PER = 8, OP_CHUNK = OP_THREADS * OP_PER;
+// One launch: a block takes a tile of 2048 frames of one voice (ticket order, tiles of all voices side by side), runs it
+// from rest, publishes its end value, sums the end values of the tiles before it -- decayed, in a fixed order, in double,
+// as far back as a^(2048 j) is not yet nothing in single precision -- and writes the tile from that state.  Nothing waits
+// for anything but end values, which need no wait themselves, so there is no chain along time, and x is read once: bound
+// by HBM, short of it by the latency of a tile (load, scan, end value, store) over eight resident blocks.  64 x 262144
+// frames: 36 us = 3.7 TB/s, against 66 us for a pass for the end values, a serial carry and a second pass; 1 x 65536: one
+// launch of 4 us instead of three of 11.
+constexpr int OP_THREADS = 128, OP_PER = 16, OP_TILE = OP_THREADS * OP_PER, OP_WARPS = OP_THREADS / 32;
+constexpr int OP_BLOCKS = 8;    // resident per SM
 
-// inclusive scan over the block of v_t = sum_{s<=t} r^(t-s) * e_s   (r = a^OP_PER), via shuffles
-__device__ __forceinline__ float block_decay_scan(float e, const float *rpow /* r^(2^i), i<8 */, float *warp_tot,
-                                                  int tid) {
-  float v = e;
-#pragma unroll
-  for (int i = 0; i < 5; ++i) {
-    float o = __shfl_up_sync(0xffffffffu, v, 1 << i);
-    if ((tid & 31) >= (1 << i)) v = fmaf(rpow[i], o, v);
+// powers of the coefficient, evaluated in double on the host and rounded once
+struct OnepolePowers {
+  float a, r[7];          // a, and r^(2^i) with r = a^OP_PER
+  double tile[6];         // A^(2^i) with A = a^OP_TILE
+  int reach;              // tiles whose end values still matter: |A|^reach vanishes in single precision
+};
+
+OnepolePowers onepole_powers(float a) {
+  OnepolePowers p;
+  p.a = a;
+  double r = 1.0;
+  for (int i = 0; i < OP_PER; ++i) r *= (double)a;
+  for (int i = 0; i < 7; ++i) {
+    p.r[i] = (float)r;
+    r *= r;
   }
-  if ((tid & 31) == 31) warp_tot[tid >> 5] = v;
-  __syncthreads();
-  if (tid < 32) {
-    float w = tid < OP_THREADS / 32 ? warp_tot[tid] : 0.0f;
-    // scan over warps with multiplier r^32 = rpow[5], r^64, r^128
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      float o = __shfl_up_sync(0xffffffffu, w, 1 << i);
-      if (tid >= (1 << i)) w = fmaf(rpow[5 + i], o, w);
-    }
-    if (tid < OP_THREADS / 32) warp_tot[tid] = w;
+  for (int i = 0; i < 6; ++i) {                      // r is now a^(OP_PER 2^7) = a^OP_TILE
+    p.tile[i] = r;
+    r *= r;
   }
-  __syncthreads();
-  if (tid >= 32) {
-    // add the carry of all previous warps, decayed by r^(lane+1)
-    float carry = warp_tot[(tid >> 5) - 1];
-    float d = rpow[8 + (tid & 31)];
-    v = fmaf(d, carry, v);
-  }
-  return v;
+  static_assert(OP_TILE == OP_PER << 7, "the powers double from a thread's run to a tile");
+  const double lg = fabs(p.tile[0]) > 0.0 ? log2(fabs(p.tile[0])) : -1e30;
+  p.reach = lg >= -1e-7 ? 0x7fffffff : (int)fmin(ceil(-160.0 / lg), 1e9);
+  return p;
 }
 
-// phase 0: chunk end values with zero carry-in; phase 1: final output using carry[chunk]
-// REV: the same scan run backwards in time (frame n of the scan is memory index T-1-n): the adjoint recursion
-// lam[n] = g[n] + a lam[n+1] of the filter's backward pass.
-template <int PHASE, bool REV = false>
-__global__ void __launch_bounds__(OP_THREADS)
-onepole_kernel(const float *__restrict__ x, int T, int NC, float a, const float *__restrict__ carry_in,
-               float *__restrict__ chunk_end, float *__restrict__ y) {
-  __shared__ float rpow[8 + 32];
-  __shared__ float warp_tot[OP_THREADS / 32];
-  const int tid = threadIdx.x, c = blockIdx.x, b = blockIdx.y;
-  if (tid == 0) {
-    float r = 1.0f;
-    for (int i = 0; i < OP_PER; ++i) r *= a;  // a^OP_PER
-    float p = r;
-    for (int i = 0; i < 8; ++i) { rpow[i] = p; p *= p; }
-    float q = r;
-    for (int i = 0; i < 32; ++i) { rpow[8 + i] = q; q *= r; }  // r^(i+1)
-  }
-  __syncthreads();
-  const float *xb = x + (size_t)b * T;
-  const int n0 = c * OP_CHUNK + tid * OP_PER;
-  float loc[OP_PER];
-  float prev = 0.0f;
-  static_assert(OP_PER == 8, "the vector path moves a thread's run as two 128-bit words");
-  // a thread's run of eight frames is 32 contiguous bytes: two 128-bit accesses when the voice row is aligned
-  // memory index of the run's lowest address: n0 forwards, T - n0 - 8 backwards (the run is then read high to low)
+// A thread's run of sixteen frames is 64 contiguous bytes: four 128-bit accesses when it lies on a 16-byte boundary.
+// REV: the scan's frame n is memory index T-1-n, the run is then read high to low.
+template <bool REV>
+__device__ __forceinline__ void onepole_load(const float *xb, int T, int n0, float *v) {
   const int m0 = REV ? T - n0 - OP_PER : n0;
-  const bool vec = n0 + OP_PER <= T && ((((uintptr_t)(xb + m0)) | (PHASE == 1 ? (uintptr_t)(y + (size_t)b * T + m0) : 0)) & 15) == 0;
-  if (vec) {
-    const float4 u = __ldg(reinterpret_cast<const float4 *>(xb + m0)), w = __ldg(reinterpret_cast<const float4 *>(xb + m0) + 1);
-    if (REV) {
-      loc[7] = u.x; loc[6] = u.y; loc[5] = u.z; loc[4] = u.w;
-      loc[3] = w.x; loc[2] = w.y; loc[1] = w.z; loc[0] = w.w;
-    } else {
-      loc[0] = u.x; loc[1] = u.y; loc[2] = u.z; loc[3] = u.w;
-      loc[4] = w.x; loc[5] = w.y; loc[6] = w.z; loc[7] = w.w;
+  if (n0 + OP_PER <= T && ((uintptr_t)(xb + m0) & 15) == 0) {
+#pragma unroll
+    for (int q = 0; q < OP_PER / 4; ++q) {
+      const float4 u = *(reinterpret_cast<const float4 *>(xb + m0) + q);
+      const int k = REV ? OP_PER - 1 - 4 * q : 4 * q, d = REV ? -1 : 1;
+      v[k] = u.x; v[k + d] = u.y; v[k + 2 * d] = u.z; v[k + 3 * d] = u.w;
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < OP_PER; ++j) loc[j] = (n0 + j < T) ? xb[REV ? T - 1 - (n0 + j) : n0 + j] : 0.0f;
+    for (int j = 0; j < OP_PER; ++j) v[j] = (n0 + j < T) ? xb[REV ? T - 1 - (n0 + j) : n0 + j] : 0.0f;
   }
+}
+
+template <bool REV>
+__device__ __forceinline__ void onepole_store(float *yb, int T, int n0, const float *v) {
+  const int m0 = REV ? T - n0 - OP_PER : n0;
+  if (n0 + OP_PER <= T && ((uintptr_t)(yb + m0) & 15) == 0) {
 #pragma unroll
-  for (int j = 0; j < OP_PER; ++j) {
-    prev = fmaf(a, prev, loc[j]);
-    loc[j] = prev;
-  }
-  float incl = block_decay_scan(prev, rpow, warp_tot, tid);  // state at the end of this thread's run
-  if (PHASE == 0) {
-    if (tid == OP_THREADS - 1) chunk_end[(size_t)b * NC + c] = incl;
-    return;
-  }
-  // state entering this thread's run = (incl - prev)/... simpler: exclusive value via shuffle
-  float excl = __shfl_up_sync(0xffffffffu, incl, 1);
-  __shared__ float last_of_warp[OP_THREADS / 32];
-  if ((tid & 31) == 31) last_of_warp[tid >> 5] = incl;
-  __syncthreads();
-  if ((tid & 31) == 0) excl = tid == 0 ? 0.0f : last_of_warp[(tid >> 5) - 1];
-  // carry from previous chunks decays by a^(tid*OP_PER) before reaching this thread
-  float cin = carry_in[(size_t)b * NC + c];
-  float dec = 1.0f;
-  {
-    // a^(tid*OP_PER) = r^tid from the binary powers
-    int e = tid;
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (e & (1 << i)) dec *= rpow[i];
-  }
-  float state = fmaf(dec, cin, excl);
-  float *yb = y + (size_t)b * T;
-  float ap = a;
-#pragma unroll
-  for (int j = 0; j < OP_PER; ++j) {
-    loc[j] = fmaf(ap, state, loc[j]);
-    ap *= a;
-  }
-  if (vec && REV) {
-    __stcs(reinterpret_cast<float4 *>(yb + m0), make_float4(loc[7], loc[6], loc[5], loc[4]));
-    __stcs(reinterpret_cast<float4 *>(yb + m0) + 1, make_float4(loc[3], loc[2], loc[1], loc[0]));
-  } else if (vec) {
-    __stcs(reinterpret_cast<float4 *>(yb + n0), make_float4(loc[0], loc[1], loc[2], loc[3]));
-    __stcs(reinterpret_cast<float4 *>(yb + n0) + 1, make_float4(loc[4], loc[5], loc[6], loc[7]));
+    for (int q = 0; q < OP_PER / 4; ++q) {
+      const int k = REV ? OP_PER - 1 - 4 * q : 4 * q, d = REV ? -1 : 1;
+      __stcs(reinterpret_cast<float4 *>(yb + m0) + q, make_float4(v[k], v[k + d], v[k + 2 * d], v[k + 3 * d]));
+    }
   } else {
 #pragma unroll
     for (int j = 0; j < OP_PER; ++j)
-      if (n0 + j < T) yb[REV ? T - 1 - (n0 + j) : n0 + j] = loc[j];
+      if (n0 + j < T) yb[REV ? T - 1 - (n0 + j) : n0 + j] = v[j];
   }
 }
 
-// carry[c] = state entering chunk c; serial over chunks (few), one thread per voice
-// y0_dev (optional): per-voice state entering the first chunk (the history cell before the call), else y0
-__global__ void onepole_carry_kernel(const float *__restrict__ chunk_end, int B, int NC, float a, float y0,
-                                     float *__restrict__ carry, const float *__restrict__ y0_dev = nullptr) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= B) return;
-  float ac = 1.0f;
-  for (int i = 0; i < OP_CHUNK; ++i) ac *= a;
-  float s = y0_dev ? y0_dev[b] : y0;
-  for (int c = 0; c < NC; ++c) {
-    carry[(size_t)b * NC + c] = s;
-    s = fmaf(ac, s, chunk_end[(size_t)b * NC + c]);
+// REV: the same scan run backwards in time, the adjoint recursion lam[n] = g[n] + a lam[n+1] of the filter's backward
+// pass.  y may be x.  state (optional): per voice the state entering the first frame, and on return the one after the
+// last.  The blocks stay: while a tile is scanned the loads of the block's next one are in flight and the ticket after
+// that is being drawn, else every tile pays the ticket's, the loads' and the end values' latency one after the other.
+template <bool REV>
+__global__ void __launch_bounds__(OP_THREADS, OP_BLOCKS)
+onepole_kernel(const float *x, int B, int T, int NT, const OnepolePowers pw, float *state, float *y,
+               unsigned long long *__restrict__ chain, int32_t *status) {
+  __shared__ float warp_end[2][OP_WARPS];
+  __shared__ float sh_in[2];
+  __shared__ uint32_t sh_index[2], sh_epoch;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t total = (uint32_t)B * (uint32_t)NT, tickets = total + gridDim.x;   // every block draws one too many
+  if (tid == 0) {
+    const dgchain::Ticket t = dgchain::take_ticket(chain, tickets);
+    sh_epoch = t.epoch;
+    sh_index[0] = t.index;
+    sh_index[1] = t.index < total ? dgchain::take_ticket(chain, tickets).index : total;
   }
+  __syncthreads();
+  const uint32_t epoch = sh_epoch;
+  uint32_t index = sh_index[0], next = sh_index[1];
+  const float a = pw.a;
+  float loc[OP_PER], ahead[OP_PER];
+  if (index < total) {
+    const int tile = (int)(index / (uint32_t)B), b = (int)(index - (uint32_t)tile * B);
+    onepole_load<REV>(x + (size_t)b * T, T, tile * OP_TILE + tid * OP_PER, loc);
+  }
+  for (int par = 0; index < total; par ^= 1) {
+    const int tile = (int)(index / (uint32_t)B), b = (int)(index - (uint32_t)tile * B);
+    const int n0 = tile * OP_TILE + tid * OP_PER;
+    unsigned long long *cells = chain + 1 + (size_t)b * NT;
+    uint32_t after = total;
+    if (next < total) {
+      const int t1 = (int)(next / (uint32_t)B), b1 = (int)(next - (uint32_t)t1 * B);
+      onepole_load<REV>(x + (size_t)b1 * T, T, t1 * OP_TILE + tid * OP_PER, ahead);
+      if (tid == 0) after = dgchain::take_ticket(chain, tickets).index;
+    }
+    float prev = 0.0f;
+#pragma unroll
+    for (int j = 0; j < OP_PER; ++j) {
+      prev = fmaf(a, prev, loc[j]);
+      loc[j] = prev;
+    }
+    // state at the end of this thread's run, the tile started from rest: decayed scan over the warp, then over the warps
+    float v = prev;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const float o = __shfl_up_sync(0xffffffffu, v, 1 << i);
+      if (lane >= (1 << i)) v = fmaf(pw.r[i], o, v);
+    }
+    float excl = __shfl_up_sync(0xffffffffu, v, 1);
+    if (lane == 0) excl = 0.0f;
+    if (lane == 31) warp_end[par][warp] = v;
+    __syncthreads();
+    if (warp == 0) {
+      float w = lane < OP_WARPS ? warp_end[par][lane] : 0.0f;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float o = __shfl_up_sync(0xffffffffu, w, 1 << i);
+        if (lane >= (1 << i)) w = fmaf(pw.r[5 + i], o, w);
+      }
+      float in = 0.0f;
+      if (tile == 0) {
+        if (state) in = state[b];
+        if (lane == OP_WARPS - 1 && NT > 1) dgchain::publish(cells, epoch, fmaf((float)pw.tile[0], in, w));
+      } else {
+        if (lane == OP_WARPS - 1 && tile < NT - 1) dgchain::publish(cells + tile, epoch, w);
+        // sum over j of A^j end[tile - 1 - j]
+        double decay = 1.0, acc = 0.0;
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+          if (lane & (1 << i)) decay *= pw.tile[i];
+        const int far = min(tile, pw.reach);
+        for (int j = lane; j < far; j += 32) {
+          acc += decay * (double)dgchain::await(cells + tile - 1 - j, epoch, status);
+          decay *= pw.tile[5];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        in = (float)acc;
+        // the first tile has read the state cell before this, the last, tile writes it
+        if (state && tile == NT - 1 && lane == 0) dgchain::await(cells, epoch, status);
+      }
+      if (lane < OP_WARPS) warp_end[par][lane] = w;
+      if (lane == 0) {
+        sh_in[par] = in;
+        sh_index[par] = after;
+      }
+    }
+    __syncthreads();
+    // state entering this thread's run: what its warp gathered, what the warps before left, what entered the tile
+    float d = 1.0f;
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+      if (lane & (1 << i)) d *= pw.r[i];
+    if (warp > 0) excl = fmaf(d, warp_end[par][warp - 1], excl);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (warp & (1 << i)) d *= pw.r[5 + i];
+    float s = fmaf(d, sh_in[par], excl);
+#pragma unroll
+    for (int j = 0; j < OP_PER; ++j) {
+      s *= a;
+      loc[j] += s;
+    }
+    onepole_store<REV>(y + (size_t)b * T, T, n0, loc);
+    if (state && tile == NT - 1) {
+#pragma unroll
+      for (int j = 0; j < OP_PER; ++j)
+        if (n0 + j == T - 1) state[b] = loc[j];
+    }
+    index = next;
+    next = sh_index[par];
+#pragma unroll
+    for (int j = 0; j < OP_PER; ++j) loc[j] = ahead[j];
+  }
+}
+
+template <bool REV>
+int32_t launch_onepole(dgc_ctx *ctx, const float *x, int B, int T, float a, float *state, float *y, const char *what) {
+  const int NT = dgc_div_up(T, OP_TILE);
+  const uint64_t tiles = (uint64_t)B * NT, room = (uint64_t)ctx->sm_count * OP_BLOCKS;
+  DGC_REQUIRE(ctx, tiles <= 0x7fffffffull, "B * T too large");
+  unsigned long long *chain = dgc_ctx_chain(ctx, tiles);
+  if (!chain) return DGC_ERR_OOM;
+  onepole_kernel<REV><<<(unsigned)(tiles < room ? tiles : room), OP_THREADS, 0, ctx->stream>>>(x, B, T, NT, onepole_powers(a), state, y, chain,
+                                                                        ctx->status_dev);
+  DGC_LAUNCHED(ctx, what);
+  return DGC_OK;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -701,46 +770,15 @@ __global__ void sum_doubles_kernel(const double *__restrict__ v, int n, double *
 }  // namespace
 
 DGC_EXPORT int32_t dgc_onepole_fwd(dgc_ctx *ctx, const float *x_dev, int32_t B, int32_t T, float a, float *y_dev) {
-  if (!ctx) return DGC_ERR_INVALID;
-  DGC_REQUIRE(ctx, x_dev && y_dev, "null pointer");
-  DGC_REQUIRE(ctx, B > 0 && T > 0, "size out of range");
-  const int NC = dgc_div_up(T, OP_CHUNK);
-  float *scr = dgc_ctx_scratch(ctx, 2ull * B * NC + 8);
-  if (!scr) return DGC_ERR_OOM;
-  float *chunk_end = scr, *carry = scr + (size_t)B * NC;
-  onepole_kernel<0><<<dim3(NC, B), OP_THREADS, 0, ctx->stream>>>(x_dev, T, NC, a, nullptr, chunk_end, nullptr);
-  DGC_LAUNCHED(ctx, "onepole_pass0");
-  onepole_carry_kernel<<<dgc_div_up(B, 64), 64, 0, ctx->stream>>>(chunk_end, B, NC, a, 0.0f, carry);
-  DGC_LAUNCHED(ctx, "onepole_carry");
-  onepole_kernel<1><<<dim3(NC, B), OP_THREADS, 0, ctx->stream>>>(x_dev, T, NC, a, carry, nullptr, y_dev);
-  DGC_LAUNCHED(ctx, "onepole_pass1");
-  return DGC_OK;
-}
-
-__global__ void onepole_final_state_kernel(const float *__restrict__ y, int B, int T, float *__restrict__ state) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < B) state[b] = y[(size_t)b * T + T - 1];
+  return dgc_onepole_fwd_state(ctx, x_dev, B, T, a, nullptr, y_dev);
 }
 
 DGC_EXPORT int32_t dgc_onepole_fwd_state(dgc_ctx *ctx, const float *x_dev, int32_t B, int32_t T, float a,
                                          float *state_dev, float *y_dev) {
   if (!ctx) return DGC_ERR_INVALID;
-  if (!state_dev) return dgc_onepole_fwd(ctx, x_dev, B, T, a, y_dev);
   DGC_REQUIRE(ctx, x_dev && y_dev, "null pointer");
   DGC_REQUIRE(ctx, B > 0 && T > 0, "size out of range");
-  const int NC = dgc_div_up(T, OP_CHUNK);
-  float *scr = dgc_ctx_scratch(ctx, 2ull * B * NC + 8);
-  if (!scr) return DGC_ERR_OOM;
-  float *chunk_end = scr, *carry = scr + (size_t)B * NC;
-  onepole_kernel<0><<<dim3(NC, B), OP_THREADS, 0, ctx->stream>>>(x_dev, T, NC, a, nullptr, chunk_end, nullptr);
-  DGC_LAUNCHED(ctx, "onepole_pass0");
-  onepole_carry_kernel<<<dgc_div_up(B, 64), 64, 0, ctx->stream>>>(chunk_end, B, NC, a, 0.0f, carry, state_dev);
-  DGC_LAUNCHED(ctx, "onepole_carry");
-  onepole_kernel<1><<<dim3(NC, B), OP_THREADS, 0, ctx->stream>>>(x_dev, T, NC, a, carry, nullptr, y_dev);
-  DGC_LAUNCHED(ctx, "onepole_pass1");
-  onepole_final_state_kernel<<<dgc_div_up(B, 128), 128, 0, ctx->stream>>>(y_dev, B, T, state_dev);
-  DGC_LAUNCHED(ctx, "onepole_final_state");
-  return DGC_OK;
+  return launch_onepole<false>(ctx, x_dev, B, T, a, state_dev, y_dev, "onepole");
 }
 
 static int32_t biquad_validate(dgc_ctx *ctx, const dgc_biquad_params *p) {
@@ -916,19 +954,14 @@ DGC_EXPORT int32_t dgc_onepole_bwd(dgc_ctx *ctx, const float *y_dev, const float
   DGC_REQUIRE(ctx, grad_a_dev == nullptr || y_dev != nullptr, "the coefficient gradient needs the forward output");
   DGC_REQUIRE(ctx, B > 0 && T > 0, "size out of range");
   DGC_REQUIRE(ctx, gy_dev != grad_x_dev, "in-place operation is not supported");
-  const int NC = dgc_div_up(T, OP_CHUNK);
-  DGC_REQUIRE(ctx, NC <= 65535 * 32 && B <= 65535, "size out of range");
-  const uint64_t need = 2ull * B * NC + 2ull * B * OPG_SEGS + 8;
-  float *scr = dgc_ctx_scratch(ctx, need);
-  if (!scr) return DGC_ERR_OOM;
-  float *chunk_end = scr, *carry = scr + (size_t)B * NC;
-  double *part = reinterpret_cast<double *>(scr + (((size_t)2 * B * NC + 1) & ~(size_t)1));
-  onepole_kernel<0, true><<<dim3(NC, B), OP_THREADS, 0, ctx->stream>>>(gy_dev, T, NC, a, nullptr, chunk_end, nullptr);
-  DGC_LAUNCHED(ctx, "onepole_bwd_pass0");
-  onepole_carry_kernel<<<dgc_div_up(B, 64), 64, 0, ctx->stream>>>(chunk_end, B, NC, a, 0.0f, carry);
-  DGC_LAUNCHED(ctx, "onepole_bwd_carry");
-  onepole_kernel<1, true><<<dim3(NC, B), OP_THREADS, 0, ctx->stream>>>(gy_dev, T, NC, a, carry, nullptr, grad_x_dev);
-  DGC_LAUNCHED(ctx, "onepole_bwd_pass1");
+  DGC_REQUIRE(ctx, B <= 65535, "size out of range");
+  double *part = nullptr;
+  if (grad_a_dev) {
+    part = reinterpret_cast<double *>(dgc_ctx_scratch(ctx, 2ull * B * OPG_SEGS));
+    if (!part) return DGC_ERR_OOM;
+  }
+  const int32_t rc = launch_onepole<true>(ctx, gy_dev, B, T, a, nullptr, grad_x_dev, "onepole_bwd");
+  if (rc != DGC_OK) return rc;
   if (grad_a_dev) {
     onepole_ga_kernel<<<dim3(OPG_SEGS, B), 256, 0, ctx->stream>>>(grad_x_dev, y_dev, T, part);
     DGC_LAUNCHED(ctx, "onepole_grad_a");
@@ -994,15 +1027,15 @@ DGC_EXPORT int32_t dgc_biquad_bwd(dgc_ctx *ctx, const dgc_biquad_params *p, cons
 
 namespace {
 constexpr int STATIC_MAX_CHUNKS = DGC_ONEPOLE_STATIC_MAX_CHUNKS;
-// [0, MAX): end value of every chunk; [MAX, 2 MAX): carry entering every chunk
-static __device__ __align__(256) float g_onepole_static_scratch[2 * STATIC_MAX_CHUNKS];
+// the ticket word and a cell per tile (chain.cuh); zero when the library is loaded, never cleared after that
+static __device__ __align__(256) unsigned long long g_onepole_static_scratch[1 + STATIC_MAX_CHUNKS];
 
 constexpr int STATIC_MAX_DEVICES = 64;
 // Resolved device address of the array, per device.  Published once with release ordering; every later call
 // reads it with one acquire load and takes no lock, so a caller on a real-time thread never waits for another
 // thread that is still in its own first call on some other device.
 std::mutex g_static_mutex;   // serialises the one-time look-ups only
-std::atomic<float *> g_static_ptr[STATIC_MAX_DEVICES];
+std::atomic<unsigned long long *> g_static_ptr[STATIC_MAX_DEVICES];
 
 void static_msg(char *buf, uint32_t len, const char *fmt, long long a = 0, long long b = 0) {
   if (buf && len) snprintf(buf, len, fmt, a, b);
@@ -1020,7 +1053,7 @@ DGC_EXPORT int32_t dgc_onepole_fwd_static(void *cuda_stream, const float *x_dev,
     static_msg(err_buf, err_len, "dgc_onepole_fwd_static: B and T must be positive");
     return DGC_ERR_INVALID;
   }
-  const long long NC = ((long long)T + OP_CHUNK - 1) / OP_CHUNK;
+  const long long NC = ((long long)T + 2047) / 2048;   // the slots of the documented limit; a tile is two of them
   if ((long long)B * NC > STATIC_MAX_CHUNKS || B > 65535) {
     static_msg(err_buf, err_len,
                "dgc_onepole_fwd_static: B*ceil(T/2048) = %lld exceeds the built-in scratch of %lld chunk slots; "
@@ -1034,14 +1067,14 @@ DGC_EXPORT int32_t dgc_onepole_fwd_static(void *cuda_stream, const float *x_dev,
     static_msg(err_buf, err_len, "dgc_onepole_fwd_static: no usable current device (cudaGetDevice = %lld)", (long long)e);
     return DGC_ERR_CUDA;
   }
-  float *scratch = g_static_ptr[dev].load(std::memory_order_acquire);
+  unsigned long long *scratch = g_static_ptr[dev].load(std::memory_order_acquire);
   if (!scratch) {
     // Set-up, once per device, with that device current: the array's name is only a host-side
     // handle for the symbol; the address a kernel can use comes from cudaGetSymbolAddress.
     std::lock_guard<std::mutex> lock(g_static_mutex);
     scratch = g_static_ptr[dev].load(std::memory_order_relaxed);
     if (!scratch) {
-      float *p = nullptr;
+      unsigned long long *p = nullptr;
       e = cudaGetSymbolAddress((void **)&p, g_onepole_static_scratch);
       if (e != cudaSuccess || !p) {
         static_msg(err_buf, err_len, "dgc_onepole_fwd_static: cudaGetSymbolAddress failed (%lld) on device %lld",
@@ -1055,12 +1088,10 @@ DGC_EXPORT int32_t dgc_onepole_fwd_static(void *cuda_stream, const float *x_dev,
   // an error left behind by an unrelated earlier call must not be reported as a failure of these launches
   (void)cudaGetLastError();
   cudaStream_t st = (cudaStream_t)cuda_stream;
-  float *chunk_end = scratch, *carry = scratch + STATIC_MAX_CHUNKS;
-  // Every slot that is read below is written first by this call (chunk ends by pass 0, carries by the
-  // carry kernel), so nothing has to be cleared although the array keeps the previous call's contents.
-  onepole_kernel<0><<<dim3((unsigned)NC, B), OP_THREADS, 0, st>>>(x_dev, T, (int)NC, a, nullptr, chunk_end, nullptr);
-  onepole_carry_kernel<<<dgc_div_up(B, 64), 64, 0, st>>>(chunk_end, B, (int)NC, a, 0.0f, carry);
-  onepole_kernel<1><<<dim3((unsigned)NC, B), OP_THREADS, 0, st>>>(x_dev, T, (int)NC, a, carry, nullptr, y_dev);
+  const int NT = dgc_div_up(T, OP_TILE);   // at most ceil(T / 2048): the cells suffice
+  const long long tiles = (long long)B * NT;
+  onepole_kernel<false><<<(unsigned)(tiles < 148 * OP_BLOCKS ? tiles : 148 * OP_BLOCKS), OP_THREADS, 0, st>>>(x_dev, B, T, NT, onepole_powers(a), nullptr, y_dev,
+                                                                            scratch, nullptr);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     static_msg(err_buf, err_len, "dgc_onepole_fwd_static: launch failed (%lld)", (long long)e);
