@@ -24,14 +24,49 @@ def dev(a):
 @pytest.mark.parametrize("B,T,a", [(1, 2047, 0.9), (1, 2048, 0.9), (2, 2049, 0.9), (3, 4097, 0.0), (2, 70003, 0.9999),
                                    (1, 200000, 0.999999), (700, 6000, -0.97)])
 def test_onepole_tiles(ctx, B, T, a):
+    a = float(f32(a))
     rng = np.random.default_rng(B + T)
     x = rng.standard_normal((B, T)).astype(f32)
     y0 = rng.standard_normal(B).astype(f32)
     first = x.copy()
-    first[:, 0] += f32(a) * y0
+    first[:, 0] += f32(a) * y0          # what the carried state adds
     want = np.stack([orc.onepole(first[b].astype(np.float64), a, double=True) for b in range(B)])
     state = dev(y0)
     got = ctx.onepole_fwd(dev(x), a, state=state)
     assert np.abs(got.cpu().numpy() - want).max() <= 1e-5 * max(1.0, np.abs(want).max())
     assert torch.equal(state, got[:, -1])
     assert torch.equal(ctx.onepole_fwd(dev(first), a), ctx.onepole_fwd(dev(first), a))
+
+
+LEVELS = {"tones": lambda n, r: 0.8 * np.sin(n * 0.031) * (1 + 0.5 * np.sin(n * 0.0007)) + 0.02 * r,
+          "steps": lambda n, r: np.where((n // 700) % 3 == 0, 0.9, 0.02) + 0.0 * r,
+          "steady": lambda n, r: np.full(n.shape, 0.9),
+          "noise": lambda n, r: 0.5 * r}
+
+
+@pytest.mark.parametrize("kind", sorted(LEVELS))
+@pytest.mark.parametrize("T,att,rel", [(4095, 0.005, 0.05), (8193, 0.001, 0.01), (16385, 0.05, 0.005), (40000, 0.0001, 1.0),
+                                       (49152, 0.005, 0.05)])
+def test_compressor_tiles(ctx, kind, T, att, rel):
+    """Against the smoother walked in order in double: one tile, several, attack slower than release, a release that
+    outlives a tile, levels that meet the state exactly."""
+    sr, ratio, thr, knee = 48000.0, 4.0, -20.0, 6.0
+    rng = np.random.default_rng(T)
+    x = np.stack([LEVELS[kind](np.arange(T, dtype=np.float64) + 50 * b, rng.standard_normal(T)) for b in range(3)]).astype(f32)
+    state0 = np.array([0.0, 7.5, 1e-3], f32)
+    m = np.maximum(np.abs(x.astype(np.float64)), 1e-5)
+    db = 20 * np.log10(m)
+    pos = (db - (thr - knee / 2)) / knee
+    soft = (db - (thr - knee / 2 + pos * knee / 2)) * (1 - 1 / (1 + pos * (ratio - 1)))
+    g = np.where(db <= thr - knee / 2, 0.0, np.where(db >= thr + knee / 2, (db - thr) * (1 - 1 / ratio), soft))
+    ca, cr = (float(f32(np.exp(np.log(0.01) / (t * sr)))) for t in (att, rel))
+    s, want = state0.astype(np.float64), np.empty((3, T))
+    for n in range(T):
+        c = np.where(g[:, n] > s, ca, cr)
+        s = c * s + (1 - c) * g[:, n]
+        want[:, n] = s
+    want = np.sign(x) * m * 10 ** (-want / 20)
+    state = dev(state0)
+    got = ctx.compressor(dev(x), ratio, thr, knee, att, rel, sr, state=state).cpu().numpy()
+    assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max()
+    assert np.abs(state.cpu().numpy() - s).max() <= 1e-3 * max(1.0, np.abs(s).max())
