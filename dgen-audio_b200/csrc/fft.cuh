@@ -18,8 +18,12 @@ __device__ __forceinline__ int pad(int i) { return i + (i >> 4); }
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// Complex sums as packed pairs: one instruction of two additions.  The lanes' arithmetic rate is the same, the issue slots,
+// which the transforms run out of first, are half.
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+// a + s b, s real
+__device__ __forceinline__ float2 cfma(float s, float2 b, float2 a) { return __ffma2_rn(b, make_float2(s, s), a); }
 // multiply by -i (forward) or +i (inverse)
 template <bool INV>
 __device__ __forceinline__ float2 rot90(float2 a) {
@@ -35,11 +39,12 @@ __device__ __forceinline__ void dft2(float2 &a, float2 &b) {
 
 template <bool INV>
 __device__ __forceinline__ void dft4(float2 &a, float2 &b, float2 &c, float2 &d) {
-  float2 s0 = cadd(a, c), s1 = csub(a, c), s2 = cadd(b, d), s3 = rot90<INV>(csub(b, d));
+  const float2 s0 = cadd(a, c), s1 = csub(a, c), s2 = cadd(b, d), s3 = rot90<INV>(csub(b, d));
   a = cadd(s0, s2);
-  b = cadd(s1, s3);
   c = csub(s0, s2);
-  d = csub(s1, s3);
+  // halves changed places: a packed pair would have to be put together first
+  b = make_float2(s1.x + s3.x, s1.y + s3.y);
+  d = make_float2(s1.x - s3.x, s1.y - s3.y);
 }
 
 template <bool INV>
@@ -49,15 +54,16 @@ __device__ __forceinline__ void dft8(float2 *v) {
   dft4<INV>(v[1], v[3], v[5], v[7]);
   const float h = 0.70710678118654752f;
   float2 o1 = v[3], o2 = v[5], o3 = v[7];
-  // W8^1 = h(1 -+ i), W8^2 = -+ i, W8^3 = h(-1 -+ i)
-  float2 w1 = INV ? make_float2(h * (o1.x - o1.y), h * (o1.x + o1.y)) : make_float2(h * (o1.x + o1.y), h * (o1.y - o1.x));
-  float2 w2 = rot90<INV>(o2);
-  float2 w3 = INV ? make_float2(-h * (o3.x + o3.y), h * (o3.x - o3.y)) : make_float2(h * (o3.y - o3.x), -h * (o3.x + o3.y));
-  float2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1];
+  // W8^1 = h(1 -+ i), W8^2 = -+ i, W8^3 = h(-1 -+ i), the factor h inside the last sums
+  const float2 w1 = INV ? make_float2(o1.x - o1.y, o1.x + o1.y) : make_float2(o1.x + o1.y, o1.y - o1.x);
+  const float2 w2 = rot90<INV>(o2);
+  const float2 w3 = INV ? make_float2(o3.x + o3.y, o3.y - o3.x) : make_float2(o3.x - o3.y, o3.x + o3.y);   // -W8^3 / h
+  const float2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1];
   v[0] = cadd(e0, o0); v[4] = csub(e0, o0);
-  v[1] = cadd(e1, w1); v[5] = csub(e1, w1);
-  v[2] = cadd(e2, w2); v[6] = csub(e2, w2);
-  v[3] = cadd(e3, w3); v[7] = csub(e3, w3);
+  v[1] = cfma(h, w1, e1); v[5] = cfma(-h, w1, e1);
+  v[2] = make_float2(e2.x + w2.x, e2.y + w2.y);
+  v[6] = make_float2(e2.x - w2.x, e2.y - w2.y);
+  v[3] = cfma(-h, w3, e3); v[7] = cfma(h, w3, e3);
 }
 
 template <int R, bool INV>
