@@ -98,6 +98,8 @@ int32_t dgc_gemm_nt(dgc_ctx *ctx, const float *a, const float *b, int M, int N, 
 // true when dgc_gemm_nt() runs this shape on its persistent short-reduction tensor-core kernel
 bool dgc_gemm_nt_persistent(const dgc_ctx *ctx, const float *a, int M, int N, int K);
 const float2 *dgc_ctx_twiddles(dgc_ctx *ctx, int N);
+// dgc_onepole_fwd as three launches (linrec.cu)
+int32_t dgc_onepole_in_passes(dgc_ctx *ctx, const float *x_dev, int32_t B, int32_t T, float a, float *y_dev);
 // dgc_mss_loss_fwd with the prediction given as the sum of two signals (pred_b may be null)
 int32_t dgc_mss_loss_fwd_sum(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev, const float *pred_b_dev,
                              const float *target_dev, float *partial_dev, double *loss_dev);

@@ -56,7 +56,7 @@ unsigned long long *dgc_ctx_chain(dgc_ctx *ctx, uint64_t n) {
     ctx->chain_cells[side] = 0;
     ctx->buffer_generation++;
   }
-  const uint64_t want = n < 4096 ? 4096 : n;
+  const uint64_t want = n < 256 ? 256 : n;
   unsigned long long *p = nullptr;
   cudaError_t e = cudaMalloc(&p, (want + 1) * sizeof(*p));
   if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, (want + 1) * sizeof(*p), ctx->stream);

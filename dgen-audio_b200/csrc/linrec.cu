@@ -207,6 +207,55 @@ onepole_kernel(const float *x, int B, int T, int NT, const OnepolePowers pw, flo
   }
 }
 
+// The filter in three launches: end value of every tile, the states entering the tiles, the output.  What a plan's step runs
+// (onepole_in_passes below).
+template <bool OUT>
+__global__ void __launch_bounds__(OP_THREADS)
+onepole_pass_kernel(const float *x, int T, int NT, const OnepolePowers pw, float *__restrict__ tiles, float *y) {
+  __shared__ float warp_end[OP_WARPS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const size_t at = (size_t)blockIdx.y * T, cell = (size_t)blockIdx.y * NT + blockIdx.x;
+  const int n0 = blockIdx.x * OP_TILE + tid * OP_PER;
+  float loc[OP_PER], prev = 0.0f;
+  onepole_load<false>(x + at, T, n0, loc);
+#pragma unroll
+  for (int j = 0; j < OP_PER; ++j) loc[j] = prev = fmaf(pw.a, prev, loc[j]);
+  float v = prev, d = 1.0f;
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const float o = __shfl_up_sync(0xffffffffu, v, 1 << i);
+    if (lane >= (1 << i)) v = fmaf(pw.r[i], o, v);
+    if (lane & (1 << i)) d *= pw.r[i];
+  }
+  if (lane == 31) warp_end[warp] = v;
+  __syncthreads();
+  float in = OUT ? tiles[cell] : 0.0f;         // state entering the warp
+  for (int w = 0; w < warp; ++w) in = fmaf(pw.r[5], in, warp_end[w]);
+  if (!OUT) {
+    if (tid == OP_THREADS - 1) tiles[cell] = fmaf(pw.r[5], in, v);
+    return;
+  }
+  float s = __shfl_up_sync(0xffffffffu, v, 1);
+  s = fmaf(d, in, lane == 0 ? 0.0f : s);
+#pragma unroll
+  for (int j = 0; j < OP_PER; ++j) {
+    s *= pw.a;
+    loc[j] += s;
+  }
+  onepole_store<false>(y + at, T, n0, loc);
+}
+
+__global__ void onepole_carry_kernel(float *__restrict__ tiles, int B, int NT, float across) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= B) return;
+  float s = 0.0f;
+  for (int c = 0; c < NT; ++c) {
+    const float end = tiles[(size_t)b * NT + c];
+    tiles[(size_t)b * NT + c] = s;
+    s = fmaf(across, s, end);
+  }
+}
+
 template <bool REV>
 int32_t launch_onepole(dgc_ctx *ctx, const float *x, int B, int T, float a, float *state, float *y, const char *what) {
   const int NT = dgc_div_up(T, OP_TILE);
@@ -779,6 +828,23 @@ DGC_EXPORT int32_t dgc_onepole_fwd_state(dgc_ctx *ctx, const float *x_dev, int32
   DGC_REQUIRE(ctx, x_dev && y_dev, "null pointer");
   DGC_REQUIRE(ctx, B > 0 && T > 0, "size out of range");
   return launch_onepole<false>(ctx, x_dev, B, T, a, state_dev, y_dev, "onepole");
+}
+
+int32_t dgc_onepole_in_passes(dgc_ctx *ctx, const float *x_dev, int32_t B, int32_t T, float a, float *y_dev) {
+  if (!ctx) return DGC_ERR_INVALID;
+  DGC_REQUIRE(ctx, x_dev && y_dev, "null pointer");
+  DGC_REQUIRE(ctx, B > 0 && T > 0, "size out of range");
+  const int NT = dgc_div_up(T, OP_TILE);
+  float *tiles = dgc_ctx_scratch(ctx, (uint64_t)B * NT);
+  if (!tiles) return DGC_ERR_OOM;
+  const OnepolePowers pw = onepole_powers(a);
+  onepole_pass_kernel<false><<<dim3(NT, B), OP_THREADS, 0, ctx->stream>>>(x_dev, T, NT, pw, tiles, y_dev);
+  DGC_LAUNCHED(ctx, "onepole_ends");
+  onepole_carry_kernel<<<dgc_div_up(B, 64), 64, 0, ctx->stream>>>(tiles, B, NT, (float)pw.tile[0]);
+  DGC_LAUNCHED(ctx, "onepole_carry");
+  onepole_pass_kernel<true><<<dim3(NT, B), OP_THREADS, 0, ctx->stream>>>(x_dev, T, NT, pw, tiles, y_dev);
+  DGC_LAUNCHED(ctx, "onepole_out");
+  return DGC_OK;
 }
 
 static int32_t biquad_validate(dgc_ctx *ctx, const dgc_biquad_params *p) {

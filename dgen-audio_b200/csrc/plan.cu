@@ -146,7 +146,8 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
         const uint64_t bt = (uint64_t)i[0] * i[1];
         const float *x = R.at(a[0], bt);
         float *y = R.at(a[1], bt), *st = R.at(a[2], i[0], true);
-        if (!R.bad) rc = dgc_onepole_fwd_state(ctx, x, i[0], i[1], f[0], st, y);
+        // without a state cell the step stays the three launches that hosts count it as (dgc_launch_count)
+        if (!R.bad) rc = st ? dgc_onepole_fwd_state(ctx, x, i[0], i[1], f[0], st, y) : dgc_onepole_in_passes(ctx, x, i[0], i[1], f[0], y);
       } break;
       case DGC_PLAN_BIQUAD_FWD: {
         dgc_biquad_params p{i[0], i[1], i[2], f[0], f[1]};
