@@ -180,11 +180,18 @@ __device__ __forceinline__ void stage_middle(const float2 *in, float2 *out, int 
   }
 }
 
+struct SyncBlock {
+  __device__ static __forceinline__ void wait() { __syncthreads(); }
+};
+template <int N> struct SyncTransform {
+  __device__ static __forceinline__ void wait() { sync_transform<N>(); }
+};
+
 // The middle stage IN PLACE: every thread first reads all sixteen of its inputs, the threads of the transform wait
 // for each other, then the butterflies run from the registers and their outputs go back into the same buffer.  One
 // more wait per transform, half the shared memory: the transforms of a block then leave room for more resident
 // blocks.
-template <int N, bool INV, class LAY = LayoutClassic>
+template <int N, bool INV, class LAY = LayoutClassic, class SYNC = SyncTransform<N>>
 __device__ __forceinline__ void stage_middle_inplace(float2 *buf, int tid, const float2 *__restrict__ tw) {
   constexpr int R = Plan<N>::R2, PER = 16 / R, T = N / 16, Ns = Plan<N>::R1;
   float2 v[PER][R];
@@ -194,7 +201,7 @@ __device__ __forceinline__ void stage_middle_inplace(float2 *buf, int tid, const
 #pragma unroll
     for (int t = 0; t < R; ++t) v[q][t] = buf[LAY::template l1<N>(j + t * (N / R))];
   }
-  sync_transform<N>();
+  SYNC::wait();
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
     const int j = tid + q * T, k = j & (Ns - 1);
@@ -298,6 +305,28 @@ __device__ __forceinline__ void stage_middle_T(const float2 *in, float2 *out, in
     twiddle<R, INV>(v, tw, k * (N / (Ns * R)));
 #pragma unroll
     for (int t = 0; t < R; ++t) out[LAY::template l1<N>(j + t * (N / R))] = v[t];
+  }
+}
+
+// the same in place (see stage_middle_inplace)
+template <int N, bool INV, class LAY = LayoutClassic, class SYNC = SyncTransform<N>>
+__device__ __forceinline__ void stage_middle_T_inplace(float2 *buf, int tid, const float2 *__restrict__ tw) {
+  constexpr int R = Plan<N>::R2, PER = 16 / R, T = N / 16, Ns = Plan<N>::R1;
+  float2 v[PER][R];
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int j = tid + q * T, k = j & (Ns - 1), j0 = (j - k) * R + k;
+#pragma unroll
+    for (int t = 0; t < R; ++t) v[q][t] = buf[LAY::template l2<N>(j0 + t * Ns)];
+  }
+  SYNC::wait();
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int j = tid + q * T, k = j & (Ns - 1);
+    dftN<R, INV>(v[q]);
+    twiddle<R, INV>(v[q], tw, k * (N / (Ns * R)));
+#pragma unroll
+    for (int t = 0; t < R; ++t) buf[LAY::template l1<N>(j + t * (N / R))] = v[q][t];
   }
 }
 

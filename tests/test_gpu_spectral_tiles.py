@@ -1,0 +1,68 @@
+"""Spectral blocks at the edges of their tiles: every window size and hop ratio of the synthesis that adds its frames in
+registers, the transforms along the hops of the partitioned convolution with their gradients, runs of silence."""
+import numpy as np
+import pytest
+import torch
+
+import dgen_b200
+from oracle import torch_oracle as to
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = dgen_b200.Context(0)
+    yield c
+    c.close()
+
+
+def windows(x, N, hop, H):
+    pad = torch.nn.functional.pad(x, (N - 1, N))
+    return pad[:, torch.arange(H)[:, None] * hop + torch.arange(N)[None, :]]
+
+
+@pytest.mark.parametrize("N", [16, 64, 128, 256, 512, 1024, 2048])
+@pytest.mark.parametrize("div", [1, 2, 4, 8, 0])
+def test_stft_and_overlap_add(ctx, N, div):
+    hop = N // div if div else N // 3
+    V, T = 3, 11 * hop + hop // 2 + 1
+    H = -(-T // hop)
+    g = torch.Generator().manual_seed(N + div)
+    x, w = torch.randn(V, T, generator=g, dtype=torch.float64), torch.rand(N, generator=g, dtype=torch.float64)
+    x[1, : T // 2] = 0.0
+    re, im = ctx.stft(x.float().cuda(), N, hop, w.float().cuda())
+    want = torch.fft.fft(windows(x.float().double(), N, hop, H) * w.float().double(), dim=2)
+    got = torch.complex(re.double().cpu(), im.double().cpu())
+    assert float((got - want).abs().max()) <= 2e-6 * float(want.abs().max())
+    spec = torch.randn(2, V, H, N, generator=g)          # any complex spectrum: the real part of its inverse is kept
+    out = ctx.istft_ola(spec[0].cuda(), spec[1].cuda(), T, hop, w.float().cuda(), gain=0.7)
+    fr = torch.fft.ifft(torch.complex(spec[0].double(), spec[1].double()), dim=2).real * w.float().double() * 0.7
+    ref = torch.zeros(V, H * hop + N, dtype=torch.float64)
+    for h in range(H):
+        ref[:, h * hop:h * hop + N] += fr[:, h]
+    assert float((out.double().cpu() - ref[:, :T]).abs().max()) <= 2e-6 * float(ref.abs().max())
+    twice = ctx.istft_ola(spec[0].cuda(), spec[1].cuda(), T, hop, w.float().cuda(), gain=0.7, out=out.clone(), accumulate=True)
+    assert torch.equal(twice, 2 * out)
+
+
+# partitions and hops that take the direct sum, and every transform size along the hops with one segment and with several
+@pytest.mark.parametrize("N,hop,H,K,V", [(64, 32, 7, 2, 2), (64, 32, 40, 16, 2), (64, 32, 40, 17, 2), (64, 32, 900, 3, 5), (64, 32, 200, 20, 1),
+                                         (64, 32, 33, 33, 2), (128, 64, 150, 60, 1), (64, 16, 400, 130, 1), (64, 32, 5, 90, 2),
+                                         (64, 32, 700, 300, 1)])
+def test_partitioned_convolution_and_gradients(ctx, N, hop, H, K, V):
+    T, n_ir = H * hop - 3, K * hop - 5
+    g = torch.Generator().manual_seed(H + K)
+    x = torch.randn(V, T, generator=g)
+    x[:, :T // 3] = 0.0
+    ir = torch.randn(n_ir, generator=g) * torch.exp(-3.0 * torch.arange(n_ir) / n_ir)
+    up = torch.randn(V, T, generator=g)
+    x64, ir64 = x.double().requires_grad_(True), ir.double().requires_grad_(True)
+    y64 = to.partconv(x64, ir64, N, hop)
+    (y64 * up.double()).sum().backward()
+    y = ctx.partconv(x.cuda(), ir.cuda(), N, hop)
+    gx, gir = ctx.partconv_bwd(x.cuda(), ir.cuda(), N, hop, up.cuda())
+    for got, want in ((y, y64.detach()), (gx, x64.grad), (gir, ir64.grad)):
+        assert float((got.double().cpu() - want).abs().max()) <= 5e-6 * float(want.abs().max())
+    onset = (T // 3) // hop * hop - N
+    assert onset <= 0 or float(y[:, :onset].abs().max()) == 0.0       # silence before the onset stays exact
