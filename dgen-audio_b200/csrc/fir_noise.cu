@@ -575,49 +575,55 @@ tap_map_tile_kernel(const float *__restrict__ A, const float *__restrict__ W, in
   }
 }
 
-// taps[r][i] = sum_j W[i][j] * bands[r][j]; W is staged once per block and reused for BT_PASSES
-// groups of 16 rows; thread = taps i, i+256, ...
-constexpr int BT_PASSES = 8;
+// taps[r][i] = sum_j W[i][j] * bands[r][j], j ascending, for maps below 2^24 multiply-adds.  These are a few hundred rows: what
+// counts is that every SM gets a piece, that the piece is short and that its loads are all in flight at once.  Block = 64
+// rows x 32 taps, a warp eight rows with a lane per tap (a row of W from shared memory at an odd stride, the rows' bands as
+// broadcast 16-byte loads), bands taken 72 at a time by asynchronous copies.  254 rows x 33 x 129:
+// 4 us, 20 us when a block staged all of W for 128 rows; 750 x 65 x 257, beside the render: 16 us and 66.
+constexpr int BT_ROWS = 64, BT_TAPS = 32, BT_DEPTH = 72, BT_STRIDE = BT_ROWS + 4;
 
 __global__ void __launch_bounds__(256)
 bands_to_taps_kernel(const float *__restrict__ bands, const float *__restrict__ w, int rows, int nb, int nt,
                      float *__restrict__ out) {
-  extern __shared__ float sh[];
-  const int ws = nb | 1;                 // odd row stride: conflict-free column walks
-  float *wsh = sh;                       // [nt][ws]
-  float *bsh = sh + (((size_t)nt * ws + 3) & ~(size_t)3);  // [nb][16], row index fastest, 16-byte aligned
-  for (int i = threadIdx.x; i < nt * nb; i += 256) wsh[(i / nb) * ws + (i % nb)] = w[i];
-  for (int pass = 0; pass < BT_PASSES; ++pass) {
-    const int r0 = (blockIdx.x * BT_PASSES + pass) * 16;
-    if (r0 >= rows) break;
+  __shared__ float wsh[BT_TAPS][BT_DEPTH | 1];
+  __shared__ __align__(16) float bsh[BT_DEPTH][BT_STRIDE];   // row index fastest
+  const int n0 = blockIdx.y * BT_TAPS, r0 = blockIdx.x * BT_ROWS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto copy4 = [](float *dst, const float *src, bool take) {   // one float, or zero
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(take ? 4 : 0)
+                 : "memory");
+  };
+  float acc[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) acc[r] = 0.0f;
+  for (int j0 = 0; j0 < nb; j0 += BT_DEPTH) {
+    const int depth = min(BT_DEPTH, nb - j0);
+    for (int i = threadIdx.x; i < BT_TAPS * depth; i += 256) {
+      const int n = i / depth, j = i - n * depth;
+      const bool in = n0 + n < nt;
+      copy4(&wsh[n][j], in ? w + (size_t)(n0 + n) * nb + j0 + j : w, in);
+    }
+    for (int i = threadIdx.x; i < BT_ROWS * depth; i += 256) {
+      const int r = i / depth, j = i - r * depth;
+      const bool in = r0 + r < rows;
+      copy4(&bsh[j][r], in ? bands + (size_t)(r0 + r) * nb + j0 + j : bands, in);
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    for (int i = threadIdx.x; i < 16 * nb; i += 256) {
-      int r = i / nb, j = i - r * nb;
-      bsh[j * 16 + r] = (r0 + r < rows) ? bands[(size_t)(r0 + r) * nb + j] : 0.0f;
+#pragma unroll 4
+    for (int j = 0; j < depth; ++j) {
+      const float wv = wsh[lane][j];
+      const float4 *bp = reinterpret_cast<const float4 *>(&bsh[j][warp * 8]);
+      const float4 u = bp[0], v = bp[1];
+      acc[0] = fmaf(wv, u.x, acc[0]); acc[1] = fmaf(wv, u.y, acc[1]); acc[2] = fmaf(wv, u.z, acc[2]); acc[3] = fmaf(wv, u.w, acc[3]);
+      acc[4] = fmaf(wv, v.x, acc[4]); acc[5] = fmaf(wv, v.y, acc[5]); acc[6] = fmaf(wv, v.z, acc[6]); acc[7] = fmaf(wv, v.w, acc[7]);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < nt; i += 256) {
-      float acc[16];
-#pragma unroll
-      for (int r = 0; r < 16; ++r) acc[r] = 0.0f;
-      const float *wr = wsh + (size_t)i * ws;
-      for (int j = 0; j < nb; ++j) {
-        float wv = wr[j];
-        const float4 *bp = reinterpret_cast<const float4 *>(bsh + j * 16);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float4 v = bp[q];
-          acc[4 * q + 0] = fmaf(wv, v.x, acc[4 * q + 0]);
-          acc[4 * q + 1] = fmaf(wv, v.y, acc[4 * q + 1]);
-          acc[4 * q + 2] = fmaf(wv, v.z, acc[4 * q + 2]);
-          acc[4 * q + 3] = fmaf(wv, v.w, acc[4 * q + 3]);
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < 16; ++r)
-        if (r0 + r < rows) out[(size_t)(r0 + r) * nt + i] = acc[r];
-    }
   }
+  if (n0 + lane >= nt) return;
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+    if (r0 + warp * 8 + r < rows) out[(size_t)(r0 + warp * 8 + r) * nt + n0 + lane] = acc[r];
 }
 
 }  // namespace
@@ -747,11 +753,9 @@ DGC_EXPORT int32_t dgc_bands_to_taps(dgc_ctx *ctx, const float *bands_dev, const
     // asynchronous copies instead of 16-byte ones, which is cheaper than a padding pass over the bands)
     return dgc_gemm_nt(ctx, bands_dev, w_dev, rows, taps, nbands, taps_dev);
   }
-  size_t smem = ((((size_t)taps * (nbands | 1) + 3) & ~(size_t)3) + (size_t)nbands * 16) * sizeof(float);
-  DGC_REQUIRE(ctx, smem <= 200 * 1024, "taps*nbands too large for shared memory");
-  DGC_CUDA(ctx, cudaFuncSetAttribute(bands_to_taps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  bands_to_taps_kernel<<<dgc_div_up(rows, 16 * BT_PASSES), 256, smem, ctx->stream>>>(bands_dev, w_dev, rows, nbands, taps,
-                                                                          taps_dev);
+  const dim3 grid(dgc_div_up(rows, BT_ROWS), dgc_div_up(taps, BT_TAPS));
+  DGC_REQUIRE(ctx, grid.y <= 65535, "too many taps");
+  bands_to_taps_kernel<<<grid, 256, 0, ctx->stream>>>(bands_dev, w_dev, rows, nbands, taps, taps_dev);
   DGC_LAUNCHED(ctx, "bands_to_taps");
   return DGC_OK;
 }
