@@ -223,7 +223,10 @@ int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *
   } else if (tc) {
     // tensor-core kernel: operand A is K-major in memory when it is NOT transposed ([M][K]);
     // operand B is K-major in memory when it IS given transposed ([N][K])
-    auto kern = dgtc::tc_gemm_kernel<!TA, TB, EPI>;
+    // a product of so few tiles that their halves fit the chip too takes 64-column ones
+    const bool halves = tiles * splits * 2 <= ctx->sm_count && N > 64;
+    auto kern = halves ? dgtc::tc_gemm_kernel<!TA, TB, EPI, 64> : dgtc::tc_gemm_kernel<!TA, TB, EPI>;
+    if (halves) grid.x = dgc_div_up(N, 64);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dgtc::SMEM_BYTES);
     if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));
     kern<<<grid, dgtc::THREADS, dgtc::SMEM_BYTES, ctx->stream>>>(A, B, bias, M, N, K, kps, dst, ctx->status_dev);

@@ -116,12 +116,16 @@ __device__ __forceinline__ void split_tf32_rn(float x, float &hi, float &lo) {
 //   layout with scalar stores; a warp moves 8 k x 4 units (16 rows), a store instruction hits 8 k x 4 rows
 //   with 2-way bank conflicts.  (An MN-major shared-memory descriptor with no swizzle was tried instead of
 //   this transposition and produced zeros on this part, so both operands always use the K-major descriptor.)
-template <bool ROWMAJOR_K>
+// ROWS: 128, or 64 for the B operand of a 64-column output tile (P float4 per thread).
+template <bool ROWMAJOR_K, int ROWS, int P>
 __device__ __forceinline__ void fetch(const float *__restrict__ src, int ld, int rows, int r0, int k0, int k_end,
-                                      int tid, float4 (&v)[4]) {
+                                      int tid, float4 (&v)[P]) {
+  static_assert(P == ROWS * TBK / 4 / THREADS, "a 32-deep tile, four values at a time");
+  constexpr int UG = ROWS / 16, UGS = UG == 8 ? 8 : 7;   // groups of four units along the rows
+  static_assert(UG == 8 || UG == 4, "128 or 64 rows");
   const bool vec_ok = ((ld & 3) == 0) && ((((uintptr_t)src) & 15) == 0);
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
+  for (int p = 0; p < P; ++p) {
     v[p] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (ROWMAJOR_K) {
       const int kc = tid & 7, r = (tid >> 3) + 32 * p, gr = r0 + r, gk = k0 + 4 * kc;
@@ -137,7 +141,7 @@ __device__ __forceinline__ void fetch(const float *__restrict__ src, int ld, int
       }
     } else {
       const int idx = p * THREADS + tid;
-      const int kk = (idx & 7) + 8 * (idx >> 8), u = ((idx >> 3) & 3) + 4 * ((idx >> 5) & 7);
+      const int kk = (idx & 7) + 8 * (idx >> UGS), u = ((idx >> 3) & 3) + 4 * ((idx >> 5) & (UG - 1));
       const int gk = k0 + kk, gr = r0 + 4 * u;
       if (gk < k_end) {
         const float *q = src + (size_t)gk * ld + gr;
@@ -153,10 +157,11 @@ __device__ __forceinline__ void fetch(const float *__restrict__ src, int ld, int
   }
 }
 
-template <bool ROWMAJOR_K>
-__device__ __forceinline__ void stash(const float4 (&v)[4], char *hi_part, char *lo_part, int tid) {
+template <bool ROWMAJOR_K, int ROWS, int P>
+__device__ __forceinline__ void stash(const float4 (&v)[P], char *hi_part, char *lo_part, int tid) {
+  constexpr int UG = ROWS / 16, UGS = UG == 8 ? 8 : 7;
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
+  for (int p = 0; p < P; ++p) {
     if (ROWMAJOR_K) {
       const int kc = tid & 7, r = (tid >> 3) + 32 * p;
       float4 h, l;
@@ -166,7 +171,7 @@ __device__ __forceinline__ void stash(const float4 (&v)[4], char *hi_part, char 
       *reinterpret_cast<float4 *>(lo_part + off) = l;
     } else {
       const int idx = p * THREADS + tid;
-      const int kk = (idx & 7) + 8 * (idx >> 8), u = ((idx >> 3) & 3) + 4 * ((idx >> 5) & 7);
+      const int kk = (idx & 7) + 8 * (idx >> UGS), u = ((idx >> 3) & 3) + 4 * ((idx >> 5) & (UG - 1));
       const float vv[4] = {v[p].x, v[p].y, v[p].z, v[p].w};
       const int base = (kk >> 2) * LBO_BYTES + (kk & 3) * 4 + (4 * u) * 16;
 #pragma unroll
@@ -260,7 +265,10 @@ __device__ __forceinline__ void epilogue(uint32_t tmem_d, const float *__restric
 
 // A_KMAJOR: A stored [M][K]; else stored [K][M].  B_KMAJOR: B stored [N][K]; else stored [K][N].
 // EPI 0: C = acc ; 1: + bias[n] ; 2: tanh(acc + bias[n]).  blockIdx.z selects a k-slice (split-K slab of C).
-template <bool A_KMAJOR, bool B_KMAJOR, int EPI>
+// BN 64: half as wide an output tile, for products that are only a few tiles (the order of the products an output element
+// adds up is the same).  The loads run three k tiles ahead in registers: with one CTA on an SM and nothing beside it a k tile
+// otherwise costs a round trip to memory.  128 x 128 over 750 k: 51 -> 38 us, 750 x 128 over 128 k: 13 -> 9.5 us.
+template <bool A_KMAJOR, bool B_KMAJOR, int EPI, int BN = TBN>
 __global__ void __launch_bounds__(THREADS, 1)
 tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const float *__restrict__ bias, int M, int N,
                int K, int k_per_split, float *__restrict__ C, int32_t *status) {
@@ -268,7 +276,7 @@ tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const f
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * STAGE_BYTES);      // two mbarriers
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 2 * STAGE_BYTES + 32);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * TBM, n0 = blockIdx.x * TBN;
+  const int m0 = blockIdx.y * TBM, n0 = blockIdx.x * BN;
   const int k_begin = blockIdx.z * k_per_split, k_end = min(K, k_begin + k_per_split);
   C += (size_t)blockIdx.z * M * N;
   const int KT = (k_end - k_begin + TBK - 1) / TBK;
@@ -280,7 +288,7 @@ tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const f
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"((uint32_t)TBN)
+                 "r"((uint32_t)BN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -290,32 +298,34 @@ tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const f
   const uint32_t tmem_d = *tmem_slot;
   bool ok = true;
 
-  float4 va[4], vb[4], na[4], nb[4];
-  if (KT > 0) {
-    fetch<A_KMAJOR>(A, A_KMAJOR ? K : M, M, m0, k_begin, k_end, tid, va);
-    fetch<B_KMAJOR>(B, B_KMAJOR ? K : N, N, n0, k_begin, k_end, tid, vb);
-  }
-  for (int kt = 0; kt < KT; ++kt) {
+  constexpr int AHEAD = 3, PA = 4, PB = BN / 32;
+  float4 va[AHEAD][PA], vb[AHEAD][PB];
+  auto load = [&](int kt, float4 (&fa)[PA], float4 (&fb)[PB]) {
+    if (kt >= KT) return;
+    fetch<A_KMAJOR, TBM>(A, A_KMAJOR ? K : M, M, m0, k_begin + kt * TBK, k_end, tid, fa);
+    fetch<B_KMAJOR, BN>(B, B_KMAJOR ? K : N, N, n0, k_begin + kt * TBK, k_end, tid, fb);
+  };
+#pragma unroll
+  for (int j = 0; j < AHEAD; ++j) load(j, va[j], vb[j]);
+  // returns false when the tensor core stopped answering: no further MMAs are issued, TMEM is still released below
+  auto tile = [&](int kt, float4 (&fa)[PA], float4 (&fb)[PB]) -> bool {
     const int s = kt & 1;
-    if (kt + 1 < KT) {  // next tile's global loads fly while this tile is stored and multiplied
-      fetch<A_KMAJOR>(A, A_KMAJOR ? K : M, M, m0, k_begin + (kt + 1) * TBK, k_end, tid, na);
-      fetch<B_KMAJOR>(B, B_KMAJOR ? K : N, N, n0, k_begin + (kt + 1) * TBK, k_end, tid, nb);
-    }
     if (kt >= 2) {
       ok = mbar_wait(smem_u32(&bars[s]), (uint32_t)(((kt >> 1) - 1) & 1));
       ok = __syncthreads_and(ok);   // same decision in every thread
-      if (!ok) break;               // give up: no further MMAs are issued, TMEM is still released below
+      if (!ok) return false;
     }
     char *st = smem + s * STAGE_BYTES;
-    stash<A_KMAJOR>(va, st, st + OPER_BYTES, tid);
-    stash<B_KMAJOR>(vb, st + 2 * OPER_BYTES, st + 3 * OPER_BYTES, tid);
+    stash<A_KMAJOR, TBM>(fa, st, st + OPER_BYTES, tid);
+    stash<B_KMAJOR, BN>(fb, st + 2 * OPER_BYTES, st + 3 * OPER_BYTES, tid);
+    load(kt + AHEAD, fa, fb);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> async proxy (tensor core)
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (tid == 0 && ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t a_hi = smem_u32(st), a_lo = a_hi + OPER_BYTES, b_hi = a_hi + 2 * OPER_BYTES, b_lo = a_hi + 3 * OPER_BYTES;
-      constexpr uint32_t ID = IDesc<true, true>::value;
+      constexpr uint32_t ID = IDesc<true, true, BN>::value;
 #pragma unroll
       for (int ks = 0; ks < TBK / 8; ++ks) {
         // 8 tf32 along k = two 16-byte k-chunks
@@ -328,11 +338,12 @@ tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const f
       }
       commit_to(smem_u32(&bars[s]));
     }
+    return true;
+  };
+  for (int kt = 0; kt < KT && ok; kt += AHEAD) {
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      va[p] = na[p];
-      vb[p] = nb[p];
-    }
+    for (int j = 0; j < AHEAD; ++j)
+      if (kt + j < KT && !tile(kt + j, va[j], vb[j])) break;
   }
   // the last commit covers every MMA issued before it
   if (KT > 0 && ok) ok = mbar_wait(smem_u32(&bars[(KT - 1) & 1]), (uint32_t)(((KT - 1) >> 1) & 1));
@@ -340,19 +351,19 @@ tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const f
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
   if (ok && KT > 0) {
-    epilogue<EPI>(tmem_d, bias, M, N, m0, n0, C, warp, lane, nullptr, reinterpret_cast<float *>(smem));
+    epilogue<EPI, BN>(tmem_d, bias, M, N, m0, n0, C, warp, lane, nullptr, reinterpret_cast<float *>(smem));
   } else if (KT == 0) {
     // empty reduction range: the slab is zero
     const int gm = m0 + (warp & 3) * 32 + lane;
     if (gm < M && warp < 4)
-      for (int c = 0; c < TBN; ++c)
+      for (int c = 0; c < BN; ++c)
         if (n0 + c < N) C[(size_t)gm * N + n0 + c] = 0.0f;
   }
   if (!ok && tid == 0) atomicExch(status, 201);  // an MMA completion never arrived within the spin limit
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"((uint32_t)TBN) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"((uint32_t)BN) : "memory");
   }
 }
 
