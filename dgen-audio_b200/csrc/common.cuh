@@ -13,6 +13,9 @@
 
 #define DGC_EXPORT extern "C" __attribute__((visibility("default")))
 
+// upload events of a host-buffer step: harmonic controls, noise branch, then one per group of voices of the target
+constexpr int DGC_COPY_EVENTS = 2 + 4;
+
 struct dgc_ctx {
   int device = 0;
   cudaStream_t own_stream = nullptr;
@@ -50,13 +53,19 @@ struct dgc_ctx {
   cudaStream_t aux_stream = nullptr;   // second stream of the composite steps (noise branch beside the harmonic one)
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   cudaStream_t copy_stream = nullptr;
-  cudaEvent_t copy_ev[3] = {nullptr, nullptr, nullptr};
+  cudaEvent_t copy_ev[DGC_COPY_EVENTS] = {};
+  cudaStream_t out_stream = nullptr;   // results on their way to the host while the step goes on
+  cudaEvent_t audio_ev = nullptr, out_ev = nullptr;
+  // small inputs are gathered here and cross PCIe as one copy: the blocking call's block and one per step in flight
+  float *pinned[3] = {nullptr, nullptr, nullptr};
+  uint64_t pinned_floats[3] = {0, 0, 0};
+  int32_t *status_host = nullptr;      // page-locked copy of the status word
   float *stage_dev = nullptr;
   uint64_t stage_floats = 0;
   // two host-buffer steps in flight (plans.cu): per-slot input staging, upload events, end-of-step event
   float *pipe_in[2] = {nullptr, nullptr};
   uint64_t pipe_in_floats[2] = {0, 0};
-  cudaEvent_t pipe_ev[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
+  cudaEvent_t pipe_ev[2][DGC_COPY_EVENTS] = {};
   cudaEvent_t pipe_done[2] = {nullptr, nullptr};
   bool pipe_used[2] = {false, false}, pipe_pending[2] = {false, false};
   // NCCL communicator of the gradient exchange (comm.cu); nullptr = a world of one
@@ -83,6 +92,8 @@ struct dgc_arena {
 
 int32_t dgc_fail(dgc_ctx *ctx, int32_t code, const char *fmt, ...);
 int32_t dgc_check_launch(dgc_ctx *ctx, const char *what);
+// DGC_ERR_DEVICE (the word is cleared) when a kernel left something in the status word
+int32_t dgc_report_status(dgc_ctx *ctx, int32_t status);
 // returns device pointer to at least n floats of context scratch (nullptr + error set on failure)
 float *dgc_ctx_scratch(dgc_ctx *ctx, uint64_t nfloats);
 // 1 + n zero-initialised 64-bit words for a launch on the current stream: the ticket word, then n cells (chain.cuh)
@@ -103,6 +114,11 @@ int32_t dgc_onepole_in_passes(dgc_ctx *ctx, const float *x_dev, int32_t B, int32
 // dgc_mss_loss_fwd with the prediction given as the sum of two signals (pred_b may be null)
 int32_t dgc_mss_loss_fwd_sum(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev, const float *pred_b_dev,
                              const float *target_dev, float *partial_dev, double *loss_dev);
+// ... with the voices in groups, each after its own event (mss_loss.cu)
+constexpr int DGC_MSS_MAX_GROUPS = 4;
+static inline int dgc_mss_group_start(int B, int q, int groups) { return (int)((int64_t)B * q / groups); }
+int32_t dgc_mss_loss_fwd_groups(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev, const float *target_dev, int groups,
+                                const cudaEvent_t *ready, double *loss_dev);
 
 #define DGC_CUDA(ctx, call)                                                                  \
   do {                                                                                       \

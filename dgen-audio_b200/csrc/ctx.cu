@@ -216,6 +216,12 @@ DGC_EXPORT int32_t dgc_ctx_destroy(dgc_ctx *c) {
   for (auto &e : c->copy_ev)
     if (e) cudaEventDestroy(e);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
+  if (c->audio_ev) cudaEventDestroy(c->audio_ev);
+  if (c->out_ev) cudaEventDestroy(c->out_ev);
+  if (c->out_stream) cudaStreamDestroy(c->out_stream);
+  for (auto &p : c->pinned)
+    if (p) cudaFreeHost(p);
+  if (c->status_host) cudaFreeHost(c->status_host);
   if (c->fork_ev) cudaEventDestroy(c->fork_ev);
   if (c->join_ev) cudaEventDestroy(c->join_ev);
   if (c->aux_stream) cudaStreamDestroy(c->aux_stream);
@@ -259,6 +265,10 @@ DGC_EXPORT int32_t dgc_sync(dgc_ctx *ctx, uint32_t timeout_ms) {
   }
   int32_t st = 0;
   DGC_CUDA(ctx, cudaMemcpy(&st, ctx->status_dev, sizeof(st), cudaMemcpyDeviceToHost));
+  return dgc_report_status(ctx, st);
+}
+
+int32_t dgc_report_status(dgc_ctx *ctx, int32_t st) {
   if (st != 0) {
     cudaMemset(ctx->status_dev, 0, sizeof(int32_t));
     return dgc_fail(ctx, DGC_ERR_DEVICE, "device status word = %d", st);

@@ -325,8 +325,8 @@ mss_fwd16_kernel(const float *__restrict__ pred, const float *__restrict__ pred_
 // total = sum_s (w_lin * sum(lin_s) + w_log * sum(log_s)) / B / nscales / T
 struct ReduceDesc {
   int nscales;
-  long long off[DGC_MSS_MAX_SCALES];  // offset of the lin block of scale s; log block follows
-  long long cnt[DGC_MSS_MAX_SCALES];  // H_s * B
+  // offset of the lin block of a scale (of a group of voices), the log block follows; H_s x voices
+  long long off[DGC_MSS_MAX_SCALES * DGC_MSS_MAX_GROUPS], cnt[DGC_MSS_MAX_SCALES * DGC_MSS_MAX_GROUPS];
 };
 
 constexpr int RED_BLOCKS = 256, RED_THREADS = 256;
@@ -841,25 +841,9 @@ DGC_EXPORT int32_t dgc_mss_loss_fwd(dgc_ctx *ctx, const dgc_mss_params *p, const
   return dgc_mss_loss_fwd_sum(ctx, p, pred_dev, nullptr, target_dev, partial_dev, loss_dev);
 }
 
-// prediction = pred_dev + pred_b_dev (pred_b_dev may be null): lets two synthesis branches that ran
-// concurrently feed the loss without a pass that adds them
-int32_t dgc_mss_loss_fwd_sum(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev, const float *pred_b_dev,
-                             const float *target_dev, float *partial_dev, double *loss_dev) {
-  if (!ctx) return DGC_ERR_INVALID;
-  DGC_REQUIRE(ctx, p && pred_dev && target_dev && loss_dev, "null pointer");
-  int32_t rc = validate(ctx, p);
-  if (rc != DGC_OK) return rc;
-  float *part = partial_dev ? partial_dev : dgc_ctx_scratch(ctx, dgc_mss_partial_floats(p) + 4);
-  if (!part) return DGC_ERR_OOM;
-  ReduceDesc d;
-  d.nscales = 0;
-  long long off = 0;
-  int used = 0;
-  for (int s = 0; s < p->nscales; ++s) {
-    const int N = p->sizes[s];
-    if (N > p->T) continue;
-    ++used;
-  }
+// The windows of one group of voices (p->B of them, at pred_dev and target_dev): partial sums at part + off, added to d.
+static int32_t mss_fwd_windows(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev, const float *pred_b_dev,
+                               const float *target_dev, float *part, long long &off, ReduceDesc &d) {
   // partial layout and summation order follow the caller's scale order; the launch runs the usable
   // scales largest window first
   int order[DGC_MSS_MAX_SCALES], no = 0;
@@ -948,6 +932,12 @@ int32_t dgc_mss_loss_fwd_sum(dgc_ctx *ctx, const dgc_mss_params *p, const float 
                                                                                                 target_dev, p->B, p->T, fd8);
     DGC_LAUNCHED(ctx, "mss_fwd");
   }
+  return DGC_OK;
+}
+
+static int32_t mss_fwd_reduce(dgc_ctx *ctx, const dgc_mss_params *p, const float *part, const ReduceDesc &d, double *loss_dev) {
+  int used = 0;
+  for (int s = 0; s < p->nscales; ++s) used += p->sizes[s] <= p->T;
   // weights: (w / nscales) with nscales = number of usable windows, normalize:true divides by T
   // (Examples/HarmonicE2E/Trainer.swift:553-586, Sources/DGenLazy/Functions.swift:951-954);
   // the batched loss is the mean over voices (Emit+SpectralLoss.swift:937-938)
@@ -956,6 +946,44 @@ int32_t dgc_mss_loss_fwd_sum(dgc_ctx *ctx, const dgc_mss_params *p, const float 
                                                                   ctx->loss_accum + 64, ctx->ticket_dev, loss_dev);
   DGC_LAUNCHED(ctx, "mss_reduce");
   return DGC_OK;
+}
+
+// prediction = pred_dev + pred_b_dev (pred_b_dev may be null): lets two synthesis branches that ran
+// concurrently feed the loss without a pass that adds them
+int32_t dgc_mss_loss_fwd_sum(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev, const float *pred_b_dev,
+                             const float *target_dev, float *partial_dev, double *loss_dev) {
+  if (!ctx) return DGC_ERR_INVALID;
+  DGC_REQUIRE(ctx, p && pred_dev && target_dev && loss_dev, "null pointer");
+  int32_t rc = validate(ctx, p);
+  if (rc != DGC_OK) return rc;
+  float *part = partial_dev ? partial_dev : dgc_ctx_scratch(ctx, dgc_mss_partial_floats(p) + 4);
+  if (!part) return DGC_ERR_OOM;
+  ReduceDesc d;
+  d.nscales = 0;
+  long long off = 0;
+  rc = mss_fwd_windows(ctx, p, pred_dev, pred_b_dev, target_dev, part, off, d);
+  return rc == DGC_OK ? mss_fwd_reduce(ctx, p, part, d, loss_dev) : rc;
+}
+
+// The same in up to DGC_MSS_MAX_GROUPS groups of voices, group q after ready[q]: a target that is still arriving in parts
+int32_t dgc_mss_loss_fwd_groups(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev, const float *target_dev, int groups,
+                                const cudaEvent_t *ready, double *loss_dev) {
+  int32_t rc = validate(ctx, p);
+  if (rc != DGC_OK) return rc;
+  float *part = dgc_ctx_scratch(ctx, dgc_mss_partial_floats(p) + 4);
+  if (!part) return DGC_ERR_OOM;
+  ReduceDesc d;
+  d.nscales = 0;
+  long long off = 0;
+  for (int q = 0; q < groups; ++q) {
+    const int b0 = dgc_mss_group_start(p->B, q, groups), b1 = dgc_mss_group_start(p->B, q + 1, groups);
+    dgc_mss_params g = *p;
+    g.B = b1 - b0;
+    DGC_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ready[q], 0));
+    rc = mss_fwd_windows(ctx, &g, pred_dev + (size_t)b0 * p->T, nullptr, target_dev + (size_t)b0 * p->T, part, off, d);
+    if (rc != DGC_OK) return rc;
+  }
+  return mss_fwd_reduce(ctx, p, part, d, loss_dev);
 }
 
 DGC_EXPORT int32_t dgc_mss_loss_bwd(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev,

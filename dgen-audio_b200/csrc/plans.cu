@@ -55,13 +55,19 @@ DGC_EXPORT uint64_t dgc_hn_forward_loss_work_floats(const dgc_hn_step *s) {
 // (band -> tap map, FIR) share no data until the loss, so they run on two streams: the small or latency-bound
 // kernels of one chain (the 64-block phase scan, the band -> tap matmul) and the last waves of the big ones fill
 // under the other chain's work.  The loss reads the prediction as the sum of the two branch outputs.
-// ev_noise_inputs / ev_target (optional): events after which the noise-branch inputs / the target are in device
-// memory (the host-buffer variant uploads them on its own stream while the first kernels already run)
+// The host-buffer variant uploads on its own stream while the first kernels already run, and reads the audio back while the
+// loss is still being computed:
+struct HostEvents {
+  cudaEvent_t noise_inputs;       // the noise branch's inputs are in device memory
+  const cudaEvent_t *target;      // group q of the target's voices is
+  int groups;
+  cudaEvent_t audio;              // recorded when the audio is complete
+};
 static int32_t hn_forward_loss_impl(dgc_ctx *ctx, const dgc_hn_step *s, const float *f0_dev, const float *uv_dev,
                                     const float *amps_dev, const float *gain_dev, const float *noise_gain_dev,
                                     const float *taps_or_bands_dev, const float *w_dev, const float *noise_dev,
                                     const float *target_dev, float *work_dev, double *loss_dev, float *audio_dev,
-                                    cudaEvent_t ev_noise_inputs, cudaEvent_t ev_target) {
+                                    const HostEvents *ev) {
   if (!ctx) return DGC_ERR_INVALID;
   DGC_REQUIRE(ctx, s && f0_dev && uv_dev && amps_dev && gain_dev && target_dev && loss_dev && work_dev, "null pointer");
   const int B = s->harm.B, T = s->harm.T, K = s->harm.K, F = s->harm.F;
@@ -106,11 +112,13 @@ static int32_t hn_forward_loss_impl(dgc_ctx *ctx, const dgc_hn_step *s, const fl
     return !e ? 0 : strcmp(e, "side") == 0 ? 1 : strcmp(e, "serial") == 0 ? 2 : 0;
   }();
   const bool serial_fir = noise && (fir_mode == 2 || (fir_mode == 0 && nBT >= (4ull << 20)));
+  // nothing is added later: the branch (and the FIR behind it) writes where the caller wants the audio
+  if (audio_dev && (serial_fir || !noise) && (((uintptr_t)audio_dev) & 15) == 0) d_harm = audio_dev;
   if (noise) {
     // fork: the noise branch starts where the caller's stream stands now
     DGC_CUDA(ctx, cudaEventRecord(ctx->fork_ev, main_stream));
     DGC_CUDA(ctx, cudaStreamWaitEvent(ctx->aux_stream, ctx->fork_ev, 0));
-    if (ev_noise_inputs) DGC_CUDA(ctx, cudaStreamWaitEvent(ctx->aux_stream, ev_noise_inputs, 0));
+    if (ev) DGC_CUDA(ctx, cudaStreamWaitEvent(ctx->aux_stream, ev->noise_inputs, 0));
     forked = true;
     ctx->stream = ctx->aux_stream;
     if (NB > 0) rc = dgc_bands_to_taps(ctx, taps_or_bands_dev, w_dev, (int32_t)nFB, NB, NT, d_taps);
@@ -138,29 +146,20 @@ static int32_t hn_forward_loss_impl(dgc_ctx *ctx, const dgc_hn_step *s, const fl
     rc = dgc_fir_noise(ctx, &fp, noise_dev, d_taps, noise_gain_dev, d_harm);
     if (rc != DGC_OK) return rc;
   }
-  if (ev_target) DGC_CUDA(ctx, cudaStreamWaitEvent(main_stream, ev_target, 0));
-  if (audio_dev) {
-    if (noise && !serial_fir) {
-      add2_kernel<<<dgc_div_up((int64_t)nBT, 256), 256, 0, ctx->stream>>>(d_harm, d_noise, nBT, audio_dev);
-      DGC_LAUNCHED(ctx, "add_branches");
-    } else {
-      DGC_CUDA(ctx, cudaMemcpyAsync(audio_dev, d_harm, nBT * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
-    }
-    return dgc_mss_loss_fwd_sum(ctx, &s->mss, audio_dev, nullptr, target_dev, nullptr, loss_dev);
-  }
-  // Sum the branches in place first, then the plain loss kernel: measured 0.349 ms per step against 0.360 ms
-  // with the loss kernel adding the two signals as it loads them (DGC_HN_SUM=fused selects that variant).
-  static const bool add_first = [] {
-    const char *e = getenv("DGC_HN_SUM");
-    return !(e && strcmp(e, "fused") == 0);
-  }();
-  if (serial_fir) return dgc_mss_loss_fwd_sum(ctx, &s->mss, d_harm, nullptr, target_dev, nullptr, loss_dev);
-  if (add_first && noise) {
-    add2_kernel<<<dgc_div_up((int64_t)nBT, 256), 256, 0, ctx->stream>>>(d_harm, d_noise, nBT, d_harm);
+  // the sum of the branches: in the audio buffer when the caller wants it, else in place (measured 0.349 ms per step
+  // against 0.360 ms with the loss kernel adding the two signals as it loads them)
+  float *mix = audio_dev ? audio_dev : d_harm;
+  if (noise && !serial_fir) {
+    add2_kernel<<<dgc_div_up((int64_t)nBT, 256), 256, 0, ctx->stream>>>(d_harm, d_noise, nBT, mix);
     DGC_LAUNCHED(ctx, "add_branches");
-    return dgc_mss_loss_fwd_sum(ctx, &s->mss, d_harm, nullptr, target_dev, nullptr, loss_dev);
+  } else if (mix != d_harm) {
+    DGC_CUDA(ctx, cudaMemcpyAsync(mix, d_harm, nBT * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
   }
-  return dgc_mss_loss_fwd_sum(ctx, &s->mss, d_harm, d_noise, target_dev, nullptr, loss_dev);
+  if (ev) {
+    DGC_CUDA(ctx, cudaEventRecord(ev->audio, main_stream));
+    return dgc_mss_loss_fwd_groups(ctx, &s->mss, mix, target_dev, ev->groups, ev->target, loss_dev);
+  }
+  return dgc_mss_loss_fwd_sum(ctx, &s->mss, mix, nullptr, target_dev, nullptr, loss_dev);
 }
 
 DGC_EXPORT int32_t dgc_hn_forward_loss(dgc_ctx *ctx, const dgc_hn_step *s, const float *f0_dev, const float *uv_dev,
@@ -168,7 +167,7 @@ DGC_EXPORT int32_t dgc_hn_forward_loss(dgc_ctx *ctx, const dgc_hn_step *s, const
                                        const float *taps_or_bands_dev, const float *w_dev, const float *noise_dev,
                                        const float *target_dev, float *work_dev, double *loss_dev, float *audio_dev) {
   return hn_forward_loss_impl(ctx, s, f0_dev, uv_dev, amps_dev, gain_dev, noise_gain_dev, taps_or_bands_dev, w_dev,
-                              noise_dev, target_dev, work_dev, loss_dev, audio_dev, nullptr, nullptr);
+                              noise_dev, target_dev, work_dev, loss_dev, audio_dev, nullptr);
 }
 
 // slot < 0: the blocking call (one staging area, returns after the loss has arrived).
@@ -208,7 +207,11 @@ static int32_t hn_host_enqueue(dgc_ctx *ctx, const dgc_hn_step *s, const float *
 
   if (!ctx->copy_stream) {
     DGC_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
+    DGC_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->out_stream, cudaStreamNonBlocking));
     for (auto &e : ctx->copy_ev) DGC_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    DGC_CUDA(ctx, cudaEventCreateWithFlags(&ctx->audio_ev, cudaEventDisableTiming));
+    DGC_CUDA(ctx, cudaEventCreateWithFlags(&ctx->out_ev, cudaEventDisableTiming));
+    DGC_CUDA(ctx, cudaMallocHost(&ctx->status_host, sizeof(int32_t)));
   }
   cudaEvent_t *ev = ctx->copy_ev;
   if (piped) {
@@ -239,11 +242,7 @@ static int32_t hn_host_enqueue(dgc_ctx *ctx, const dgc_hn_step *s, const float *
   // area; work the caller queued on the context stream before this call does not touch it either.
   Carver dc(piped ? ctx->pipe_in[slot] : ctx->stage_dev);
   cudaError_t cp_err = cudaSuccess;
-  static const bool inline_upload = [] {
-    const char *e = getenv("DGC_UPLOAD");
-    return e && strcmp(e, "inline") == 0;
-  }();
-  cudaStream_t up = inline_upload ? ctx->stream : ctx->copy_stream;
+  cudaStream_t up = ctx->copy_stream;
   auto put = [&](const float *src, uint64_t n) -> float * {
     float *d = dc.take(n);
     cudaError_t e = cudaMemcpyAsync(d, src, n * sizeof(float), cudaMemcpyHostToDevice, up);
@@ -254,20 +253,59 @@ static int32_t hn_host_enqueue(dgc_ctx *ctx, const dgc_hn_step *s, const float *
     cudaError_t e = cudaEventRecord(ev[i], up);
     if (e != cudaSuccess && cp_err == cudaSuccess) cp_err = e;
   };
-  // group 0: harmonic controls; group 1: noise branch; group 2: target
-  float *d_f0 = put(f0_host, nFB), *d_uv = put(uv_host, nFB), *d_gain = put(gain_host, nFB);
+  // The small inputs cost 5 us and a gap each on the link whatever their size: up to 512 KB of them are gathered in
+  // page-locked memory, while the amplitudes are already crossing, and go up as one copy.
+  const uint64_t small_floats = (noise ? 4 : 3) * ((nFB + 63) & ~63ull) + ((n_w + 63) & ~63ull);
+  float *gather = nullptr;
+  if (small_floats <= (128u << 10)) {
+    const int k = piped ? 1 + slot : 0;
+    if (ctx->pinned_floats[k] < small_floats) {
+      if (ctx->pinned[k]) cudaFreeHost(ctx->pinned[k]);
+      ctx->pinned[k] = nullptr;
+      ctx->pinned_floats[k] = 0;
+      DGC_CUDA(ctx, cudaMallocHost(&ctx->pinned[k], small_floats * sizeof(float)));
+      ctx->pinned_floats[k] = small_floats;
+    }
+    gather = ctx->pinned[k];
+  }
+  // group 0: harmonic controls; group 1: noise branch; then the target, in groups of voices so that the loss of the first
+  // ones is computed while the last are on their way
   float *d_amps = put(amps_host, nFB * K);
+  float *d_small = dc.take(small_floats), *d_next = d_small;
+  auto put_small = [&](const float *src, uint64_t n) -> float * {
+    float *d = d_next;
+    d_next += (n + 63) & ~63ull;
+    if (gather) memcpy(gather + (d - d_small), src, n * sizeof(float));
+    else {
+      cudaError_t e = cudaMemcpyAsync(d, src, n * sizeof(float), cudaMemcpyHostToDevice, up);
+      if (e != cudaSuccess && cp_err == cudaSuccess) cp_err = e;
+    }
+    return d;
+  };
+  float *d_f0 = put_small(f0_host, nFB), *d_uv = put_small(uv_host, nFB), *d_gain = put_small(gain_host, nFB);
+  float *d_ng = noise ? put_small(noise_gain_host, nFB) : nullptr, *d_w = n_w ? put_small(w_host, n_w) : nullptr;
+  if (gather) {
+    cudaError_t e = cudaMemcpyAsync(d_small, gather, small_floats * sizeof(float), cudaMemcpyHostToDevice, up);
+    if (e != cudaSuccess && cp_err == cudaSuccess) cp_err = e;
+  }
   mark(0);
-  float *d_ng = nullptr, *d_tab = nullptr, *d_w = nullptr, *d_noise = nullptr;
+  float *d_tab = nullptr, *d_noise = nullptr;
   if (noise) {
-    d_ng = put(noise_gain_host, nFB);
     d_tab = put(taps_or_bands_host, n_tab);
-    if (NB > 0) d_w = put(w_host, n_w);
     d_noise = gen_noise ? dc.take(nBT) : put(noise_host, nBT);
   }
   mark(1);
-  float *d_target = resident_target ? const_cast<float *>(s->target_dev) : put(target_host, nBT);
-  mark(2);
+  // four groups, each loss launch still a few waves of blocks; a resident target is one group that waits for nothing
+  const int groups = !resident_target && B >= 8 && nBT >= (1u << 18) ? DGC_MSS_MAX_GROUPS : 1;
+  float *d_target = resident_target ? const_cast<float *>(s->target_dev) : dc.take(nBT);
+  for (int q = 0; q < groups; ++q) {
+    const uint64_t t0 = (uint64_t)dgc_mss_group_start(B, q, groups) * T, t1 = (uint64_t)dgc_mss_group_start(B, q + 1, groups) * T;
+    if (!resident_target) {
+      cudaError_t e = cudaMemcpyAsync(d_target + t0, target_host + t0, (t1 - t0) * sizeof(float), cudaMemcpyHostToDevice, up);
+      if (e != cudaSuccess && cp_err == cudaSuccess) cp_err = e;
+    }
+    mark(2 + q);
+  }
   if (cp_err != cudaSuccess) {
     cudaStreamSynchronize(ctx->copy_stream);
     return dgc_fail(ctx, DGC_ERR_CUDA, "input upload: %s", cudaGetErrorString(cp_err));
@@ -276,6 +314,7 @@ static int32_t hn_host_enqueue(dgc_ctx *ctx, const dgc_hn_step *s, const float *
   // its buffers as soon as this function returns)
   auto bail = [&](int32_t code) {
     cudaStreamSynchronize(ctx->copy_stream);
+    cudaStreamSynchronize(ctx->out_stream);
     return code;
   };
   // device work area of the two-branch step, and (only when the caller wants the audio back) the summed signal
@@ -292,13 +331,23 @@ static int32_t hn_host_enqueue(dgc_ctx *ctx, const dgc_hn_step *s, const float *
     if (rc != DGC_OK) return bail(rc);
   }
   double *loss_dev = ctx->loss_accum + (piped ? 1 + slot : 0);
+  const HostEvents events = {ev[1], ev + 2, groups, ctx->audio_ev};
   rc = hn_forward_loss_impl(ctx, &st, d_f0, d_uv, d_amps, d_gain, d_ng, d_tab, d_w, d_noise, d_target, d_work, loss_dev,
-                            d_audio, inline_upload ? nullptr : ev[1], inline_upload ? nullptr : ev[2]);
+                            d_audio, &events);
   if (rc != DGC_OK) return bail(rc);
+  if (audio_host) {   // the way down is free while the target comes up and the loss is computed
+    DGC_CUDA(ctx, cudaStreamWaitEvent(ctx->out_stream, ctx->audio_ev, 0));
+    DGC_CUDA(ctx, cudaMemcpyAsync(audio_host, d_audio, nBT * sizeof(float), cudaMemcpyDeviceToHost, ctx->out_stream));
+    DGC_CUDA(ctx, cudaEventRecord(ctx->out_ev, ctx->out_stream));
+  }
   DGC_CUDA(ctx, cudaMemcpyAsync(loss_host, loss_dev, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  if (audio_host)
-    DGC_CUDA(ctx, cudaMemcpyAsync(audio_host, d_audio, nBT * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-  if (!piped) return dgc_sync(ctx, 0);
+  if (!piped) DGC_CUDA(ctx, cudaMemcpyAsync(ctx->status_host, ctx->status_dev, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+  // the step ends when its audio is down too: the next one writes the same buffer
+  if (audio_host) DGC_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->out_ev, 0));
+  if (!piped) {
+    DGC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return dgc_report_status(ctx, *ctx->status_host);
+  }
   DGC_CUDA(ctx, cudaEventRecord(ctx->pipe_done[slot], ctx->stream));
   ctx->pipe_used[slot] = true;
   ctx->pipe_pending[slot] = true;
