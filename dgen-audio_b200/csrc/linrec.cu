@@ -10,6 +10,8 @@
 // linearity the sums are corrected for the carried adjoint state without re-reading the signals).
 #include <math.h>
 
+#include <type_traits>
+
 #include "chain.cuh"
 #include "common.cuh"
 
@@ -298,10 +300,8 @@ __device__ __forceinline__ Dual dselect(float mode1, const Dual *opt, int n) {
 
 // Graph.biquad coefficient DAG (Sources/DGen/HigherOps.swift:444-555), all eight modes, node by node.
 // coef layout per lane: b0 b1 b2 a1 a2, then d/dcutoff of the five, then d/dq of the five.
-__global__ void biquad_coef_kernel(const float *__restrict__ cutoff, const float *__restrict__ q, int L, float gain,
-                                   float mode, float *__restrict__ coef) {
-  int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= L) return;
+__device__ __noinline__ void biquad_coef(const float *__restrict__ cutoff, const float *__restrict__ q, int l, float gain,
+                                         float mode, float *__restrict__ coef) {
   Dual cut = {cutoff[l], 1.f, 0.f}, res = {q[l], 0.f, 1.f};
   float add4 = mode + 1.0f;
   Dual mult7 = dmul(dabs(cut), dconst(0.00014247585730565955f));
@@ -357,6 +357,11 @@ __global__ void biquad_coef_kernel(const float *__restrict__ cutoff, const float
   c[5] = b0.dc; c[6] = b1.dc; c[7] = b2.dc; c[8] = a1.dc; c[9] = a2.dc;
   c[10] = b0.dq; c[11] = b1.dq; c[12] = b2.dq; c[13] = a1.dq; c[14] = a2.dq;
 }
+__global__ void biquad_coef_kernel(const float *__restrict__ cutoff, const float *__restrict__ q, int L, float gain,
+                                   float mode, float *__restrict__ coef) {
+  int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l < L) biquad_coef(cutoff, q, l, gain, mode, coef);
+}
 
 struct Coef {
   float b0, b1, b2, a1, a2;
@@ -373,45 +378,42 @@ __device__ __forceinline__ float biquad_step(const Coef &c, float x0, float x1, 
   return __fsub_rn(add39, add45);
 }
 
-// Per lane: the homogeneous transition over one chunk, M = [[m11 m12],[m21 m22]] with
-// (y1,y2)_end = M (y1,y2)_start for zero input.  Poles close to the unit circle make the entries of
-// M large with cancelling signs, so M and the chunk-to-chunk carry are kept in double precision.
-__global__ void biquad_trans_kernel(const float *__restrict__ coef, int L, int len, double *__restrict__ trans) {
-  int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= L) return;
-  Coef c = load_coef(coef, l);
-  const double a1 = c.a1, a2 = c.a2;
-  double m[4];
-  for (int col = 0; col < 2; ++col) {
-    double y1 = col == 0 ? 1.0 : 0.0, y2 = col == 0 ? 0.0 : 1.0;
-    for (int n = 0; n < len; ++n) {
-      double v = -(a2 * y2 + a1 * y1);
-      y2 = y1;
-      y1 = v;
-    }
-    m[col] = y1;      // m11, m12
-    m[2 + col] = y2;  // m21, m22
-  }
-  for (int i = 0; i < 4; ++i) trans[(size_t)l * 4 + i] = m[i];
+// The samples x[c0 BQ_CHUNK - 2 ..] of the chunks that a block's consecutive (chunk, lane) pairs touch, staged in shared
+// memory; returns this thread's pair, or false.  xc[n] is the chunk's frame n.  A bank of few lanes so fills its warps with
+// several chunks (37 lanes left 91 of 128 threads without work).
+__device__ __forceinline__ bool biquad_stage(const float *__restrict__ xb, int T, int L, int NC, float *sm, int &c, int &l,
+                                             const float *&xc) {
+  const int64_t i0 = (int64_t)blockIdx.x * blockDim.x, i = i0 + threadIdx.x, pairs = (int64_t)NC * L;
+  const int c0 = (int)(i0 / L), c1 = (int)((min(i0 + blockDim.x, pairs) - 1) / L);
+  const int span = (c1 - c0 + 1) * BQ_CHUNK + 2, t0 = c0 * BQ_CHUNK - 2;
+  for (int j = threadIdx.x; j < span; j += blockDim.x) sm[j] = t0 + j >= 0 && t0 + j < T ? xb[t0 + j] : 0.0f;
+  __syncthreads();
+  if (i >= pairs) return false;
+  c = (int)(i / L);
+  l = (int)(i - (int64_t)c * L);
+  xc = sm + (c - c0) * BQ_CHUNK + 2;
+  return true;
+}
+// pairs per block (fewer where a bank of one lane would make a block's chunks too many for shared memory), staged bytes
+int biquad_pairs(int L) { return L == 1 ? 64 : BQ_THREADS; }
+int biquad_stage_bytes(int L) {
+  const int n = biquad_pairs(L);
+  return ((L % n == 0 ? 1 : n / L + 2) * BQ_CHUNK + 4) * (int)sizeof(float);
 }
 
 // Forward sweep.  PHASE 0: end state of every (voice, lane, chunk) from a zero y-state.
 //                 PHASE 1: rerun from the carried state and write y[b][n][l] (lanes fastest).
 template <int PHASE>
 __global__ void __launch_bounds__(BQ_THREADS)
-biquad_fwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, int B, int T, int L, int NC,
+biquad_fwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, int T, int L, int NC,
                   float *__restrict__ state /* [B][NC][L][2] */, float *__restrict__ y,
                   const float *__restrict__ st0 = nullptr /* [B][4][L]: history cells before the call */) {
-  const int l = blockIdx.x * BQ_THREADS + threadIdx.x, c = blockIdx.y, b = blockIdx.z;
-  __shared__ float xs[BQ_CHUNK + 2];
-  const float *xb = x + (size_t)b * T;
+  extern __shared__ float sm[];
+  const int b = blockIdx.y;
+  int c, l;
+  const float *xc;
+  if (!biquad_stage(x + (size_t)b * T, T, L, NC, sm, c, l, xc)) return;
   const int n0 = c * BQ_CHUNK, len = min(BQ_CHUNK, T - n0);
-  for (int i = threadIdx.x; i < len + 2; i += BQ_THREADS) {
-    int t = n0 - 2 + i;
-    xs[i] = t >= 0 ? xb[t] : 0.0f;
-  }
-  __syncthreads();
-  if (l >= L) return;
   const Coef cf = load_coef(coef, l);
   float *st = state + (((size_t)b * NC + c) * L + l) * 2;
   float y1 = 0.f, y2 = 0.f;
@@ -419,7 +421,7 @@ biquad_fwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, i
     y1 = st[0];
     y2 = st[1];
   }
-  float x2 = xs[0], x1 = xs[1];
+  float x2 = xc[-2], x1 = xc[-1];
   if (st0 && c == 0) {   // x[-1], x[-2] come from the history cells
     x1 = st0[((size_t)b * 4 + 2) * L + l];
     x2 = st0[((size_t)b * 4 + 3) * L + l];
@@ -427,7 +429,7 @@ biquad_fwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, i
   float *yo = y + ((size_t)b * T + n0) * L + l;
 #pragma unroll 4
   for (int n = 0; n < len; ++n) {
-    float x0 = xs[n + 2];
+    float x0 = xc[n];
     float v = biquad_step(cf, x0, x1, x2, y1, y2);
     if (PHASE == 1) yo[(size_t)n * L] = v;
     x2 = x1; x1 = x0; y2 = y1; y1 = v;
@@ -448,53 +450,59 @@ biquad_fwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, i
 // product X[B*NC][C] * G^T[C][2L] on the tensor cores (its result lands directly in the [B][NC][L][2] state
 // layout) instead of a second run of the serial recurrence.  The table is evaluated in double per call (the
 // coefficients are inputs) and rounded once.
-__global__ void biquad_endstate_table_kernel(const float *__restrict__ coef, int L, float *__restrict__ G,
-                                             float *__restrict__ hist /* [L][4] */) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+// Coefficients, the homogeneous transition M over one chunk, (y1, y2)_end = M (y1, y2)_start for zero input, and (G not null)
+// the table, in one launch: a warp per lane, whose first two threads walk the recursion from (1, 0) -- those are the hy[k]
+// -- and from (0, 1).  M's entries are large with cancelling signs where the poles are close to the unit circle: double.
+// Bound by the walk, 512 dependent steps: 11 us for 256 lanes; 54 us when a thread per lane did all of it in three kernels
+// and wrote its row of G value by value.
+__global__ void __launch_bounds__(128)
+biquad_tables_kernel(const float *__restrict__ cutoff, const float *__restrict__ q, int L, float gain, float mode,
+                     float *__restrict__ coef, double *__restrict__ trans, float *__restrict__ G,
+                     float *__restrict__ hist /* [L][4] */) {
+  __shared__ double hys[4][BQ_CHUNK + 2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = blockIdx.x * 4 + warp;
   if (l >= L) return;
-  const Coef c = load_coef(coef, l);
-  const double a1 = c.a1, a2 = c.a2, b0 = c.b0, b1 = c.b1, b2 = c.b2;
-  float *g1 = G + (size_t)(2 * l) * BQ_CHUNK, *g2 = g1 + BQ_CHUNK;
-  double hm1 = 0.0, hm2 = 0.0;   // hy[k-1], hy[k-2]
-  double hprev = 0.0;            // h[k-1]
-  double hyC1 = 0, hyC2 = 0, hyC3 = 0;
-  for (int k = 0; k < BQ_CHUNK; ++k) {
-    const double hy = k == 0 ? 1.0 : -(a2 * hm2 + a1 * hm1);
-    const double h = b0 * hy + b1 * hm1 + b2 * hm2;
-    // h[k] multiplies x[n0 + C-1-k] in y[end] and x[n0 + C-2-k] in y[end-1]
-    g1[BQ_CHUNK - 1 - k] = (float)h;
-    if (k >= 1) g2[BQ_CHUNK - 1 - k] = (float)hprev;   // h[k-1] at m = C-1-k  <=>  h[C-2-m]
-    if (k == BQ_CHUNK - 1) {
-      g2[BQ_CHUNK - 1] = 0.0f;                         // m = C-1: h[-1] = 0
-      hyC1 = hy; hyC2 = hm1; hyC3 = hm2;
+  if (lane == 0) biquad_coef(cutoff, q, l, gain, mode, coef);
+  __syncwarp();
+  const float *cp = coef + (size_t)l * 15;
+  const double b0 = __ldcg(cp), b1 = __ldcg(cp + 1), b2 = __ldcg(cp + 2), a1 = __ldcg(cp + 3), a2 = __ldcg(cp + 4);
+  double *hy = hys[warp] + 2;                  // hy[-2], hy[-1]: zero
+  if (lane < 2) {
+    double y1 = lane == 0 ? 1.0 : 0.0, y2 = lane == 0 ? 0.0 : 1.0;
+    if (lane == 0) {
+      hy[-2] = hy[-1] = 0.0;
+      hy[0] = 1.0;
     }
-    hprev = h;
-    hm2 = hm1;
-    hm1 = hy;
+    for (int n = 0; n < BQ_CHUNK; n += 4) {    // the order of rounding of four steps as it always was, see BiquadSweep
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const double v = j == 0 ? -__fma_rn(a1, y1, __dmul_rn(a2, y2)) : -__fma_rn(a2, y2, __dmul_rn(a1, y1));
+        y2 = y1;
+        y1 = v;
+        if (lane == 0 && n + j + 1 < BQ_CHUNK) hy[n + j + 1] = v;
+      }
+    }
+    trans[(size_t)l * 4 + lane] = y1;          // m11, m12
+    trans[(size_t)l * 4 + 2 + lane] = y2;      // m21, m22
   }
-  hist[l * 4 + 0] = (float)(b1 * hyC1 + b2 * hyC2);
-  hist[l * 4 + 1] = (float)(b1 * hyC2 + b2 * hyC3);
-  hist[l * 4 + 2] = (float)(b2 * hyC1);
-  hist[l * 4 + 3] = (float)(b2 * hyC2);
-}
-
-// adds the x-history terms to the matrix-product states
-__global__ void biquad_state_hist_kernel(const float *__restrict__ x, const float *__restrict__ hist, int B, int T, int L,
-                                         int NC, float *__restrict__ state, const float *__restrict__ st0 = nullptr) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)B * NC * L) return;
-  const int l = (int)(idx % L);
-  const size_t bc = idx / L;
-  const int c = (int)(bc % NC), b = (int)(bc / NC);
-  if (c == 0 && !st0) return;   // no history before the first chunk
-  const float *xb = x + (size_t)b * T + (size_t)c * BQ_CHUNK;
-  const float x1 = c == 0 ? st0[((size_t)b * 4 + 2) * L + l] : xb[-1];
-  const float x2 = c == 0 ? st0[((size_t)b * 4 + 3) * L + l] : xb[-2];
-  float2 *st = reinterpret_cast<float2 *>(state) + idx;
-  float2 v = *st;
-  v.x += hist[l * 4 + 0] * x1 + hist[l * 4 + 2] * x2;
-  v.y += hist[l * 4 + 1] * x1 + hist[l * 4 + 3] * x2;
-  *st = v;
+  __syncwarp();
+  if (!G) return;
+  float *g1 = G + (size_t)(2 * l) * BQ_CHUNK, *g2 = g1 + BQ_CHUNK;
+  for (int k = lane; k < BQ_CHUNK; k += 32) {
+    const double h0 = hy[k], h1 = hy[k - 1], h2 = hy[k - 2];
+    const float h = (float)(b0 * h0 + b1 * h1 + b2 * h2);
+    // h[k] multiplies x[n0 + C-1-k] in y[end] and x[n0 + C-2-k] in y[end-1]
+    g1[BQ_CHUNK - 1 - k] = h;
+    if (k + 1 < BQ_CHUNK) g2[BQ_CHUNK - 2 - k] = h;
+    else g2[BQ_CHUNK - 1] = 0.0f;              // m = C-1: h[-1] = 0
+  }
+  if (lane == 0) {
+    const double y1 = hy[BQ_CHUNK - 1], y2 = hy[BQ_CHUNK - 2], y3 = hy[BQ_CHUNK - 3];
+    hist[l * 4 + 0] = (float)(b1 * y1 + b2 * y2);
+    hist[l * 4 + 1] = (float)(b1 * y2 + b2 * y3);
+    hist[l * 4 + 2] = (float)(b2 * y1);
+    hist[l * 4 + 3] = (float)(b2 * y2);
+  }
 }
 
 // The same sweep with FOUR lanes per thread (L a multiple of 4): four independent recurrences hide the
@@ -554,25 +562,60 @@ biquad_fwd4_kernel(const float *__restrict__ x, const float *__restrict__ coef, 
   }
 }
 
-// state[c] <- state entering chunk c (exclusive scan of the affine maps), thread per (voice, lane)
-__global__ void biquad_carry_kernel(const double *__restrict__ trans, int B, int L, int NC,
-                                    float *__restrict__ state, const float *__restrict__ st0 = nullptr) {
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= B * L) return;
-  int b = idx / L, l = idx - b * L;
+// state[c] <- state entering chunk c: the affine maps s <- M s + e one after the other, in double, a thread per (voice, lane).
+// The next BQ_AHEAD chunks are in flight while the present ones are walked.  Not a scan by runs: a last-bit change of a
+// state is 140 times as much in the output of a low, sharp lane, and 10000 times in the gradient of its cutoff.
+// hist (optional): the end states come from the matrix product, which knows nothing of the x-history before a chunk: its
+// two terms are added here.  32 voices x 512 chunks x 256 lanes: 70 us, 110 us as two kernels with a load in every step.
+constexpr int BQ_AHEAD = 16;
+__global__ void __launch_bounds__(32)
+biquad_carry_kernel(const double *__restrict__ trans, const float *__restrict__ x, const float *__restrict__ hist, int T, int L,
+                    int NC, float2 *__restrict__ state, const float *__restrict__ st0) {
+  const int l = blockIdx.x * 32 + threadIdx.x, b = blockIdx.y;
+  if (l >= L) return;
   const double m11 = trans[(size_t)l * 4], m12 = trans[(size_t)l * 4 + 1], m21 = trans[(size_t)l * 4 + 2],
                m22 = trans[(size_t)l * 4 + 3];
+  float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (hist) h = make_float4(hist[l * 4], hist[l * 4 + 1], hist[l * 4 + 2], hist[l * 4 + 3]);
+  const float *xb = x + (size_t)b * T;
+  float2 *st = state + (size_t)b * NC * L + l;
   // y[-1], y[-2]: the history cells before the call, else rest
   double s1 = st0 ? (double)st0[((size_t)b * 4 + 0) * L + l] : 0.0, s2 = st0 ? (double)st0[((size_t)b * 4 + 1) * L + l] : 0.0;
-  for (int c = 0; c < NC; ++c) {
-    float *st = state + (((size_t)b * NC + c) * L + l) * 2;
-    double e1 = st[0], e2 = st[1];
-    st[0] = (float)s1;
-    st[1] = (float)s2;
-    // every chunk but possibly the last has full length; the state after the last chunk is unused
-    double n1 = m11 * s1 + m12 * s2 + e1, n2 = m21 * s1 + m22 * s2 + e2;
-    s1 = n1;
-    s2 = n2;
+  float2 e[BQ_AHEAD], xx[BQ_AHEAD];
+  auto fetch = [&](int c0) {
+#pragma unroll
+    for (int j = 0; j < BQ_AHEAD; ++j) {
+      const int c = c0 + j;
+      if (c < NC) {
+        e[j] = st[(size_t)c * L];
+        if (hist && c > 0) xx[j] = make_float2(__ldg(xb + (size_t)c * BQ_CHUNK - 1), __ldg(xb + (size_t)c * BQ_CHUNK - 2));
+      }
+    }
+    if (hist && c0 == 0 && st0) xx[0] = make_float2(st0[((size_t)b * 4 + 2) * L + l], st0[((size_t)b * 4 + 3) * L + l]);
+  };
+  fetch(0);
+  for (int c0 = 0; c0 < NC; c0 += BQ_AHEAD) {
+    float2 v[BQ_AHEAD];
+#pragma unroll
+    for (int j = 0; j < BQ_AHEAD; ++j) {
+      v[j] = e[j];
+      if (hist && (c0 + j > 0 || st0)) {
+        v[j].x += h.x * xx[j].x + h.z * xx[j].y;
+        v[j].y += h.y * xx[j].x + h.w * xx[j].y;
+      }
+    }
+    fetch(c0 + BQ_AHEAD);
+#pragma unroll
+    for (int j = 0; j < BQ_AHEAD; ++j) {
+      if (c0 + j < NC) {
+        st[(size_t)(c0 + j) * L] = make_float2((float)s1, (float)s2);
+        // every chunk but possibly the last has full length; the state after the last chunk is unused
+        const double e1 = v[j].x, e2 = v[j].y;
+        const double n1 = m11 * s1 + m12 * s2 + e1, n2 = m21 * s1 + m22 * s2 + e2;
+        s1 = n1;
+        s2 = n2;
+      }
+    }
   }
 }
 
@@ -586,49 +629,28 @@ __global__ void biquad_carry_kernel(const double *__restrict__ trans, int B, int
 // S_loc + s1*S_h1 + s2*S_h2.  Record per (voice, chunk, lane): 15 sums + local start adjoint (2) + sq error.
 constexpr int BW_REC = 18;
 
-// UP = false: g = gscale * (y - tgt) (the MSE loss, squared error summed on the way);  UP = true: `tgt` IS the
-// upstream gradient dL/dy [B][T][L] of an arbitrary loss.
+// The order in which a1 p + a2 q is rounded is spelled out: lam and one frame in sixteen (in the edge chunks every odd one)
+// multiply a2 q first, the rest a1 p.  The gradient of a low cutoff is a difference of these sums that loses four digits,
+// so another order is another gradient there (6e-3 at 32 voices x 256 lanes); this one is kept as it is.
+__device__ __forceinline__ float feedback(const Coef &c, float p, float q, bool a2_first) {
+  return a2_first ? __fmaf_rn(c.a1, p, __fmul_rn(c.a2, q)) : __fmaf_rn(c.a2, q, __fmul_rn(c.a1, p));
+}
+
 template <bool UP>
-__global__ void __launch_bounds__(BQ_THREADS)
-biquad_bwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, const float *__restrict__ y,
-                  const float *__restrict__ tgt, int B, int T, int L, int NC, float gscale,
-                  float *__restrict__ rec /* [B][NC][BW_REC][L] */) {
-  const int l = blockIdx.x * BQ_THREADS + threadIdx.x, c = blockIdx.y, b = blockIdx.z;
-  __shared__ float xs[BQ_CHUNK + 2];
-  const float *xb = x + (size_t)b * T;
-  const int n0 = c * BQ_CHUNK, len = min(BQ_CHUNK, T - n0);
-  for (int i = threadIdx.x; i < len + 2; i += BQ_THREADS) {
-    int t = n0 - 2 + i;
-    xs[i] = t >= 0 ? xb[t] : 0.0f;
-  }
-  __syncthreads();
-  if (l >= L) return;
-  const Coef cf = load_coef(coef, l);
-  const float *yb = y + (size_t)b * T * L + l, *tb = tgt + (size_t)b * T * L + l;
-  float la1 = 0.f, la2 = 0.f;            // lam[n+1], lam[n+2] (local)
-  float h1a = 1.f, h1b = 0.f;            // homogeneous response to terminal (lam[n_end+1], lam[n_end+2]) = (1,0)
-  float h2a = 0.f, h2b = 1.f;            // ... = (0,1)
-  float S[15];
-#pragma unroll
-  for (int i = 0; i < 15; ++i) S[i] = 0.f;
-  float sq = 0.f;
-  // y[n-1], y[n-2] sliding from the top: prefetch y at n, n-1, n-2
-  int nt = n0 + len - 1;
-  float yc = yb[(size_t)nt * L];
-  float ym1 = nt - 1 >= 0 ? yb[(size_t)(nt - 1) * L] : 0.f;
-  auto body = [&](int n, float ym2, float tv) {
-    float g;
-    if (UP) {
-      g = tv;
-    } else {
-      float d = yc - tv;
-      sq = fmaf(d, d, sq);
-      g = gscale * d;
-    }
-    float lam = g - (cf.a1 * la1 + cf.a2 * la2);
-    float h1 = -(cf.a1 * h1a + cf.a2 * h1b);
-    float h2 = -(cf.a1 * h2a + cf.a2 * h2b);
-    float x0 = xs[n + 2], x1 = xs[n + 1], x2 = xs[n];
+struct BiquadSweep {
+  Coef cf;
+  float gscale, yc, ym1;                     // y[n], y[n-1]
+  float la1 = 0.f, la2 = 0.f;                // lam[n+1], lam[n+2] (local)
+  float h1a = 1.f, h1b = 0.f;                // homogeneous response to terminal (lam[n_end+1], lam[n_end+2]) = (1,0)
+  float h2a = 0.f, h2b = 1.f;                // ... = (0,1)
+  float S[15] = {}, sq = 0.f;
+
+  // frame n: x[n], x[n-1], x[n-2], y[n-2], target
+  __device__ __forceinline__ void step(float x0, float x1, float x2, float ym2, float tv, bool a2_first) {
+    const float fed = feedback(cf, la1, la2, true), d = UP ? 0.0f : __fsub_rn(yc, tv);
+    if (!UP) sq = fmaf(d, d, sq);
+    const float lam = UP ? __fsub_rn(tv, fed) : __fmaf_rn(gscale, d, -fed);
+    const float h1 = -feedback(cf, h1a, h1b, a2_first), h2 = -feedback(cf, h2a, h2b, a2_first);
     S[0] = fmaf(lam, x0, S[0]); S[1] = fmaf(lam, x1, S[1]); S[2] = fmaf(lam, x2, S[2]);
     S[3] = fmaf(lam, ym1, S[3]); S[4] = fmaf(lam, ym2, S[4]);
     S[5] = fmaf(h1, x0, S[5]); S[6] = fmaf(h1, x1, S[6]); S[7] = fmaf(h1, x2, S[7]);
@@ -639,79 +661,150 @@ biquad_bwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, c
     h1b = h1a; h1a = h1;
     h2b = h2a; h2a = h2;
     yc = ym1; ym1 = ym2;
-  };
+  }
+  __device__ __forceinline__ void record(float *r, int L) const {
+#pragma unroll
+    for (int i = 0; i < 15; ++i) r[(size_t)i * L] = S[i];
+    r[(size_t)15 * L] = la1;  // local adjoint at the first frame of the chunk: lam[n0]
+    r[(size_t)16 * L] = la2;  // lam[n0+1]
+    r[(size_t)17 * L] = sq;
+  }
+};
+
+// UP = false: g = gscale * (y - tgt) (the MSE loss, squared error summed on the way);  UP = true: `tgt` IS the
+// upstream gradient dL/dy [B][T][L] of an arbitrary loss.
+// A group of sixteen frames issues its 32 loads before the dependent recurrence steps: the sweep is bound by loads in
+// flight (32 voices x 262144 x 256 lanes: 17.2 GB in 3.20 ms, 82 % of the copy rate).  In the first and the last chunk frames
+// outside the chunk or the signal are zeros; with a load in every step those two took three times as long as the others,
+// and a bank of few lanes as long as they: 5 voices x 50001 x 37 lanes 124 us, now 76.  Asynchronous copies to a ring in
+// shared memory were measured: 6 % slower on the large bank, 66 us on this one but 80 for 61 with 64 lanes.
+template <bool UP>
+__global__ void __launch_bounds__(BQ_THREADS)
+biquad_bwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, const float *__restrict__ y,
+                  const float *__restrict__ tgt, int T, int L, int NC, float gscale,
+                  float *__restrict__ rec /* [B][NC][BW_REC][L] */) {
+  extern __shared__ float sm[];
+  constexpr int G = 16;
+  const int b = blockIdx.y;
+  int c, l;
+  const float *xc;
+  if (!biquad_stage(x + (size_t)b * T, T, L, NC, sm, c, l, xc)) return;
+  const int n0 = c * BQ_CHUNK, len = min(BQ_CHUNK, T - n0);
+  const float *yb = y + ((size_t)b * T + n0) * L + l, *tb = tgt + ((size_t)b * T + n0) * L + l;
+  auto y_at = [&](int n) { return n0 + n >= 0 ? yb[(ptrdiff_t)n * L] : 0.0f; };
+  BiquadSweep<UP> w{load_coef(coef, l), gscale, y_at(len - 1), y_at(len - 2)};
   if (len == BQ_CHUNK && n0 >= 2) {
-    // interior chunk: every load is in range, so a group of sixteen frames issues its 32 loads before the
-    // dependent recurrence steps (the sweep is bound by loads in flight, not by arithmetic)
-    constexpr int G = 16;
-    for (int nb = BQ_CHUNK - G; nb >= 0; nb -= G) {
+    auto group = [&](int nb, auto first) {
       float yv[G], tv[G];
 #pragma unroll
       for (int j = 0; j < G; ++j) {
-        const int t = n0 + nb + j;
-        yv[j] = __ldcs(yb + (size_t)(t - 2) * L);
-        tv[j] = __ldcs(tb + (size_t)t * L);
+        yv[j] = __ldcs(yb + (ptrdiff_t)(nb + j - 2) * L);
+        tv[j] = __ldcs(tb + (ptrdiff_t)(nb + j) * L);
       }
 #pragma unroll
-      for (int j = G - 1; j >= 0; --j) body(nb + j, yv[j], tv[j]);
-    }
+      for (int j = G - 1; j >= 0; --j)
+        w.step(xc[nb + j], xc[nb + j - 1], xc[nb + j - 2], yv[j], tv[j], j == G - 1 || (decltype(first)::value && j == G - 2));
+    };
+    group(BQ_CHUNK - G, std::true_type());
+    for (int nb = BQ_CHUNK - 2 * G; nb >= 0; nb -= G) group(nb, std::false_type());
   } else {
-    for (int n = len - 1; n >= 0; --n) {
-      int t = n0 + n;
-      float ym2 = t - 2 >= 0 ? yb[(size_t)(t - 2) * L] : 0.f;
-      body(n, ym2, tb[(size_t)t * L]);
+    for (int nb = (len - 1) / G * G; nb >= 0; nb -= G) {
+      float yv[G], tv[G];
+#pragma unroll
+      for (int j = 0; j < G; ++j) {
+        const int n = nb + j;
+        yv[j] = n < len && n0 + n >= 2 ? __ldcs(yb + (ptrdiff_t)(n - 2) * L) : 0.0f;
+        tv[j] = n < len ? __ldcs(tb + (ptrdiff_t)n * L) : 0.0f;
+      }
+#pragma unroll
+      for (int j = G - 1; j >= 0; --j)
+        if (nb + j < len) w.step(xc[nb + j], xc[nb + j - 1], xc[nb + j - 2], yv[j], tv[j], j & 1);
     }
   }
-  float *r = rec + ((size_t)b * NC + c) * BW_REC * L + l;
-#pragma unroll
-  for (int i = 0; i < 15; ++i) r[(size_t)i * L] = S[i];
-  r[(size_t)15 * L] = la1;  // local adjoint at the first frame of the chunk: lam[n0]
-  r[(size_t)16 * L] = la2;  // lam[n0+1]
-  r[(size_t)17 * L] = sq;
+  w.record(rec + ((size_t)b * NC + c) * BW_REC * L + l, L);
 }
 
-// Reverse carry over chunks, thread per (voice, lane): resolves the terminal adjoint of every chunk,
-// combines the sums, and writes per (voice, lane) the five coefficient-gradient sums and the squared error.
-__global__ void biquad_bwd_carry_kernel(const float *__restrict__ rec, const float *__restrict__ coef, int B, int L,
-                                        int NC, int T, double *__restrict__ acc /* [B][L][6] */,
-                                        float2 *__restrict__ term /* [B][NC][L] or null */) {
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= B * L) return;
-  int b = idx / L, l = idx - b * L;
-  const Coef cf = load_coef(coef, l);
-  // adjoint transition over a full chunk: (lam[n0], lam[n0+1]) = A (s1, s2) + local, with A from the
-  // homogeneous responses; recompute A by running the recurrence (cheap, per thread)
-  const double da1 = cf.a1, da2 = cf.a2;
-  auto homog = [&](int len, double &a11, double &a12, double &a21, double &a22) {
-    double p1 = 1.0, p2 = 0.0, q1 = 0.0, q2 = 1.0;
-    for (int n = 0; n < len; ++n) {
-      double v = -(da1 * p1 + da2 * p2);
-      p2 = p1; p1 = v;
-      double w = -(da1 * q1 + da2 * q2);
-      q2 = q1; q1 = w;
-    }
-    a11 = p1; a21 = p2; a12 = q1; a22 = q2;
-  };
-  double f11, f12, f21, f22;
-  homog(BQ_CHUNK, f11, f12, f21, f22);
-  double G[5] = {0, 0, 0, 0, 0}, sq = 0;
-  double s1 = 0.0, s2 = 0.0;  // terminal adjoint (lam[n_end+1], lam[n_end+2]) of the current chunk
-  for (int c = NC - 1; c >= 0; --c) {
-    const float *r = rec + ((size_t)b * NC + c) * BW_REC * L + l;
-    if (term) term[((size_t)b * NC + c) * L + l] = make_float2((float)s1, (float)s2);
-    for (int i = 0; i < 5; ++i)
-      G[i] += (double)r[(size_t)i * L] + s1 * (double)r[(size_t)(5 + i) * L] + s2 * (double)r[(size_t)(10 + i) * L];
-    sq += (double)r[(size_t)17 * L];
-    int len = min(BQ_CHUNK, T - c * BQ_CHUNK);
-    double a11 = f11, a12 = f12, a21 = f21, a22 = f22;
-    if (len != BQ_CHUNK) homog(len, a11, a12, a21, a22);
-    double n1 = a11 * s1 + a12 * s2 + (double)r[(size_t)15 * L];
-    double n2 = a21 * s1 + a22 * s2 + (double)r[(size_t)16 * L];
-    s1 = n1;
-    s2 = n2;
+struct Mat2 {
+  double a, b, c, d;      // [[a, b], [c, d]]
+};
+__device__ __forceinline__ Mat2 mat_mul(const Mat2 &p, const Mat2 &q) {
+  return {p.a * q.a + p.b * q.c, p.a * q.b + p.b * q.d, p.c * q.a + p.d * q.c, p.c * q.b + p.d * q.d};
+}
+// m^n by squaring
+__device__ __forceinline__ Mat2 mat_pow(Mat2 m, int n) {
+  Mat2 r = {1.0, 0.0, 0.0, 1.0};
+  for (; n > 0; n >>= 1) {
+    if (n & 1) r = mat_mul(r, m);
+    m = mat_mul(m, m);
   }
-  double *o = acc + ((size_t)b * L + l) * 6;
-  o[0] = G[0]; o[1] = G[1]; o[2] = G[2]; o[3] = -G[3]; o[4] = -G[4]; o[5] = sq;
+  return r;
+}
+
+// Reverse carry over chunks, in double: resolves the terminal adjoint of every chunk, combines the sums, and writes per
+// (voice, lane) the five coefficient-gradient sums and the squared error.  Block = 32 lanes of a voice x BQ_RUNS warps: a
+// warp walks its run of consecutive chunks from rest, the ends of the runs are carried over by A^run, and the warp walks
+// its run again from the true terminal adjoint; the warps' sums are added in a fixed order.  (Nothing here is rounded to
+// single precision but the results.)  32 voices x 512 chunks x 256 lanes: 80 us, the record's 302 MB at 3.8 TB/s; 914 us when
+// a thread per (voice, lane) walked all chunks, two warps on an SM.
+constexpr int BQ_RUNS = 16;
+__global__ void __launch_bounds__(32 * BQ_RUNS)
+biquad_bwd_carry_kernel(const float *__restrict__ rec, const float *__restrict__ coef, int L, int NC,
+                        double *__restrict__ acc /* [B][L][6] */, float2 *__restrict__ term /* [B][NC][L] or null */) {
+  __shared__ double2 ends[BQ_RUNS][32];
+  __shared__ double sums[BQ_RUNS][6][32];
+  const int l = blockIdx.x * 32 + threadIdx.x, run = threadIdx.y, b = blockIdx.y;
+  // run 0 takes the LAST chunks, the ones the reverse pass meets first
+  const int per = (NC + BQ_RUNS - 1) / BQ_RUNS, d0 = min(run * per, NC), d1 = min(d0 + per, NC);
+  const bool live = l < L;
+  const Coef cf = live ? load_coef(coef, l) : Coef{};
+  const float *rb = rec + (size_t)b * NC * BW_REC * L + l;
+  // (lam[n0], lam[n0+1]) = A (terminal adjoint) + local, A = [[h1[0], h2[0]], [h1[1], h2[1]]] over a full chunk.  The one
+  // chunk that may be shorter is the last, whose terminal adjoint is zero.
+  const Mat2 A = mat_pow({-(double)cf.a1, -(double)cf.a2, 1.0, 0.0}, BQ_CHUNK);
+  double s1 = 0.0, s2 = 0.0;
+  if (live) {
+#pragma unroll 8
+    for (int d = d0; d < d1; ++d) {
+      const float *r = rb + (size_t)(NC - 1 - d) * BW_REC * L;
+      const double n1 = A.a * s1 + A.b * s2 + (double)r[(size_t)15 * L], n2 = A.c * s1 + A.d * s2 + (double)r[(size_t)16 * L];
+      s1 = n1;
+      s2 = n2;
+    }
+  }
+  ends[run][threadIdx.x] = make_double2(s1, s2);
+  __syncthreads();
+  double g[6] = {0, 0, 0, 0, 0, 0};
+  if (live && d0 < d1) {
+    s1 = s2 = 0.0;
+    const Mat2 Ar = mat_pow(A, per);
+    for (int q = 0; q < run; ++q) {
+      const double2 e = ends[q][threadIdx.x];
+      const double n1 = Ar.a * s1 + Ar.b * s2 + e.x, n2 = Ar.c * s1 + Ar.d * s2 + e.y;
+      s1 = n1;
+      s2 = n2;
+    }
+#pragma unroll 2
+    for (int d = d0; d < d1; ++d) {
+      const int c = NC - 1 - d;
+      const float *r = rb + (size_t)c * BW_REC * L;
+      if (term) term[((size_t)b * NC + c) * L + l] = make_float2((float)s1, (float)s2);
+#pragma unroll
+      for (int i = 0; i < 5; ++i)
+        g[i] += (double)r[(size_t)i * L] + s1 * (double)r[(size_t)(5 + i) * L] + s2 * (double)r[(size_t)(10 + i) * L];
+      g[5] += (double)r[(size_t)17 * L];
+      const double n1 = A.a * s1 + A.b * s2 + (double)r[(size_t)15 * L], n2 = A.c * s1 + A.d * s2 + (double)r[(size_t)16 * L];
+      s1 = n1;
+      s2 = n2;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 6; ++i) sums[run][i][threadIdx.x] = g[i];
+  __syncthreads();
+  if (live && run < 6) {
+    double t = 0.0;
+    for (int q = 0; q < BQ_RUNS; ++q) t += sums[q][run][threadIdx.x];
+    acc[((size_t)b * L + l) * 6 + run] = run == 3 || run == 4 ? -t : t;
+  }
 }
 
 // Gradient with respect to the INPUT x[b][n] (shared by the lanes): sum over lanes of
@@ -786,34 +879,56 @@ __global__ void sum_partial_rows_kernel(const float *__restrict__ part, int npar
   out[i] = s;
 }
 
-// Sum over voices (fixed order), chain rule to cutoff and q, total loss.
-__global__ void biquad_bwd_final_kernel(const double *__restrict__ acc, const float *__restrict__ coef, int B, int L,
-                                        float loss_scale, float *__restrict__ gcut, float *__restrict__ gq,
-                                        double *__restrict__ lane_loss) {
-  int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= L) return;
-  double G[5] = {0, 0, 0, 0, 0}, sq = 0;
-  for (int b = 0; b < B; ++b) {
-    const double *a = acc + ((size_t)b * L + l) * 6;
-    for (int i = 0; i < 5; ++i) G[i] += a[i];
-    sq += a[5];
+// Sum over voices, chain rule to cutoff and q, total loss: a warp per lane, the voices over its threads and a fixed tree;
+// the block that finishes last adds the lanes' losses.
+__global__ void __launch_bounds__(256)
+biquad_bwd_final_kernel(const double *__restrict__ acc, const float *__restrict__ coef, int B, int L,
+                        float loss_scale, float *__restrict__ gcut, float *__restrict__ gq,
+                        double *__restrict__ lane_loss, unsigned int *__restrict__ ticket, double *__restrict__ loss) {
+  const int l = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (l < L) {
+    double G[6] = {0, 0, 0, 0, 0, 0};
+    for (int b = lane; b < B; b += 32)
+#pragma unroll
+      for (int i = 0; i < 6; ++i) G[i] += acc[((size_t)b * L + l) * 6 + i];
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) G[i] += __shfl_xor_sync(0xffffffffu, G[i], o);
+    if (lane == 0) {
+      const float *c = coef + (size_t)l * 15;
+      double dc = 0, dq = 0;
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        dc += G[i] * (double)c[5 + i];
+        dq += G[i] * (double)c[10 + i];
+      }
+      gcut[l] = (float)dc;
+      gq[l] = (float)dq;
+      lane_loss[l] = G[5] * (double)loss_scale;
+    }
   }
-  const float *c = coef + (size_t)l * 15;
-  double dc = 0, dq = 0;
-  for (int i = 0; i < 5; ++i) {
-    dc += G[i] * (double)c[5 + i];
-    dq += G[i] * (double)c[10 + i];
+  if (!loss) return;
+  __shared__ bool last;
+  __shared__ double part[256];
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double t = 0.0;
+  for (int i = threadIdx.x; i < L; i += 256) t += __ldcg(lane_loss + i);
+  part[threadIdx.x] = t;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if (threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
+    __syncthreads();
   }
-  gcut[l] = (float)dc;
-  gq[l] = (float)dq;
-  lane_loss[l] = sq * (double)loss_scale;
-}
-
-__global__ void sum_doubles_kernel(const double *__restrict__ v, int n, double *__restrict__ out) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  double t = 0;
-  for (int i = 0; i < n; ++i) t += v[i];
-  out[0] = t;
+  if (threadIdx.x == 0) {
+    *loss = part[0];
+    *ticket = 0u;
+  }
 }
 
 }  // namespace
@@ -912,37 +1027,68 @@ static int32_t biquad_fwd_impl(dgc_ctx *ctx, const dgc_biquad_params *p, const f
   float *coef = scr;
   double *trans = reinterpret_cast<double *>(scr + (size_t)L * 16);
   float *state = scr + ((((size_t)L * 24) + 3) & ~(size_t)3);
-  biquad_coef_kernel<<<dgc_div_up(L, 128), 128, 0, ctx->stream>>>(cutoff_dev, q_dev, L, p->gain, p->mode, coef);
-  DGC_LAUNCHED(ctx, "biquad_coef");
-  biquad_trans_kernel<<<dgc_div_up(L, 128), 128, 0, ctx->stream>>>(coef, L, BQ_CHUNK, trans);
-  DGC_LAUNCHED(ctx, "biquad_trans");
   // four lanes per thread when the lane count and the output alignment allow 128-bit accesses
   const bool quad = (L & 3) == 0 && L >= 16 && ((((uintptr_t)y_dev) | ((uintptr_t)state)) & 15) == 0;
   const int qx = quad ? (L / 4 >= 64 ? 64 : L / 4) : 0;
-  dim3 grid(dgc_div_up(L, BQ_THREADS), NC, B);
+  const int nth = biquad_pairs(L), smem = biquad_stage_bytes(L);
+  const dim3 grid((unsigned)(((int64_t)NC * L + nth - 1) / nth), B);
   dim3 grid4(quad ? dgc_div_up(L / 4, qx) : 1, dgc_div_up(NC, BQ4_CHUNKS), B), block4(quad ? qx : 1, BQ4_CHUNKS);
+  if (!quad && smem > 48 * 1024) {
+    DGC_CUDA(ctx, cudaFuncSetAttribute(biquad_fwd_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    DGC_CUDA(ctx, cudaFuncSetAttribute(biquad_fwd_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  }
   // first pass: chunk end states from a zero y-state -- as one tensor-core product when the chunks tile T exactly
   // and the problem is large enough for that path, else by running the recurrence
   const bool by_matmul = (T % BQ_CHUNK) == 0 && (double)B * NC * L >= (double)(1 << 16) && (((uintptr_t)x_dev) & 15) == 0;
+  float *G = by_matmul ? state + ((((size_t)B * NC * L * 2) + 3) & ~(size_t)3) : nullptr;
+  float *hist = by_matmul ? G + (size_t)L * 2 * BQ_CHUNK : nullptr;
+  biquad_tables_kernel<<<dgc_div_up(L, 4), 128, 0, ctx->stream>>>(cutoff_dev, q_dev, L, p->gain, p->mode, coef, trans, G, hist);
+  DGC_LAUNCHED(ctx, "biquad_tables");
   if (by_matmul) {
-    float *G = state + ((((size_t)B * NC * L * 2) + 3) & ~(size_t)3), *hist = G + (size_t)L * 2 * BQ_CHUNK;
-    biquad_endstate_table_kernel<<<dgc_div_up(L, 64), 64, 0, ctx->stream>>>(coef, L, G, hist);
-    DGC_LAUNCHED(ctx, "biquad_endstate_table");
     rc = dgc_gemm_nt(ctx, x_dev, G, B * NC, 2 * L, BQ_CHUNK, state);
     if (rc != DGC_OK) return rc;
-    biquad_state_hist_kernel<<<dgc_div_up((int64_t)B * NC * L, 256), 256, 0, ctx->stream>>>(x_dev, hist, B, T, L, NC, state, st0);
-  } else if (quad) biquad_fwd4_kernel<0><<<grid4, block4, 0, ctx->stream>>>(x_dev, coef, B, T, L, NC, state, nullptr, st0);
-  else biquad_fwd_kernel<0><<<grid, BQ_THREADS, 0, ctx->stream>>>(x_dev, coef, B, T, L, NC, state, nullptr, st0);
-  DGC_LAUNCHED(ctx, "biquad_fwd_state");
-  biquad_carry_kernel<<<dgc_div_up(B * L, 128), 128, 0, ctx->stream>>>(trans, B, L, NC, state, st0);
+  } else {
+    if (quad) biquad_fwd4_kernel<0><<<grid4, block4, 0, ctx->stream>>>(x_dev, coef, B, T, L, NC, state, nullptr, st0);
+    else biquad_fwd_kernel<0><<<grid, nth, smem, ctx->stream>>>(x_dev, coef, T, L, NC, state, nullptr, st0);
+    DGC_LAUNCHED(ctx, "biquad_fwd_state");
+  }
+  biquad_carry_kernel<<<dim3(dgc_div_up(L, 32), B), 32, 0, ctx->stream>>>(trans, x_dev, hist, T, L, NC,
+                                                                         reinterpret_cast<float2 *>(state), st0);
   DGC_LAUNCHED(ctx, "biquad_carry");
   if (quad) biquad_fwd4_kernel<1><<<grid4, block4, 0, ctx->stream>>>(x_dev, coef, B, T, L, NC, state, y_dev, st0);
-  else biquad_fwd_kernel<1><<<grid, BQ_THREADS, 0, ctx->stream>>>(x_dev, coef, B, T, L, NC, state, y_dev, st0);
+  else biquad_fwd_kernel<1><<<grid, nth, smem, ctx->stream>>>(x_dev, coef, T, L, NC, state, y_dev, st0);
   DGC_LAUNCHED(ctx, "biquad_fwd_out");
   if (st0) {
     biquad_final_state_kernel<<<dgc_div_up(B * L, 128), 128, 0, ctx->stream>>>(x_dev, y_dev, B, T, L, st0);
     DGC_LAUNCHED(ctx, "biquad_final_state");
   }
+  return DGC_OK;
+}
+
+// The reverse-time pass both backward entry points share: coefficients, sweep, carry, gradients (and the loss)
+template <bool UP>
+static int32_t biquad_backward(dgc_ctx *ctx, const dgc_biquad_params *p, const float *x, const float *cutoff, const float *q,
+                               const float *y, const float *up, float gscale, float loss_scale, float *scr, float2 *term,
+                               float *gcut, float *gq, double *loss) {
+  const int B = p->B, T = p->T, L = p->L, NC = dgc_div_up(T, BQ_CHUNK);
+  float *coef = scr;
+  float *rec = scr + ((((size_t)L * 24) + 3) & ~(size_t)3);
+  const size_t rec_n = ((size_t)B * NC * BW_REC * L + 3) & ~(size_t)3;
+  double *acc = reinterpret_cast<double *>(rec + rec_n);
+  double *lane_loss = acc + (size_t)B * L * 6;
+  biquad_coef_kernel<<<dgc_div_up(L, 32), 32, 0, ctx->stream>>>(cutoff, q, L, p->gain, p->mode, coef);
+  DGC_LAUNCHED(ctx, "biquad_coef");
+  const int nth = biquad_pairs(L), smem = biquad_stage_bytes(L);
+  if (smem > 48 * 1024)
+    DGC_CUDA(ctx, cudaFuncSetAttribute(biquad_bwd_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  const dim3 grid((unsigned)(((int64_t)NC * L + nth - 1) / nth), B);
+  biquad_bwd_kernel<UP><<<grid, nth, smem, ctx->stream>>>(x, coef, y, up, T, L, NC, gscale, rec);
+  DGC_LAUNCHED(ctx, "biquad_bwd");
+  biquad_bwd_carry_kernel<<<dim3(dgc_div_up(L, 32), B), dim3(32, BQ_RUNS), 0, ctx->stream>>>(rec, coef, L, NC, acc, term);
+  DGC_LAUNCHED(ctx, "biquad_bwd_carry");
+  biquad_bwd_final_kernel<<<dgc_div_up(L, 8), 256, 0, ctx->stream>>>(acc, coef, B, L, loss_scale, gcut, gq, lane_loss,
+                                                                    ctx->ticket_dev, loss);
+  DGC_LAUNCHED(ctx, "biquad_bwd_final");
   return DGC_OK;
 }
 
@@ -955,30 +1101,12 @@ DGC_EXPORT int32_t dgc_biquad_mse_bwd(dgc_ctx *ctx, const dgc_biquad_params *p, 
                        loss_dev, "null pointer");
   int32_t rc = biquad_validate(ctx, p);
   if (rc != DGC_OK) return rc;
-  const int B = p->B, T = p->T, L = p->L, NC = dgc_div_up(T, BQ_CHUNK);
-  DGC_REQUIRE(ctx, NC <= 65535, "T too large");
+  DGC_REQUIRE(ctx, dgc_div_up(p->T, BQ_CHUNK) <= 65535, "T too large");
   float *scr = scratch_dev ? scratch_dev : dgc_ctx_scratch(ctx, dgc_biquad_scratch_floats(p, 1));
   if (!scr) return DGC_ERR_OOM;
   DGC_REQUIRE(ctx, (((uintptr_t)scr) & 15) == 0, "scratch must be 16-byte aligned");
-  float *coef = scr;
-  float *rec = scr + ((((size_t)L * 24) + 3) & ~(size_t)3);
-  size_t rec_n = ((size_t)B * NC * BW_REC * L + 3) & ~(size_t)3;
-  double *acc = reinterpret_cast<double *>(rec + rec_n);
-  double *lane_loss = acc + (size_t)B * L * 6;
-  biquad_coef_kernel<<<dgc_div_up(L, 128), 128, 0, ctx->stream>>>(cutoff_dev, q_dev, L, p->gain, p->mode, coef);
-  DGC_LAUNCHED(ctx, "biquad_coef");
-  dim3 grid(dgc_div_up(L, BQ_THREADS), NC, B);
-  biquad_bwd_kernel<false><<<grid, BQ_THREADS, 0, ctx->stream>>>(x_dev, coef, y_dev, target_dev, B, T, L, NC,
-                                                                 2.0f * loss_scale, rec);
-  DGC_LAUNCHED(ctx, "biquad_bwd");
-  biquad_bwd_carry_kernel<<<dgc_div_up(B * L, 128), 128, 0, ctx->stream>>>(rec, coef, B, L, NC, T, acc, nullptr);
-  DGC_LAUNCHED(ctx, "biquad_bwd_carry");
-  biquad_bwd_final_kernel<<<dgc_div_up(L, 128), 128, 0, ctx->stream>>>(acc, coef, B, L, loss_scale, grad_cutoff_dev,
-                                                                        grad_q_dev, lane_loss);
-  DGC_LAUNCHED(ctx, "biquad_bwd_final");
-  sum_doubles_kernel<<<1, 32, 0, ctx->stream>>>(lane_loss, L, loss_dev);
-  DGC_LAUNCHED(ctx, "biquad_loss_sum");
-  return DGC_OK;
+  return biquad_backward<false>(ctx, p, x_dev, cutoff_dev, q_dev, y_dev, target_dev, 2.0f * loss_scale, loss_scale, scr, nullptr,
+                                grad_cutoff_dev, grad_q_dev, loss_dev);
 }
 
 namespace {
@@ -1050,26 +1178,15 @@ DGC_EXPORT int32_t dgc_biquad_bwd(dgc_ctx *ctx, const dgc_biquad_params *p, cons
   float *scr = scratch_dev ? scratch_dev : dgc_ctx_scratch(ctx, dgc_biquad_scratch_floats(p, grad_x_dev ? 2 : 1));
   if (!scr) return DGC_ERR_OOM;
   DGC_REQUIRE(ctx, (((uintptr_t)scr) & 15) == 0, "scratch must be 16-byte aligned");
-  float *coef = scr;
-  float *rec = scr + ((((size_t)L * 24) + 3) & ~(size_t)3);
-  size_t rec_n = ((size_t)B * NC * BW_REC * L + 3) & ~(size_t)3;
-  double *acc = reinterpret_cast<double *>(rec + rec_n);
-  double *lane_loss = acc + (size_t)B * L * 6;
   float *after = scr + dgc_biquad_scratch_floats(p, 1);
   float2 *term = grad_x_dev ? reinterpret_cast<float2 *>(after) : nullptr;
   float *part = after + (size_t)2 * B * NC * L;
-  biquad_coef_kernel<<<dgc_div_up(L, 128), 128, 0, ctx->stream>>>(cutoff_dev, q_dev, L, p->gain, p->mode, coef);
-  DGC_LAUNCHED(ctx, "biquad_coef");
-  dim3 grid(dgc_div_up(L, BQ_THREADS), NC, B);
-  biquad_bwd_kernel<true><<<grid, BQ_THREADS, 0, ctx->stream>>>(x_dev, coef, y_dev, gy_dev, B, T, L, NC, 1.0f, rec);
-  DGC_LAUNCHED(ctx, "biquad_bwd");
-  biquad_bwd_carry_kernel<<<dgc_div_up(B * L, 128), 128, 0, ctx->stream>>>(rec, coef, B, L, NC, T, acc, term);
-  DGC_LAUNCHED(ctx, "biquad_bwd_carry");
-  biquad_bwd_final_kernel<<<dgc_div_up(L, 128), 128, 0, ctx->stream>>>(acc, coef, B, L, 0.0f, grad_cutoff_dev, grad_q_dev,
-                                                                        lane_loss);
-  DGC_LAUNCHED(ctx, "biquad_bwd_final");
+  rc = biquad_backward<true>(ctx, p, x_dev, cutoff_dev, q_dev, y_dev, gy_dev, 1.0f, 0.0f, scr, term, grad_cutoff_dev, grad_q_dev,
+                             nullptr);
+  if (rc != DGC_OK) return rc;
   if (grad_x_dev) {
-    biquad_gx_kernel<true><<<grid, BQ_THREADS, 0, ctx->stream>>>(coef, y_dev, gy_dev, term, B, T, L, NC, 1.0f, part);
+    const dim3 grid(dgc_div_up(L, BQ_THREADS), NC, B);
+    biquad_gx_kernel<true><<<grid, BQ_THREADS, 0, ctx->stream>>>(scr, y_dev, gy_dev, term, B, T, L, NC, 1.0f, part);
     DGC_LAUNCHED(ctx, "biquad_grad_x");
     const size_t n = (size_t)B * T;
     sum_partial_rows_kernel<<<dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream>>>(part, (int)grid.x, n, grad_x_dev);
