@@ -562,25 +562,27 @@ __device__ __forceinline__ void grad_self(float2 z, float c_lin, float c_log2, i
   if (lane == 0) Y.x += gre; else Y.y += gre;
 }
 
-// MINB: resident blocks per SM the registers are capped for (3: 168 registers, nothing spilled; 4: 128 registers,
-// a few spilled words in the middle sizes; 5: 102 registers).  4 is the default: measured 0.315 / 0.498 / 3.53 ms
-// at 16 / 32 / 256 voices against 0.336 / 0.550 / 3.91 ms for 3.
-template <int N, int MINB>
-__global__ void __launch_bounds__(LOSS16_THREADS, MINB)
-mss_bwd16_kernel(const float *__restrict__ pred, const float *__restrict__ target, int B, int T, int hop, int H,
-                 int S /* windows whose first-covered frames this block owns */, const float *__restrict__ window,
-                 const float2 *__restrict__ tw, float c_lin, float c_log, int accumulate, float *__restrict__ grad) {
+inline int hop_of(const dgc_mss_params *p, int s) {
+  int hop = p->sizes[s] / p->hop_div;
+  return hop < 1 ? 1 : hop;
+}
+
+// One block's windows of one scale: block bx of voice b.
+template <int N>
+__device__ __forceinline__ void mss_bwd16_body(float2 *sm2, int bx, int b, const float *__restrict__ pred,
+                                               const float *__restrict__ target, int T, int hop, int H,
+                                               int S /* windows whose first-covered frames this block owns */,
+                                               const float *__restrict__ window, const float2 *__restrict__ tw, float c_lin,
+                                               float c_log, int accumulate, float *__restrict__ grad) {
   using Gm = Bwd16Geom<N>;
   using Ge = dgfft16::Geo<N>;
   constexpr int TT = Gm::TT, NF = Gm::NF, WR = Gm::WR, RL = Ge::RL;
-  extern __shared__ float2 sm2[];
   using Lay = dgfft16::LayoutFree;   // conflict-free exchange layouts (the windowed results below keep pad())
   constexpr int PN = Lay::template size<N>();
   float2 *bufa_all = sm2, *bufb_all = sm2 + NF * PN;
   float *tile = reinterpret_cast<float *>(sm2 + 2 * NF * PN);
   const int tid = threadIdx.x, f = tid / TT, lt = tid % TT;
-  const int b = blockIdx.y;
-  const int hA = blockIdx.x * S;
+  const int hA = bx * S;
   const int p0 = (hA - 1) * hop + 1;          // first owned frame (may be negative for the first block)
   const int owned = S * hop;
   const float *x1 = pred + (size_t)b * T, *x2 = target + (size_t)b * T;
@@ -686,28 +688,92 @@ mss_bwd16_kernel(const float *__restrict__ pred, const float *__restrict__ targe
   }
 }
 
-template <int N, int MINB>
-int32_t launch_bwd16(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred, const float *target, int hop, int H,
+// Scales of one launch, scale-major in the grid (the blocks resident together run the same instructions)
+struct Bwd16Desc {
+  int nscales;
+  int N[DGC_MSS_MAX_SCALES], hop[DGC_MSS_MAX_SCALES], H[DGC_MSS_MAX_SCALES], S[DGC_MSS_MAX_SCALES];
+  int first_block[DGC_MSS_MAX_SCALES + 1];
+  const float *window[DGC_MSS_MAX_SCALES];
+  const float2 *tw[DGC_MSS_MAX_SCALES];
+  float *out[DGC_MSS_MAX_SCALES];
+};
+
+// 4 resident blocks per SM: 128 registers, a few spilled words in the middle sizes; measured 0.315 / 0.498 / 3.53 ms at 16 /
+// 32 / 256 voices against 0.336 / 0.550 / 3.91 ms for 3 (168 registers, nothing spilled).
+__global__ void __launch_bounds__(LOSS16_THREADS, 4)
+mss_bwd16_kernel(const float *__restrict__ pred, const float *__restrict__ target, int B, int T, const Bwd16Desc d, float c_lin,
+                 float c_log, int accumulate) {
+  extern __shared__ float2 bwd_sm[];
+  int s = 0;
+  while (s + 1 < d.nscales && (int)blockIdx.x >= d.first_block[s + 1]) ++s;
+  const int r = blockIdx.x - d.first_block[s], per_voice = (d.first_block[s + 1] - d.first_block[s]) / B;
+  const int b = r / per_voice, bx = r - b * per_voice;
+  switch (d.N[s]) {
+#define CASE(NN) \
+  case NN: mss_bwd16_body<NN>(bwd_sm, bx, b, pred, target, T, d.hop[s], d.H[s], d.S[s], d.window[s], d.tw[s], c_lin, c_log, accumulate, d.out[s]); break;
+    CASE(64) CASE(128) CASE(256) CASE(512) CASE(1024) CASE(2048)
+#undef CASE
+    default: break;
+  }
+}
+
+// grad = ((part 0 + part 1) + part 2) + ..: the order in which launches of one scale each add up
+__global__ void __launch_bounds__(256)
+mss_bwd_sum_kernel(float *__restrict__ grad, const float *__restrict__ parts, int n_parts, size_t n) {
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  float g = grad[i];
+  for (int k = 0; k < n_parts; ++k) g = __fadd_rn(g, parts[(size_t)k * n + i]);
+  grad[i] = g;
+}
+
+// Geometry of the kernel per window size: windows per round, windows per block at full rounds, shared memory without the tile
+struct Bwd16Size {
+  int WR, WB;
+  size_t base;
+};
+template <int N> constexpr Bwd16Size bwd16_size_of() {
+  return {Bwd16Geom<N>::WR, Bwd16Geom<N>::WB, (size_t)2 * Bwd16Geom<N>::NF * dgfft16::LayoutFree::size<N>() * sizeof(float2)};
+}
+Bwd16Size bwd16_size(int N) {
+  switch (N) {
+    case 64: return bwd16_size_of<64>();
+    case 128: return bwd16_size_of<128>();
+    case 256: return bwd16_size_of<256>();
+    case 512: return bwd16_size_of<512>();
+    case 1024: return bwd16_size_of<1024>();
+    default: return bwd16_size_of<2048>();
+  }
+}
+
+// Below 4 M samples all scales run in ONE launch into buffers of their own, which a last pass adds to the gradient in the
+// scales' order: a launch per scale mostly waits for its last blocks there.  Six scales, 3 x 16001: 107 us in six launches, 51 in one and
+// the pass; 32 x 64000: 468 and 409.  Above, the buffers' traffic is
+// the larger cost and every launch fills the chip by itself.
+constexpr size_t BWD16_TOGETHER = (size_t)4 << 20, BWD16_SMEM_4 = 56 * 1024;   // shared memory of 4 resident blocks
+
+int32_t launch_bwd16(dgc_ctx *ctx, const dgc_mss_params *p, const int *scales, int n, const float *pred, const float *target,
                      float c_lin, float c_log, int accumulate, float *grad) {
-  using Gm = Bwd16Geom<N>;
-  const float *win = dgc_ctx_hann_sym(ctx, N);
-  const float2 *tw = dgc_ctx_twiddles(ctx, N);
-  if (!win || !tw) return DGC_ERR_OOM;
-  const int E = (N - 1) / hop;
-  const int S0 = Gm::WB - E;
-  if (S0 < 1) return dgc_fail(ctx, DGC_ERR_UNSUPPORTED, "hop %d too small for window %d", hop, N);
-  auto smem_of = [&](int S_) {
-    return (size_t)2 * Gm::NF * dgfft16::LayoutFree::size<N>() * sizeof(float2) + (size_t)S_ * hop * sizeof(float);
-  };
-  if (smem_of(S0) > 200 * 1024) return dgc_fail(ctx, DGC_ERR_UNSUPPORTED, "backward tile does not fit shared memory");
-  cudaError_t e = cudaFuncSetAttribute(mss_bwd16_kernel<N, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "mss_bwd smem opt-in: %s", cudaGetErrorString(e));
-  cudaFuncSetAttribute(mss_bwd16_kernel<N, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  // windows owned per block: the choice that minimises (waves of resident blocks x rounds per block), see launch_bwd;
-  // the summation order per output frame does not depend on it
-  int S = S0;
-  {
-    const auto key = std::make_pair(std::make_pair(N, -hop * 8 - MINB), std::make_pair(H, p->B));   // (-hop: this kernel's own entries)
+  const size_t nBT = (size_t)p->B * p->T;
+  static const bool opted = [] {
+    cudaFuncSetAttribute(mss_bwd16_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return cudaFuncSetAttribute(mss_bwd16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess;
+  }();
+  if (!opted) return dgc_fail(ctx, DGC_ERR_CUDA, "mss_bwd smem opt-in");
+  Bwd16Desc all;
+  all.nscales = n;
+  size_t smem[DGC_MSS_MAX_SCALES], most = 0;
+  for (int k = 0; k < n; ++k) {
+    const int N = p->sizes[scales[k]], hop = hop_of(p, scales[k]), H = dgc_div_up(p->T, hop), E = (N - 1) / hop;
+    const Bwd16Size g = bwd16_size(N);
+    const int S0 = g.WB - E;
+    auto smem_of = [&](int S) { return g.base + (size_t)S * hop * sizeof(float); };
+    if (S0 < 1) return dgc_fail(ctx, DGC_ERR_UNSUPPORTED, "hop %d too small for window %d", hop, N);
+    if (smem_of(S0) > 200 * 1024) return dgc_fail(ctx, DGC_ERR_UNSUPPORTED, "backward tile does not fit shared memory");
+    // Windows owned per block: the choice that minimises (waves of resident blocks x rounds per block) of a launch of this
+    // scale, see launch_bwd.  (It decides which windows share a transform, so the last bits depend on it.)
+    int S = S0;
+    const auto key = std::make_pair(std::make_pair(N, -hop), std::make_pair(H, p->B));   // (-hop: this kernel's own entries)
     auto it = ctx->mss_bwd_owned.find(key);
     if (it != ctx->mss_bwd_owned.end()) {
       S = it->second;
@@ -718,15 +784,13 @@ int32_t launch_bwd16(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred, c
       // candidates too; ties go to the larger S (less revisiting).
       long long best = -1;
       for (int cand = 1; cand <= S0 + 24 && cand <= H + E; ++cand) {
-        const size_t sm = smem_of(cand);
-        if (sm > 200 * 1024) break;
+        if (smem_of(cand) > 200 * 1024) break;
         int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mss_bwd16_kernel<N, MINB>, LOSS16_THREADS, sm) != cudaSuccess ||
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mss_bwd16_kernel, LOSS16_THREADS, smem_of(cand)) != cudaSuccess ||
             per_sm < 1)
           break;
         const long long blocks = (long long)dgc_div_up(H + 1, cand) * p->B, slots = (long long)per_sm * ctx->sm_count;
-        const long long waves = (blocks + slots - 1) / slots;
-        const long long cost = waves * dgc_div_up(cand + E, Gm::WR);
+        const long long cost = ((blocks + slots - 1) / slots) * dgc_div_up(cand + E, g.WR);
         if (best < 0 || cost <= best) {
           best = cost;
           S = cand;
@@ -734,15 +798,50 @@ int32_t launch_bwd16(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred, c
       }
       ctx->mss_bwd_owned[key] = S;
     }
+    all.N[k] = N;
+    all.hop[k] = hop;
+    all.H[k] = H;
+    all.S[k] = S;
+    all.window[k] = dgc_ctx_hann_sym(ctx, N);
+    all.tw[k] = dgc_ctx_twiddles(ctx, N);
+    if (!all.window[k] || !all.tw[k]) return DGC_ERR_OOM;
+    smem[k] = smem_of(S);
+    most = std::max(most, smem[k]);
   }
-  const size_t smem = smem_of(S);
+  const bool together = n > 1 && !accumulate && nBT < BWD16_TOGETHER && most <= BWD16_SMEM_4;
+  float *parts = nullptr;
+  if (together && !(parts = dgc_ctx_scratch(ctx, (uint64_t)(n - 1) * nBT))) return DGC_ERR_OOM;
   // block j owns the frames whose first covering window is in [j S, (j+1) S).  The frames behind the last window
   // ((H-1) hop, T-1] are covered by no window at all -- their "first covering window" would be number H -- and must
   // still be written (zero, or left as accumulated): the grid spans window indices 0 .. H.
-  mss_bwd16_kernel<N, MINB><<<dim3(dgc_div_up(H + 1, S), p->B), LOSS16_THREADS, smem, ctx->stream>>>(
-      pred, target, p->B, p->T, hop, H, S, win, tw, c_lin, c_log, accumulate, grad);
-  ctx->launches++;
-  return dgc_check_launch(ctx, "mss_bwd16");
+  auto launch = [&](const Bwd16Desc &d, size_t bytes, int add) -> int32_t {
+    mss_bwd16_kernel<<<d.first_block[d.nscales], LOSS16_THREADS, bytes, ctx->stream>>>(pred, target, p->B, p->T, d, c_lin, c_log, add);
+    ctx->launches++;
+    return dgc_check_launch(ctx, "mss_bwd16");
+  };
+  if (together) {
+    all.first_block[0] = 0;
+    for (int k = 0; k < n; ++k) {
+      all.out[k] = k ? parts + (size_t)(k - 1) * nBT : grad;
+      all.first_block[k + 1] = all.first_block[k] + dgc_div_up(all.H[k] + 1, all.S[k]) * p->B;
+    }
+    int32_t rc = launch(all, most, 0);
+    if (rc != DGC_OK) return rc;
+    mss_bwd_sum_kernel<<<dgc_div_up((int64_t)nBT, 256), 256, 0, ctx->stream>>>(grad, parts, n - 1, nBT);
+    DGC_LAUNCHED(ctx, "mss_bwd_sum");
+    return DGC_OK;
+  }
+  for (int k = 0; k < n; ++k) {
+    Bwd16Desc d;
+    d.nscales = 1;
+    d.N[0] = all.N[k]; d.hop[0] = all.hop[k]; d.H[0] = all.H[k]; d.S[0] = all.S[k];
+    d.window[0] = all.window[k]; d.tw[0] = all.tw[k]; d.out[0] = grad;
+    d.first_block[0] = 0;
+    d.first_block[1] = dgc_div_up(all.H[k] + 1, all.S[k]) * p->B;
+    int32_t rc = launch(d, smem[k], accumulate || k > 0);
+    if (rc != DGC_OK) return rc;
+  }
+  return DGC_OK;
 }
 
 template <int N>
@@ -816,11 +915,6 @@ int32_t validate(dgc_ctx *ctx, const dgc_mss_params *p) {
     DGC_REQUIRE(ctx, dgc_is_pow2(p->sizes[s]) && p->sizes[s] >= 16 && p->sizes[s] <= 2048,
                 "window sizes must be powers of two in 16..2048");
   return DGC_OK;
-}
-
-inline int hop_of(const dgc_mss_params *p, int s) {
-  int hop = p->sizes[s] / p->hop_div;
-  return hop < 1 ? 1 : hop;
 }
 
 }  // namespace
@@ -1002,34 +1096,29 @@ DGC_EXPORT int32_t dgc_mss_loss_bwd(dgc_ctx *ctx, const dgc_mss_params *p, const
   const double den = (double)p->B * (double)used * (double)p->T;
   const float c_lin = (float)((double)upstream * (double)p->w_lin / den);
   const float c_log = (float)((double)upstream * (double)p->w_log / den);
+  // windows of 64 points and more run on the sixteen-points-per-thread kernel
+  static const bool bwd_old = [] {
+    const char *e = getenv("DGC_MSS_BWD");
+    return e && strcmp(e, "r8") == 0;
+  }();
+  int scales[DGC_MSS_MAX_SCALES], n = 0;
+  bool wide = !bwd_old;
+  for (int s = 0; s < p->nscales; ++s)
+    if (p->sizes[s] <= p->T) {
+      const int N = p->sizes[s];
+      if (N < 16 || N > 2048 || (N & (N - 1))) return dgc_fail(ctx, DGC_ERR_UNSUPPORTED, "window size %d", N);
+      wide = wide && N >= 64;
+      scales[n++] = s;
+    }
+  if (wide) return launch_bwd16(ctx, p, scales, n, pred_dev, target_dev, c_lin, c_log, 0, grad_pred_dev);
   int accumulate = 0;
-  for (int s = 0; s < p->nscales; ++s) {
-    const int N = p->sizes[s];
-    if (N > p->T) continue;
-    const int hop = hop_of(p, s), H = dgc_div_up(p->T, hop);
-    static const bool bwd_old = [] {
-      const char *e = getenv("DGC_MSS_BWD");
-      return e && strcmp(e, "r8") == 0;
-    }();
-    // windows of 64 points and more run on the sixteen-points-per-thread kernel
-    const bool wide = N >= 64 && !bwd_old;
-    static const int bwd_minb = [] {
-      const char *e = getenv("DGC_MSS_BWD_BLOCKS");
-      return e ? atoi(e) : 4;
-    }();
-    switch (wide ? N : -N) {
-#define CASE(NN) case -NN: rc = launch_bwd<NN>(ctx, p, pred_dev, target_dev, hop, H, c_lin, c_log, accumulate, grad_pred_dev); break;
+  for (int k = 0; k < n; ++k) {
+    const int N = p->sizes[scales[k]], hop = hop_of(p, scales[k]), H = dgc_div_up(p->T, hop);
+    if (N >= 64 && !bwd_old) rc = launch_bwd16(ctx, p, scales + k, 1, pred_dev, target_dev, c_lin, c_log, accumulate, grad_pred_dev);
+    else switch (N) {
+#define CASE(NN) case NN: rc = launch_bwd<NN>(ctx, p, pred_dev, target_dev, hop, H, c_lin, c_log, accumulate, grad_pred_dev); break;
       CASE(16) CASE(32) CASE(64) CASE(128) CASE(256) CASE(512) CASE(1024) CASE(2048)
 #undef CASE
-#define CASE(NN)                                                                                                          \
-  case NN:                                                                                                                \
-    rc = bwd_minb >= 5 ? launch_bwd16<NN, 5>(ctx, p, pred_dev, target_dev, hop, H, c_lin, c_log, accumulate, grad_pred_dev) \
-       : bwd_minb == 4 ? launch_bwd16<NN, 4>(ctx, p, pred_dev, target_dev, hop, H, c_lin, c_log, accumulate, grad_pred_dev) \
-                       : launch_bwd16<NN, 3>(ctx, p, pred_dev, target_dev, hop, H, c_lin, c_log, accumulate, grad_pred_dev); \
-    break;
-      CASE(64) CASE(128) CASE(256) CASE(512) CASE(1024) CASE(2048)
-#undef CASE
-      default: return dgc_fail(ctx, DGC_ERR_UNSUPPORTED, "window size %d", N);
     }
     if (rc != DGC_OK) return rc;
     accumulate = 1;
