@@ -253,30 +253,74 @@ __global__ void transpose_kernel(const float *__restrict__ in, int R, int Cc, fl
     if (c0 + i < Cc && r < R) out[(size_t)(c0 + i) * R + r] = t[threadIdx.x][i];
 }
 
-// dZ = dC * act'(C) written twice: dZ[m][n] and the transposed copy dZt[n][m] (32 x 32 tiles through shared
-// memory), so that the weight-gradient product can read both of its operands along the reduction index
-__global__ void act_bwd_t_kernel(const float *__restrict__ dC, const float *__restrict__ Cv, int M, int N, int act,
-                                 float *__restrict__ dZ, float *__restrict__ dZt) {
-  __shared__ float t[32][33];
-  const int n = blockIdx.x * 32 + threadIdx.x, m0 = blockIdx.y * 32;
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int m = m0 + i;
-    float g = 0.0f;
-    if (m < M && n < N) {
-      const size_t idx = (size_t)m * N + n;
-      g = dC[idx];
-      if (act == 1) {
-        const float c = Cv[idx];
-        g *= (1.0f - c * c);
+// The transposed copy of a tile t[m][n] of 64 x 64 values, out[n][m] (M a multiple of 4, out 16-byte aligned)
+constexpr int TT = 64;
+__device__ __forceinline__ void store_tile_t(const float (*t)[TT + 1], int m0, int n0, int M, int N, float *__restrict__ out) {
+  const int m = (threadIdx.x & 15) * 4;
+  if (m0 + m >= M) return;
+#pragma unroll
+  for (int i = 0; i < TT; i += 16) {
+    const int n = i + (threadIdx.x >> 4);
+    if (n0 + n < N)
+      *reinterpret_cast<float4 *>(out + (size_t)(n0 + n) * M + m0 + m) = make_float4(t[m][n], t[m + 1][n], t[m + 2][n], t[m + 3][n]);
+  }
+}
+
+// dZ = dC * act'(C) written twice: dZ[m][n] and the transposed copy dZt[n][m] (64 x 64 tiles through shared
+// memory), so that the weight-gradient product can read both of its operands along the reduction index.  Four passes
+// over the layer and nothing else: 32000 x 512 in 39 us (6.6 TB/s; 61 us in 32 x 32 tiles of single loads).  M a
+// multiple of 4; VEC: N too, and every buffer on 16 bytes.
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+act_bwd_t_kernel(const float *__restrict__ dC, const float *__restrict__ Cv, int M, int N, int act,
+                 float *__restrict__ dZ, float *__restrict__ dZt) {
+  __shared__ float t[TT][TT + 1];
+  const int n0 = blockIdx.x * TT, m0 = blockIdx.y * TT;
+  if (VEC) {
+    const int n = (threadIdx.x & 15) * 4, mr = threadIdx.x >> 4;
+    float4 g[4], c[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + 16 * i + mr;
+      g[i] = c[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (m < M && n0 + n < N) {
+        g[i] = *reinterpret_cast<const float4 *>(dC + (size_t)m * N + n0 + n);
+        if (act == 1) c[i] = *reinterpret_cast<const float4 *>(Cv + (size_t)m * N + n0 + n);
       }
-      dZ[idx] = g;
     }
-    t[i][threadIdx.x] = g;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = 16 * i + mr;
+      if (act == 1) {
+        g[i].x *= (1.0f - c[i].x * c[i].x);
+        g[i].y *= (1.0f - c[i].y * c[i].y);
+        g[i].z *= (1.0f - c[i].z * c[i].z);
+        g[i].w *= (1.0f - c[i].w * c[i].w);
+      }
+      if (m0 + m < M && n0 + n < N) *reinterpret_cast<float4 *>(dZ + (size_t)(m0 + m) * N + n0 + n) = g[i];
+      t[m][n] = g[i].x;
+      t[m][n + 1] = g[i].y;
+      t[m][n + 2] = g[i].z;
+      t[m][n + 3] = g[i].w;
+    }
+  } else {
+    const int n = threadIdx.x & 63;
+    for (int m = threadIdx.x >> 6; m < TT; m += 4) {
+      float g = 0.0f;
+      if (m0 + m < M && n0 + n < N) {
+        const size_t idx = (size_t)(m0 + m) * N + n0 + n;
+        g = dC[idx];
+        if (act == 1) {
+          const float c = Cv[idx];
+          g *= (1.0f - c * c);
+        }
+        dZ[idx] = g;
+      }
+      t[m][n] = g;
+    }
   }
   __syncthreads();
-  const int m = m0 + threadIdx.x, nb = blockIdx.x * 32;
-  for (int i = threadIdx.y; i < 32; i += 8)
-    if (nb + i < N && m < M) dZt[(size_t)(nb + i) * M + m] = t[threadIdx.x][i];
+  store_tile_t(t, m0, n0, M, N, dZt);
 }
 
 // dZ = dC * (1 - C^2) in place-compatible form (tanh'), or copy when act == 0
@@ -313,13 +357,8 @@ __global__ void act_bwd4_kernel(const float4 *__restrict__ dC, const float4 *__r
 // inputs of the row are broadcast loads, W and the bias stay in L1, the store is 16 bytes.  Same operation order as
 // the tile kernel (k ascending from zero, then the bias, then the library tanh).
 template <int KK, int EPI>
-__global__ void __launch_bounds__(256)
-smallk_fwd_kernel(const float *__restrict__ A, const float *__restrict__ W, const float *__restrict__ bias, int M, int N,
-                  float *__restrict__ C) {
-  const int nq = N >> 2;
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)M * nq) return;
-  const int m = (int)(idx / nq), n = (int)(idx - (size_t)m * nq) * 4;
+__device__ __forceinline__ float4 smallk_quad(const float *__restrict__ A, const float *__restrict__ W,
+                                              const float *__restrict__ bias, int N, int m, int n) {
   float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
   for (int k = 0; k < KK; ++k) {
@@ -338,7 +377,43 @@ smallk_fwd_kernel(const float *__restrict__ A, const float *__restrict__ W, cons
 #pragma unroll
     for (int j = 0; j < 4; ++j) v[j] = tanhf(v[j]);
   }
-  *reinterpret_cast<float4 *>(C + (size_t)m * N + n) = make_float4(v[0], v[1], v[2], v[3]);
+  return make_float4(v[0], v[1], v[2], v[3]);
+}
+
+template <int KK, int EPI>
+__global__ void __launch_bounds__(256)
+smallk_fwd_kernel(const float *__restrict__ A, const float *__restrict__ W, const float *__restrict__ bias, int M, int N,
+                  float *__restrict__ C) {
+  const int nq = N >> 2;
+  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (size_t)M * nq) return;
+  const int m = (int)(idx / nq), n = (int)(idx - (size_t)m * nq) * 4;
+  *reinterpret_cast<float4 *>(C + (size_t)m * N + n) = smallk_quad<KK, EPI>(A, W, bias, N, m, n);
+}
+
+// With the transposed copy Ct[n][m] that the weight gradient of the next layer reads, in tiles of 64 x 64: 25 us for
+// 32000 x 512, 58 us with a transposing pass over C behind it
+template <int KK, int EPI>
+__global__ void __launch_bounds__(256)
+smallk_fwd_t_kernel(const float *__restrict__ A, const float *__restrict__ W, const float *__restrict__ bias, int M, int N,
+                    float *__restrict__ C, float *__restrict__ Ct) {
+  __shared__ float t[TT][TT + 1];
+  const int n0 = blockIdx.x * TT, m0 = blockIdx.y * TT, n = (threadIdx.x & 15) * 4;
+  if (n0 + n < N) {
+#pragma unroll
+    for (int i = 0; i < TT; i += 16) {
+      const int m = i + (threadIdx.x >> 4);
+      if (m0 + m >= M) break;
+      const float4 v = smallk_quad<KK, EPI>(A, W, bias, N, m0 + m, n0 + n);
+      *reinterpret_cast<float4 *>(C + (size_t)(m0 + m) * N + n0 + n) = v;
+      t[m][n] = v.x;
+      t[m][n + 1] = v.y;
+      t[m][n + 2] = v.z;
+      t[m][n + 3] = v.w;
+    }
+  }
+  __syncthreads();
+  store_tile_t(t, m0, n0, M, N, Ct);
 }
 
 // Its backward: db[n] = sum_m dZ[m][n] and dW[k][n] = sum_m A[m][k] dZ[m][n] from ONE pass over dZ (a matmul
@@ -357,7 +432,7 @@ smallk_grad_kernel(const float *__restrict__ A, const float *__restrict__ dZ, in
 #pragma unroll
   for (int q = 0; q <= KK; ++q) acc[q] = 0.0f;
   if (col < N) {
-#pragma unroll 4
+#pragma unroll 16
     for (int m = m_begin + rg; m < m_end; m += 8) {
       const float d = dZ[(size_t)m * N + col];
       acc[0] += d;
@@ -402,6 +477,7 @@ bias_grad_kernel(const float *__restrict__ dZ, int M, int N, float *__restrict__
   const int m_begin = blockIdx.y * 1024, m_end = min(M, m_begin + 1024);
   float acc = 0.0f;
   if (col < N)
+#pragma unroll 16
     for (int m = m_begin + rg; m < m_end; m += 8) acc += dZ[(size_t)m * N + col];
   sh[rg][threadIdx.x & 31] = acc;
   __syncthreads();
@@ -478,18 +554,27 @@ DGC_EXPORT int32_t dgc_linear_fwd(dgc_ctx *ctx, const float *a_dev, const float 
   } else if (K <= 4 && (N & 3) == 0 && ((((uintptr_t)w_dev) | ((uintptr_t)c_dev) | ((uintptr_t)bias_dev)) & 15) == 0) {
     // a handful of inputs: the streaming map
     const int64_t work = (int64_t)M * (N >> 2);
-    const dim3 grid((unsigned)dgc_div_up(work, 256));
+    ct_done = ct_dev && (M & 3) == 0 && (((uintptr_t)ct_dev) & 15) == 0 && dgc_div_up(M, TT) <= 65535;
+#define DGC_SMALLK_EPI(KKV, EPI, BIAS)                                                                                \
+  do {                                                                                                               \
+    if (ct_done)                                                                                                     \
+      smallk_fwd_t_kernel<KKV, EPI><<<dim3(dgc_div_up(N, TT), dgc_div_up(M, TT)), 256, 0, ctx->stream>>>(            \
+          a_dev, w_dev, BIAS, M, N, c_dev, ct_dev);                                                                  \
+    else                                                                                                             \
+      smallk_fwd_kernel<KKV, EPI><<<(unsigned)dgc_div_up(work, 256), 256, 0, ctx->stream>>>(a_dev, w_dev, BIAS, M, N, c_dev); \
+  } while (0)
 #define DGC_SMALLK_FWD(KKV)                                                                                           \
   do {                                                                                                               \
-    if (act == 1) smallk_fwd_kernel<KKV, 2><<<grid, 256, 0, ctx->stream>>>(a_dev, w_dev, bias_dev, M, N, c_dev);      \
-    else if (bias_dev) smallk_fwd_kernel<KKV, 1><<<grid, 256, 0, ctx->stream>>>(a_dev, w_dev, bias_dev, M, N, c_dev); \
-    else smallk_fwd_kernel<KKV, 0><<<grid, 256, 0, ctx->stream>>>(a_dev, w_dev, nullptr, M, N, c_dev);                \
+    if (act == 1) DGC_SMALLK_EPI(KKV, 2, bias_dev);                                                                  \
+    else if (bias_dev) DGC_SMALLK_EPI(KKV, 1, bias_dev);                                                             \
+    else DGC_SMALLK_EPI(KKV, 0, nullptr);                                                                            \
   } while (0)
     if (K == 1) DGC_SMALLK_FWD(1);
     else if (K == 2) DGC_SMALLK_FWD(2);
     else if (K == 3) DGC_SMALLK_FWD(3);
     else DGC_SMALLK_FWD(4);
 #undef DGC_SMALLK_FWD
+#undef DGC_SMALLK_EPI
     rc = DGC_OK;
   } else
   if (act == 1) rc = launch_sgemm<false, false, 2>(ctx, a_dev, w_dev, bias_dev, M, N, K, c_dev);
@@ -527,8 +612,9 @@ DGC_EXPORT int32_t dgc_linear_bwd(dgc_ctx *ctx, const float *a_dev, const float 
       DGC_CUDA(ctx, cudaMalloc(&ctx->dzt_buf, n * sizeof(float)));
       ctx->dzt_floats = n;
     }
-    act_bwd_t_kernel<<<dim3(dgc_div_up(N, 32), dgc_div_up(M, 32)), dim3(32, 8), 0, ctx->stream>>>(dc_dev, c_dev, M, N, act,
-                                                                                                dz_dev, ctx->dzt_buf);
+    const bool vec = (N & 3) == 0 && ((((uintptr_t)dc_dev) | ((uintptr_t)dz_dev) | (act == 1 ? (uintptr_t)c_dev : 0)) & 15) == 0;
+    auto kern = vec ? act_bwd_t_kernel<true> : act_bwd_t_kernel<false>;
+    kern<<<dim3(dgc_div_up(N, TT), dgc_div_up(M, TT)), 256, 0, ctx->stream>>>(dc_dev, c_dev, M, N, act, dz_dev, ctx->dzt_buf);
   } else {
     const bool vec = (n & 3) == 0 && ((((uintptr_t)dc_dev) | ((uintptr_t)dz_dev) | (act == 1 ? (uintptr_t)c_dev : 0)) & 15) == 0;
     if (vec)
