@@ -111,10 +111,7 @@ bool dgc_gemm_nt_persistent(const dgc_ctx *ctx, const float *a, int M, int N, in
 const float2 *dgc_ctx_twiddles(dgc_ctx *ctx, int N);
 // dgc_onepole_fwd as three launches (linrec.cu)
 int32_t dgc_onepole_in_passes(dgc_ctx *ctx, const float *x_dev, int32_t B, int32_t T, float a, float *y_dev);
-// dgc_mss_loss_fwd with the prediction given as the sum of two signals (pred_b may be null)
-int32_t dgc_mss_loss_fwd_sum(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev, const float *pred_b_dev,
-                             const float *target_dev, float *partial_dev, double *loss_dev);
-// ... with the voices in groups, each after its own event (mss_loss.cu)
+// dgc_mss_loss_fwd with the voices in groups, each after its own event (mss_loss.cu)
 constexpr int DGC_MSS_MAX_GROUPS = 4;
 static inline int dgc_mss_group_start(int B, int q, int groups) { return (int)((int64_t)B * q / groups); }
 int32_t dgc_mss_loss_fwd_groups(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev, const float *target_dev, int groups,

@@ -53,9 +53,8 @@ __device__ __forceinline__ void unpack(float2 zk, float2 znk, float2 &x1, float2
 
 // One block of one scale: LOSS_THREADS / (N/8) windows of one voice, prediction and target in the real
 // and imaginary lane of one transform; sm holds 2 * NF * padded(N) float2 (the same 34.8 KB for every N).
-template <int N, bool SUM2>
+template <int N>
 __device__ __forceinline__ void mss_fwd_body(float2 *sm, float *red, int bx, int b, const float *__restrict__ pred,
-                                             const float *__restrict__ pred_b,
                                              const float *__restrict__ target, int B, int T, int hop, int H,
                                              const float *__restrict__ window, const float2 *__restrict__ tw,
                                              float *__restrict__ part_lin, float *__restrict__ part_log) {
@@ -68,7 +67,6 @@ __device__ __forceinline__ void mss_fwd_body(float2 *sm, float *red, int bx, int
   const bool valid = h < H;
   const int t_base = h * hop - (N - 1);
   const float *x1 = pred + (size_t)b * T, *x2 = target + (size_t)b * T;
-  const float *x1b = SUM2 ? pred_b + (size_t)b * T : nullptr;   // prediction given as a sum of two signals
   float2 *a = bufa + f * PN, *bb = bufb + f * PN;
   // the windowed samples a thread loads (stride G) are exactly its inputs of the first radix-8 stage: they stay
   // in registers
@@ -79,8 +77,7 @@ __device__ __forceinline__ void mss_fwd_body(float2 *sm, float *red, int bx, int
     float2 v = make_float2(0.0f, 0.0f);
     if (valid && t >= 0 && t < T) {
       float w = __ldg(&window[i]);
-      const float xp = SUM2 ? __fadd_rn(x1[t], x1b[t]) : x1[t];
-      v = make_float2(xp * w, x2[t] * w);
+      v = make_float2(x1[t] * w, x2[t] * w);
     }
     vin[q] = v;
   }
@@ -123,10 +120,8 @@ struct FwdDesc {
 
 constexpr int FWD_SMEM_BYTES = 2 * (LOSS_THREADS / (2048 / 8)) * padded(2048) * (int)sizeof(float2);
 
-template <bool SUM2>
 __global__ void __launch_bounds__(LOSS_THREADS, 6)
-mss_fwd_kernel(const float *__restrict__ pred, const float *__restrict__ pred_b, const float *__restrict__ target,
-               int B, int T, const FwdDesc d) {
+mss_fwd_kernel(const float *__restrict__ pred, const float *__restrict__ target, int B, int T, const FwdDesc d) {
   extern __shared__ float2 fwd_sm[];
   __shared__ float red[LOSS_THREADS / 32];
   int s = 0;
@@ -134,7 +129,7 @@ mss_fwd_kernel(const float *__restrict__ pred, const float *__restrict__ pred_b,
   const int bx = blockIdx.x - d.first_block[s], b = blockIdx.y;
   switch (d.N[s]) {
 #define CASE(NN) \
-  case NN: mss_fwd_body<NN, SUM2>(fwd_sm, red, bx, b, pred, pred_b, target, B, T, d.hop[s], d.H[s], d.window[s], d.tw[s], d.lin[s], d.lg[s]); break;
+  case NN: mss_fwd_body<NN>(fwd_sm, red, bx, b, pred, target, B, T, d.hop[s], d.H[s], d.window[s], d.tw[s], d.lin[s], d.lg[s]); break;
     CASE(16) CASE(32) CASE(64) CASE(128) CASE(256) CASE(512) CASE(1024) CASE(2048)
 #undef CASE
     default: break;
@@ -174,9 +169,8 @@ __device__ __forceinline__ void pair_terms(float2 zk, float2 zn, float &lin, flo
 constexpr int SPAN_BOX = 128, SPAN_BOXES = 17;
 static_assert(2 * SPAN_BOX * SPAN_BOXES * sizeof(float) <= padded(2048) * sizeof(float2), "the staged runs must fit the buffer");
 
-template <int N, bool SUM2, bool TMA>
+template <int N, bool TMA>
 __device__ __forceinline__ void mss_fwd16_body(float2 *sm, float *red, int bx, int b, const float *__restrict__ pred,
-                                               const float *__restrict__ pred_b,
                                                const float *__restrict__ target, int B, int T, int hop, int H,
                                                const float *__restrict__ window, const float2 *__restrict__ tw,
                                                float *__restrict__ part_lin, float *__restrict__ part_log,
@@ -193,7 +187,6 @@ __device__ __forceinline__ void mss_fwd16_body(float2 *sm, float *red, int bx, i
   const bool valid = h < H;
   const int t_base = h * hop - (N - 1);
   const float *x1 = pred + (size_t)b * T, *x2 = target + (size_t)b * T;
-  const float *x1b = SUM2 ? pred_b + (size_t)b * T : nullptr;   // prediction given as a sum of two signals
   // one buffer per transform (in-place middle stage): 17 KB per block instead of 33, room for 8 resident blocks;
   // the variant that stages the sample runs with the copy engine keeps the second buffer for them
   float2 *bufa = sm + f * PN, *bufb = TMA ? sm + (NF + f) * PN : bufa;
@@ -236,8 +229,7 @@ __device__ __forceinline__ void mss_fwd16_body(float2 *sm, float *red, int bx, i
 #pragma unroll
     for (int m = 0; m < 16; ++m) {
       const float w = __ldg(wp + m * TT);
-      const float xp = SUM2 ? __fadd_rn(p1[m * TT], x1b[t_base + lt + m * TT]) : p1[m * TT];
-      x[m] = make_float2(xp * w, p2[m * TT] * w);
+      x[m] = make_float2(p1[m * TT] * w, p2[m * TT] * w);
     }
   } else {
 #pragma unroll
@@ -246,8 +238,7 @@ __device__ __forceinline__ void mss_fwd16_body(float2 *sm, float *red, int bx, i
       float2 v = make_float2(0.0f, 0.0f);
       if (valid && t >= 0) {
         const float w = __ldg(&window[i]);
-        const float xp = SUM2 ? __fadd_rn(x1[t], x1b[t]) : x1[t];
-        v = make_float2(xp * w, x2[t] * w);
+        v = make_float2(x1[t] * w, x2[t] * w);
       }
       x[m] = v;
     }
@@ -293,9 +284,9 @@ constexpr int FWD16_SMEM_BYTES = 32 * 76 * (int)sizeof(float2);
 static_assert(FWD16_SMEM_BYTES >= padded(2048) * (int)sizeof(float2) && FWD16_SMEM_BYTES >= 4 * 568 * (int)sizeof(float2) &&
               FWD16_SMEM_BYTES >= 8 * 280 * (int)sizeof(float2), "one buffer per transform must fit");
 
-template <bool SUM2, bool TMA>
+template <bool TMA>
 __global__ void __launch_bounds__(LOSS16_THREADS, TMA ? 6 : 8)
-mss_fwd16_kernel(const float *__restrict__ pred, const float *__restrict__ pred_b, const float *__restrict__ target,
+mss_fwd16_kernel(const float *__restrict__ pred, const float *__restrict__ target,
                  int B, int T, const FwdDesc d, const __grid_constant__ CUtensorMap map_pred,
                  const __grid_constant__ CUtensorMap map_target, int32_t *status) {
   extern __shared__ __align__(128) float2 fwd_sm[];
@@ -315,7 +306,7 @@ mss_fwd16_kernel(const float *__restrict__ pred, const float *__restrict__ pred_
   const int b = r / per_voice, bx = r - b * per_voice;
   switch (d.N[s]) {
 #define CASE(NN) \
-  case NN: mss_fwd16_body<NN, SUM2, TMA>(fwd_sm, red, bx, b, pred, pred_b, target, B, T, d.hop[s], d.H[s], d.window[s], d.tw[s], d.lin[s], d.lg[s], &map_pred, &map_target, &span_bar, status); break;
+  case NN: mss_fwd16_body<NN, TMA>(fwd_sm, red, bx, b, pred, target, B, T, d.hop[s], d.H[s], d.window[s], d.tw[s], d.lin[s], d.lg[s], &map_pred, &map_target, &span_bar, status); break;
     CASE(64) CASE(128) CASE(256) CASE(512) CASE(1024) CASE(2048)
 #undef CASE
     default: break;
@@ -747,9 +738,9 @@ Bwd16Size bwd16_size(int N) {
 }
 
 // Below 4 M samples all scales run in ONE launch into buffers of their own, which a last pass adds to the gradient in the
-// scales' order: a launch per scale mostly waits for its last blocks there.  Six scales, 3 x 16001: 107 us in six launches, 51 in one and
-// the pass; 32 x 64000: 468 and 409.  Above, the buffers' traffic is
-// the larger cost and every launch fills the chip by itself.
+// scales' order: a launch per scale mostly waits for its last blocks there.  Six scales, 3 x 16001: 107 us in six
+// launches, 51 in one and the pass; 32 x 64000: 468 and 409.  Above, the buffers' traffic is the larger cost and every
+// launch fills the chip by itself.
 constexpr size_t BWD16_TOGETHER = (size_t)4 << 20, BWD16_SMEM_4 = 56 * 1024;   // shared memory of 4 resident blocks
 
 int32_t launch_bwd16(dgc_ctx *ctx, const dgc_mss_params *p, const int *scales, int n, const float *pred, const float *target,
@@ -930,13 +921,8 @@ DGC_EXPORT uint64_t dgc_mss_partial_floats(const dgc_mss_params *p) {
   return n;
 }
 
-DGC_EXPORT int32_t dgc_mss_loss_fwd(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev,
-                                    const float *target_dev, float *partial_dev, double *loss_dev) {
-  return dgc_mss_loss_fwd_sum(ctx, p, pred_dev, nullptr, target_dev, partial_dev, loss_dev);
-}
-
 // The windows of one group of voices (p->B of them, at pred_dev and target_dev): partial sums at part + off, added to d.
-static int32_t mss_fwd_windows(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev, const float *pred_b_dev,
+static int32_t mss_fwd_windows(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev,
                                const float *target_dev, float *part, long long &off, ReduceDesc &d) {
   // partial layout and summation order follow the caller's scale order; the launch runs the usable
   // scales largest window first
@@ -985,11 +971,9 @@ static int32_t mss_fwd_windows(dgc_ctx *ctx, const dgc_mss_params *p, const floa
   }
   // resident blocks per SM are limited by shared memory (6 x 34 KB): ask for the largest carve-out
   static const bool carved = [] {
-    cudaFuncSetAttribute(mss_fwd_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(mss_fwd_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(mss_fwd16_kernel<true, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(mss_fwd16_kernel<false, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(mss_fwd16_kernel<false, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(mss_fwd_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(mss_fwd16_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(mss_fwd16_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     return true;
   }();
   (void)carved;
@@ -1004,26 +988,18 @@ static int32_t mss_fwd_windows(dgc_ctx *ctx, const dgc_mss_params *p, const floa
     CUtensorMap mp, mt;
     memset(&mp, 0, sizeof(mp));
     memset(&mt, 0, sizeof(mt));
-    bool tma = tma_on && !pred_b_dev && p->hop_div >= 1;
+    bool tma = tma_on && p->hop_div >= 1;
     tma = tma && dgtma::make_map_2d(&mp, pred_dev, p->B, p->T, SPAN_BOX) && dgtma::make_map_2d(&mt, target_dev, p->B, p->T, SPAN_BOX);
-    if (pred_b_dev)
-      mss_fwd16_kernel<true, false><<<blocks16, LOSS16_THREADS, FWD16_SMEM_BYTES, ctx->stream>>>(
-          pred_dev, pred_b_dev, target_dev, p->B, p->T, fd16, mp, mt, ctx->status_dev);
-    else if (tma)
-      mss_fwd16_kernel<false, true><<<blocks16, LOSS16_THREADS, 2 * padded(2048) * (int)sizeof(float2), ctx->stream>>>(
-          pred_dev, nullptr, target_dev, p->B, p->T, fd16, mp, mt, ctx->status_dev);
+    if (tma)
+      mss_fwd16_kernel<true><<<blocks16, LOSS16_THREADS, 2 * padded(2048) * (int)sizeof(float2), ctx->stream>>>(
+          pred_dev, target_dev, p->B, p->T, fd16, mp, mt, ctx->status_dev);
     else
-      mss_fwd16_kernel<false, false><<<blocks16, LOSS16_THREADS, FWD16_SMEM_BYTES, ctx->stream>>>(
-          pred_dev, nullptr, target_dev, p->B, p->T, fd16, mp, mt, ctx->status_dev);
+      mss_fwd16_kernel<false><<<blocks16, LOSS16_THREADS, FWD16_SMEM_BYTES, ctx->stream>>>(pred_dev, target_dev, p->B, p->T, fd16,
+                                                                                           mp, mt, ctx->status_dev);
     DGC_LAUNCHED(ctx, tma ? "mss_fwd16_tma" : "mss_fwd16");
   }
   if (fd8.nscales > 0) {
-    if (pred_b_dev)
-      mss_fwd_kernel<true><<<dim3(blocks8, p->B), LOSS_THREADS, FWD_SMEM_BYTES, ctx->stream>>>(pred_dev, pred_b_dev,
-                                                                                               target_dev, p->B, p->T, fd8);
-    else
-      mss_fwd_kernel<false><<<dim3(blocks8, p->B), LOSS_THREADS, FWD_SMEM_BYTES, ctx->stream>>>(pred_dev, nullptr,
-                                                                                                target_dev, p->B, p->T, fd8);
+    mss_fwd_kernel<<<dim3(blocks8, p->B), LOSS_THREADS, FWD_SMEM_BYTES, ctx->stream>>>(pred_dev, target_dev, p->B, p->T, fd8);
     DGC_LAUNCHED(ctx, "mss_fwd");
   }
   return DGC_OK;
@@ -1042,10 +1018,8 @@ static int32_t mss_fwd_reduce(dgc_ctx *ctx, const dgc_mss_params *p, const float
   return DGC_OK;
 }
 
-// prediction = pred_dev + pred_b_dev (pred_b_dev may be null): lets two synthesis branches that ran
-// concurrently feed the loss without a pass that adds them
-int32_t dgc_mss_loss_fwd_sum(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev, const float *pred_b_dev,
-                             const float *target_dev, float *partial_dev, double *loss_dev) {
+DGC_EXPORT int32_t dgc_mss_loss_fwd(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred_dev,
+                                    const float *target_dev, float *partial_dev, double *loss_dev) {
   if (!ctx) return DGC_ERR_INVALID;
   DGC_REQUIRE(ctx, p && pred_dev && target_dev && loss_dev, "null pointer");
   int32_t rc = validate(ctx, p);
@@ -1055,7 +1029,7 @@ int32_t dgc_mss_loss_fwd_sum(dgc_ctx *ctx, const dgc_mss_params *p, const float 
   ReduceDesc d;
   d.nscales = 0;
   long long off = 0;
-  rc = mss_fwd_windows(ctx, p, pred_dev, pred_b_dev, target_dev, part, off, d);
+  rc = mss_fwd_windows(ctx, p, pred_dev, target_dev, part, off, d);
   return rc == DGC_OK ? mss_fwd_reduce(ctx, p, part, d, loss_dev) : rc;
 }
 
@@ -1074,7 +1048,7 @@ int32_t dgc_mss_loss_fwd_groups(dgc_ctx *ctx, const dgc_mss_params *p, const flo
     dgc_mss_params g = *p;
     g.B = b1 - b0;
     DGC_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ready[q], 0));
-    rc = mss_fwd_windows(ctx, &g, pred_dev + (size_t)b0 * p->T, nullptr, target_dev + (size_t)b0 * p->T, part, off, d);
+    rc = mss_fwd_windows(ctx, &g, pred_dev + (size_t)b0 * p->T, target_dev + (size_t)b0 * p->T, part, off, d);
     if (rc != DGC_OK) return rc;
   }
   return mss_fwd_reduce(ctx, p, part, d, loss_dev);

@@ -159,7 +159,7 @@ static int32_t hn_forward_loss_impl(dgc_ctx *ctx, const dgc_hn_step *s, const fl
     DGC_CUDA(ctx, cudaEventRecord(ev->audio, main_stream));
     return dgc_mss_loss_fwd_groups(ctx, &s->mss, mix, target_dev, ev->groups, ev->target, loss_dev);
   }
-  return dgc_mss_loss_fwd_sum(ctx, &s->mss, mix, nullptr, target_dev, nullptr, loss_dev);
+  return dgc_mss_loss_fwd(ctx, &s->mss, mix, target_dev, nullptr, loss_dev);
 }
 
 DGC_EXPORT int32_t dgc_hn_forward_loss(dgc_ctx *ctx, const dgc_hn_step *s, const float *f0_dev, const float *uv_dev,
