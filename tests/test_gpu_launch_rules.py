@@ -1,0 +1,101 @@
+"""Sizes on both sides of the launch rules: tap maps in small blocks, matmuls in half-width tiles, the spectral gradient in
+one launch, the host-buffer step in groups of voices, banks of odd lane counts."""
+import numpy as np
+import pytest
+import torch
+
+import dgen_b200
+from dgen_b200 import workloads as wl
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+f32 = np.float32
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = dgen_b200.Context(0)
+    yield c
+    c.close()
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+@pytest.mark.parametrize("F,B,NB,NT", [(1, 1, 1, 1), (63, 1, 65, 31), (64, 1, 64, 32), (13, 5, 33, 257), (125, 3, 65, 255),
+                                       (500, 2, 9, 33)])
+def test_small_tap_maps(ctx, F, B, NB, NT):
+    rng = np.random.default_rng(F + NT)
+    bands, w = rng.uniform(0, 1, (F, B, NB)).astype(f32), rng.standard_normal((NT, NB)).astype(f32)
+    want = bands.astype(np.float64) @ w.astype(np.float64).T
+    got = ctx.bands_to_taps(dev(bands), dev(w)).cpu().numpy()
+    assert np.abs(got - want).max() <= 2e-6 * max(1.0, np.abs(want).max())
+
+
+# the weight gradient reduces over M rows of either parity; outputs of one, of a few and of more tiles than half the chip
+@pytest.mark.parametrize("M,K,N", [(750, 128, 128), (997, 130, 65), (257, 96, 129), (33, 512, 512), (321, 1100, 1030)])
+def test_weight_gradient_tiles(ctx, M, K, N):
+    rng = np.random.default_rng(M)
+    a, w = rng.standard_normal((M, K)).astype(f32), (rng.standard_normal((K, N)) / np.sqrt(K)).astype(f32)
+    dc = rng.standard_normal((M, N)).astype(f32)
+    c = ctx.linear_fwd(dev(a), dev(w))
+    da, dw, db = ctx.linear_bwd(dev(a), dev(w), c, dev(dc))
+    a64, w64, dc64 = a.astype(np.float64), w.astype(np.float64), dc.astype(np.float64)
+    for got, want in ((c, a64 @ w64), (da, dc64 @ w64.T), (dw, a64.T @ dc64), (db, dc64.sum(0))):
+        assert np.abs(got.cpu().numpy() - want).max() <= 5e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("B,T,sizes", [(1, 2048, (2048, 64)), (3, 2047, (2048, 512, 64)), (2, 16001, (64, 2048, 256, 1024)),
+                                       (64, 65536, (1024, 128)), (64, 65535, (1024, 128)), (1, 64, (64, 128))])
+def test_spectral_gradient_of_several_scales_is_the_sum_of_each(ctx, B, T, sizes):
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x, y = (torch.randn(B, T, generator=g, device="cuda") for _ in range(2))
+    got = ctx.mss_loss_bwd(x, y, sizes=sizes)
+    used = [n for n in sizes if n <= T]
+    want = sum(ctx.mss_loss_bwd(x, y, sizes=(n,)).double() for n in used) / len(used)
+    assert float((got - want).abs().max()) <= 2e-6 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("B", [1, 3, 4, 9])
+def test_host_step_equals_the_device_step(ctx, B):
+    T, K, F, NB, NT = 4097, 20, 33, 9, 33
+    st = dgen_b200.HnStep()
+    st.harm = dgen_b200.HarmonicParams(B, T, K, F, 16000.0, 1.0, dgen_b200.PHASE_SCAN, 0)
+    st.fir = dgen_b200.FirParams(B, T, F, NT, 0.12, 1)
+    st.mss = dgen_b200.mss_params(B, T, (512, 128, 64))
+    st.nbands = NB
+    d = wl.harmonic_noise_inputs(B, B=B, T=T, K=K, F=F, nbands=NB, taps=NT)
+    P = [d[k] for k in ("f0", "uv", "amps", "gain", "noise_gain", "bands", "W", "noise")]
+    P.append(np.random.default_rng(B).standard_normal((B, T)).astype(f32) * f32(0.1))
+    audio = torch.empty(B, T, device="cuda")
+    loss, _ = ctx.hn_forward_loss(st, *[dev(p) for p in P], audio=audio)
+    pinned = [torch.from_numpy(np.ascontiguousarray(p)).pin_memory() for p in P]
+    out = torch.zeros(B, T).pin_memory()
+    got = ctx.hn_forward_loss_host(st, *pinned, audio_out=out)
+    assert torch.equal(out, audio.cpu())
+    assert abs(got - float(loss)) <= 1e-6 * float(loss)
+
+
+@pytest.mark.parametrize("B,L,T", [(1, 1, 1), (2, 1, 1537), (1, 37, 512), (1, 37, 8193), (1, 300, 1025)])
+def test_biquad_banks_of_odd_lanes(ctx, B, L, T):
+    d = wl.biquad_bank_inputs(L + T, B=B, L=L, T=T)
+    x, q = d["x"], d["q"]
+    cut = np.exp(np.random.default_rng(L).uniform(np.log(400.0), np.log(8000.0), L)).astype(f32)
+    want = orc.biquad_bank(x, cut, q)
+    X, C_, Q_ = dev(x), dev(cut), dev(q)
+    y = ctx.biquad_fwd(X, C_, Q_)
+    assert np.abs(y.cpu().numpy().transpose(0, 2, 1) - want).max() < 1e-4 * max(1.0, np.abs(want).max())
+    target = orc.biquad_bank(x, cut * f32(1.05), q)
+    scale = 1.0 / (B * T)
+    _, gc64, gq64 = orc.biquad_bank_mse_grad(x, cut, q, target, scale=scale)
+    t = dev(target.transpose(0, 2, 1))
+    gc, gq, _ = ctx.biquad_mse_bwd(X, C_, Q_, y, t, loss_scale=scale)
+    assert np.abs(gc.cpu().numpy() - gc64).max() <= 1e-3 * np.abs(gc64).max()
+    assert np.abs(gq.cpu().numpy() - gq64).max() <= 1e-3 * np.abs(gq64).max()
+    gy = (2.0 * scale) * (y - t)
+    _, _, gx = ctx.biquad_bwd(X, C_, Q_, y, gy)
+    g64 = gy.cpu().numpy().astype(np.float64)
+    ref = np.stack([sum(orc.biquad(g64[b, ::-1, l].copy(), float(cut[l]), float(q[l]), double=True)[::-1] for l in range(L))
+                    for b in range(B)])
+    assert np.abs(gx.cpu().numpy() - ref).max() <= 1e-3 * max(np.abs(ref).max(), 1e-30)
