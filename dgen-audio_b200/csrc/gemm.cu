@@ -223,13 +223,20 @@ int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *
   } else if (tc) {
     // tensor-core kernel: operand A is K-major in memory when it is NOT transposed ([M][K]);
     // operand B is K-major in memory when it IS given transposed ([N][K])
-    // a product of so few tiles that their halves fit the chip too takes 64-column ones
-    const bool halves = tiles * splits * 2 <= ctx->sm_count && N > 64;
-    auto kern = halves ? dgtc::tc_gemm_kernel<!TA, TB, EPI, 64> : dgtc::tc_gemm_kernel<!TA, TB, EPI>;
-    if (halves) grid.x = dgc_div_up(N, 64);
+    // the smallest tile whose grid the chip still takes at once
+    auto kern = dgtc::tc_gemm_kernel<!TA, TB, EPI, 128, 128>;
+    auto fits = [&](int tm, int tn) {
+      if ((int64_t)dgc_div_up(M, tm) * dgc_div_up(N, tn) * splits > ctx->sm_count) return false;
+      grid.x = dgc_div_up(N, tn);
+      grid.y = dgc_div_up(M, tm);
+      return true;
+    };
+    if (fits(32, 32)) kern = dgtc::tc_gemm_kernel<!TA, TB, EPI, 32, 32>;
+    else if (fits(64, 64)) kern = dgtc::tc_gemm_kernel<!TA, TB, EPI, 64, 64>;
+    else if (fits(128, 64)) kern = dgtc::tc_gemm_kernel<!TA, TB, EPI, 128, 64>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dgtc::SMEM_BYTES);
     if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));
-    kern<<<grid, dgtc::THREADS, dgtc::SMEM_BYTES, ctx->stream>>>(A, B, bias, M, N, K, kps, dst, ctx->status_dev);
+    kern<<<grid, dgtc::THREADS + 32, dgtc::SMEM_BYTES, ctx->stream>>>(A, B, bias, M, N, K, kps, dst, ctx->status_dev);
   } else {
     sgemm_kernel<TA, TB, EPI><<<grid, 256, 0, ctx->stream>>>(A, B, bias, M, N, K, kps, dst);
   }

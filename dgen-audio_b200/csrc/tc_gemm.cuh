@@ -73,6 +73,10 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
 // true when the phase with the given parity has completed; bounded
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   for (uint32_t it = 0; it < SPIN_LIMIT; ++it) {
@@ -121,8 +125,8 @@ template <bool ROWMAJOR_K, int ROWS, int P>
 __device__ __forceinline__ void fetch(const float *__restrict__ src, int ld, int rows, int r0, int k0, int k_end,
                                       int tid, float4 (&v)[P]) {
   static_assert(P == ROWS * TBK / 4 / THREADS, "a 32-deep tile, four values at a time");
-  constexpr int UG = ROWS / 16, UGS = UG == 8 ? 8 : 7;   // groups of four units along the rows
-  static_assert(UG == 8 || UG == 4, "128 or 64 rows");
+  constexpr int UG = ROWS / 16, UGS = UG == 8 ? 8 : UG == 4 ? 7 : 6;   // groups of four units along the rows
+  static_assert(UG == 8 || UG == 4 || UG == 2, "128, 64 or 32 rows");
   const bool vec_ok = ((ld & 3) == 0) && ((((uintptr_t)src) & 15) == 0);
 #pragma unroll
   for (int p = 0; p < P; ++p) {
@@ -159,7 +163,7 @@ __device__ __forceinline__ void fetch(const float *__restrict__ src, int ld, int
 
 template <bool ROWMAJOR_K, int ROWS, int P>
 __device__ __forceinline__ void stash(const float4 (&v)[P], char *hi_part, char *lo_part, int tid) {
-  constexpr int UG = ROWS / 16, UGS = UG == 8 ? 8 : 7;
+  constexpr int UG = ROWS / 16, UGS = UG == 8 ? 8 : UG == 4 ? 7 : 6;
 #pragma unroll
   for (int p = 0; p < P; ++p) {
     if (ROWMAJOR_K) {
@@ -204,16 +208,18 @@ constexpr int EPI_STAGE_FLOATS = 32 * 33;   // per warp: a 32 x 32 block, rows p
 // now) and writes full 128-byte row segments.  EPI 0: C = acc ; 1: + bias[n] ; 2: tanh(acc + bias[n]).
 // Ct (optional): a second, transposed copy Ct[n][m] of the result, written straight from the registers
 // (lanes = consecutive m: already 128-byte stores).
-template <int EPI, int BN = TBN>
+template <int EPI, int BN = TBN, int BM = TBM>
 __device__ __forceinline__ void epilogue(uint32_t tmem_d, const float *__restrict__ bias, int M, int N, int m0, int n0,
                                          float *__restrict__ C, int warp, int lane, float *__restrict__ Ct,
                                          float *__restrict__ stage_all) {
-  const int lane_base = (warp & 3) * 32, col_base = (warp >> 2) * (BN / 2);
+  constexpr int SPAN = BN >= 64 ? BN / 2 : BN;           // columns of a warp
+  const int lane_base = (warp & 3) * 32, col_base = (warp >> 2) * SPAN;
+  if (lane_base >= BM || col_base >= BN) return;
   const int gm = m0 + lane_base + lane;
   float *stage = stage_all + warp * EPI_STAGE_FLOATS;
   const bool aligned = ((N & 3) == 0) && ((((uintptr_t)C) & 15) == 0);
 #pragma unroll 1
-  for (int c0 = col_base; c0 < col_base + BN / 2; c0 += 32) {
+  for (int c0 = col_base; c0 < col_base + SPAN; c0 += 32) {
     if (n0 + c0 >= N) break;   // the rest of this tile lies beyond the last column (warp-uniform)
     uint32_t r[32];
     const uint32_t taddr = tmem_d + ((uint32_t)lane_base << 16) + (uint32_t)c0;
@@ -265,25 +271,35 @@ __device__ __forceinline__ void epilogue(uint32_t tmem_d, const float *__restric
 
 // A_KMAJOR: A stored [M][K]; else stored [K][M].  B_KMAJOR: B stored [N][K]; else stored [K][N].
 // EPI 0: C = acc ; 1: + bias[n] ; 2: tanh(acc + bias[n]).  blockIdx.z selects a k-slice (split-K slab of C).
-// BN 64: half as wide an output tile, for products that are only a few tiles (the order of the products an output element
-// adds up is the same).  The loads run three k tiles ahead in registers: with one CTA on an SM and nothing beside it a k tile
-// otherwise costs a round trip to memory.  128 x 128 over 750 k: 51 -> 38 us, 750 x 128 over 128 k: 13 -> 9.5 us.
-template <bool A_KMAJOR, bool B_KMAJOR, int EPI, int BN = TBN>
-__global__ void __launch_bounds__(THREADS, 1)
+// BM x BN: the output tile.  Products of few tiles take smaller ones: a CTA alone on its SM waits for its own loads, 24 KB a
+// k tile for 128 x 64 at the 45 bytes a cycle that one SM gets, 8 KB for 32 x 32.  The MMA stays 128 rows high (what the rows
+// past BM hold goes to accumulator rows that nobody reads) and an output element adds up the same products in the same order.
+// The loads run three k tiles ahead in registers, and a ninth warp issues the MMAs: from a worker, the 900 cycles that twelve
+// of them and the commit take stood between two tiles of splitting and loading.
+// 128 x 128 over 750 k: 51 us in one 128 x 128 tile with one k tile ahead, 38 in 128 x 64 with three, 27 in 64 x 64, 20 in
+// 32 x 32; 750 x 128 over 128 k: 13 and 7.7 us.
+template <bool A_KMAJOR, bool B_KMAJOR, int EPI, int BM, int BN>
+__global__ void __launch_bounds__(THREADS + 32, 1)
 tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const float *__restrict__ bias, int M, int N,
                int K, int k_per_split, float *__restrict__ C, int32_t *status) {
   extern __shared__ __align__(128) char smem[];
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * STAGE_BYTES);      // two mbarriers
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * STAGE_BYTES);      // two "stage multiplied" mbarriers
+  uint64_t *ready = bars + 2;                                                 // two "stage written"
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 2 * STAGE_BYTES + 32);
+  volatile int *failed = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * TBM, n0 = blockIdx.x * BN;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const int k_begin = blockIdx.z * k_per_split, k_end = min(K, k_begin + k_per_split);
   C += (size_t)blockIdx.z * M * N;
   const int KT = (k_end - k_begin + TBK - 1) / TBK;
 
   if (tid == 0) {
-    mbar_init(smem_u32(&bars[0]), 1);
-    mbar_init(smem_u32(&bars[1]), 1);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&bars[i]), 1);
+      mbar_init(smem_u32(&ready[i]), THREADS / 32);   // one arrival per worker warp
+    }
+    *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -296,36 +312,46 @@ tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const f
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_d = *tmem_slot;
-  bool ok = true;
 
-  constexpr int AHEAD = 3, PA = 4, PB = BN / 32;
-  float4 va[AHEAD][PA], vb[AHEAD][PB];
-  auto load = [&](int kt, float4 (&fa)[PA], float4 (&fb)[PB]) {
-    if (kt >= KT) return;
-    fetch<A_KMAJOR, TBM>(A, A_KMAJOR ? K : M, M, m0, k_begin + kt * TBK, k_end, tid, fa);
-    fetch<B_KMAJOR, BN>(B, B_KMAJOR ? K : N, N, n0, k_begin + kt * TBK, k_end, tid, fb);
-  };
+  if (warp < THREADS / 32) {
+    constexpr int AHEAD = 3, PA = BM / 32, PB = BN / 32;
+    float4 va[AHEAD][PA], vb[AHEAD][PB];
+    auto load = [&](int kt, float4 (&fa)[PA], float4 (&fb)[PB]) {
+      if (kt >= KT) return;
+      fetch<A_KMAJOR, BM>(A, A_KMAJOR ? K : M, M, m0, k_begin + kt * TBK, k_end, tid, fa);
+      fetch<B_KMAJOR, BN>(B, B_KMAJOR ? K : N, N, n0, k_begin + kt * TBK, k_end, tid, fb);
+    };
 #pragma unroll
-  for (int j = 0; j < AHEAD; ++j) load(j, va[j], vb[j]);
-  // returns false when the tensor core stopped answering: no further MMAs are issued, TMEM is still released below
-  auto tile = [&](int kt, float4 (&fa)[PA], float4 (&fb)[PB]) -> bool {
-    const int s = kt & 1;
-    if (kt >= 2) {
-      ok = mbar_wait(smem_u32(&bars[s]), (uint32_t)(((kt >> 1) - 1) & 1));
-      ok = __syncthreads_and(ok);   // same decision in every thread
-      if (!ok) return false;
+    for (int j = 0; j < AHEAD; ++j) load(j, va[j], vb[j]);
+    auto tile = [&](int kt, float4 (&fa)[PA], float4 (&fb)[PB]) {
+      const int s = kt & 1;
+      // bounded; a thread that gives up raises the shared flag and everybody stops waiting
+      if (kt >= 2 && !*failed && !mbar_wait(smem_u32(&bars[s]), (uint32_t)(((kt >> 1) - 1) & 1))) *failed = 1;
+      char *st = smem + s * STAGE_BYTES;
+      stash<A_KMAJOR, BM>(fa, st, st + OPER_BYTES, tid);
+      stash<B_KMAJOR, BN>(fb, st + 2 * OPER_BYTES, st + 3 * OPER_BYTES, tid);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> async proxy (tensor core)
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ready[s]));
+      load(kt + AHEAD, fa, fb);
+    };
+    for (int kt = 0; kt < KT; kt += AHEAD) {
+#pragma unroll
+      for (int j = 0; j < AHEAD; ++j)
+        if (kt + j < KT) tile(kt + j, va[j], vb[j]);
     }
-    char *st = smem + s * STAGE_BYTES;
-    stash<A_KMAJOR, TBM>(fa, st, st + OPER_BYTES, tid);
-    stash<B_KMAJOR, BN>(fb, st + 2 * OPER_BYTES, st + 3 * OPER_BYTES, tid);
-    load(kt + AHEAD, fa, fb);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> async proxy (tensor core)
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (tid == 0 && ok) {
+  } else if (lane == 0) {
+    constexpr uint32_t ID = IDesc<true, true, BN>::value;
+    for (int kt = 0; kt < KT; ++kt) {
+      const int s = kt & 1;
+      // when the workers or the tensor core stop answering no further MMAs are issued, TMEM is still released below
+      if (*failed || !mbar_wait(smem_u32(&ready[s]), (uint32_t)((kt >> 1) & 1))) {
+        *failed = 1;
+        break;
+      }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a_hi = smem_u32(st), a_lo = a_hi + OPER_BYTES, b_hi = a_hi + 2 * OPER_BYTES, b_lo = a_hi + 3 * OPER_BYTES;
-      constexpr uint32_t ID = IDesc<true, true, BN>::value;
+      const uint32_t a_hi = smem_u32(smem + s * STAGE_BYTES), a_lo = a_hi + OPER_BYTES, b_hi = a_hi + 2 * OPER_BYTES,
+                     b_lo = a_hi + 3 * OPER_BYTES;
 #pragma unroll
       for (int ks = 0; ks < TBK / 8; ++ks) {
         // 8 tf32 along k = two 16-byte k-chunks
@@ -338,24 +364,20 @@ tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const f
       }
       commit_to(smem_u32(&bars[s]));
     }
-    return true;
-  };
-  for (int kt = 0; kt < KT && ok; kt += AHEAD) {
-#pragma unroll
-    for (int j = 0; j < AHEAD; ++j)
-      if (kt + j < KT && !tile(kt + j, va[j], vb[j])) break;
+    // the last commit covers every MMA issued before it
+    if (KT > 0 && !*failed && !mbar_wait(smem_u32(&bars[(KT - 1) & 1]), (uint32_t)(((KT - 1) >> 1) & 1))) *failed = 1;
   }
-  // the last commit covers every MMA issued before it
-  if (KT > 0 && ok) ok = mbar_wait(smem_u32(&bars[(KT - 1) & 1]), (uint32_t)(((KT - 1) >> 1) & 1));
-  ok = __syncthreads_and(ok);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  const bool ok = !*failed;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
   if (ok && KT > 0) {
-    epilogue<EPI, BN>(tmem_d, bias, M, N, m0, n0, C, warp, lane, nullptr, reinterpret_cast<float *>(smem));
+    if (warp < THREADS / 32) epilogue<EPI, BN, BM>(tmem_d, bias, M, N, m0, n0, C, warp, lane, nullptr, reinterpret_cast<float *>(smem));
   } else if (KT == 0) {
     // empty reduction range: the slab is zero
     const int gm = m0 + (warp & 3) * 32 + lane;
-    if (gm < M && warp < 4)
+    if (gm < M && warp < BM / 32)
       for (int c = 0; c < BN; ++c)
         if (n0 + c < N) C[(size_t)gm * N + n0 + c] = 0.0f;
   }
@@ -436,10 +458,6 @@ __device__ __forceinline__ unsigned long long gtime() {
 #endif
 
 constexpr int KK_THREADS = THREADS + 32;   // 8 worker warps + 1 warp whose lane 0 issues the MMAs
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 
 // A4: the operands' rows are only 4-byte aligned (K % 4 != 0): every 16-byte unit is fetched as four 4-byte copies.
 template <int EPI, int BK, bool SW, int BN = TBN, bool A4 = false>

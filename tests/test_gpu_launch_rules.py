@@ -1,4 +1,4 @@
-"""Sizes on both sides of the launch rules: tap maps in small blocks, matmuls in half-width tiles, the spectral gradient in
+"""Sizes on both sides of the launch rules: tap maps in small blocks, matmuls in every tile shape, the spectral gradient in
 one launch, the host-buffer step in groups of voices, banks of odd lane counts."""
 import numpy as np
 import pytest
@@ -33,8 +33,9 @@ def test_small_tap_maps(ctx, F, B, NB, NT):
     assert np.abs(got - want).max() <= 2e-6 * max(1.0, np.abs(want).max())
 
 
-# the weight gradient reduces over M rows of either parity; outputs of one, of a few and of more tiles than half the chip
-@pytest.mark.parametrize("M,K,N", [(750, 128, 128), (997, 130, 65), (257, 96, 129), (33, 512, 512), (321, 1100, 1030)])
+# the weight gradient reduces over M rows of either parity; outputs that take each of the four tile shapes
+@pytest.mark.parametrize("M,K,N", [(750, 128, 128), (997, 130, 65), (257, 96, 129), (33, 512, 512), (40, 1024, 1000),
+                                   (321, 1100, 1030)])
 def test_weight_gradient_tiles(ctx, M, K, N):
     rng = np.random.default_rng(M)
     a, w = rng.standard_normal((M, K)).astype(f32), (rng.standard_normal((K, N)) / np.sqrt(K)).astype(f32)
