@@ -189,8 +189,12 @@ int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *
     if (!dst) return DGC_ERR_OOM;
   }
   dim3 grid(dgc_div_up(N, bn), dgc_div_up(M, bm), splits);
-  ctx->gemm_paths[(kk && (splits == 1 || kps % 32 == 0)) ? (wide ? 3 : 2) : (tc ? 1 : 0)]++;
-  if (kk && (splits == 1 || kps % 32 == 0)) {
+  // a whole reduction whose 64 x 64 tiles the chip takes at once: smaller tiles beat the pipeline (750 x 128 over 128 k: 10 -> 7 us,
+  // 750 x 512 over 512 k: 30 -> 17 us)
+  const bool few = tc && splits == 1 && (int64_t)dgc_div_up(M, 64) * dgc_div_up(N, 64) <= ctx->sm_count;
+  const bool piped = kk && !few && (splits == 1 || kps % 32 == 0);
+  ctx->gemm_paths[piped ? (wide ? 3 : 2) : (tc ? 1 : 0)]++;
+  if (piped) {
     // both operands contiguous along k: the cp.async pipeline
 #define DGC_KK_LAUNCH(BKV, SWV)                                                                                      \
   do {                                                                                                              \
@@ -236,7 +240,9 @@ int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *
     else if (fits(128, 64)) kern = dgtc::tc_gemm_kernel<!TA, TB, EPI, 128, 64>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dgtc::SMEM_BYTES);
     if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));
-    kern<<<grid, dgtc::THREADS + 32, dgtc::SMEM_BYTES, ctx->stream>>>(A, B, bias, M, N, K, kps, dst, ctx->status_dev);
+    kern<<<grid, dgtc::THREADS + 32, dgtc::SMEM_BYTES, ctx->stream>>>(A, B, bias, M, N, K, kps, dst,
+                                                                              splits == 1 ? Ct : nullptr, ctx->status_dev);
+    if (ct_written) *ct_written = Ct && splits == 1;
   } else {
     sgemm_kernel<TA, TB, EPI><<<grid, 256, 0, ctx->stream>>>(A, B, bias, M, N, K, kps, dst);
   }

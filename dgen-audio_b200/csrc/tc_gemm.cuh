@@ -281,7 +281,7 @@ __device__ __forceinline__ void epilogue(uint32_t tmem_d, const float *__restric
 template <bool A_KMAJOR, bool B_KMAJOR, int EPI, int BM, int BN>
 __global__ void __launch_bounds__(THREADS + 32, 1)
 tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const float *__restrict__ bias, int M, int N,
-               int K, int k_per_split, float *__restrict__ C, int32_t *status) {
+               int K, int k_per_split, float *__restrict__ C, float *__restrict__ Ct, int32_t *status) {
   extern __shared__ __align__(128) char smem[];
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * STAGE_BYTES);      // two "stage multiplied" mbarriers
   uint64_t *ready = bars + 2;                                                 // two "stage written"
@@ -373,7 +373,7 @@ tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const f
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
   if (ok && KT > 0) {
-    if (warp < THREADS / 32) epilogue<EPI, BN, BM>(tmem_d, bias, M, N, m0, n0, C, warp, lane, nullptr, reinterpret_cast<float *>(smem));
+    if (warp < THREADS / 32) epilogue<EPI, BN, BM>(tmem_d, bias, M, N, m0, n0, C, warp, lane, Ct, reinterpret_cast<float *>(smem));
   } else if (KT == 0) {
     // empty reduction range: the slab is zero
     const int gm = m0 + (warp & 3) * 32 + lane;
