@@ -106,6 +106,8 @@ const float *dgc_ctx_hann_sym(dgc_ctx *ctx, int N);
 const float *dgc_ctx_hann_per(dgc_ctx *ctx, int N);
 // C[M][N] = A[M][K] * B[N][K]^T on the matmul path of gemm.cu
 int32_t dgc_gemm_nt(dgc_ctx *ctx, const float *a, const float *b, int M, int N, int K, float *c);
+// whether dgc_linear_bwd has a use for a transposed copy of the layer's input
+bool dgc_linear_bwd_reads_t(int64_t M, int64_t K, int64_t N);
 // true when dgc_gemm_nt() runs this shape on its persistent short-reduction tensor-core kernel
 bool dgc_gemm_nt_persistent(const dgc_ctx *ctx, const float *a, int M, int N, int K);
 const float2 *dgc_ctx_twiddles(dgc_ctx *ctx, int N);

@@ -527,6 +527,10 @@ __global__ void adam_kernel(float *__restrict__ theta, const float *__restrict__
 
 }  // namespace
 
+bool dgc_linear_bwd_reads_t(int64_t M, int64_t K, int64_t N) {
+  return use_tensor_cores() && (M & 3) == 0 && (double)M * N * K >= (double)(1 << 24);
+}
+
 bool dgc_gemm_nt_persistent(const dgc_ctx *ctx, const float *a, int M, int N, int K) { return smallk_shape(ctx, a, M, N, K); }
 
 // C[M][N] = A[M][K] * B[N][K]^T, no epilogue (used for the band -> tap map)
@@ -612,8 +616,7 @@ DGC_EXPORT int32_t dgc_linear_bwd(dgc_ctx *ctx, const float *a_dev, const float 
   const size_t n = (size_t)M * N;
   // With a transposed copy of the layer input at hand, the weight gradient reads both operands along the
   // reduction index m (the asynchronous K-major pipeline): dZ is then written in both orientations.
-  const bool dw_kmajor = at_dev && use_tensor_cores() && (M & 3) == 0 && (double)M * N * K >= (double)(1 << 24) &&
-                         (((uintptr_t)at_dev) & 15) == 0;
+  const bool dw_kmajor = at_dev && dgc_linear_bwd_reads_t(M, K, N) && (((uintptr_t)at_dev) & 15) == 0;
   if (dw_kmajor) {
     if (!ctx->dzt_buf || ctx->dzt_floats < n) {
       if (ctx->dzt_buf) {

@@ -158,6 +158,7 @@ SIGNATURES = {
     "dgc_launch_count": (_i64, [_vp]),
     "dgc_arena_create": (_i32, [_vp, _u64, C.POINTER(_vp)]),
     "dgc_arena_wrap": (_i32, [_vp, _vp, _u64, C.POINTER(_vp)]),
+    "dgc_copy_many": (_i32, [_vp, _vp, _i32, C.POINTER(_vp), C.POINTER(_vp), C.POINTER(C.c_uint64)]),
     "dgc_plan_run": (_i32, [_vp, _vp, C.POINTER(Plan), _i32, _i32]),
     "dgc_hn_train_plan": (_i32, [C.POINTER(HnTrainConfig), C.POINTER(HnTrainLayout), C.POINTER(PlanStep), _i32]),
     "dgc_arena_destroy": (_i32, [_vp]),

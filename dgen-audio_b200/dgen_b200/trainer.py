@@ -121,10 +121,20 @@ class HarmonicModel:
     # ------------------------------------------------------------------------------------------
     def _load(self, args):
         """Inputs given as other tensors are copied into their arena slots (device to device)."""
+        torch, plain = self.torch, []
         for k, a in zip(self.INPUTS, args):
             v = self.inputs[k]
-            if a.data_ptr() != v.data_ptr():
+            if a.data_ptr() == v.data_ptr():
+                continue
+            if a.dtype == v.dtype and a.device == v.device and a.is_contiguous() and a.numel() == v.numel():
+                plain.append((a.data_ptr(), v.data_ptr(), v.numel()))
+            else:
                 v.copy_(a.reshape(v.shape))
+        if plain:
+            n = len(plain)
+            src, dst, floats = zip(*plain)
+            self.ctx.check(self.ctx.lib.dgc_copy_many(self.ctx.h, torch.cuda.current_stream(self.ctx.device).cuda_stream, n,
+                                                      (C.c_void_p * n)(*src), (C.c_void_p * n)(*dst), (C.c_uint64 * n)(*floats)))
 
     def _run(self, first, count):
         self.ctx.check(self.ctx.lib.dgc_plan_run(self.ctx.h, self.arena, C.byref(self.plan), first, count))

@@ -627,6 +627,11 @@ typedef struct dgc_plan {
   const char *const *kernels;
   int32_t n_kernels;
 } dgc_plan;
+/* Copies floats[k] floats from src[k] to dst[k], k < count <= DGC_COPY_MAX, in one launch on `stream` (a cudaStream_t).
+ * Device memory; the destinations overlap nothing. */
+#define DGC_COPY_MAX 16
+int32_t dgc_copy_many(dgc_ctx *ctx, void *stream, int32_t count, const float *const *src, float *const *dst,
+                      const uint64_t *floats);
 /* Runs steps [first, first + count) of the plan on the arena (count < 0: to the end).  On an error the step index is
  * part of dgc_last_error and nothing after it is enqueued; a side stream that was forked is joined first. */
 int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *plan, int32_t first, int32_t count);

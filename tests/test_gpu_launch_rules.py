@@ -1,5 +1,7 @@
 """Sizes on both sides of the launch rules: tap maps in small blocks, matmuls in every tile shape, the spectral gradient in
 one launch, the host-buffer step in groups of voices, banks of odd lane counts."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -100,3 +102,16 @@ def test_biquad_banks_of_odd_lanes(ctx, B, L, T):
     ref = np.stack([sum(orc.biquad(g64[b, ::-1, l].copy(), float(cut[l]), float(q[l]), double=True)[::-1] for l in range(L))
                     for b in range(B)])
     assert np.abs(gx.cpu().numpy() - ref).max() <= 1e-3 * max(np.abs(ref).max(), 1e-30)
+
+
+def test_many_copies_in_one_launch(ctx):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    sizes = [1, 3, 4, 1023, 700001, 64, 17, 2]
+    src = [torch.randn(n + 2, generator=g, device="cuda") for n in sizes]
+    dst = [torch.zeros(n + 2, device="cuda") for n in sizes]
+    off = [k % 2 for k in range(len(sizes))]                       # every other pair is not 16-byte aligned
+    ptr = lambda ts: (C.c_void_p * len(sizes))(*[t.data_ptr() + 4 * o for t, o in zip(ts, off)])
+    ctx.check(ctx.lib.dgc_copy_many(ctx.h, torch.cuda.current_stream().cuda_stream, len(sizes), ptr(src), ptr(dst),
+                                    (C.c_uint64 * len(sizes))(*sizes)))
+    for n, o, s, d in zip(sizes, off, src, dst):
+        assert torch.equal(d[o:o + n], s[o:o + n]) and float(d[:o].abs().sum()) + float(d[o + n:].abs().sum()) == 0.0
