@@ -244,9 +244,9 @@ int32_t dgc_onepole_fwd_state(dgc_ctx *ctx, const float *x_dev, int32_t B, int32
 /* The same filter for callers that must not allocate.  No counterpart in the reference: it exists
  * because a real-time audio thread (a plug-in render callback, a driver I/O thread) cannot call
  * cudaMalloc -- it may block without bound -- and creating or growing a dgc_ctx does.  This call takes
- * no context and allocates nothing, on the host or on the device: its chunk-carry scratch is a fixed
- * 256 KiB array inside the library's device image, present on every GPU that loads the library until
- * the process exits.
+ * no context and allocates nothing, on the host or on the device: its scratch (a ticket and the tiles'
+ * cells) is a fixed array of 256 KiB inside the library's device image, present on every GPU that loads
+ * the library until the process exits.
  *   limit     B * ceil(T / 2048) <= DGC_ONEPOLE_STATIC_MAX_CHUNKS (and B <= 65535); larger requests
  *             return DGC_ERR_INVALID with the reason in err_buf (err_buf may be NULL).
  *   set-up    the first call on each device looks up the array's device address
@@ -255,8 +255,8 @@ int32_t dgc_onepole_fwd_state(dgc_ctx *ctx, const float *x_dev, int32_t B, int32
  *             (a cudaStream_t; NULL = default stream) of the CURRENT device and take no lock (the
  *             resolved address is read with one atomic load).
  *   in place  x_dev == y_dev is allowed: every thread reads its run of samples before it writes it.
- *   sharing   all calls on a device use the same array, which keeps the last call's contents; the
- *             filter overwrites every slot before reading it, so nothing needs clearing, but two
+ *   sharing   all calls on a device use the same array, which keeps the last call's contents; a cell
+ *             carries the number of the launch that wrote it, so nothing needs clearing, but two
  *             calls that overlap on the GPU (different streams, no ordering) race: serialise them. */
 #define DGC_ONEPOLE_STATIC_MAX_CHUNKS 32768
 int32_t dgc_onepole_fwd_static(void *cuda_stream, const float *x_dev, int32_t B, int32_t T, float a, float *y_dev,
