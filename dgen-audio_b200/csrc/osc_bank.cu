@@ -299,11 +299,12 @@ __device__ __forceinline__ unsigned long long inc_q64(float f0v, float sr, float
 // How many partials k = 1, 2, .. pass the Nyquist mask fl(k f0) < nyq of the reference (Examples/HarmonicE2E/
 // Synth.swift:161-170): the products are monotone in k for f0 >= 0, so the passing partials are a prefix 1 .. kcut
 // and one count per frame replaces a multiply and a compare per partial and frame.  Decided on the reference's own
-// single-precision product, so a partial exactly at Nyquist flips exactly where the reference flips it.
+// single-precision product, so a partial exactly at Nyquist flips exactly where the reference flips it.  The quotient only
+// has to start the walk down no lower than the count, so the approximate one does (2 ulp against steps of one in K).
 __device__ __forceinline__ int nyquist_count(float f0v, float nyq, int K) {
   if (!(f0v == f0v)) return 0;            // NaN: every comparison is false
   if (!(f0v > 0.0f)) return K;            // zero or negative: every product is <= 0 < nyq
-  const float r = nyq / f0v;
+  const float r = __fdividef(nyq, f0v);
   if (!(r < (float)(K + 2))) return K;
   int k = (int)r + 1;
   if (k > K) k = K;
@@ -315,46 +316,80 @@ __device__ __forceinline__ int nyquist_count(float f0v, float nyq, int K) {
 // the chunk's total phase advance of the fundamental (Q0.64), and per frame the pair (phase advance of the
 // fundamental from the chunk's first frame to this one: the wrapping sum of the frames' increments rounded to
 // Q0.32; number of partials below Nyquist) that the render and its backward read instead of deriving them.
+// Bound by instruction issue; a lane takes two neighbouring frames, which mostly share their control rows, so the chunk
+// takes one scan and half the stores: 256 voices x 64000 frames 113 -> 100 us beside the map, 32 x 64000 31 -> 18.
 __global__ void __launch_bounds__(128)
 f0_track_fund_kernel(const float2 *__restrict__ rowtab, const float *__restrict__ f0, int B, int T, int F, int K, float sr,
                      float rsr, float *__restrict__ f0t, const float *__restrict__ uv,
                      const float *__restrict__ gain, float scale, float *__restrict__ env,
                      unsigned long long *__restrict__ chunk_sum /* [B][C] */, int2 *__restrict__ trk /* [B][T] */) {
+  static_assert(CH == 64, "two frames per lane");
   const int C = (T + CH - 1) / CH;
   const int c = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, b = blockIdx.y;
   if (c >= C) return;
+  const int n = c * CH + 2 * lane;
+  const float *f0b = f0 + b, *gb = gain + b, *ub = uv + b;
   unsigned long long tot = 0ull;
-  uint32_t carry = 0u;   // sum of the rounded increments of the chunk's frames before this half
+  float f0v[2] = {0.0f, 0.0f}, ev[2] = {0.0f, 0.0f};
+  uint32_t dq[2] = {0u, 0u};
+  int cnt[2] = {0, 0}, row = -1;
+  float fl = 0.0f, fh = 0.0f, gl = 0.0f, gh = 0.0f, ul = 0.0f, uh = 0.0f;
 #pragma unroll
-  for (int h = 0; h < CH / 32; ++h) {
-    const int n = c * CH + h * 32 + lane;
-    uint32_t dq = 0u;
-    int cnt = 0;
-    if (n < T) {
-      const float2 rt = rowtab[n];
-      const int lo = __float_as_int(rt.x), hi = lo + 1 >= F ? 0 : lo + 1;
-      const float fr = rt.y, omf = __fsub_rn(1.0f, fr);
-      const float f0v = lerp_strict(omf, f0[(size_t)lo * B + b], fr, f0[(size_t)hi * B + b]);
-      f0t[(size_t)b * T + n] = f0v;
+  for (int u = 0; u < 2; ++u) {
+    if (n + u >= T) continue;
+    const float2 rt = rowtab[n + u];
+    const int lo = __float_as_int(rt.x);
+    if (lo != row) {
+      const size_t ol = (size_t)lo * B, oh = lo + 1 >= F ? 0 : ol + B;
+      fl = f0b[ol];
+      fh = f0b[oh];
       if (env) {
-        const float gt = fmaf(fr, gain[(size_t)hi * B + b], omf * gain[(size_t)lo * B + b]);
-        const float uvt = fmaf(fr, uv[(size_t)hi * B + b], omf * uv[(size_t)lo * B + b]);
-        env[(size_t)b * T + n] = gt * uvt * scale;
+        gl = gb[ol];
+        gh = gb[oh];
+        ul = ub[ol];
+        uh = ub[oh];
       }
-      const unsigned long long d64 = inc_q64(f0v, sr, rsr);
-      tot += d64;
-      dq = (uint32_t)((d64 + 0x80000000ull) >> 32);
-      cnt = nyquist_count(f0v, sr * 0.5f, K);
+      row = lo;
     }
-    if (trk) {   // warp-uniform
-      uint32_t inc = dq;
+    const float fr = rt.y, omf = __fsub_rn(1.0f, fr);
+    f0v[u] = lerp_strict(omf, fl, fr, fh);
+    if (env) {
+      const float gt = fmaf(fr, gh, omf * gl);
+      const float uvt = fmaf(fr, uh, omf * ul);
+      ev[u] = gt * uvt * scale;
+    }
+    const unsigned long long d64 = inc_q64(f0v[u], sr, rsr);
+    tot += d64;
+    dq[u] = (uint32_t)((d64 + 0x80000000ull) >> 32);
+    cnt[u] = nyquist_count(f0v[u], sr * 0.5f, K);
+  }
+  uint32_t inc = dq[0] + dq[1];
+  if (trk) {   // warp-uniform
 #pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, off);
-        if (lane >= off) inc += v;
-      }
-      if (n < T) trk[(size_t)b * T + n] = make_int2((int)(carry + inc - dq), cnt);
-      carry += __shfl_sync(0xffffffffu, inc, 31);
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, inc, off);
+      if (lane >= off) inc += v;
+    }
+  }
+  const uint32_t before = inc - dq[0] - dq[1];
+  const size_t at = (size_t)b * T + n;
+  const bool two = n + 1 < T;
+  if (two && (at & 1) == 0) {
+    *reinterpret_cast<float2 *>(f0t + at) = make_float2(f0v[0], f0v[1]);
+    if (env) *reinterpret_cast<float2 *>(env + at) = make_float2(ev[0], ev[1]);
+  } else if (n < T) {
+    f0t[at] = f0v[0];
+    if (two) f0t[at + 1] = f0v[1];
+    if (env) env[at] = ev[0];
+    if (env && two) env[at + 1] = ev[1];
+  }
+  if (trk && n < T) {
+    const int2 t0 = make_int2((int)before, cnt[0]), t1 = make_int2((int)(before + dq[0]), cnt[1]);
+    if (two && (((uintptr_t)(trk + at)) & 15) == 0) {
+      *reinterpret_cast<int4 *>(trk + at) = make_int4(t0.x, t0.y, t1.x, t1.y);
+    } else {
+      trk[at] = t0;
+      if (two) trk[at + 1] = t1;
     }
   }
 #pragma unroll
