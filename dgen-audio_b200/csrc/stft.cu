@@ -180,66 +180,6 @@ istft_kernel(const float2 *__restrict__ Y, int H, const float *__restrict__ wind
   }
 }
 
-// The same with the overlap-add in registers: a thread's elements of a frame are lt + q N/8, and a hop of S N/8 keeps them
-// in the thread, so its eight running sums take the frames oldest first and S of them are final after each.  The threads
-// of a transform walk `run` hop pairs of one signal, after the WARM pairs before them that reach into their first hop.
-// out[v][t], t = position on the overlap-add grid + offset.  Every value is formed, and every sum taken, as the two kernels
-// istft and overlap_add do it, to the last bit.
-template <int N, int S>
-__global__ void __launch_bounds__(ST_THREADS)
-istft_ola_kernel(const float2 *__restrict__ Y, int H, int T, const float *__restrict__ window, const float2 *__restrict__ tw,
-                 float gain, int offset, int accumulate, int run, float *__restrict__ out) {
-  constexpr int G = N / 8, NF = ST_THREADS / G, NB = N / 2 + 1, PN = padded(N), WARM = (8 / S) / 2;
-  __shared__ float2 bufa[NF * PN];
-  __shared__ float2 bufb[NF * PN];
-  const int tid = threadIdx.x, f = tid / G, lt = tid % G, v = blockIdx.y;
-  const int first = (blockIdx.x * NF + f) * run;
-  float2 *a = bufa + f * PN, *bb = bufb + f * PN;
-  const float invn = 1.0f / (float)N;
-  float acc[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) acc[q] = 0.0f;
-  for (int p = first - WARM; p < first + run; ++p) {
-    const int h0 = 2 * p, h1 = h0 + 1;
-    const bool live0 = h0 >= 0 && h0 < H, live1 = h0 >= 0 && h1 < H;
-    const size_t row = ((size_t)v * H + (live0 ? h0 : 0)) * NB;
-    float2 vin[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      int k = lt + q * G;
-      int ks = k <= N / 2 ? k : N - k;
-      float2 y0 = make_float2(0.f, 0.f), y1 = y0;
-      if (live0) y0 = Y[row + ks];
-      if (live1) y1 = Y[row + NB + ks];
-      if (k > N / 2) { y0.y = -y0.y; y1.y = -y1.y; }
-      vin[q] = make_float2(y0.x - y1.y, y0.y + y1.x);
-    }
-    fft_sync<N>();      // the previous pair's frames have been read
-    float2 *z = fft_block_regs<N, true>(vin, a, bb, lt, tw);
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      if (half ? live1 : live0) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int i = lt + q * G;
-          const float w = window ? __ldg(&window[i]) : 1.0f;
-          const float2 val = z[pad(i)];
-          acc[q] = __fadd_rn(acc[q], __fmul_rn(__fmul_rn(__fmul_rn(half ? val.y : val.x, invn), w), gain));
-        }
-      }
-      if (p >= first) {
-        const int t0 = (h0 + half) * (S * G) + offset + lt;
-        float *o = out + (size_t)v * T + t0;
-#pragma unroll
-        for (int q = 0; q < S; ++q)
-          if (t0 + q * G >= 0 && t0 + q * G < T) o[q * G] = accumulate ? o[q * G] + acc[q] : acc[q];
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) acc[q] = q + S < 8 ? acc[(q + S) & 7] : 0.0f;
-    }
-  }
-}
-
 // out[v][t] (+)= sum over hops h with 0 <= t - h*hop - offset < N of frames[v][h][t - h*hop - offset],
 // oldest first.  offset 0: the forward overlap-add; offset -(N-1): the adjoint of the bufferView gather.
 __global__ void overlap_add_kernel(const float *__restrict__ frames, int T, int N, int hop, int H, int offset,
@@ -455,22 +395,13 @@ int32_t istft16_ola(dgc_ctx *ctx, int N, const float *Y, const float *Yim, int V
   return dgc_fail(ctx, DGC_ERR_UNSUPPORTED, "FFT size %d (powers of two 64..2048)", N);
 }
 
-// The same on the eight-point transforms, half spectra only
+// The same on the eight-point transforms, half spectra only, through frames in memory
 template <int N>
 int32_t launch_istft_ola(dgc_ctx *ctx, const float2 *Y, int V, int H, int T, int hop, const float *window, float gain, int offset,
                          int accumulate, float *frames, float *out) {
   const float2 *tw = dgc_ctx_twiddles(ctx, N);
   if (!tw) return DGC_ERR_OOM;
-  constexpr int G = N / 8, NF = ST_THREADS / G;
-  const int pairs = (dgc_div_up((int64_t)T - offset, hop) + 1) / 2, run = ola_run(ctx, V, pairs, 5, NF);
-  const dim3 grid(dgc_div_up(dgc_div_up(pairs, run), NF), V);
-#define STEP(SS) if (hop == SS * G) {                                                                               \
-    istft_ola_kernel<N, SS><<<grid, ST_THREADS, 0, ctx->stream>>>(Y, H, T, window, tw, gain, offset, accumulate, run, out); \
-    ctx->launches++;                                                                                                \
-    return dgc_check_launch(ctx, "istft_overlap_add");                                                              \
-  }
-  STEP(4) STEP(2) STEP(1) STEP(8)
-#undef STEP
+  constexpr int NF = ST_THREADS / (N / 8);
   istft_kernel<N><<<dim3(dgc_div_up((H + 1) / 2, NF), V), ST_THREADS, 0, ctx->stream>>>(Y, H, window, tw, gain, frames);
   ctx->launches++;
   int32_t rc = dgc_check_launch(ctx, "istft");
