@@ -812,12 +812,13 @@ biquad_bwd_carry_kernel(const float *__restrict__ rec, const float *__restrict__
 // A second reverse sweep per (voice, lane, chunk), now from the chunk's TRUE terminal adjoint (resolved by the carry
 // kernel), recomputes lam; the sum over the block's 128 lanes goes through a shared-memory tile of 32 frames, the
 // sum over lane blocks through per-block partial rows that a last kernel adds in a fixed order.
+// Bound by the walk's instructions: no tests in a whole group of frames, a pointer that steps, nothing to walk for a warp
+// without lanes: 5 voices x 50001 x 37 lanes 42 -> 27 us, 300 lanes 120 -> 80.  (The next group's loads sent ahead: 46 and 115.)
 constexpr int GX_FRAMES = 32;
 
-template <bool UP>
 __global__ void __launch_bounds__(BQ_THREADS)
-biquad_gx_kernel(const float *__restrict__ coef, const float *__restrict__ y, const float *__restrict__ tgt,
-                 const float2 *__restrict__ term, int B, int T, int L, int NC, float gscale,
+biquad_gx_kernel(const float *__restrict__ coef, const float *__restrict__ gy, const float2 *__restrict__ term, int B, int T,
+                 int L, int NC,
                  float *__restrict__ part /* [gridDim.x][B][T] */) {
   __shared__ float red[GX_FRAMES][BQ_THREADS + 1];
   const int tid = threadIdx.x, l = blockIdx.x * BQ_THREADS + tid, c = blockIdx.y, b = blockIdx.z;
@@ -831,30 +832,33 @@ biquad_gx_kernel(const float *__restrict__ coef, const float *__restrict__ y, co
     la1 = s.x;
     la2 = s.y;
   }
-  const float *yb = y + (size_t)b * T * L + l, *tb = tgt + (size_t)b * T * L + l;
+  const float *gb = gy + ((size_t)b * T + n0) * L + l;
   float *pb = part + ((size_t)blockIdx.x * B + b) * T;
+  if (!live)
+    for (int j = 0; j < GX_FRAMES; ++j) red[j][tid] = 0.f;
   // groups of 32 frames from the end of the chunk; the last group (lowest frames) may be shorter
   for (int hi = len; hi > 0; hi -= GX_FRAMES) {
     const int lo = max(hi - GX_FRAMES, 0), cnt = hi - lo;
-    float gv[GX_FRAMES];
+    auto walk = [&](auto whole) {
+      float gv[GX_FRAMES];
+      const float *p = gb + (size_t)lo * L;
+#pragma unroll
+      for (int j = 0; j < GX_FRAMES; ++j, p += L) gv[j] = decltype(whole)::value || j < cnt ? __ldcs(p) : 0.f;
+#pragma unroll
+      for (int j = GX_FRAMES - 1; j >= 0; --j) {
+        float contrib = 0.f;
+        if (decltype(whole)::value || j < cnt) {
+          const float lam = __fsub_rn(gv[j], fmaf(cf.a1, la1, __fmul_rn(cf.a2, la2)));
+          contrib = fmaf(cf.b0, lam, fmaf(cf.b1, la1, cf.b2 * la2));
+          la2 = la1;
+          la1 = lam;
+        }
+        red[j][tid] = contrib;
+      }
+    };
     if (live) {
-#pragma unroll
-      for (int j = 0; j < GX_FRAMES; ++j) {
-        const int t = n0 + lo + j;
-        if (j < cnt) gv[j] = UP ? __ldcs(tb + (size_t)t * L) : gscale * (__ldcs(yb + (size_t)t * L) - __ldcs(tb + (size_t)t * L));
-        else gv[j] = 0.f;
-      }
-    }
-#pragma unroll
-    for (int j = GX_FRAMES - 1; j >= 0; --j) {
-      float contrib = 0.f;
-      if (live && j < cnt) {
-        const float lam = gv[j] - (cf.a1 * la1 + cf.a2 * la2);
-        contrib = fmaf(cf.b0, lam, fmaf(cf.b1, la1, cf.b2 * la2));
-        la2 = la1;
-        la1 = lam;
-      }
-      red[j][tid] = contrib;
+      if (cnt == GX_FRAMES) walk(std::true_type());
+      else walk(std::false_type());
     }
     __syncthreads();
     // thread -> (frame j = tid / 4, quarter of the lanes): 32 adds, then the four quarters by shuffles
@@ -1186,7 +1190,7 @@ DGC_EXPORT int32_t dgc_biquad_bwd(dgc_ctx *ctx, const dgc_biquad_params *p, cons
   if (rc != DGC_OK) return rc;
   if (grad_x_dev) {
     const dim3 grid(dgc_div_up(L, BQ_THREADS), NC, B);
-    biquad_gx_kernel<true><<<grid, BQ_THREADS, 0, ctx->stream>>>(scr, y_dev, gy_dev, term, B, T, L, NC, 1.0f, part);
+    biquad_gx_kernel<<<grid, BQ_THREADS, 0, ctx->stream>>>(scr, gy_dev, term, B, T, L, NC, part);
     DGC_LAUNCHED(ctx, "biquad_grad_x");
     const size_t n = (size_t)B * T;
     sum_partial_rows_kernel<<<dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream>>>(part, (int)grid.x, n, grad_x_dev);
