@@ -168,25 +168,30 @@ __device__ __forceinline__ float cond_at(const float *__restrict__ cond, int con
   return cond_mode == 1 ? cond[n] : cond[n * W + e];
 }
 
-// last[c][e] = the last frame of chunk c whose trigger is positive, or -1
+// last[c][e] = the last frame of chunk c whose trigger is positive, or -1.  Sixteen frames are read at a time: one after
+// another each waits for memory (64 lanes x 262144 frames, 3 % of them triggers: 11 -> 9 us).
 __global__ void latch_last_kernel(const float *__restrict__ cond, int cond_mode, int64_t T, int W, int NC,
                                   int *__restrict__ last) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
   if (e >= W) return;
   const int64_t n0 = (int64_t)c * LATCH_CHUNK, n1 = min(n0 + (int64_t)LATCH_CHUNK, T);
+  constexpr int G = 16;
   int found = -1;
-  for (int64_t n = n1 - 1; n >= n0; --n)
-    if (cond_at(cond, cond_mode, n, e, W) > 0.0f) {
-      found = (int)(n - n0);
-      break;
-    }
+  for (int64_t n = n1 - 1; n >= n0 && found < 0; n -= G) {
+    float v[G];
+#pragma unroll
+    for (int j = 0; j < G; ++j) v[j] = cond_at(cond, cond_mode, max(n - j, n0), e, W);
+#pragma unroll
+    for (int j = G - 1; j >= 0; --j)
+      if (n - j >= n0 && v[j] > 0.0f) found = (int)(n - j - n0);
+  }
   last[(size_t)c * W + e] = found;
 }
 
-// Exclusive "most recent trigger" over chunks in three coalesced steps (threads run along the lanes):
+// Exclusive "most recent trigger" over chunks in two coalesced steps (threads run along the lanes):
 //   segments of LATCH_SEG chunks: (chunk, offset) of the last trigger inside each segment;
-//   one thread per lane walks the segment summaries (NC / LATCH_SEG of them) into "most recent before the segment";
-//   each (segment, lane) thread then walks its chunks: last[c][e] becomes the offset and src_chunk[c][e] the chunk of
+//   each (segment, lane) thread then looks back through the summaries, eight at a time, for the last one with a trigger
+//   (mostly the one before it; a walk of one thread per lane over all of them was a launch of 9 us) and walks its chunks: last[c][e] becomes the offset and src_chunk[c][e] the chunk of
 //   the most recent trigger BEFORE chunk c (chunk -1: none yet, the state cell holds the value).
 constexpr int LATCH_SEG = 32;
 
@@ -208,27 +213,28 @@ __global__ void latch_seg_kernel(const int *__restrict__ last, int W, int NC, in
   seg_off[(size_t)sgm * W + e] = off;
 }
 
-__global__ void latch_seg_carry_kernel(int *seg_chunk, int *seg_off, int W, int NS) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= W) return;
-  int run = -1, run_off = 0;
-  for (int sgm = 0; sgm < NS; ++sgm) {
-    const int ch = seg_chunk[(size_t)sgm * W + e], off = seg_off[(size_t)sgm * W + e];
-    seg_chunk[(size_t)sgm * W + e] = run;
-    seg_off[(size_t)sgm * W + e] = run_off;
-    if (ch >= 0) {
-      run = ch;
-      run_off = off;
-    }
-  }
-}
-
 __global__ void latch_carry_kernel(int *last, int *src_chunk, const int *__restrict__ seg_chunk,
                                    const int *__restrict__ seg_off, int W, int NC) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x, sgm = blockIdx.y;
   if (e >= W) return;
   const int c0 = sgm * LATCH_SEG, c1 = min(c0 + LATCH_SEG, NC);
-  int run = seg_chunk[(size_t)sgm * W + e], run_off = seg_off[(size_t)sgm * W + e];
+  int run = -1, run_off = 0;
+  constexpr int BACK = 8;
+  for (int s = sgm - 1; s >= 0 && run < 0; s -= BACK) {
+    int ch[BACK], off[BACK];
+#pragma unroll
+    for (int j = 0; j < BACK; ++j) {
+      const size_t at = (size_t)max(s - j, 0) * W + e;
+      ch[j] = seg_chunk[at];
+      off[j] = seg_off[at];
+    }
+#pragma unroll
+    for (int j = BACK - 1; j >= 0; --j)
+      if (s - j >= 0 && ch[j] >= 0) {
+        run = ch[j];
+        run_off = off[j];
+      }
+  }
 #pragma unroll 8
   for (int c = c0; c < c1; ++c) {
     const int here = last[(size_t)c * W + e];
@@ -754,8 +760,6 @@ DGC_EXPORT int32_t dgc_latch(dgc_ctx *ctx, const float *value_dev, const float *
   dim3 sgrid(dgc_div_up(lanes, 128), NS);
   latch_seg_kernel<<<sgrid, 128, 0, ctx->stream>>>(last, lanes, NC, NS, seg_chunk, seg_off);
   DGC_LAUNCHED(ctx, "latch_segments");
-  latch_seg_carry_kernel<<<dgc_div_up(lanes, 128), 128, 0, ctx->stream>>>(seg_chunk, seg_off, lanes, NS);
-  DGC_LAUNCHED(ctx, "latch_segment_carry");
   latch_carry_kernel<<<sgrid, 128, 0, ctx->stream>>>(last, src_chunk, seg_chunk, seg_off, lanes, NC);
   DGC_LAUNCHED(ctx, "latch_carry");
   const bool quad = (lanes & 3) == 0 &&

@@ -115,3 +115,17 @@ def test_many_copies_in_one_launch(ctx):
                                     (C.c_uint64 * len(sizes))(*sizes)))
     for n, o, s, d in zip(sizes, off, src, dst):
         assert torch.equal(d[o:o + n], s[o:o + n]) and float(d[:o].abs().sum()) + float(d[o + n:].abs().sum()) == 0.0
+
+
+# the trigger a segment of 4096 frames starts from: many segments back, the very first frame, none at all
+@pytest.mark.parametrize("T,W,triggers", [(70001, 3, [100, 69000]), (70001, 4, [0]), (40000, 5, []), (4097, 8, [4095, 4096])])
+def test_latch_far_triggers(ctx, T, W, triggers):
+    g = torch.Generator().manual_seed(T + W)
+    value, cond = torch.randn(T, W, generator=g), torch.zeros(T)
+    cond[triggers] = 1.0
+    state = torch.randn(W, generator=g)
+    src = torch.cummax(torch.where(cond > 0, torch.arange(T), torch.full((T,), -1)), 0).values
+    want = torch.where(src[:, None] >= 0, value[src.clamp(min=0)], state)
+    held = state.cuda()
+    assert torch.equal(ctx.latch(value.cuda(), cond.cuda(), state=held).cpu(), want)
+    assert torch.equal(held.cpu(), want[-1])
