@@ -292,6 +292,7 @@ namespace {
 // waits on an mbarrier that nothing ever arrives on, with the library's bounded wait cut down to `polls`:
 // the wait gives up, the kernel records status 201 (the code of an expired pipeline wait) and returns
 __global__ void selftest_expired_wait_kernel(uint32_t polls, int32_t *status) {
+  dgc_after_previous();
   __shared__ __align__(8) uint64_t bar;
   if (threadIdx.x == 0) dgtma::mbar_init(&bar, 1);
   __syncthreads();
@@ -314,6 +315,7 @@ __global__ void selftest_expired_wait_kernel(uint32_t polls, int32_t *status) {
 }
 // keeps one thread busy for about `us` microseconds of the global timer (capped by the caller)
 __global__ void selftest_busy_kernel(unsigned long long us) {
+  dgc_after_previous();
   unsigned long long t0, t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
   do {
@@ -325,7 +327,7 @@ __global__ void selftest_busy_kernel(unsigned long long us) {
 DGC_EXPORT int32_t dgc_selftest_expired_wait(dgc_ctx *ctx, uint32_t polls) {
   if (!ctx) return DGC_ERR_INVALID;
   DGC_REQUIRE(ctx, polls >= 1 && polls <= (1u << 20), "polls must be in 1 .. 2^20");
-  selftest_expired_wait_kernel<<<1, 32, 0, ctx->stream>>>(polls, ctx->status_dev);
+  dgc_launch(selftest_expired_wait_kernel, 1, 32, 0, ctx->stream, polls, ctx->status_dev);
   DGC_LAUNCHED(ctx, "selftest_expired_wait");
   return DGC_OK;
 }
@@ -333,7 +335,7 @@ DGC_EXPORT int32_t dgc_selftest_expired_wait(dgc_ctx *ctx, uint32_t polls) {
 DGC_EXPORT int32_t dgc_selftest_busy(dgc_ctx *ctx, uint32_t milliseconds) {
   if (!ctx) return DGC_ERR_INVALID;
   DGC_REQUIRE(ctx, milliseconds >= 1 && milliseconds <= 500, "milliseconds must be in 1 .. 500");
-  selftest_busy_kernel<<<1, 1, 0, ctx->stream>>>((unsigned long long)milliseconds * 1000ull);
+  dgc_launch(selftest_busy_kernel, 1, 1, 0, ctx->stream, (unsigned long long)milliseconds * 1000ull);
   DGC_LAUNCHED(ctx, "selftest_busy");
   return DGC_OK;
 }
@@ -417,6 +419,7 @@ __device__ __forceinline__ float sanitize_bits(float v) {
 // (in and out may be the same buffer: no restrict, every element is read before it is written by the same thread)
 __global__ void __launch_bounds__(256) sanitize_kernel(const float *in, float *out,
                                                        uint64_t n, uint64_t head, int vec_ok) {
+  dgc_after_previous();
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (uint64_t)gridDim.x * blockDim.x;
   if (!vec_ok) {
     for (uint64_t i = tid; i < n; i += nth) out[i] = sanitize_bits(in[i]);
@@ -457,7 +460,7 @@ DGC_EXPORT int32_t dgc_sanitize(dgc_ctx *ctx, const float *in_dev, uint64_t n, f
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   uint64_t want = dgc_div_up((int64_t)((n >> 2) + 1), 256);
   int grid = (int)(want < (uint64_t)sms * 8 ? want : (uint64_t)sms * 8);
-  sanitize_kernel<<<grid, 256, 0, ctx->stream>>>(in_dev, out_dev, n, head, vec_ok);
+  dgc_launch(sanitize_kernel, grid, 256, 0, ctx->stream, in_dev, out_dev, n, head, vec_ok);
   DGC_LAUNCHED(ctx, "sanitize");
   return DGC_OK;
 }
@@ -472,6 +475,7 @@ constexpr int RF_SEG = 256;   // frames per segment
 
 __global__ void reduce_frames_seg_kernel(const float *__restrict__ x, int64_t T, int64_t E, int NS,
                                          double *__restrict__ part /* [NS][E] */) {
+  dgc_after_previous();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int sgm = blockIdx.y;
   if (e >= E) return;
@@ -491,6 +495,7 @@ __global__ void reduce_frames_seg_kernel(const float *__restrict__ x, int64_t T,
 
 __global__ void reduce_frames_sum_kernel(const double *__restrict__ part, int64_t E, int NS, float scale, int accumulate,
                                          float *__restrict__ out) {
+  dgc_after_previous();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= E) return;
   double acc = 0.0;
@@ -511,9 +516,9 @@ DGC_EXPORT int32_t dgc_reduce_frames(dgc_ctx *ctx, const float *x_dev, int64_t T
   float *scr = dgc_ctx_scratch(ctx, 2ull * (uint64_t)NS * (uint64_t)E + 4);
   if (!scr) return DGC_ERR_OOM;
   double *part = reinterpret_cast<double *>(scr);
-  reduce_frames_seg_kernel<<<dim3((unsigned)((E + 127) / 128), NS), 128, 0, ctx->stream>>>(x_dev, T, E, NS, part);
+  dgc_launch(reduce_frames_seg_kernel, dim3((unsigned)((E + 127) / 128), NS), 128, 0, ctx->stream, x_dev, T, E, NS, part);
   DGC_LAUNCHED(ctx, "reduce_frames_segments");
-  reduce_frames_sum_kernel<<<(unsigned)((E + 127) / 128), 128, 0, ctx->stream>>>(part, E, NS, scale, accumulate, out_dev);
+  dgc_launch(reduce_frames_sum_kernel, (unsigned)((E + 127) / 128), 128, 0, ctx->stream, part, E, NS, scale, accumulate, out_dev);
   DGC_LAUNCHED(ctx, "reduce_frames_sum");
   return DGC_OK;
 }

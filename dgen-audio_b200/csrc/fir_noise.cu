@@ -20,6 +20,7 @@ __global__ void __launch_bounds__(NTH, 4)
 fir_noise_kernel(dgc_fir_params prm, const float2 *__restrict__ rowtab, const float *__restrict__ noise,
                  const float *__restrict__ taps_tab, const float *__restrict__ ngain, float *__restrict__ audio,
                  int max_rows, int32_t *status) {
+  dgc_after_previous();
   extern __shared__ float sh[];
   const int B = prm.B, T = prm.T, F = prm.F, NT = prm.taps;
   constexpr int TILE = NTH * SPT;
@@ -225,6 +226,7 @@ __global__ void __launch_bounds__(NTH, RB ? RB : (SPT == 8 ? 768 : 512) / NTH)
 fir_noise8_kernel(dgc_fir_params prm, const float2 *__restrict__ rowtab, const float *__restrict__ noise,
                   const float *__restrict__ taps_tab, const float *__restrict__ ngain, float *__restrict__ audio,
                   int max_rows, int NTP, int32_t *status) {
+  dgc_after_previous();
   extern __shared__ __align__(16) float sh[];
   constexpr int TILE = NTH * SPT, GROUPS = NTH / 8;
   const int B = prm.B, T = prm.T, F = prm.F, NT = prm.taps;
@@ -487,6 +489,7 @@ __host__ __device__ constexpr int tmap_stride(int K) { return ((K + 3) & ~3) % 8
 
 __global__ void __launch_bounds__(256, 2)
 tap_map_tile_kernel(const float *__restrict__ A, const float *__restrict__ W, int M, int N, int K, float *__restrict__ C) {
+  dgc_after_previous();
   extern __shared__ __align__(16) float tmap_sh[];
   const int tid = threadIdx.x, m0 = blockIdx.y * 128, n0 = blockIdx.x * 128;
   // columns of this tile; a remainder of at most TMAP_NARROW columns behind the last full tile (N = 257 = 2 x 128 + 1)
@@ -585,6 +588,7 @@ constexpr int BT_ROWS = 64, BT_TAPS = 32, BT_DEPTH = 72, BT_STRIDE = BT_ROWS + 4
 __global__ void __launch_bounds__(256)
 bands_to_taps_kernel(const float *__restrict__ bands, const float *__restrict__ w, int rows, int nb, int nt,
                      float *__restrict__ out) {
+  dgc_after_previous();
   __shared__ float wsh[BT_TAPS][BT_DEPTH | 1];
   __shared__ __align__(16) float bsh[BT_DEPTH][BT_STRIDE];   // row index fastest
   const int n0 = blockIdx.y * BT_TAPS, r0 = blockIdx.x * BT_ROWS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -648,9 +652,8 @@ DGC_EXPORT int32_t dgc_fir_noise(dgc_ctx *ctx, const dgc_fir_params *p, const fl
     if (smem > 200 * 1024) return DGC_ERR_UNSUPPORTED;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "fir smem opt-in: %s", cudaGetErrorString(e));
-    kern<<<dim3(dgc_div_up(p->T, tile), p->B), nth, smem, ctx->stream>>>(*p, play, noise_dev, taps_dev,
-                                                                          noise_gain_dev, audio_dev, max_rows,
-                                                                          ctx->status_dev);
+    dgc_launch(kern, dim3(dgc_div_up(p->T, tile), p->B), nth, smem, ctx->stream, *p, play, noise_dev, taps_dev, noise_gain_dev,
+               audio_dev, max_rows, ctx->status_dev);
     ctx->launches++;
     return dgc_check_launch(ctx, "fir_noise");
   };
@@ -679,8 +682,8 @@ DGC_EXPORT int32_t dgc_fir_noise(dgc_ctx *ctx, const dgc_fir_params *p, const fl
       if (smem > 160 * 1024) return DGC_ERR_UNSUPPORTED;
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "fir smem opt-in: %s", cudaGetErrorString(e));
-      kern<<<dim3(dgc_div_up(p->T, tile), p->B), nth, smem, ctx->stream>>>(*p, play, noise_dev, taps_dev, noise_gain_dev,
-                                                                            audio_dev, max_rows, NTP, ctx->status_dev);
+      dgc_launch(kern, dim3(dgc_div_up(p->T, tile), p->B), nth, smem, ctx->stream, *p, play, noise_dev, taps_dev, noise_gain_dev,
+                 audio_dev, max_rows, NTP, ctx->status_dev);
       ctx->launches++;
       return dgc_check_launch(ctx, "fir_noise8");
     };
@@ -743,8 +746,8 @@ DGC_EXPORT int32_t dgc_bands_to_taps(dgc_ctx *ctx, const float *bands_dev, const
     DGC_CUDA(ctx, cudaFuncSetAttribute(tap_map_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int rem = taps % 128;
     const int ntx = (taps >= 128 && rem > 0 && rem <= TMAP_NARROW) ? taps / 128 : dgc_div_up(taps, 128);
-    tap_map_tile_kernel<<<dim3(ntx, dgc_div_up(rows, 128)), 256, smem, ctx->stream>>>(bands_dev, w_dev, rows, taps,
-                                                                                     nbands, taps_dev);
+    dgc_launch(tap_map_tile_kernel, dim3(ntx, dgc_div_up(rows, 128)), 256, smem, ctx->stream, bands_dev, w_dev, rows, taps,
+               nbands, taps_dev);
     DGC_LAUNCHED(ctx, "tap_map_tile");
     return DGC_OK;
   }
@@ -755,7 +758,7 @@ DGC_EXPORT int32_t dgc_bands_to_taps(dgc_ctx *ctx, const float *bands_dev, const
   }
   const dim3 grid(dgc_div_up(rows, BT_ROWS), dgc_div_up(taps, BT_TAPS));
   DGC_REQUIRE(ctx, grid.y <= 65535, "too many taps");
-  bands_to_taps_kernel<<<grid, 256, 0, ctx->stream>>>(bands_dev, w_dev, rows, nbands, taps, taps_dev);
+  dgc_launch(bands_to_taps_kernel, grid, 256, 0, ctx->stream, bands_dev, w_dev, rows, nbands, taps, taps_dev);
   DGC_LAUNCHED(ctx, "bands_to_taps");
   return DGC_OK;
 }

@@ -23,6 +23,7 @@ template <bool TA, bool TB, int EPI>
 __global__ void __launch_bounds__(256)
 sgemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const float *__restrict__ bias, int M, int N,
              int K, int k_per_split, float *__restrict__ C) {
+  dgc_after_previous();
   __shared__ float As[BK][BM + 4];
   __shared__ float Bs[BK][BN + 4];
   const int tid = threadIdx.x;
@@ -102,6 +103,7 @@ sgemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const flo
 
 // C[m][n] = sum_z part[z][m][n], z ascending: fixed order, bit-reproducible
 __global__ void splitk_reduce_kernel(const float *__restrict__ part, size_t mn, int splits, float *__restrict__ C) {
+  dgc_after_previous();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= mn) return;
   float acc = 0.0f;
@@ -166,8 +168,8 @@ int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dgtc::SK::SMEM);
     if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));
     ctx->gemm_paths[2]++;
-    kern<<<nblk * per, dgtc::SK::THREADS_ALL, dgtc::SK::SMEM, ctx->stream>>>(A, B, M, N, K, nblk, n_extra, per, C,
-                                                                             ctx->status_dev);
+    dgc_launch(kern, nblk * per, dgtc::SK::THREADS_ALL, dgtc::SK::SMEM, ctx->stream, A, B, M, N, K, nblk, n_extra, per, C,
+               ctx->status_dev);
     return DGC_OK;
   }
   const int bm = tc ? dgtc::TBM : BM, bn = wide ? 256 : (tc ? dgtc::TBN : BN);
@@ -202,7 +204,7 @@ int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *
     constexpr int SM = dgtc::KK<BKV, SWV, dgtc::TBN>::SMEM;                                                         \
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);                    \
     if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));     \
-    kern<<<grid, dgtc::KK_THREADS, SM, ctx->stream>>>(A, B, bias, M, N, K, kps, dst, splits == 1 ? Ct : nullptr,    \
+    dgc_launch(kern, grid, dgtc::KK_THREADS, SM, ctx->stream, A, B, bias, M, N, K, kps, dst, splits == 1 ? Ct : nullptr,    \
                                                    ctx->status_dev);                                                \
   } while (0)
     if (kk4) {
@@ -210,14 +212,14 @@ int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *
       constexpr int SM = dgtc::KK<16, true, dgtc::TBN>::SMEM;
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
       if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));
-      kern<<<grid, dgtc::KK_THREADS, SM, ctx->stream>>>(A, B, nullptr, M, N, K, kps, dst, nullptr, ctx->status_dev);
+      dgc_launch(kern, grid, dgtc::KK_THREADS, SM, ctx->stream, A, B, nullptr, M, N, K, kps, dst, nullptr, ctx->status_dev);
     } else if (wide) {
       auto kern = dgtc::tc_gemm_kk_kernel<EPI, 16, true, 256>;
       constexpr int SM = dgtc::KK<16, true, 256>::SMEM;
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
       if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));
-      kern<<<grid, dgtc::KK_THREADS, SM, ctx->stream>>>(A, B, bias, M, N, K, kps, dst, splits == 1 ? Ct : nullptr,
-                                                         ctx->status_dev);
+      dgc_launch(kern, grid, dgtc::KK_THREADS, SM, ctx->stream, A, B, bias, M, N, K, kps, dst, splits == 1 ? Ct : nullptr,
+                 ctx->status_dev);
     } else if (kk_bk == 16 || kk_bk == 256) DGC_KK_LAUNCH(16, true);
     else if (kk_bk == 17) DGC_KK_LAUNCH(16, false);
     else if (kk_bk == 33) DGC_KK_LAUNCH(32, false);
@@ -240,22 +242,23 @@ int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *
     else if (fits(128, 64)) kern = dgtc::tc_gemm_kernel<!TA, TB, EPI, 128, 64>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dgtc::SMEM_BYTES);
     if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));
-    kern<<<grid, dgtc::THREADS + 32, dgtc::SMEM_BYTES, ctx->stream>>>(A, B, bias, M, N, K, kps, dst,
-                                                                              splits == 1 ? Ct : nullptr, ctx->status_dev);
+    dgc_launch(kern, grid, dgtc::THREADS + 32, dgtc::SMEM_BYTES, ctx->stream, A, B, bias, M, N, K, kps, dst,
+               splits == 1 ? Ct : nullptr, ctx->status_dev);
     if (ct_written) *ct_written = Ct && splits == 1;
   } else {
-    sgemm_kernel<TA, TB, EPI><<<grid, 256, 0, ctx->stream>>>(A, B, bias, M, N, K, kps, dst);
+    dgc_launch(sgemm_kernel<TA, TB, EPI>, grid, 256, 0, ctx->stream, A, B, bias, M, N, K, kps, dst);
   }
   if (splits > 1) {
     ctx->launches++;
     size_t mn = (size_t)M * N;
-    splitk_reduce_kernel<<<dgc_div_up((int64_t)mn, 256), 256, 0, ctx->stream>>>(dst, mn, splits, C);
+    dgc_launch(splitk_reduce_kernel, dgc_div_up((int64_t)mn, 256), 256, 0, ctx->stream, dst, mn, splits, C);
   }
   return DGC_OK;
 }
 
 // out[c][r] = in[r][c] (small weight matrices only), 32 x 32 tiles through shared memory
 __global__ void transpose_kernel(const float *__restrict__ in, int R, int Cc, float *__restrict__ out) {
+  dgc_after_previous();
   __shared__ float t[32][33];
   int c = blockIdx.x * 32 + threadIdx.x, r0 = blockIdx.y * 32;
   for (int i = threadIdx.y; i < 32; i += 8)
@@ -287,6 +290,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(256)
 act_bwd_t_kernel(const float *__restrict__ dC, const float *__restrict__ Cv, int M, int N, int act,
                  float *__restrict__ dZ, float *__restrict__ dZt) {
+  dgc_after_previous();
   __shared__ float t[TT][TT + 1];
   const int n0 = blockIdx.x * TT, m0 = blockIdx.y * TT;
   if (VEC) {
@@ -339,6 +343,7 @@ act_bwd_t_kernel(const float *__restrict__ dC, const float *__restrict__ Cv, int
 // dZ = dC * (1 - C^2) in place-compatible form (tanh'), or copy when act == 0
 __global__ void act_bwd_kernel(const float *__restrict__ dC, const float *__restrict__ Cv, size_t n, int act,
                                float *__restrict__ dZ) {
+  dgc_after_previous();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float g = dC[i];
@@ -352,6 +357,7 @@ __global__ void act_bwd_kernel(const float *__restrict__ dC, const float *__rest
 // the same, four elements per thread (n a multiple of 4, 16-byte aligned buffers)
 __global__ void act_bwd4_kernel(const float4 *__restrict__ dC, const float4 *__restrict__ Cv, size_t n4, int act,
                                 float4 *__restrict__ dZ) {
+  dgc_after_previous();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n4) return;
   float4 g = dC[i];
@@ -397,6 +403,7 @@ template <int KK, int EPI>
 __global__ void __launch_bounds__(256)
 smallk_fwd_kernel(const float *__restrict__ A, const float *__restrict__ W, const float *__restrict__ bias, int M, int N,
                   float *__restrict__ C) {
+  dgc_after_previous();
   const int nq = N >> 2;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)M * nq) return;
@@ -410,6 +417,7 @@ template <int KK, int EPI>
 __global__ void __launch_bounds__(256)
 smallk_fwd_t_kernel(const float *__restrict__ A, const float *__restrict__ W, const float *__restrict__ bias, int M, int N,
                     float *__restrict__ C, float *__restrict__ Ct) {
+  dgc_after_previous();
   __shared__ float t[TT][TT + 1];
   const int n0 = blockIdx.x * TT, m0 = blockIdx.y * TT, n = (threadIdx.x & 15) * 4;
   if (n0 + n < N) {
@@ -454,6 +462,7 @@ __device__ __forceinline__ void sum_rows(const float *__restrict__ column, int N
 template <int KK>
 __global__ void __launch_bounds__(256)
 smallk_grad_kernel(const float *__restrict__ A, const float *__restrict__ dZ, int M, int N, float *__restrict__ part) {
+  dgc_after_previous();
   __shared__ float sh[KK + 1][8][33];
   __shared__ float as[1024 * KK];          // the chunk's rows of A: one coalesced read, then broadcast loads
   const int lane = threadIdx.x & 31, col = blockIdx.x * 32 + lane, rg = threadIdx.x >> 5;
@@ -487,6 +496,7 @@ smallk_grad_kernel(const float *__restrict__ A, const float *__restrict__ dZ, in
 // db (may be null) and dW from the chunk sums, chunks in index order
 __global__ void smallk_grad_reduce_kernel(const float *__restrict__ part, int chunks, int KK, int N, float *__restrict__ db,
                                           float *__restrict__ dW) {
+  dgc_after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (KK + 1) * N) return;
   const int q = i / N, col = i - q * N;
@@ -502,6 +512,7 @@ __global__ void smallk_grad_reduce_kernel(const float *__restrict__ part, int ch
 // part[chunk][n]; stage 2 adds the chunks in index order: bit-reproducible.
 __global__ void __launch_bounds__(256)
 bias_grad_kernel(const float *__restrict__ dZ, int M, int N, float *__restrict__ part) {
+  dgc_after_previous();
   __shared__ float sh[8][33];
   const int col = blockIdx.x * 32 + (threadIdx.x & 31), rg = threadIdx.x >> 5;
   const int m_begin = blockIdx.y * 1024, m_end = min(M, m_begin + 1024);
@@ -519,6 +530,7 @@ bias_grad_kernel(const float *__restrict__ dZ, int M, int N, float *__restrict__
 }
 
 __global__ void bias_grad_reduce_kernel(const float *__restrict__ part, int chunks, int N, float *__restrict__ db) {
+  dgc_after_previous();
   int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= N) return;
   float t = 0.0f;
@@ -529,6 +541,7 @@ __global__ void bias_grad_reduce_kernel(const float *__restrict__ part, int chun
 __global__ void adam_kernel(float *__restrict__ theta, const float *__restrict__ g, float *__restrict__ m,
                             float *__restrict__ v, size_t n, float lr, float b1, float b2, float eps, float c1,
                             float c2) {
+  dgc_after_previous();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   // operation order of Optimizers.swift:188-203
@@ -579,7 +592,8 @@ DGC_EXPORT int32_t dgc_linear_fwd(dgc_ctx *ctx, const float *a_dev, const float 
       DGC_CUDA(ctx, cudaMalloc(&ctx->wt_buf, (size_t)K * N * sizeof(float)));
       ctx->wt_floats = (uint64_t)K * N;
     }
-    transpose_kernel<<<dim3(dgc_div_up(N, 32), dgc_div_up(K, 32)), dim3(32, 8), 0, ctx->stream>>>(w_dev, K, N, ctx->wt_buf);
+    dgc_launch(transpose_kernel, dim3(dgc_div_up(N, 32), dgc_div_up(K, 32)), dim3(32, 8), 0, ctx->stream, w_dev, K, N,
+               ctx->wt_buf);
     DGC_LAUNCHED(ctx, "transpose_w");
     if (act == 1) rc = launch_sgemm<false, true, 2>(ctx, a_dev, ctx->wt_buf, bias_dev, M, N, K, c_dev, ct_dev, &ct_done);
     else if (bias_dev) rc = launch_sgemm<false, true, 1>(ctx, a_dev, ctx->wt_buf, bias_dev, M, N, K, c_dev, ct_dev, &ct_done);
@@ -591,10 +605,11 @@ DGC_EXPORT int32_t dgc_linear_fwd(dgc_ctx *ctx, const float *a_dev, const float 
 #define DGC_SMALLK_EPI(KKV, EPI, BIAS)                                                                                \
   do {                                                                                                               \
     if (ct_done)                                                                                                     \
-      smallk_fwd_t_kernel<KKV, EPI><<<dim3(dgc_div_up(N, TT), dgc_div_up(M, TT)), 256, 0, ctx->stream>>>(            \
+      dgc_launch(smallk_fwd_t_kernel<KKV, EPI>, dim3(dgc_div_up(N, TT), dgc_div_up(M, TT)), 256, 0, ctx->stream, \
           a_dev, w_dev, BIAS, M, N, c_dev, ct_dev);                                                                  \
     else                                                                                                             \
-      smallk_fwd_kernel<KKV, EPI><<<(unsigned)dgc_div_up(work, 256), 256, 0, ctx->stream>>>(a_dev, w_dev, BIAS, M, N, c_dev); \
+      dgc_launch(smallk_fwd_kernel<KKV, EPI>, (unsigned)dgc_div_up(work, 256), 256, 0, ctx->stream, a_dev, w_dev, BIAS, M, N, \
+                 c_dev);                                                                                              \
   } while (0)
 #define DGC_SMALLK_FWD(KKV)                                                                                           \
   do {                                                                                                               \
@@ -616,7 +631,7 @@ DGC_EXPORT int32_t dgc_linear_fwd(dgc_ctx *ctx, const float *a_dev, const float 
   if (rc != DGC_OK) return rc;
   DGC_LAUNCHED(ctx, "linear_fwd");
   if (ct_dev && !ct_done) {  // the matmul kernel that ran has no transposed store: one extra pass
-    transpose_kernel<<<dim3(dgc_div_up(N, 32), dgc_div_up(M, 32)), dim3(32, 8), 0, ctx->stream>>>(c_dev, M, N, ct_dev);
+    dgc_launch(transpose_kernel, dim3(dgc_div_up(N, 32), dgc_div_up(M, 32)), dim3(32, 8), 0, ctx->stream, c_dev, M, N, ct_dev);
     DGC_LAUNCHED(ctx, "transpose_c");
   }
   return DGC_OK;
@@ -646,15 +661,16 @@ DGC_EXPORT int32_t dgc_linear_bwd(dgc_ctx *ctx, const float *a_dev, const float 
     }
     const bool vec = (N & 3) == 0 && ((((uintptr_t)dc_dev) | ((uintptr_t)dz_dev) | (act == 1 ? (uintptr_t)c_dev : 0)) & 15) == 0;
     auto kern = vec ? act_bwd_t_kernel<true> : act_bwd_t_kernel<false>;
-    kern<<<dim3(dgc_div_up(N, TT), dgc_div_up(M, TT)), 256, 0, ctx->stream>>>(dc_dev, c_dev, M, N, act, dz_dev, ctx->dzt_buf);
+    dgc_launch(kern, dim3(dgc_div_up(N, TT), dgc_div_up(M, TT)), 256, 0, ctx->stream, dc_dev, c_dev, M, N, act, dz_dev,
+               ctx->dzt_buf);
   } else {
     const bool vec = (n & 3) == 0 && ((((uintptr_t)dc_dev) | ((uintptr_t)dz_dev) | (act == 1 ? (uintptr_t)c_dev : 0)) & 15) == 0;
     if (vec)
-      act_bwd4_kernel<<<dgc_div_up((int64_t)(n / 4), 256), 256, 0, ctx->stream>>>(
-          reinterpret_cast<const float4 *>(dc_dev), reinterpret_cast<const float4 *>(c_dev), n / 4, act,
-          reinterpret_cast<float4 *>(dz_dev));
+      dgc_launch(act_bwd4_kernel, dgc_div_up((int64_t)(n / 4), 256), 256, 0, ctx->stream,
+                 reinterpret_cast<const float4 *>(dc_dev), reinterpret_cast<const float4 *>(c_dev), n / 4, act,
+                 reinterpret_cast<float4 *>(dz_dev));
     else
-      act_bwd_kernel<<<dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream>>>(dc_dev, c_dev, n, act, dz_dev);
+      dgc_launch(act_bwd_kernel, dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream, dc_dev, c_dev, n, act, dz_dev);
   }
   DGC_LAUNCHED(ctx, "act_bwd");
   const bool smallk = K <= 4;   // bias and weight gradient from one pass over dZ
@@ -663,20 +679,21 @@ DGC_EXPORT int32_t dgc_linear_bwd(dgc_ctx *ctx, const float *a_dev, const float 
     float *part = dgc_ctx_scratch(ctx, (uint64_t)chunks * (K + 1) * N + 4);
     if (!part) return DGC_ERR_OOM;
     const dim3 grid(dgc_div_up(N, 32), chunks);
-    if (K == 1) smallk_grad_kernel<1><<<grid, 256, 0, ctx->stream>>>(a_dev, dz_dev, M, N, part);
-    else if (K == 2) smallk_grad_kernel<2><<<grid, 256, 0, ctx->stream>>>(a_dev, dz_dev, M, N, part);
-    else if (K == 3) smallk_grad_kernel<3><<<grid, 256, 0, ctx->stream>>>(a_dev, dz_dev, M, N, part);
-    else smallk_grad_kernel<4><<<grid, 256, 0, ctx->stream>>>(a_dev, dz_dev, M, N, part);
+    if (K == 1) dgc_launch(smallk_grad_kernel<1>, grid, 256, 0, ctx->stream, a_dev, dz_dev, M, N, part);
+    else if (K == 2) dgc_launch(smallk_grad_kernel<2>, grid, 256, 0, ctx->stream, a_dev, dz_dev, M, N, part);
+    else if (K == 3) dgc_launch(smallk_grad_kernel<3>, grid, 256, 0, ctx->stream, a_dev, dz_dev, M, N, part);
+    else dgc_launch(smallk_grad_kernel<4>, grid, 256, 0, ctx->stream, a_dev, dz_dev, M, N, part);
     DGC_LAUNCHED(ctx, "smallk_grad");
-    smallk_grad_reduce_kernel<<<dgc_div_up((K + 1) * N, 128), 128, 0, ctx->stream>>>(part, chunks, K, N, dbias_dev, dw_dev);
+    dgc_launch(smallk_grad_reduce_kernel, dgc_div_up((K + 1) * N, 128), 128, 0, ctx->stream, part, chunks, K, N, dbias_dev,
+               dw_dev);
     DGC_LAUNCHED(ctx, "smallk_grad_reduce");
   } else if (dbias_dev) {
     const int chunks = dgc_div_up(M, 1024);
     float *part = dgc_ctx_scratch(ctx, (uint64_t)chunks * N + 4);
     if (!part) return DGC_ERR_OOM;
-    bias_grad_kernel<<<dim3(dgc_div_up(N, 32), chunks), 256, 0, ctx->stream>>>(dz_dev, M, N, part);
+    dgc_launch(bias_grad_kernel, dim3(dgc_div_up(N, 32), chunks), 256, 0, ctx->stream, dz_dev, M, N, part);
     DGC_LAUNCHED(ctx, "bias_grad");
-    bias_grad_reduce_kernel<<<dgc_div_up(N, 128), 128, 0, ctx->stream>>>(part, chunks, N, dbias_dev);
+    dgc_launch(bias_grad_reduce_kernel, dgc_div_up(N, 128), 128, 0, ctx->stream, part, chunks, N, dbias_dev);
     DGC_LAUNCHED(ctx, "bias_grad_reduce");
   }
   // dW[K][N] = A^T[K][M] * dZ[M][N]
@@ -701,8 +718,8 @@ DGC_EXPORT int32_t dgc_adam_step(dgc_ctx *ctx, float *theta_dev, const float *gr
   if (n == 0) return DGC_OK;
   // bias corrections as the reference computes them: 1 - pow(beta, Float(t)) in single precision
   float c1 = 1.0f - powf(beta1, (float)t), c2 = 1.0f - powf(beta2, (float)t);
-  adam_kernel<<<dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream>>>(theta_dev, grad_dev, m_dev, v_dev, n, lr, beta1,
-                                                                    beta2, eps, c1, c2);
+  dgc_launch(adam_kernel, dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream, theta_dev, grad_dev, m_dev, v_dev, n, lr, beta1,
+             beta2, eps, c1, c2);
   DGC_LAUNCHED(ctx, "adam");
   return DGC_OK;
 }
@@ -712,6 +729,7 @@ DGC_EXPORT int32_t dgc_adam_step(dgc_ctx *ctx, float *theta_dev, const float *gr
 // rounded: the correctly rounded single-precision power), the update kernel reads them.
 namespace {
 __global__ void adam_tick_kernel(int32_t *t_dev, float beta1, float beta2, float *corr) {
+  dgc_after_previous();
   const int32_t t = *t_dev + 1;
   *t_dev = t;
   corr[0] = 1.0f - (float)pow((double)beta1, (double)t);
@@ -721,6 +739,7 @@ __global__ void adam_tick_kernel(int32_t *t_dev, float beta1, float beta2, float
 __global__ void adam_counted_kernel(float *__restrict__ theta, const float *__restrict__ g, float *__restrict__ m,
                                     float *__restrict__ v, uint64_t n, float lr, float b1, float b2, float eps,
                                     const float *__restrict__ corr) {
+  dgc_after_previous();
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float c1 = corr[0], c2 = corr[1];
@@ -739,11 +758,11 @@ DGC_EXPORT int32_t dgc_adam_step_counted(dgc_ctx *ctx, float *theta_dev, const f
                                          float beta1, float beta2, float eps) {
   if (!ctx) return DGC_ERR_INVALID;
   DGC_REQUIRE(ctx, theta_dev && grad_dev && m_dev && v_dev && t_dev && corr_dev, "null pointer");
-  adam_tick_kernel<<<1, 1, 0, ctx->stream>>>(t_dev, beta1, beta2, corr_dev);
+  dgc_launch(adam_tick_kernel, 1, 1, 0, ctx->stream, t_dev, beta1, beta2, corr_dev);
   DGC_LAUNCHED(ctx, "adam_tick");
   if (n == 0) return DGC_OK;
-  adam_counted_kernel<<<dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream>>>(theta_dev, grad_dev, m_dev, v_dev, n, lr,
-                                                                            beta1, beta2, eps, corr_dev);
+  dgc_launch(adam_counted_kernel, dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream, theta_dev, grad_dev, m_dev, v_dev, n, lr,
+             beta1, beta2, eps, corr_dev);
   DGC_LAUNCHED(ctx, "adam");
   return DGC_OK;
 }

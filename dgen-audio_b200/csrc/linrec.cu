@@ -139,6 +139,7 @@ template <bool REV>
 __global__ void __launch_bounds__(OP_THREADS, OP_BLOCKS)
 onepole_kernel(const float *x, int B, int T, int NT, const OnepolePowers pw, float *state, float *y,
                unsigned long long *__restrict__ chain, int32_t *status) {
+  dgc_after_previous();
   __shared__ float warp_end[2][OP_WARPS];
   __shared__ float sh_in[2];
   __shared__ uint32_t sh_index[2];
@@ -260,6 +261,7 @@ onepole_kernel(const float *x, int B, int T, int NT, const OnepolePowers pw, flo
 template <bool REV, bool OUT>
 __global__ void __launch_bounds__(OP_THREADS)
 onepole_pass_kernel(const float *x, int T, int NT, const OnepolePowers pw, float *__restrict__ tiles, float *state, float *y) {
+  dgc_after_previous();
   __shared__ float warp_end[OP_WARPS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int b = blockIdx.x / NT, tile = blockIdx.x - b * NT;
@@ -306,6 +308,7 @@ onepole_pass_kernel(const float *x, int T, int NT, const OnepolePowers pw, float
 // The states entering the tiles, in double, a thread per voice with the next end values in flight
 __global__ void __launch_bounds__(32)
 onepole_carry_kernel(float *__restrict__ tiles, int B, int NT, double across, const float *__restrict__ state) {
+  dgc_after_previous();
   constexpr int AHEAD = 32;
   const int b = blockIdx.x * 32 + threadIdx.x;
   if (b >= B) return;
@@ -334,9 +337,9 @@ onepole_carry_kernel(float *__restrict__ tiles, int B, int NT, double across, co
 template <bool REV>
 void onepole_passes(cudaStream_t stream, const float *x, int B, int T, int NT, const OnepolePowers &pw, float *tiles, float *state,
                     float *y) {
-  onepole_pass_kernel<REV, false><<<B * NT, OP_THREADS, 0, stream>>>(x, T, NT, pw, tiles, nullptr, y);
-  onepole_carry_kernel<<<dgc_div_up(B, 32), 32, 0, stream>>>(tiles, B, NT, pw.tile[0], state);
-  onepole_pass_kernel<REV, true><<<B * NT, OP_THREADS, 0, stream>>>(x, T, NT, pw, tiles, state, y);
+  dgc_launch(onepole_pass_kernel<REV, false>, B * NT, OP_THREADS, 0, stream, x, T, NT, pw, tiles, nullptr, y);
+  dgc_launch(onepole_carry_kernel, dgc_div_up(B, 32), 32, 0, stream, tiles, B, NT, pw.tile[0], state);
+  dgc_launch(onepole_pass_kernel<REV, true>, B * NT, OP_THREADS, 0, stream, x, T, NT, pw, tiles, state, y);
 }
 
 template <bool REV>
@@ -359,8 +362,8 @@ int32_t launch_onepole(dgc_ctx *ctx, const float *x, int B, int T, float a, floa
   if (NT > OP_REACH && pw.reach > OP_REACH) return launch_onepole_passes<REV>(ctx, x, B, T, pw, state, y, what);
   unsigned long long *chain = dgc_ctx_chain(ctx, tiles);
   if (!chain) return DGC_ERR_OOM;
-  onepole_kernel<REV><<<(unsigned)(tiles < room ? tiles : room), OP_THREADS, 0, ctx->stream>>>(x, B, T, NT, pw, state, y, chain,
-                                                                        ctx->status_dev);
+  dgc_launch(onepole_kernel<REV>, (unsigned)(tiles < room ? tiles : room), OP_THREADS, 0, ctx->stream, x, B, T, NT, pw, state, y,
+             chain, ctx->status_dev);
   DGC_LAUNCHED(ctx, what);
   return DGC_OK;
 }
@@ -453,6 +456,7 @@ __device__ __noinline__ void biquad_coef(const float *__restrict__ cutoff, const
 }
 __global__ void biquad_coef_kernel(const float *__restrict__ cutoff, const float *__restrict__ q, int L, float gain,
                                    float mode, float *__restrict__ coef) {
+  dgc_after_previous();
   int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l < L) biquad_coef(cutoff, q, l, gain, mode, coef);
 }
@@ -502,6 +506,7 @@ __global__ void __launch_bounds__(BQ_THREADS)
 biquad_fwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, int T, int L, int NC,
                   float *__restrict__ state /* [B][NC][L][2] */, float *__restrict__ y,
                   const float *__restrict__ st0 = nullptr /* [B][4][L]: history cells before the call */) {
+  dgc_after_previous();
   extern __shared__ float sm[];
   const int b = blockIdx.y;
   int c, l;
@@ -553,6 +558,7 @@ __global__ void __launch_bounds__(128)
 biquad_tables_kernel(const float *__restrict__ cutoff, const float *__restrict__ q, int L, float gain, float mode,
                      float *__restrict__ coef, double *__restrict__ trans, float *__restrict__ G,
                      float *__restrict__ hist /* [L][4] */) {
+  dgc_after_previous();
   __shared__ double hys[4][BQ_CHUNK + 2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = blockIdx.x * 4 + warp;
   if (l >= L) return;
@@ -608,6 +614,7 @@ __global__ void __launch_bounds__(256)
 biquad_fwd4_kernel(const float *__restrict__ x, const float *__restrict__ coef, int B, int T, int L, int NC,
                    float *__restrict__ state /* [B][NC][L][2] */, float *__restrict__ y,
                    const float *__restrict__ st0 = nullptr /* [B][4][L]: history cells before the call */) {
+  dgc_after_previous();
   __shared__ float xs[BQ4_CHUNKS][BQ_CHUNK + 2];
   const int lq = blockIdx.x * blockDim.x + threadIdx.x, cy = threadIdx.y;
   const int c = blockIdx.y * BQ4_CHUNKS + cy, b = blockIdx.z;
@@ -665,6 +672,7 @@ constexpr int BQ_AHEAD = 16;
 __global__ void __launch_bounds__(32)
 biquad_carry_kernel(const double *__restrict__ trans, const float *__restrict__ x, const float *__restrict__ hist, int T, int L,
                     int NC, float2 *__restrict__ state, const float *__restrict__ st0) {
+  dgc_after_previous();
   const int l = blockIdx.x * 32 + threadIdx.x, b = blockIdx.y;
   if (l >= L) return;
   const double m11 = trans[(size_t)l * 4], m12 = trans[(size_t)l * 4 + 1], m21 = trans[(size_t)l * 4 + 2],
@@ -777,6 +785,7 @@ __global__ void __launch_bounds__(BQ_THREADS)
 biquad_bwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, const float *__restrict__ y,
                   const float *__restrict__ tgt, int T, int L, int NC, float gscale,
                   float *__restrict__ rec /* [B][NC][BW_REC][L] */) {
+  dgc_after_previous();
   extern __shared__ float sm[];
   constexpr int G = 16;
   const int b = blockIdx.y;
@@ -844,6 +853,7 @@ constexpr int BQ_RUNS = 16;
 __global__ void __launch_bounds__(32 * BQ_RUNS)
 biquad_bwd_carry_kernel(const float *__restrict__ rec, const float *__restrict__ coef, int L, int NC,
                         double *__restrict__ acc /* [B][L][6] */, float2 *__restrict__ term /* [B][NC][L] or null */) {
+  dgc_after_previous();
   __shared__ double2 ends[BQ_RUNS][32];
   __shared__ double sums[BQ_RUNS][6][32];
   const int l = blockIdx.x * 32 + threadIdx.x, run = threadIdx.y, b = blockIdx.y;
@@ -914,6 +924,7 @@ __global__ void __launch_bounds__(BQ_THREADS)
 biquad_gx_kernel(const float *__restrict__ coef, const float *__restrict__ gy, const float2 *__restrict__ term, int B, int T,
                  int L, int NC,
                  float *__restrict__ part /* [gridDim.x][B][T] */) {
+  dgc_after_previous();
   __shared__ float red[GX_FRAMES][BQ_THREADS + 1];
   const int tid = threadIdx.x, l = blockIdx.x * BQ_THREADS + tid, c = blockIdx.y, b = blockIdx.z;
   const int n0 = c * BQ_CHUNK, len = min(BQ_CHUNK, T - n0);
@@ -970,6 +981,7 @@ biquad_gx_kernel(const float *__restrict__ coef, const float *__restrict__ gy, c
 }
 
 __global__ void sum_partial_rows_kernel(const float *__restrict__ part, int nparts, size_t n, float *__restrict__ out) {
+  dgc_after_previous();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float s = 0.f;
@@ -983,6 +995,7 @@ __global__ void __launch_bounds__(256)
 biquad_bwd_final_kernel(const double *__restrict__ acc, const float *__restrict__ coef, int B, int L,
                         float loss_scale, float *__restrict__ gcut, float *__restrict__ gq,
                         double *__restrict__ lane_loss, unsigned int *__restrict__ ticket, double *__restrict__ loss) {
+  dgc_after_previous();
   const int l = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (l < L) {
     double G[6] = {0, 0, 0, 0, 0, 0};
@@ -1076,6 +1089,7 @@ DGC_EXPORT uint64_t dgc_biquad_scratch_floats(const dgc_biquad_params *p, int32_
 // from the cells as they were
 __global__ void biquad_final_state_kernel(const float *__restrict__ x, const float *__restrict__ y, int B, int T, int L,
                                           float *__restrict__ st) {
+  dgc_after_previous();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= B * L) return;
   const int b = idx / L, l = idx - b * L;
@@ -1131,24 +1145,25 @@ static int32_t biquad_fwd_impl(dgc_ctx *ctx, const dgc_biquad_params *p, const f
   const bool by_matmul = (T % BQ_CHUNK) == 0 && (double)B * NC * L >= (double)(1 << 16) && (((uintptr_t)x_dev) & 15) == 0;
   float *G = by_matmul ? state + ((((size_t)B * NC * L * 2) + 3) & ~(size_t)3) : nullptr;
   float *hist = by_matmul ? G + (size_t)L * 2 * BQ_CHUNK : nullptr;
-  biquad_tables_kernel<<<dgc_div_up(L, 4), 128, 0, ctx->stream>>>(cutoff_dev, q_dev, L, p->gain, p->mode, coef, trans, G, hist);
+  dgc_launch(biquad_tables_kernel, dgc_div_up(L, 4), 128, 0, ctx->stream, cutoff_dev, q_dev, L, p->gain, p->mode, coef, trans, G,
+             hist);
   DGC_LAUNCHED(ctx, "biquad_tables");
   if (by_matmul) {
     rc = dgc_gemm_nt(ctx, x_dev, G, B * NC, 2 * L, BQ_CHUNK, state);
     if (rc != DGC_OK) return rc;
   } else {
-    if (quad) biquad_fwd4_kernel<0><<<grid4, block4, 0, ctx->stream>>>(x_dev, coef, B, T, L, NC, state, nullptr, st0);
-    else biquad_fwd_kernel<0><<<grid, nth, smem, ctx->stream>>>(x_dev, coef, T, L, NC, state, nullptr, st0);
+    if (quad) dgc_launch(biquad_fwd4_kernel<0>, grid4, block4, 0, ctx->stream, x_dev, coef, B, T, L, NC, state, nullptr, st0);
+    else dgc_launch(biquad_fwd_kernel<0>, grid, nth, smem, ctx->stream, x_dev, coef, T, L, NC, state, nullptr, st0);
     DGC_LAUNCHED(ctx, "biquad_fwd_state");
   }
-  biquad_carry_kernel<<<dim3(dgc_div_up(L, 32), B), 32, 0, ctx->stream>>>(trans, x_dev, hist, T, L, NC,
-                                                                         reinterpret_cast<float2 *>(state), st0);
+  dgc_launch(biquad_carry_kernel, dim3(dgc_div_up(L, 32), B), 32, 0, ctx->stream, trans, x_dev, hist, T, L, NC,
+             reinterpret_cast<float2 *>(state), st0);
   DGC_LAUNCHED(ctx, "biquad_carry");
-  if (quad) biquad_fwd4_kernel<1><<<grid4, block4, 0, ctx->stream>>>(x_dev, coef, B, T, L, NC, state, y_dev, st0);
-  else biquad_fwd_kernel<1><<<grid, nth, smem, ctx->stream>>>(x_dev, coef, T, L, NC, state, y_dev, st0);
+  if (quad) dgc_launch(biquad_fwd4_kernel<1>, grid4, block4, 0, ctx->stream, x_dev, coef, B, T, L, NC, state, y_dev, st0);
+  else dgc_launch(biquad_fwd_kernel<1>, grid, nth, smem, ctx->stream, x_dev, coef, T, L, NC, state, y_dev, st0);
   DGC_LAUNCHED(ctx, "biquad_fwd_out");
   if (st0) {
-    biquad_final_state_kernel<<<dgc_div_up(B * L, 128), 128, 0, ctx->stream>>>(x_dev, y_dev, B, T, L, st0);
+    dgc_launch(biquad_final_state_kernel, dgc_div_up(B * L, 128), 128, 0, ctx->stream, x_dev, y_dev, B, T, L, st0);
     DGC_LAUNCHED(ctx, "biquad_final_state");
   }
   return DGC_OK;
@@ -1165,18 +1180,18 @@ static int32_t biquad_backward(dgc_ctx *ctx, const dgc_biquad_params *p, const f
   const size_t rec_n = ((size_t)B * NC * BW_REC * L + 3) & ~(size_t)3;
   double *acc = reinterpret_cast<double *>(rec + rec_n);
   double *lane_loss = acc + (size_t)B * L * 6;
-  biquad_coef_kernel<<<dgc_div_up(L, 32), 32, 0, ctx->stream>>>(cutoff, q, L, p->gain, p->mode, coef);
+  dgc_launch(biquad_coef_kernel, dgc_div_up(L, 32), 32, 0, ctx->stream, cutoff, q, L, p->gain, p->mode, coef);
   DGC_LAUNCHED(ctx, "biquad_coef");
   const int nth = biquad_pairs(L), smem = biquad_stage_bytes(L);
   if (smem > 48 * 1024)
     DGC_CUDA(ctx, cudaFuncSetAttribute(biquad_bwd_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const dim3 grid((unsigned)(((int64_t)NC * L + nth - 1) / nth), B);
-  biquad_bwd_kernel<UP><<<grid, nth, smem, ctx->stream>>>(x, coef, y, up, T, L, NC, gscale, rec);
+  dgc_launch(biquad_bwd_kernel<UP>, grid, nth, smem, ctx->stream, x, coef, y, up, T, L, NC, gscale, rec);
   DGC_LAUNCHED(ctx, "biquad_bwd");
-  biquad_bwd_carry_kernel<<<dim3(dgc_div_up(L, 32), B), dim3(32, BQ_RUNS), 0, ctx->stream>>>(rec, coef, L, NC, acc, term);
+  dgc_launch(biquad_bwd_carry_kernel, dim3(dgc_div_up(L, 32), B), dim3(32, BQ_RUNS), 0, ctx->stream, rec, coef, L, NC, acc, term);
   DGC_LAUNCHED(ctx, "biquad_bwd_carry");
-  biquad_bwd_final_kernel<<<dgc_div_up(L, 8), 256, 0, ctx->stream>>>(acc, coef, B, L, loss_scale, gcut, gq, lane_loss,
-                                                                    dgc_ctx_ticket(ctx), loss);
+  dgc_launch(biquad_bwd_final_kernel, dgc_div_up(L, 8), 256, 0, ctx->stream, acc, coef, B, L, loss_scale, gcut, gq, lane_loss,
+             dgc_ctx_ticket(ctx), loss);
   DGC_LAUNCHED(ctx, "biquad_bwd_final");
   return DGC_OK;
 }
@@ -1203,6 +1218,7 @@ namespace {
 constexpr int OPG_SEGS = 32;
 __global__ void __launch_bounds__(256)
 onepole_ga_kernel(const float *__restrict__ lam, const float *__restrict__ y, int T, double *__restrict__ part) {
+  dgc_after_previous();
   const int b = blockIdx.y, sgm = blockIdx.x;
   const int64_t per = ((int64_t)T + OPG_SEGS - 1) / OPG_SEGS, lo = max((int64_t)1, sgm * per),
                 hi = min((int64_t)T, (sgm + 1) * per);
@@ -1220,6 +1236,7 @@ onepole_ga_kernel(const float *__restrict__ lam, const float *__restrict__ y, in
 }
 
 __global__ void onepole_ga_sum_kernel(const double *__restrict__ part, int B, float *__restrict__ ga) {
+  dgc_after_previous();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   double s = 0.0;
@@ -1246,9 +1263,9 @@ DGC_EXPORT int32_t dgc_onepole_bwd(dgc_ctx *ctx, const float *y_dev, const float
   const int32_t rc = launch_onepole<true>(ctx, gy_dev, B, T, a, nullptr, grad_x_dev, "onepole_bwd");
   if (rc != DGC_OK) return rc;
   if (grad_a_dev) {
-    onepole_ga_kernel<<<dim3(OPG_SEGS, B), 256, 0, ctx->stream>>>(grad_x_dev, y_dev, T, part);
+    dgc_launch(onepole_ga_kernel, dim3(OPG_SEGS, B), 256, 0, ctx->stream, grad_x_dev, y_dev, T, part);
     DGC_LAUNCHED(ctx, "onepole_grad_a");
-    onepole_ga_sum_kernel<<<dgc_div_up(B, 128), 128, 0, ctx->stream>>>(part, B, grad_a_dev);
+    dgc_launch(onepole_ga_sum_kernel, dgc_div_up(B, 128), 128, 0, ctx->stream, part, B, grad_a_dev);
     DGC_LAUNCHED(ctx, "onepole_grad_a_sum");
   }
   return DGC_OK;
@@ -1275,10 +1292,10 @@ DGC_EXPORT int32_t dgc_biquad_bwd(dgc_ctx *ctx, const dgc_biquad_params *p, cons
   if (rc != DGC_OK) return rc;
   if (grad_x_dev) {
     const dim3 grid(dgc_div_up(L, BQ_THREADS), NC, B);
-    biquad_gx_kernel<<<grid, BQ_THREADS, 0, ctx->stream>>>(scr, gy_dev, term, B, T, L, NC, part);
+    dgc_launch(biquad_gx_kernel, grid, BQ_THREADS, 0, ctx->stream, scr, gy_dev, term, B, T, L, NC, part);
     DGC_LAUNCHED(ctx, "biquad_grad_x");
     const size_t n = (size_t)B * T;
-    sum_partial_rows_kernel<<<dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream>>>(part, (int)grid.x, n, grad_x_dev);
+    dgc_launch(sum_partial_rows_kernel, dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream, part, (int)grid.x, n, grad_x_dev);
     DGC_LAUNCHED(ctx, "biquad_grad_x_sum");
   }
   return DGC_OK;
@@ -1372,8 +1389,8 @@ DGC_EXPORT int32_t dgc_onepole_fwd_static(void *cuda_stream, const float *x_dev,
       static_msg(err_buf, err_len, "dgc_onepole_fwd_static: clearing the scratch failed (%lld)", (long long)e);
       return DGC_ERR_CUDA;
     }
-    onepole_kernel<false><<<(unsigned)(tiles < 148 * OP_BLOCKS ? tiles : 148 * OP_BLOCKS), OP_THREADS, 0, st>>>(x_dev, B, T, NT, pw, nullptr,
-                                                                                                               y_dev, scratch, nullptr);
+    dgc_launch(onepole_kernel<false>, (unsigned)(tiles < 148 * OP_BLOCKS ? tiles : 148 * OP_BLOCKS), OP_THREADS, 0, st, x_dev, B,
+               T, NT, pw, nullptr, y_dev, scratch, nullptr);
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) {

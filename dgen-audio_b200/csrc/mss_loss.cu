@@ -122,6 +122,7 @@ constexpr int FWD_SMEM_BYTES = 2 * (LOSS_THREADS / (2048 / 8)) * padded(2048) * 
 
 __global__ void __launch_bounds__(LOSS_THREADS, 6)
 mss_fwd_kernel(const float *__restrict__ pred, const float *__restrict__ target, int B, int T, const FwdDesc d) {
+  dgc_after_previous();
   extern __shared__ float2 fwd_sm[];
   __shared__ float red[LOSS_THREADS / 32];
   int s = 0;
@@ -289,6 +290,7 @@ __global__ void __launch_bounds__(LOSS16_THREADS, TMA ? 6 : 8)
 mss_fwd16_kernel(const float *__restrict__ pred, const float *__restrict__ target,
                  int B, int T, const FwdDesc d, const __grid_constant__ CUtensorMap map_pred,
                  const __grid_constant__ CUtensorMap map_target, int32_t *status) {
+  dgc_after_previous();
   extern __shared__ __align__(128) float2 fwd_sm[];
   __shared__ float red[LOSS16_THREADS / 32];
   __shared__ __align__(8) uint64_t span_bar;
@@ -328,6 +330,7 @@ constexpr int RED_BLOCKS = 256, RED_THREADS = 256;
 __global__ void __launch_bounds__(RED_THREADS)
 mss_reduce_kernel(const float *__restrict__ part, ReduceDesc d, double scale_lin, double scale_log,
                   double *__restrict__ block_sums, unsigned int *__restrict__ ticket, double *__restrict__ out) {
+  dgc_after_previous();
   __shared__ double sh[RED_THREADS];
   __shared__ bool last;
   double acc = 0.0;
@@ -399,6 +402,7 @@ __global__ void __launch_bounds__(LOSS_THREADS, (N >= 256 ? 3 : 4))
 mss_bwd_kernel(const float *__restrict__ pred, const float *__restrict__ target, int B, int T, int hop, int H,
                int S /* windows whose first-covered frames this block owns */, const float *__restrict__ window,
                const float2 *__restrict__ tw, float c_lin, float c_log, int accumulate, float *__restrict__ grad) {
+  dgc_after_previous();
   using Gm = BwdGeom<N>;
   constexpr int G = Gm::G, NF = Gm::NF, WR = Gm::WR;
   extern __shared__ float2 sm2[];
@@ -694,6 +698,7 @@ struct Bwd16Desc {
 __global__ void __launch_bounds__(LOSS16_THREADS, 4)
 mss_bwd16_kernel(const float *__restrict__ pred, const float *__restrict__ target, int B, int T, const Bwd16Desc d, float c_lin,
                  float c_log, int accumulate) {
+  dgc_after_previous();
   extern __shared__ float2 bwd_sm[];
   int s = 0;
   while (s + 1 < d.nscales && (int)blockIdx.x >= d.first_block[s + 1]) ++s;
@@ -711,6 +716,7 @@ mss_bwd16_kernel(const float *__restrict__ pred, const float *__restrict__ targe
 // grad = ((part 0 + part 1) + part 2) + ..: the order in which launches of one scale each add up
 __global__ void __launch_bounds__(256)
 mss_bwd_sum_kernel(float *__restrict__ grad, const float *__restrict__ parts, int n_parts, size_t n) {
+  dgc_after_previous();
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   float g = grad[i];
@@ -804,7 +810,8 @@ int32_t launch_bwd16(dgc_ctx *ctx, const dgc_mss_params *p, const int *scales, i
   // ((H-1) hop, T-1] are covered by no window at all -- their "first covering window" would be number H -- and must
   // still be written (zero, or left as accumulated): the grid spans window indices 0 .. H.
   auto launch = [&](const Bwd16Desc &d, size_t bytes, int add) -> int32_t {
-    mss_bwd16_kernel<<<d.first_block[d.nscales], LOSS16_THREADS, bytes, ctx->stream>>>(pred, target, p->B, p->T, d, c_lin, c_log, add);
+    dgc_launch(mss_bwd16_kernel, d.first_block[d.nscales], LOSS16_THREADS, bytes, ctx->stream, pred, target, p->B, p->T, d,
+               c_lin, c_log, add);
     ctx->launches++;
     return dgc_check_launch(ctx, "mss_bwd16");
   };
@@ -816,7 +823,7 @@ int32_t launch_bwd16(dgc_ctx *ctx, const dgc_mss_params *p, const int *scales, i
     }
     int32_t rc = launch(all, most, 0);
     if (rc != DGC_OK) return rc;
-    mss_bwd_sum_kernel<<<dgc_div_up((int64_t)nBT, 256), 256, 0, ctx->stream>>>(grad, parts, n - 1, nBT);
+    dgc_launch(mss_bwd_sum_kernel, dgc_div_up((int64_t)nBT, 256), 256, 0, ctx->stream, grad, parts, n - 1, nBT);
     DGC_LAUNCHED(ctx, "mss_bwd_sum");
     return DGC_OK;
   }
@@ -890,8 +897,8 @@ int32_t launch_bwd(dgc_ctx *ctx, const dgc_mss_params *p, const float *pred, con
   const size_t smem = smem_of(S);
   // block j owns the frames whose first covering window is in [j*S, (j+1)*S); frames up to T-1 have
   // first covering window <= H-1
-  mss_bwd_kernel<N><<<dim3(dgc_div_up(H + 1, S), p->B), LOSS_THREADS, smem, ctx->stream>>>(
-      pred, target, p->B, p->T, hop, H, S, win, tw, c_lin, c_log, accumulate, grad);
+  dgc_launch(mss_bwd_kernel<N>, dim3(dgc_div_up(H + 1, S), p->B), LOSS_THREADS, smem, ctx->stream, pred, target, p->B, p->T, hop,
+             H, S, win, tw, c_lin, c_log, accumulate, grad);
   ctx->launches++;
   return dgc_check_launch(ctx, "mss_bwd");
 }
@@ -989,15 +996,16 @@ static int32_t mss_fwd_windows(dgc_ctx *ctx, const dgc_mss_params *p, const floa
     bool tma = tma_on && p->hop_div >= 1;
     tma = tma && dgtma::make_map_2d(&mp, pred_dev, p->B, p->T, SPAN_BOX) && dgtma::make_map_2d(&mt, target_dev, p->B, p->T, SPAN_BOX);
     if (tma)
-      mss_fwd16_kernel<true><<<blocks16, LOSS16_THREADS, 2 * padded(2048) * (int)sizeof(float2), ctx->stream>>>(
-          pred_dev, target_dev, p->B, p->T, fd16, mp, mt, ctx->status_dev);
+      dgc_launch(mss_fwd16_kernel<true>, blocks16, LOSS16_THREADS, 2 * padded(2048) * (int)sizeof(float2), ctx->stream, pred_dev,
+                 target_dev, p->B, p->T, fd16, mp, mt, ctx->status_dev);
     else
-      mss_fwd16_kernel<false><<<blocks16, LOSS16_THREADS, FWD16_SMEM_BYTES, ctx->stream>>>(pred_dev, target_dev, p->B, p->T, fd16,
-                                                                                           mp, mt, ctx->status_dev);
+      dgc_launch(mss_fwd16_kernel<false>, blocks16, LOSS16_THREADS, FWD16_SMEM_BYTES, ctx->stream, pred_dev, target_dev, p->B,
+                 p->T, fd16, mp, mt, ctx->status_dev);
     DGC_LAUNCHED(ctx, tma ? "mss_fwd16_tma" : "mss_fwd16");
   }
   if (fd8.nscales > 0) {
-    mss_fwd_kernel<<<dim3(blocks8, p->B), LOSS_THREADS, FWD_SMEM_BYTES, ctx->stream>>>(pred_dev, target_dev, p->B, p->T, fd8);
+    dgc_launch(mss_fwd_kernel, dim3(blocks8, p->B), LOSS_THREADS, FWD_SMEM_BYTES, ctx->stream, pred_dev, target_dev, p->B, p->T,
+               fd8);
     DGC_LAUNCHED(ctx, "mss_fwd");
   }
   return DGC_OK;
@@ -1010,8 +1018,8 @@ static int32_t mss_fwd_reduce(dgc_ctx *ctx, const dgc_mss_params *p, const float
   // (Examples/HarmonicE2E/Trainer.swift:553-586, Sources/DGenLazy/Functions.swift:951-954);
   // the batched loss is the mean over voices (Emit+SpectralLoss.swift:937-938)
   const double den = (double)p->B * (double)(used > 0 ? used : 1) * (double)p->T;
-  mss_reduce_kernel<<<RED_BLOCKS, RED_THREADS, 0, ctx->stream>>>(part, d, (double)p->w_lin / den, (double)p->w_log / den,
-                                                                  ctx->loss_accum + 64, dgc_ctx_ticket(ctx), loss_dev);
+  dgc_launch(mss_reduce_kernel, RED_BLOCKS, RED_THREADS, 0, ctx->stream, part, d, (double)p->w_lin / den, (double)p->w_log / den,
+             ctx->loss_accum + 64, dgc_ctx_ticket(ctx), loss_dev);
   DGC_LAUNCHED(ctx, "mss_reduce");
   return DGC_OK;
 }

@@ -54,6 +54,7 @@ __device__ __forceinline__ uint32_t voice_state(uint32_t seed, uint32_t b) {
 }
 
 __global__ void noise_stream_kernel(uint32_t seed, int B, int T, float *__restrict__ out) {
+  dgc_after_previous();
   const unsigned run = blockIdx.x * blockDim.x + threadIdx.x;
   const int n0 = (int)run * RUN;
   if (n0 >= T) return;
@@ -73,6 +74,7 @@ __global__ void noise_stream_kernel(uint32_t seed, int B, int T, float *__restri
 // go through a shared-memory tile instead (rows padded to 65 floats) and leave as full 128-byte row segments.
 __global__ void __launch_bounds__(64) noise_gaussian_kernel(uint32_t seed, int B, int T, float sigma,
                                                              float *__restrict__ out) {
+  dgc_after_previous();
   __shared__ float tile[64][RUN + 1];
   const unsigned run = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y, n0 = (int)run * RUN;
@@ -158,9 +160,9 @@ DGC_EXPORT int32_t dgc_noise_fill(dgc_ctx *ctx, uint32_t seed, int32_t mode, int
   if (rc != DGC_OK) return rc;
   const int runs = dgc_div_up(T, RUN);
   if (mode == DGC_NOISE_STREAM) {
-    noise_stream_kernel<<<dgc_div_up(runs, 64), 64, 0, ctx->stream>>>(seed, B, T, out_dev);
+    dgc_launch(noise_stream_kernel, dgc_div_up(runs, 64), 64, 0, ctx->stream, seed, B, T, out_dev);
   } else {
-    noise_gaussian_kernel<<<dim3(dgc_div_up(runs, 64), B), 64, 0, ctx->stream>>>(seed, B, T, sigma, out_dev);
+    dgc_launch(noise_gaussian_kernel, dim3(dgc_div_up(runs, 64), B), 64, 0, ctx->stream, seed, B, T, sigma, out_dev);
   }
   DGC_LAUNCHED(ctx, "noise_fill");
   return DGC_OK;

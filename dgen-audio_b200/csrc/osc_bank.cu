@@ -21,6 +21,7 @@ using namespace dgosc;
 // ---------------------------------------------------------------------------------------------
 __global__ void clock_accum_kernel(float incr, float mn, float mx, float state0, int T, float *out, int clip,
                                    float clip_lo, float clip_hi) {
+  dgc_after_previous();
   if (blockIdx.x != 0 || threadIdx.x != 0) return;
   float acc = state0;
   const float span = __fsub_rn(mx, mn);
@@ -42,6 +43,7 @@ __global__ void clock_accum_kernel(float incr, float mn, float mx, float state0,
 // deterministic phasor: frame-parallel, one thread per frame looping over partials
 __global__ void osc_const_det_kernel(const float *__restrict__ freq, const float *__restrict__ amp, int K, int T,
                                      float sr, float *__restrict__ audio) {
+  dgc_after_previous();
   extern __shared__ float sh[];  // inc[K], amp[K]
   for (int k = threadIdx.x; k < K; k += blockDim.x) {
     sh[k] = __fdiv_rn(freq[k], sr);
@@ -62,6 +64,7 @@ __global__ void osc_const_det_kernel(const float *__restrict__ freq, const float
 // stateful phasor, constant frequency: anchors by the serial recurrence (one thread per partial)
 __global__ void osc_const_anchor_seq_kernel(const float *__restrict__ freq, int K, int T, float sr,
                                             float *__restrict__ anchors /* [C][K] */) {
+  dgc_after_previous();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= K) return;
   float inc = __fdiv_rn(freq[k], sr);
@@ -75,6 +78,7 @@ __global__ void osc_const_anchor_seq_kernel(const float *__restrict__ freq, int 
 __global__ void osc_const_render_kernel(const float *__restrict__ freq, const float *__restrict__ amp,
                                         const float *__restrict__ anchors, int K, int T, float sr,
                                         float *__restrict__ audio) {
+  dgc_after_previous();
   // one warp per chunk; lanes stride over partials and keep 64 per-frame sums in registers; the
   // cross-lane sum is a fixed shuffle tree, so the result does not depend on scheduling
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -110,6 +114,7 @@ __global__ void osc_const_render_kernel(const float *__restrict__ freq, const fl
 // predecessor's (the control clock wrapped), or a value above every frame index when the rows only ascend:
 // preset by the host, lowered here with an atomic minimum.
 __global__ void row_table_kernel(const float *__restrict__ play, int T, int F, float2 *__restrict__ tab) {
+  dgc_after_previous();
   int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= T) return;
   int lo, hi;
@@ -129,6 +134,7 @@ __global__ void row_table_kernel(const float *__restrict__ play, int T, int F, f
 __global__ void f0_track_kernel(const float2 *__restrict__ rowtab, const float *__restrict__ f0, int B, int T, int F,
                                 float *__restrict__ f0t, const float *__restrict__ uv,
                                 const float *__restrict__ gain, float scale, float *__restrict__ env) {
+  dgc_after_previous();
   int n = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
   if (n >= T) return;
   const float2 rt = rowtab[n];
@@ -146,6 +152,7 @@ __global__ void f0_track_kernel(const float2 *__restrict__ rowtab, const float *
 // SEQUENTIAL anchors: thread = (voice, partial), partial fastest; anchors[b][c][k]
 __global__ void anchor_seq_kernel(const float *__restrict__ f0t, int B, int T, int K, float sr, float rsr,
                                   float *__restrict__ anchors) {
+  dgc_after_previous();
   int lane_id = blockIdx.x * blockDim.x + threadIdx.x;
   if (lane_id >= B * K) return;
   int b = lane_id / K, k = lane_id - b * K;
@@ -182,6 +189,7 @@ template <int LPC, int P>
 __global__ void __launch_bounds__(128)
 anchor_sum_kernel(const float *__restrict__ f0t, int B, int T, int K, float sr, float rsr,
                   unsigned long long *__restrict__ sums /* [B][C][K] */) {
+  dgc_after_previous();
   constexpr int G = 128 / LPC;
   const int C = (T + CH - 1) / CH;
   const int g = threadIdx.x / LPC, j = threadIdx.x % LPC;
@@ -252,6 +260,7 @@ constexpr int SCAN_KK = 8, SCAN_SEGS = 128;
 __global__ void __launch_bounds__(SCAN_KK * SCAN_SEGS)
 anchor_scan_kernel(const unsigned long long *__restrict__ sums, int B, int C, int K,
                    float *__restrict__ anchors, uint32_t *__restrict__ anchors_q) {
+  dgc_after_previous();
   __shared__ unsigned long long seg_tot[SCAN_SEGS][SCAN_KK + 1];
   const int kk = threadIdx.x % SCAN_KK, seg = threadIdx.x / SCAN_KK;
   const int k = blockIdx.x * SCAN_KK + kk, b = blockIdx.y;
@@ -323,6 +332,7 @@ f0_track_fund_kernel(const float2 *__restrict__ rowtab, const float *__restrict_
                      float rsr, float *__restrict__ f0t, const float *__restrict__ uv,
                      const float *__restrict__ gain, float scale, float *__restrict__ env,
                      unsigned long long *__restrict__ chunk_sum /* [B][C] */, int2 *__restrict__ trk /* [B][T] */) {
+  dgc_after_previous();
   static_assert(CH == 64, "two frames per lane");
   const int C = (T + CH - 1) / CH;
   const int c = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, b = blockIdx.y;
@@ -401,6 +411,7 @@ f0_track_fund_kernel(const float2 *__restrict__ rowtab, const float *__restrict_
 constexpr int FSCAN_THREADS = 1024;
 __global__ void __launch_bounds__(FSCAN_THREADS)
 fund_scan_kernel(const unsigned long long *__restrict__ chunk_sum, int C, unsigned long long *__restrict__ prefix) {
+  dgc_after_previous();
   __shared__ unsigned long long warp_tot[FSCAN_THREADS / 32];
   const unsigned long long *s = chunk_sum + (size_t)blockIdx.x * C;
   unsigned long long *o = prefix + (size_t)blockIdx.x * C;
@@ -444,6 +455,7 @@ harmonic_render_kernel(dgc_harmonic_params prm, float rsr, const float *__restri
                        const float *__restrict__ f0, const float *__restrict__ uv,
                        const float *__restrict__ amps, const float *__restrict__ gain,
                        const float *__restrict__ anchors, float *__restrict__ audio) {
+  dgc_after_previous();
   constexpr int G = 128 / LPC;
   const int B = prm.B, T = prm.T, K = prm.K, F = prm.F;
   const int C = (T + CH - 1) / CH;
@@ -624,6 +636,7 @@ harmonic_render_q_kernel(dgc_harmonic_params prm, float rsr, const float2 *__res
                          const float *__restrict__ amps, const uint32_t *__restrict__ anchors_q,
                          const unsigned long long *__restrict__ fund,
                          const float *__restrict__ g_audio, float *__restrict__ audio) {
+  dgc_after_previous();
   constexpr int G = 128 / LPC, FB = 8;
   constexpr float THREE_PI = 9.42477796076938f;
   const int B = prm.B, T = prm.T, K = prm.K, F = prm.F;
@@ -724,6 +737,7 @@ __global__ void __launch_bounds__(128)
 harmonic_render_frame_kernel(dgc_harmonic_params prm, const float2 *__restrict__ rowtab, const float *__restrict__ env,
                              const float *__restrict__ amps, const unsigned long long *__restrict__ fund,
                              const int2 *__restrict__ trk, float2 *__restrict__ sums, float *__restrict__ audio) {
+  dgc_after_previous();
   constexpr float THREE_PI = 9.42477796076938f;
   const int B = prm.B, T = prm.T, K = prm.K, F = prm.F;
   const int C = (T + CH - 1) / CH;
@@ -796,7 +810,7 @@ template <int LPC, int P>
 void launch_anchor_sum_t(dgc_ctx *ctx, int B, int T, int K, int C, const float *f0t, float sr, float rsr,
                          unsigned long long *sums) {
   constexpr int G = 128 / LPC;
-  anchor_sum_kernel<LPC, P><<<dim3(dgc_div_up(C, G), B), 128, 0, ctx->stream>>>(f0t, B, T, K, sr, rsr, sums);
+  dgc_launch(anchor_sum_kernel<LPC, P>, dim3(dgc_div_up(C, G), B), 128, 0, ctx->stream, f0t, B, T, K, sr, rsr, sums);
 }
 
 // lanes per (voice, chunk) group and partials per lane for K partials (K <= 512)
@@ -826,8 +840,8 @@ void launch_render(dgc_ctx *ctx, const dgc_harmonic_params &p, const float *play
   int C = (p.T + CH - 1) / CH;
   constexpr int G = 128 / LPC;
   dim3 grid(dgc_div_up(C, G), p.B);
-  harmonic_render_kernel<LPC, P><<<grid, 128, 0, ctx->stream>>>(p, 1.0f / p.sample_rate, play, f0, uv, amps, gain,
-                                                                 anchors, audio);
+  dgc_launch(harmonic_render_kernel<LPC, P>, grid, 128, 0, ctx->stream, p, 1.0f / p.sample_rate, play, f0, uv, amps, gain,
+             anchors, audio);
 }
 
 template <int LPC, int P, int MODE>
@@ -840,11 +854,13 @@ void launch_render_q(dgc_ctx *ctx, const dgc_harmonic_params &p, const float2 *r
     const dim3 fgrid(dgc_div_up(p.T, 128), p.B);
     const bool vec = (p.K & 3) == 0 && (((uintptr_t)amps) & 15) == 0;
     float2 *keep = keep_sums ? x.sums : nullptr;
-    if (vec) harmonic_render_frame_kernel<true><<<fgrid, 128, 0, ctx->stream>>>(p, rowtab, x.env, amps, x.fund, x.trk, keep, out);
-    else harmonic_render_frame_kernel<false><<<fgrid, 128, 0, ctx->stream>>>(p, rowtab, x.env, amps, x.fund, x.trk, keep, out);
+    if (vec) dgc_launch(harmonic_render_frame_kernel<true>, fgrid, 128, 0, ctx->stream, p, rowtab, x.env, amps, x.fund, x.trk,
+                        keep, out);
+    else dgc_launch(harmonic_render_frame_kernel<false>, fgrid, 128, 0, ctx->stream, p, rowtab, x.env, amps, x.fund, x.trk, keep,
+                    out);
   } else
-    harmonic_render_q_kernel<LPC, P, MODE><<<grid, 128, 0, ctx->stream>>>(p, 1.0f / p.sample_rate, rowtab, x.f0t, x.env,
-                                                                           amps, x.anchors_q, x.fund, g_audio, out);
+    dgc_launch(harmonic_render_q_kernel<LPC, P, MODE>, grid, 128, 0, ctx->stream, p, 1.0f / p.sample_rate, rowtab, x.f0t, x.env,
+               amps, x.anchors_q, x.fund, g_audio, out);
 }
 
 // The reverse scan of the reference's temporalGradScan (Sources/DGen/Emit+TemporalGradient.swift:54-88), per row e
@@ -861,6 +877,7 @@ constexpr int TSCAN_THREADS = 1024;
 __global__ void __launch_bounds__(TSCAN_THREADS)
 temporal_suffix_scan_kernel(const float *__restrict__ g, const float *__restrict__ reset, int T, float scale,
                             float *__restrict__ out) {
+  dgc_after_previous();
   __shared__ double tot[TSCAN_THREADS];
   __shared__ unsigned char pass[TSCAN_THREADS];   // a of the composed map
   const float *row = g + (size_t)blockIdx.x * T;
@@ -902,6 +919,7 @@ temporal_suffix_scan_kernel(const float *__restrict__ g, const float *__restrict
 // the floor row, fr where r is the next row (Sources/DGen/Emit+RowSelection.swift:166-199 backward).
 __global__ void f0_rows_grad_kernel(const float2 *__restrict__ rowtab, const int *__restrict__ ranges,
                                     const float *__restrict__ G, int F, int B, int T, float *__restrict__ g_f0) {
+  dgc_after_previous();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= F * B) return;
   const int r = idx / B, b = idx - r * B;
@@ -938,7 +956,7 @@ const float2 *dgc_ctx_row_table(dgc_ctx *ctx, int F, int T) {
     dgc_fail(ctx, DGC_ERR_CUDA, "row table preset failed");
     return nullptr;
   }
-  row_table_kernel<<<dgc_div_up(T, 256), 256, 0, ctx->stream>>>(play, T, F, d);
+  dgc_launch(row_table_kernel, dgc_div_up(T, 256), 256, 0, ctx->stream, play, T, F, d);
   ctx->launches++;
   if (dgc_check_launch(ctx, "row_table") != DGC_OK) {
     cudaFree(d);
@@ -953,7 +971,7 @@ DGC_EXPORT int32_t dgc_clock_accum(dgc_ctx *ctx, float incr, float mn, float mx,
   if (!ctx) return DGC_ERR_INVALID;
   DGC_REQUIRE(ctx, out_dev && T > 0, "null output or T <= 0");
   DGC_REQUIRE(ctx, mx > mn, "max must exceed min");
-  clock_accum_kernel<<<1, 32, 0, ctx->stream>>>(incr, mn, mx, state0, T, out_dev, 0, 0.f, 0.f);
+  dgc_launch(clock_accum_kernel, 1, 32, 0, ctx->stream, incr, mn, mx, state0, T, out_dev, 0, 0.f, 0.f);
   DGC_LAUNCHED(ctx, "clock_accum");
   return DGC_OK;
 }
@@ -978,7 +996,7 @@ DGC_EXPORT int32_t dgc_playhead(dgc_ctx *ctx, int32_t F, int32_t T, const float 
   if (fmax <= 0.f) {
     DGC_CUDA(ctx, cudaMemsetAsync(d, 0, (size_t)T * sizeof(float), ctx->stream));
   } else {
-    clock_accum_kernel<<<1, 32, 0, ctx->stream>>>(step, 0.f, fmax, 0.f, T, d, 1, 0.f, hi);
+    dgc_launch(clock_accum_kernel, 1, 32, 0, ctx->stream, step, 0.f, fmax, 0.f, T, d, 1, 0.f, hi);
     ctx->launches++;
     int32_t rc = dgc_check_launch(ctx, "playhead");
     if (rc != DGC_OK) {
@@ -997,8 +1015,8 @@ DGC_EXPORT int32_t dgc_osc_bank_const(dgc_ctx *ctx, const float *freq_dev, const
   DGC_REQUIRE(ctx, freq_dev && amp_dev && audio_dev, "null pointer");
   DGC_REQUIRE(ctx, K > 0 && K <= 4096 && T > 0 && sr > 0, "size out of range");
   if (phase_mode == DGC_PHASE_DETERMINISTIC) {
-    osc_const_det_kernel<<<dgc_div_up(T, 256), 256, 2 * K * sizeof(float), ctx->stream>>>(freq_dev, amp_dev, K, T, sr,
-                                                                                          audio_dev);
+    dgc_launch(osc_const_det_kernel, dgc_div_up(T, 256), 256, 2 * K * sizeof(float), ctx->stream, freq_dev, amp_dev, K, T, sr,
+               audio_dev);
     DGC_LAUNCHED(ctx, "osc_const_det");
     return DGC_OK;
   }
@@ -1007,9 +1025,9 @@ DGC_EXPORT int32_t dgc_osc_bank_const(dgc_ctx *ctx, const float *freq_dev, const
   int C = dgc_div_up(T, CH);
   float *anchors = dgc_ctx_scratch(ctx, (uint64_t)C * K);
   if (!anchors) return DGC_ERR_OOM;
-  osc_const_anchor_seq_kernel<<<dgc_div_up(K, 32), 32, 0, ctx->stream>>>(freq_dev, K, T, sr, anchors);
+  dgc_launch(osc_const_anchor_seq_kernel, dgc_div_up(K, 32), 32, 0, ctx->stream, freq_dev, K, T, sr, anchors);
   DGC_LAUNCHED(ctx, "osc_const_anchor_seq");
-  osc_const_render_kernel<<<dgc_div_up(C, 4), 128, 0, ctx->stream>>>(freq_dev, amp_dev, anchors, K, T, sr, audio_dev);
+  dgc_launch(osc_const_render_kernel, dgc_div_up(C, 4), 128, 0, ctx->stream, freq_dev, amp_dev, anchors, K, T, sr, audio_dev);
   DGC_LAUNCHED(ctx, "osc_const_render");
   return DGC_OK;
 }
@@ -1058,24 +1076,23 @@ int32_t dgc_harmonic_prepare(dgc_ctx *ctx, const dgc_harmonic_params *p, const f
   if (already_prepared) {
     // nothing to launch
   } else if (p->phase_mode == DGC_PHASE_FUNDAMENTAL) {
-    f0_track_fund_kernel<<<dim3(dgc_div_up(C, 4), B), 128, 0, ctx->stream>>>(rowtab, f0_dev, B, T, F, K, sr, rsr, f0t, uv_dev,
-                                                                          gain_dev, p->harmonic_scale,
-                                                                          want_env ? env : nullptr, fund_sum, trk);
+    dgc_launch(f0_track_fund_kernel, dim3(dgc_div_up(C, 4), B), 128, 0, ctx->stream, rowtab, f0_dev, B, T, F, K, sr, rsr, f0t,
+               uv_dev, gain_dev, p->harmonic_scale, want_env ? env : nullptr, fund_sum, trk);
     DGC_LAUNCHED(ctx, "f0_track_fund");
-    fund_scan_kernel<<<B, FSCAN_THREADS, 0, ctx->stream>>>(fund_sum, C, fund_prefix);
+    dgc_launch(fund_scan_kernel, B, FSCAN_THREADS, 0, ctx->stream, fund_sum, C, fund_prefix);
     DGC_LAUNCHED(ctx, "fund_scan");
   } else {
-  f0_track_kernel<<<dim3(dgc_div_up(T, 256), B), 256, 0, ctx->stream>>>(rowtab, f0_dev, B, T, F, f0t, uv_dev, gain_dev,
-                                                                         p->harmonic_scale, want_env ? env : nullptr);
+  dgc_launch(f0_track_kernel, dim3(dgc_div_up(T, 256), B), 256, 0, ctx->stream, rowtab, f0_dev, B, T, F, f0t, uv_dev, gain_dev,
+             p->harmonic_scale, want_env ? env : nullptr);
   DGC_LAUNCHED(ctx, "f0_track");
   if (p->phase_mode == DGC_PHASE_SEQUENTIAL) {
-    anchor_seq_kernel<<<dgc_div_up(B * K, 32), 32, 0, ctx->stream>>>(f0t, B, T, K, sr, rsr, anchors);
+    dgc_launch(anchor_seq_kernel, dgc_div_up(B * K, 32), 32, 0, ctx->stream, f0t, B, T, K, sr, rsr, anchors);
     DGC_LAUNCHED(ctx, "anchor_seq");
   } else {
     launch_anchor_sum(ctx, B, T, K, C, f0t, sr, rsr, sums);
     DGC_LAUNCHED(ctx, "anchor_sum");
-    anchor_scan_kernel<<<dim3(dgc_div_up(K, SCAN_KK), B), SCAN_KK * SCAN_SEGS, 0, ctx->stream>>>(sums, B, C, K, anchors,
-                                                                             extra ? anchors_q : nullptr);
+    dgc_launch(anchor_scan_kernel, dim3(dgc_div_up(K, SCAN_KK), B), SCAN_KK * SCAN_SEGS, 0, ctx->stream, sums, B, C, K, anchors,
+               extra ? anchors_q : nullptr);
     DGC_LAUNCHED(ctx, "anchor_scan");
   }
   }
@@ -1128,7 +1145,7 @@ DGC_EXPORT int32_t dgc_temporal_grad_scan(dgc_ctx *ctx, const float *g_dev, cons
   DGC_REQUIRE(ctx, g_dev && out_dev, "null pointer");
   DGC_REQUIRE(ctx, E > 0 && T > 0, "E and T must be positive");
   DGC_REQUIRE(ctx, g_dev != out_dev, "the scan is not in place");
-  temporal_suffix_scan_kernel<<<E, TSCAN_THREADS, 0, ctx->stream>>>(g_dev, reset_dev, T, scale, out_dev);
+  dgc_launch(temporal_suffix_scan_kernel, E, TSCAN_THREADS, 0, ctx->stream, g_dev, reset_dev, T, scale, out_dev);
   DGC_LAUNCHED(ctx, "temporal_grad_scan");
   return DGC_OK;
 }
@@ -1164,10 +1181,10 @@ DGC_EXPORT int32_t dgc_harmonic_f0_bwd(dgc_ctx *ctx, const dgc_harmonic_params *
   DGC_PICK_GROUP(K, PHGRAD);
 #undef PHGRAD
   DGC_LAUNCHED(ctx, "harmonic_phase_grad");
-  temporal_suffix_scan_kernel<<<q.B, TSCAN_THREADS, 0, ctx->stream>>>(gphi, nullptr, q.T, 1.0f / q.sample_rate, gsum);
+  dgc_launch(temporal_suffix_scan_kernel, q.B, TSCAN_THREADS, 0, ctx->stream, gphi, nullptr, q.T, 1.0f / q.sample_rate, gsum);
   DGC_LAUNCHED(ctx, "temporal_grad_scan");
-  f0_rows_grad_kernel<<<dgc_div_up((int64_t)q.F * q.B, 128), 128, 0, ctx->stream>>>(rowtab, ranges, gsum, q.F, q.B, q.T,
-                                                                                g_f0_dev);
+  dgc_launch(f0_rows_grad_kernel, dgc_div_up((int64_t)q.F * q.B, 128), 128, 0, ctx->stream, rowtab, ranges, gsum, q.F, q.B, q.T,
+             g_f0_dev);
   DGC_LAUNCHED(ctx, "f0_rows_grad");
   return DGC_OK;
 }

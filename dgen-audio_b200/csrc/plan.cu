@@ -14,6 +14,7 @@
 namespace {
 
 __global__ void plan_add_kernel(const float *a, const float *__restrict__ b, size_t n, float *out) {
+  dgc_after_previous();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = __fadd_rn(a[i], b[i]);
 }
@@ -27,6 +28,7 @@ struct CopyDesc {
 };
 constexpr int COPY_THREADS = 256, COPY_BLOCKS = 592;
 __global__ void __launch_bounds__(COPY_THREADS) copy_many_kernel(const __grid_constant__ CopyDesc d) {
+  dgc_after_previous();
   const float *s = d.src[blockIdx.y];
   float *o = d.dst[blockIdx.y];
   const size_t n = d.n[blockIdx.y], first = (size_t)blockIdx.x * COPY_THREADS + threadIdx.x, step = (size_t)gridDim.x * COPY_THREADS;
@@ -89,7 +91,7 @@ DGC_EXPORT int32_t dgc_copy_many(dgc_ctx *ctx, void *stream, int32_t count, cons
   }
   if (most == 0) return DGC_OK;
   const int64_t blocks = std::min<int64_t>(dgc_div_up((int64_t)most, 4 * COPY_THREADS), COPY_BLOCKS);
-  copy_many_kernel<<<dim3((unsigned)blocks, count), COPY_THREADS, 0, (cudaStream_t)stream>>>(d);
+  dgc_launch(copy_many_kernel, dim3((unsigned)blocks, count), COPY_THREADS, 0, (cudaStream_t)stream, d);
   DGC_LAUNCHED(ctx, "copy_many");
   return DGC_OK;
 }
@@ -168,7 +170,7 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
         const float *x = R.at(a[0], n), *y = R.at(a[1], n);
         float *out = R.at(a[2], n);
         if (!R.bad && n > 0) {
-          plan_add_kernel<<<dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream>>>(x, y, n, out);
+          dgc_launch(plan_add_kernel, dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream, x, y, n, out);
           ctx->launches++;
           rc = dgc_check_launch(ctx, "plan_add");
         }

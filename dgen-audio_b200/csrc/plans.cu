@@ -38,6 +38,7 @@ int32_t ensure_stage(dgc_ctx *ctx, uint64_t nfloats) {
 
 // out may be the same buffer as a (element i is read before it is written): no restrict on those two
 __global__ void add2_kernel(const float *a, const float *__restrict__ b, size_t n, float *out) {
+  dgc_after_previous();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = __fadd_rn(a[i], b[i]);
 }
@@ -155,7 +156,7 @@ static int32_t hn_forward_loss_impl(dgc_ctx *ctx, const dgc_hn_step *s, const fl
   // against 0.360 ms with the loss kernel adding the two signals as it loads them)
   float *mix = audio_dev ? audio_dev : d_harm;
   if (noise && !serial_fir) {
-    add2_kernel<<<dgc_div_up((int64_t)nBT, 256), 256, 0, ctx->stream>>>(d_harm, d_noise, nBT, mix);
+    dgc_launch(add2_kernel, dgc_div_up((int64_t)nBT, 256), 256, 0, ctx->stream, d_harm, d_noise, nBT, mix);
     DGC_LAUNCHED(ctx, "add_branches");
   } else if (mix != d_harm) {
     DGC_CUDA(ctx, cudaMemcpyAsync(mix, d_harm, nBT * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));

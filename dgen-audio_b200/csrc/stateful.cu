@@ -46,6 +46,7 @@ __global__ void __launch_bounds__(256)
 frac_delay_kernel(const float *__restrict__ x, const float *__restrict__ delay, int delay_mode, int fixed_k, int64_t T,
                   int W, int R, float dmax, const float *__restrict__ ring, const float *__restrict__ head,
                   float *__restrict__ y) {
+  dgc_after_previous();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= T * W) return;
   const int64_t n = idx / W;
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(256)
 frac_delay4_kernel(const float *__restrict__ x, const float *__restrict__ delay, int delay_mode, int fixed_k, int64_t T,
                    int W, int R, float dmax, const float *__restrict__ ring, const float *__restrict__ head,
                    float *__restrict__ y) {
+  dgc_after_previous();
   const int W4 = W >> 2;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, total = T * W4;
   if (idx >= total) return;
@@ -131,11 +133,11 @@ static void launch_frac_delay(cudaStream_t st, const float *x, const float *dela
                               int W, int R, float dmax, const float *ring, const float *head, float *y) {
   const bool vec = (W & 3) == 0 && ((((uintptr_t)x) | ((uintptr_t)y) | ((uintptr_t)delay)) & 15) == 0;
   if (vec)
-    frac_delay4_kernel<ROW_MAJOR><<<dgc_div_up(T * (W >> 2), 256), 256, 0, st>>>(x, delay, delay_mode, fixed_k, T, W, R, dmax,
-                                                                                ring, head, y);
+    dgc_launch(frac_delay4_kernel<ROW_MAJOR>, dgc_div_up(T * (W >> 2), 256), 256, 0, st, x, delay, delay_mode, fixed_k, T, W, R,
+               dmax, ring, head, y);
   else
-    frac_delay_kernel<ROW_MAJOR><<<dgc_div_up(T * W, 256), 256, 0, st>>>(x, delay, delay_mode, fixed_k, T, W, R, dmax, ring,
-                                                                        head, y);
+    dgc_launch(frac_delay_kernel<ROW_MAJOR>, dgc_div_up(T * W, 256), 256, 0, st, x, delay, delay_mode, fixed_k, T, W, R, dmax,
+               ring, head, y);
 }
 
 // ring slot p holds, after the call, the last row written to it: frames n = off, off + R, ... < T with
@@ -143,6 +145,7 @@ static void launch_frac_delay(cudaStream_t st, const float *x, const float *dela
 template <bool ROW_MAJOR>
 __global__ void ring_update_kernel(const float *__restrict__ x, int64_t T, int W, int R, float *__restrict__ ring,
                                    const float *__restrict__ head) {
+  dgc_after_previous();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (int64_t)W * R) return;
   // lanes fastest over threads for the row-major ring, slots fastest for the lane-major one: coalesced writes
@@ -157,6 +160,7 @@ __global__ void ring_update_kernel(const float *__restrict__ x, int64_t T, int W
 }
 
 __global__ void head_advance_kernel(float *head, int64_t T, int R) {
+  dgc_after_previous();
   const int64_t w0 = (int64_t)head[0];
   head[0] = (float)((w0 + T) % R);
 }
@@ -172,6 +176,7 @@ __device__ __forceinline__ float cond_at(const float *__restrict__ cond, int con
 // another each waits for memory (64 lanes x 262144 frames, 3 % of them triggers: 11 -> 9 us).
 __global__ void latch_last_kernel(const float *__restrict__ cond, int cond_mode, int64_t T, int W, int NC,
                                   int *__restrict__ last, int *__restrict__ span, int NP) {
+  dgc_after_previous();
   const int e = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
   if (e >= W) return;
   if (c < NP) span[(size_t)c * W + e] = 0;     // for latch_seg_kernel
@@ -209,6 +214,7 @@ __global__ void latch_last_kernel(const float *__restrict__ cond, int cond_mode,
 constexpr int LATCH_SEG = 32, LATCH_SPAN = 32;
 
 __global__ void latch_seg_kernel(const int *__restrict__ last, int W, int NC, int *__restrict__ seg, int *__restrict__ span) {
+  dgc_after_previous();
   const int e = blockIdx.x * blockDim.x + threadIdx.x, sgm = blockIdx.y;
   if (e >= W) return;
   const int c0 = sgm * LATCH_SEG, c1 = min(c0 + LATCH_SEG, NC);
@@ -224,6 +230,7 @@ __global__ void latch_seg_kernel(const int *__restrict__ last, int W, int NC, in
 
 __global__ void latch_carry_kernel(int *last, int *src_chunk, const int *__restrict__ seg, const int *__restrict__ span, int W,
                                    int NC) {
+  dgc_after_previous();
   const int e = blockIdx.x * blockDim.x + threadIdx.x, sgm = blockIdx.y;
   if (e >= W) return;
   const int c0 = sgm * LATCH_SEG, c1 = min(c0 + LATCH_SEG, NC);
@@ -260,6 +267,7 @@ __global__ void latch_out_kernel(const float *__restrict__ value, const float *_
                                  int64_t T, int W, int NC, const int *__restrict__ src_off,
                                  const int *__restrict__ src_chunk, const float *__restrict__ state,
                                  float *__restrict__ y) {
+  dgc_after_previous();
   const int e = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
   if (e >= W) return;
   const int sc = src_chunk[(size_t)c * W + e];
@@ -291,6 +299,7 @@ __global__ void __launch_bounds__(256)
 latch_out4_kernel(const float *__restrict__ value, const float *__restrict__ cond, int cond_mode, int64_t T, int W,
                   int NC, const int *__restrict__ src_off, const int *__restrict__ src_chunk,
                   const float *__restrict__ state, float *__restrict__ y) {
+  dgc_after_previous();
   const int e = (blockIdx.x * blockDim.x + threadIdx.x) * 4, c = blockIdx.y * blockDim.y + threadIdx.y;
   if (e >= W || c >= NC) return;
   float held[4];
@@ -328,6 +337,7 @@ latch_out4_kernel(const float *__restrict__ value, const float *__restrict__ con
 }
 
 __global__ void latch_state_kernel(const float *__restrict__ y, int64_t T, int W, float *__restrict__ state) {
+  dgc_after_previous();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < W) state[e] = y[(T - 1) * W + e];
 }
@@ -403,6 +413,7 @@ template <int P>
 __global__ void __launch_bounds__(COMP_THREADS, 2)
 compressor_kernel(const float *__restrict__ x, const float *__restrict__ det, int B, int64_t T, int NT, CompCoef c,
                   float *state, float *__restrict__ y, unsigned long long *__restrict__ chain, int32_t *status) {
+  dgc_after_previous();
   constexpr int TILE = COMP_THREADS * P, WARPS = COMP_THREADS / 32;
   extern __shared__ float gs[];                // TILE values, one pad float after every P: a thread's run is conflict-free
   __shared__ Affine warp_map[2][WARPS];
@@ -612,6 +623,7 @@ constexpr int PV_RUN = 8;
 __global__ void __launch_bounds__(128)
 pv_analysis_kernel(const float *__restrict__ re, const float *__restrict__ im, int64_t H, int N, float omega_scale,
                    const float *__restrict__ state, float2 *__restrict__ mag_omega) {
+  dgc_after_previous();
   const int i = blockIdx.y * blockDim.x + threadIdx.x, v = blockIdx.z;
   const int64_t h0 = (int64_t)blockIdx.x * PV_RUN;
   if (i >= N) return;
@@ -647,6 +659,7 @@ __global__ void __launch_bounds__(PV_BINS * PV_WARPS)
 pv_synthesis_kernel(const float *__restrict__ re, const float *__restrict__ im, const float2 *__restrict__ mag_omega,
                     const float *__restrict__ ratio, int ratio_mode, int64_t H, int N, float *__restrict__ state,
                     float *__restrict__ out_re, float *__restrict__ out_im) {
+  dgc_after_previous();
   __shared__ float phase[2][PV_TILE][PV_BINS];      // a tile's unscaled frequencies, then, in place, its phases
   __shared__ float ratios[2][PV_TILE];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, v = blockIdx.y;
@@ -735,6 +748,7 @@ pv_synthesis_kernel(const float *__restrict__ re, const float *__restrict__ im, 
 }
 
 __global__ void pv_mark_started_kernel(float *state, int V, int N) {
+  dgc_after_previous();
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v < V) state[(size_t)v * (2 * N + 1) + 2 * N] = 1.0f;
 }
@@ -757,10 +771,10 @@ DGC_EXPORT int32_t dgc_delay_line(dgc_ctx *ctx, const float *x_dev, const float 
                            ring_dev, head_dev, y_dev);
   DGC_LAUNCHED(ctx, "delay_line");
   if (ring_dev) {
-    ring_update_kernel<false><<<dgc_div_up((int64_t)lanes * max_delay, 256), 256, 0, ctx->stream>>>(
-        x_dev, T, lanes, max_delay, ring_dev, head_dev);
+    dgc_launch(ring_update_kernel<false>, dgc_div_up((int64_t)lanes * max_delay, 256), 256, 0, ctx->stream, x_dev, T, lanes,
+               max_delay, ring_dev, head_dev);
     DGC_LAUNCHED(ctx, "delay_line_ring");
-    head_advance_kernel<<<1, 1, 0, ctx->stream>>>(head_dev, T, max_delay);
+    dgc_launch(head_advance_kernel, 1, 1, 0, ctx->stream, head_dev, T, max_delay);
     DGC_LAUNCHED(ctx, "delay_line_head");
   }
   return DGC_OK;
@@ -781,10 +795,10 @@ DGC_EXPORT int32_t dgc_spectrum_delay(dgc_ctx *ctx, const float *spec_dev, const
                           row_dev, out_dev);
   DGC_LAUNCHED(ctx, "spectrum_delay");
   if (ring_dev) {
-    ring_update_kernel<true><<<dgc_div_up((int64_t)N * R, 256), 256, 0, ctx->stream>>>(spec_dev, H, N, R, ring_dev,
-                                                                                     row_dev);
+    dgc_launch(ring_update_kernel<true>, dgc_div_up((int64_t)N * R, 256), 256, 0, ctx->stream, spec_dev, H, N, R, ring_dev,
+               row_dev);
     DGC_LAUNCHED(ctx, "spectrum_delay_ring");
-    head_advance_kernel<<<1, 1, 0, ctx->stream>>>(row_dev, H, R);
+    dgc_launch(head_advance_kernel, 1, 1, 0, ctx->stream, row_dev, H, R);
     DGC_LAUNCHED(ctx, "spectrum_delay_row");
   }
   return DGC_OK;
@@ -811,26 +825,26 @@ DGC_EXPORT int32_t dgc_latch(dgc_ctx *ctx, const float *value_dev, const float *
   dim3 grid(dgc_div_up(lanes, 128), NC);
   const int NS = dgc_div_up(NC, LATCH_SEG), NP = dgc_div_up(NS, LATCH_SPAN);
   int *seg = src_chunk + (size_t)NC * lanes, *span = seg + (size_t)NS * lanes;
-  latch_last_kernel<<<grid, 128, 0, ctx->stream>>>(cond_dev, cond_mode, T, lanes, NC, last, span, NP);
+  dgc_launch(latch_last_kernel, grid, 128, 0, ctx->stream, cond_dev, cond_mode, T, lanes, NC, last, span, NP);
   DGC_LAUNCHED(ctx, "latch_last");
   dim3 sgrid(dgc_div_up(lanes, 128), NS);
-  latch_seg_kernel<<<sgrid, 128, 0, ctx->stream>>>(last, lanes, NC, seg, span);
+  dgc_launch(latch_seg_kernel, sgrid, 128, 0, ctx->stream, last, lanes, NC, seg, span);
   DGC_LAUNCHED(ctx, "latch_segments");
-  latch_carry_kernel<<<sgrid, 128, 0, ctx->stream>>>(last, src_chunk, seg, span, lanes, NC);
+  dgc_launch(latch_carry_kernel, sgrid, 128, 0, ctx->stream, last, src_chunk, seg, span, lanes, NC);
   DGC_LAUNCHED(ctx, "latch_carry");
   const bool quad = (lanes & 3) == 0 &&
                     ((((uintptr_t)value_dev) | ((uintptr_t)y_dev) | (cond_mode == 2 ? (uintptr_t)cond_dev : 0)) & 15) == 0;
   if (quad) {
     const int bx = lanes / 4 >= 64 ? 64 : lanes / 4, by = 256 / bx >= 1 ? (256 / bx > 8 ? 8 : 256 / bx) : 1;
-    latch_out4_kernel<<<dim3(dgc_div_up(lanes / 4, bx), dgc_div_up(NC, by)), dim3(bx, by), 0, ctx->stream>>>(
-        value_dev, cond_dev, cond_mode, T, lanes, NC, last, src_chunk, state_dev, y_dev);
+    dgc_launch(latch_out4_kernel, dim3(dgc_div_up(lanes / 4, bx), dgc_div_up(NC, by)), dim3(bx, by), 0, ctx->stream, value_dev,
+               cond_dev, cond_mode, T, lanes, NC, last, src_chunk, state_dev, y_dev);
   } else {
-    latch_out_kernel<<<grid, 128, 0, ctx->stream>>>(value_dev, cond_dev, cond_mode, T, lanes, NC, last, src_chunk,
-                                                    state_dev, y_dev);
+    dgc_launch(latch_out_kernel, grid, 128, 0, ctx->stream, value_dev, cond_dev, cond_mode, T, lanes, NC, last, src_chunk,
+               state_dev, y_dev);
   }
   DGC_LAUNCHED(ctx, "latch_out");
   if (state_dev) {
-    latch_state_kernel<<<dgc_div_up(lanes, 128), 128, 0, ctx->stream>>>(y_dev, T, lanes, state_dev);
+    dgc_launch(latch_state_kernel, dgc_div_up(lanes, 128), 128, 0, ctx->stream, y_dev, T, lanes, state_dev);
     DGC_LAUNCHED(ctx, "latch_state");
   }
   return DGC_OK;
@@ -869,12 +883,12 @@ DGC_EXPORT int32_t dgc_compressor(dgc_ctx *ctx, const dgc_compressor_params *p, 
   unsigned long long *chain = dgc_ctx_chain(ctx, 2 * blocks);
   if (!chain) return DGC_ERR_OOM;
   if (P == 8) {
-    compressor_kernel<8><<<(unsigned)blocks, COMP_THREADS, smem, ctx->stream>>>(x_dev, det, p->B, p->T, NT, c, state_dev, y_dev,
-                                                                               chain, ctx->status_dev);
+    dgc_launch(compressor_kernel<8>, (unsigned)blocks, COMP_THREADS, smem, ctx->stream, x_dev, det, p->B, p->T, NT, c, state_dev,
+               y_dev, chain, ctx->status_dev);
   } else {
     DGC_CUDA(ctx, cudaFuncSetAttribute(compressor_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    compressor_kernel<32><<<(unsigned)blocks, COMP_THREADS, smem, ctx->stream>>>(x_dev, det, p->B, p->T, NT, c, state_dev, y_dev,
-                                                                                chain, ctx->status_dev);
+    dgc_launch(compressor_kernel<32>, (unsigned)blocks, COMP_THREADS, smem, ctx->stream, x_dev, det, p->B, p->T, NT, c,
+               state_dev, y_dev, chain, ctx->status_dev);
   }
   DGC_LAUNCHED(ctx, "compressor");
   return DGC_OK;
@@ -902,14 +916,14 @@ DGC_EXPORT int32_t dgc_phase_vocoder(dgc_ctx *ctx, const float *re_dev, const fl
   if (!scr) return DGC_ERR_OOM;
   float2 *mag_omega = reinterpret_cast<float2 *>(scr);
   const float omega_scale = 2.0f * 3.14159265358979323846f * (float)hop / (float)N;
-  pv_analysis_kernel<<<dim3((unsigned)runs, dgc_div_up(N, 128), V), 128, 0, ctx->stream>>>(re_dev, im_dev, H, N, omega_scale,
-                                                                                      state_dev, mag_omega);
+  dgc_launch(pv_analysis_kernel, dim3((unsigned)runs, dgc_div_up(N, 128), V), 128, 0, ctx->stream, re_dev, im_dev, H, N,
+             omega_scale, state_dev, mag_omega);
   DGC_LAUNCHED(ctx, "phase_vocoder_analysis");
-  pv_synthesis_kernel<<<dim3(dgc_div_up(N, PV_BINS), V), PV_BINS * PV_WARPS, 0, ctx->stream>>>(re_dev, im_dev, mag_omega, ratio_dev, ratio_mode,
-                                                                           H, N, state_dev, out_re_dev, out_im_dev);
+  dgc_launch(pv_synthesis_kernel, dim3(dgc_div_up(N, PV_BINS), V), PV_BINS * PV_WARPS, 0, ctx->stream, re_dev, im_dev, mag_omega,
+             ratio_dev, ratio_mode, H, N, state_dev, out_re_dev, out_im_dev);
   DGC_LAUNCHED(ctx, "phase_vocoder_synthesis");
   if (state_dev) {
-    pv_mark_started_kernel<<<dgc_div_up(V, 128), 128, 0, ctx->stream>>>(state_dev, V, N);
+    dgc_launch(pv_mark_started_kernel, dgc_div_up(V, 128), 128, 0, ctx->stream, state_dev, V, N);
     DGC_LAUNCHED(ctx, "phase_vocoder_state");
   }
   return DGC_OK;

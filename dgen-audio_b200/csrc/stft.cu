@@ -29,6 +29,7 @@ template <int N, int SRC, int OUT>
 __global__ void __launch_bounds__(ST_THREADS)
 stft_kernel(const float *__restrict__ x, int T, int hop, int H, const float *__restrict__ window,
             const float2 *__restrict__ tw, float *__restrict__ out, float *__restrict__ out_im) {
+  dgc_after_previous();
   constexpr int G = N / 8, NF = ST_THREADS / G, NB = N / 2 + 1, PN = padded(N);
   __shared__ float2 bufa[NF * PN];
   __shared__ float2 bufb[NF * PN];
@@ -96,6 +97,7 @@ constexpr int MAC_BINS = 32, MAC_HPT = 4, MAC_HT = 8 * MAC_HPT;
 __global__ void __launch_bounds__(256)
 partconv_mac_kernel(const float2 *__restrict__ X, const float2 *__restrict__ Hs, int H, int K, int NB,
                     float2 *__restrict__ Y) {
+  dgc_after_previous();
   extern __shared__ float2 smem[];
   float2 *hs = smem;                          // [K][MAC_BINS]
   float2 *xs = smem + (size_t)K * MAC_BINS;   // [MAC_HT + K - 1][MAC_BINS], row r <-> hop hb - (K-1) + r
@@ -149,6 +151,7 @@ template <int N>
 __global__ void __launch_bounds__(ST_THREADS)
 istft_kernel(const float2 *__restrict__ Y, int H, const float *__restrict__ window, const float2 *__restrict__ tw,
              float gain, float *__restrict__ frames) {
+  dgc_after_previous();
   constexpr int G = N / 8, NF = ST_THREADS / G, NB = N / 2 + 1, PN = padded(N);
   __shared__ float2 bufa[NF * PN];
   __shared__ float2 bufb[NF * PN];
@@ -184,6 +187,7 @@ istft_kernel(const float2 *__restrict__ Y, int H, const float *__restrict__ wind
 // oldest first.  offset 0: the forward overlap-add; offset -(N-1): the adjoint of the bufferView gather.
 __global__ void overlap_add_kernel(const float *__restrict__ frames, int T, int N, int hop, int H, int offset,
                                    int accumulate, float *__restrict__ out) {
+  dgc_after_previous();
   int t = blockIdx.x * blockDim.x + threadIdx.x, v = blockIdx.y;
   if (t >= T) return;
   int u = t - offset;            // frame h covers u in [h*hop, h*hop + N)
@@ -199,6 +203,7 @@ __global__ void overlap_add_kernel(const float *__restrict__ frames, int T, int 
 __global__ void __launch_bounds__(256)
 partconv_mac_adj_kernel(const float2 *__restrict__ U, const float2 *__restrict__ Hs, int H, int K, int NB,
                         float2 *__restrict__ V) {
+  dgc_after_previous();
   extern __shared__ float2 smem[];
   float2 *hs = smem;                          // [K][MAC_BINS]
   float2 *us = smem + (size_t)K * MAC_BINS;   // [MAC_HT + K - 1][MAC_BINS], row r <-> hop hb + r
@@ -245,6 +250,7 @@ constexpr int IR_LOADS = 8;
 __global__ void __launch_bounds__(256)
 partconv_ir_grad_kernel(const float2 *__restrict__ X, const float2 *__restrict__ U, int V, int H, int NB,
                         float2 *__restrict__ G) {
+  dgc_after_previous();
   __shared__ float2 red[8][33];
   const int bin = blockIdx.x * 32 + (threadIdx.x & 31), k = blockIdx.y, grp = threadIdx.x >> 5;
   float2 acc = make_float2(0.f, 0.f);
@@ -288,6 +294,7 @@ partconv_ir_grad_kernel(const float2 *__restrict__ X, const float2 *__restrict__
 // g_ir[k*hop + i] = frames[k][i], i < hop (the zero-padded tail of each partition carries no parameter)
 __global__ void take_partitions_kernel(const float *__restrict__ frames, int ir_len, int N, int hop,
                                        float *__restrict__ g_ir) {
+  dgc_after_previous();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ir_len) return;
   int k = t / hop, i = t - k * hop;
@@ -297,6 +304,7 @@ __global__ void take_partitions_kernel(const float *__restrict__ frames, int ir_
 // half spectra float2 [rows][N/2+1] -> all N bins as split re / im [rows][N] (bins above N/2: the conjugate mirror)
 __global__ void half_to_full_kernel(const float2 *__restrict__ half, int64_t rows, int N, float *__restrict__ re,
                                     float *__restrict__ im) {
+  dgc_after_previous();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * N) return;
   const int64_t r = idx / N;
@@ -312,6 +320,7 @@ bool overlap(const float *a, uint64_t n, const float *b, uint64_t m) { return a 
 // transform is the real part of the inverse transform of the whole (the reference keeps only that real part)
 __global__ void full_to_half_kernel(const float *__restrict__ re, const float *__restrict__ im, int64_t rows, int N,
                                     float2 *__restrict__ half) {
+  dgc_after_previous();
   const int NB = N / 2 + 1;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * NB) return;
@@ -327,8 +336,8 @@ int32_t launch_stft(dgc_ctx *ctx, const float *x, int V, int T, int hop, int H, 
   if (!tw) return DGC_ERR_OOM;
   constexpr int NF = ST_THREADS / (N / 8);
   int pairs = (H + 1) / 2;
-  stft_kernel<N, SRC, OUT><<<dim3(dgc_div_up(pairs, NF), V), ST_THREADS, 0, ctx->stream>>>(x, T, hop, H, window, tw,
-                                                                                          out, out_im);
+  dgc_launch(stft_kernel<N, SRC, OUT>, dim3(dgc_div_up(pairs, NF), V), ST_THREADS, 0, ctx->stream, x, T, hop, H, window, tw, out,
+             out_im);
   ctx->launches++;
   return dgc_check_launch(ctx, "stft");
 }
@@ -351,7 +360,7 @@ int32_t stft16_half(dgc_ctx *ctx, int N, const float *x, int V, int T, int hop, 
   if (!tw) return DGC_ERR_OOM;
   const int pairs = (H + 1) / 2;
   switch (N) {
-#define CASE(NN) case NN: dgstft::stft16_kernel<NN, SRC><<<dim3(dgc_div_up(pairs, dgstft::THREADS / (NN / 16)), V), dgstft::THREADS, 0, ctx->stream>>>( \
+#define CASE(NN) case NN: dgc_launch(dgstft::stft16_kernel<NN, SRC>, dim3(dgc_div_up(pairs, dgstft::THREADS / (NN / 16)), V), dgstft::THREADS, 0, ctx->stream, \
     x, T, hop, H, window, tw, reinterpret_cast<float2 *>(out)); break;
     CASE(64) CASE(128) CASE(256) CASE(512) CASE(1024) CASE(2048)
 #undef CASE
@@ -378,7 +387,7 @@ int32_t launch_istft16_ola(dgc_ctx *ctx, const float *Y, const float *Yim, int V
   constexpr int TT = N / 16, NF = dgstft::THREADS / TT;
   const int pairs = (dgc_div_up((int64_t)T - offset, hop) + 1) / 2, run = ola_run(ctx, V, pairs, 4, NF);
   const dim3 grid(dgc_div_up(dgc_div_up(pairs, run), NF), V);
-#define RUN(FULL, SS) dgstft::istft16_kernel<N, FULL, SS><<<grid, dgstft::THREADS, 0, ctx->stream>>>(                  \
+#define RUN(FULL, SS) dgc_launch(dgstft::istft16_kernel<N, FULL, SS>, grid, dgstft::THREADS, 0, ctx->stream, \
       Y, Yim, H, T, window, tw, gain, offset, accumulate, run, out)
 #define STEP(SS) if (!in_place && hop == SS * TT) {                                                                              \
     if (Yim) RUN(true, SS); else RUN(false, SS);                                                                    \
@@ -389,12 +398,14 @@ int32_t launch_istft16_ola(dgc_ctx *ctx, const float *Y, const float *Yim, int V
 #undef STEP
 #undef RUN
   const dim3 every(dgc_div_up((H + 1) / 2, NF), V);
-  if (Yim) dgstft::istft16_kernel<N, true, 0><<<every, dgstft::THREADS, 0, ctx->stream>>>(Y, Yim, H, T, window, tw, gain, 0, 0, 1, frames);
-  else dgstft::istft16_kernel<N, false, 0><<<every, dgstft::THREADS, 0, ctx->stream>>>(Y, Yim, H, T, window, tw, gain, 0, 0, 1, frames);
+  if (Yim) dgc_launch(dgstft::istft16_kernel<N, true, 0>, every, dgstft::THREADS, 0, ctx->stream, Y, Yim, H, T, window, tw, gain,
+                      0, 0, 1, frames);
+  else dgc_launch(dgstft::istft16_kernel<N, false, 0>, every, dgstft::THREADS, 0, ctx->stream, Y, Yim, H, T, window, tw, gain, 0,
+                  0, 1, frames);
   ctx->launches++;
   int32_t rc = dgc_check_launch(ctx, "istft");
   if (rc != DGC_OK) return rc;
-  overlap_add_kernel<<<dim3(dgc_div_up(T, 256), V), 256, 0, ctx->stream>>>(frames, T, N, hop, H, offset, accumulate, out);
+  dgc_launch(overlap_add_kernel, dim3(dgc_div_up(T, 256), V), 256, 0, ctx->stream, frames, T, N, hop, H, offset, accumulate, out);
   DGC_LAUNCHED(ctx, "overlap_add");
   return DGC_OK;
 }
@@ -416,11 +427,11 @@ int32_t launch_istft_ola(dgc_ctx *ctx, const float2 *Y, int V, int H, int T, int
   const float2 *tw = dgc_ctx_twiddles(ctx, N);
   if (!tw) return DGC_ERR_OOM;
   constexpr int NF = ST_THREADS / (N / 8);
-  istft_kernel<N><<<dim3(dgc_div_up((H + 1) / 2, NF), V), ST_THREADS, 0, ctx->stream>>>(Y, H, window, tw, gain, frames);
+  dgc_launch(istft_kernel<N>, dim3(dgc_div_up((H + 1) / 2, NF), V), ST_THREADS, 0, ctx->stream, Y, H, window, tw, gain, frames);
   ctx->launches++;
   int32_t rc = dgc_check_launch(ctx, "istft");
   if (rc != DGC_OK) return rc;
-  overlap_add_kernel<<<dim3(dgc_div_up(T, 256), V), 256, 0, ctx->stream>>>(frames, T, N, hop, H, offset, accumulate, out);
+  dgc_launch(overlap_add_kernel, dim3(dgc_div_up(T, 256), V), 256, 0, ctx->stream, frames, T, N, hop, H, offset, accumulate, out);
   DGC_LAUNCHED(ctx, "overlap_add");
   return DGC_OK;
 }
@@ -441,7 +452,7 @@ int32_t istft_frames(dgc_ctx *ctx, int N, const float *Y, int H, float gain, flo
   const float2 *tw = dgc_ctx_twiddles(ctx, N), *y = reinterpret_cast<const float2 *>(Y);
   if (!tw) return DGC_ERR_OOM;
   switch (N) {
-#define CASE(NN) case NN: istft_kernel<NN><<<dgc_div_up((H + 1) / 2, ST_THREADS / (NN / 8)), ST_THREADS, 0, ctx->stream>>>( \
+#define CASE(NN) case NN: dgc_launch(istft_kernel<NN>, dgc_div_up((H + 1) / 2, ST_THREADS / (NN / 8)), ST_THREADS, 0, ctx->stream, \
     y, H, nullptr, tw, gain, frames); break;
     CASE(16) CASE(32) CASE(64) CASE(128) CASE(256) CASE(512) CASE(1024) CASE(2048)
 #undef CASE
@@ -502,9 +513,10 @@ int32_t convolve_hops(dgc_ctx *ctx, const float *in, const float *hs, int V, int
 #define CASE(MM) case MM:                                                                                            \
     if (int32_t rc = hop_smem(ctx, (const void *)dgstft::hop_spectrum_kernel<MM>, MM, &bytes)) return rc;            \
     if (int32_t rc = hop_smem(ctx, (const void *)dgstft::hop_convolve_kernel<MM, ADJ>, MM, &bytes)) return rc;       \
-    dgstft::hop_spectrum_kernel<MM><<<groups, MM, bytes, ctx->stream>>>(hs2, K, NB, tw, g);                          \
+    dgc_launch(dgstft::hop_spectrum_kernel<MM>, groups, MM, bytes, ctx->stream, hs2, K, NB, tw, g);                  \
     DGC_LAUNCHED(ctx, "hop_spectrum");                                                                               \
-    dgstft::hop_convolve_kernel<MM, ADJ><<<dim3(groups, pl.segs, V), MM, bytes, ctx->stream>>>(in2, hs2, g, H, K, NB, tw, out2); \
+    dgc_launch(dgstft::hop_convolve_kernel<MM, ADJ>, dim3(groups, pl.segs, V), MM, bytes, ctx->stream, in2, hs2, g, H, K, NB,   \
+               tw, out2);                                                                                            \
     break;
     HOP_CASES(pl.M)
 #undef CASE
@@ -515,10 +527,10 @@ int32_t convolve_hops(dgc_ctx *ctx, const float *in, const float *hs, int V, int
   const dim3 grid(dgc_div_up(NB, MAC_BINS), dgc_div_up(H, MAC_HT), V);
   if (ADJ) {
     DGC_CUDA(ctx, cudaFuncSetAttribute(partconv_mac_adj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    partconv_mac_adj_kernel<<<grid, 256, smem, ctx->stream>>>(in2, hs2, H, K, NB, out2);
+    dgc_launch(partconv_mac_adj_kernel, grid, 256, smem, ctx->stream, in2, hs2, H, K, NB, out2);
   } else {
     DGC_CUDA(ctx, cudaFuncSetAttribute(partconv_mac_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    partconv_mac_kernel<<<grid, 256, smem, ctx->stream>>>(in2, hs2, H, K, NB, out2);
+    dgc_launch(partconv_mac_kernel, grid, 256, smem, ctx->stream, in2, hs2, H, K, NB, out2);
   }
   DGC_LAUNCHED(ctx, "partconv_mac");
   return DGC_OK;
@@ -540,16 +552,17 @@ int32_t correlate_hops(dgc_ctx *ctx, const float *x, const float *u, int V, int 
 #define CASE(MM) case MM:                                                                                            \
     if (int32_t rc = hop_smem(ctx, (const void *)dgstft::hop_correlate_kernel<MM>, MM, &bytes)) return rc;           \
     if (int32_t rc = hop_smem(ctx, (const void *)dgstft::hop_lags_kernel<MM>, MM, &bytes)) return rc;                \
-    dgstft::hop_correlate_kernel<MM><<<dim3(groups, n), MM, bytes, ctx->stream>>>(x2, u2, V, H, K, NB, pl.segs, tw, p2); \
+    dgc_launch(dgstft::hop_correlate_kernel<MM>, dim3(groups, n), MM, bytes, ctx->stream, x2, u2, V, H, K, NB,       \
+               pl.segs, tw, p2);                                                                                     \
     DGC_LAUNCHED(ctx, "hop_correlate");                                                                              \
-    dgstft::hop_lags_kernel<MM><<<groups, MM, bytes, ctx->stream>>>(p2, n, x2, u2, V, H, K, NB, tw, out2);                         \
+    dgc_launch(dgstft::hop_lags_kernel<MM>, groups, MM, bytes, ctx->stream, p2, n, x2, u2, V, H, K, NB, tw, out2);     \
     break;
     HOP_CASES(pl.M)
 #undef CASE
     DGC_LAUNCHED(ctx, "hop_lags");
     return DGC_OK;
   }
-  partconv_ir_grad_kernel<<<dim3(dgc_div_up(NB, 32), K), 256, 0, ctx->stream>>>(x2, u2, V, H, NB, out2);
+  dgc_launch(partconv_ir_grad_kernel, dim3(dgc_div_up(NB, 32), K), 256, 0, ctx->stream, x2, u2, V, H, NB, out2);
   DGC_LAUNCHED(ctx, "partconv_ir_grad");
   return DGC_OK;
 }
@@ -591,8 +604,8 @@ DGC_EXPORT int32_t dgc_stft_fwd(dgc_ctx *ctx, const float *x_dev, int32_t V, int
   DGC_REQUIRE(ctx, (((uintptr_t)scr) & 7) == 0, "scratch must be 8-byte aligned");
   int32_t rc = dispatch_stft<0, 1>(ctx, N, x_dev, V, T, hop, H, window_dev, scr);
   if (rc != DGC_OK) return rc;
-  half_to_full_kernel<<<dgc_div_up((int64_t)bins, 256), 256, 0, ctx->stream>>>(reinterpret_cast<const float2 *>(scr), (int64_t)V * H, N,
-                                                                              re_dev, im_dev);
+  dgc_launch(half_to_full_kernel, dgc_div_up((int64_t)bins, 256), 256, 0, ctx->stream, reinterpret_cast<const float2 *>(scr),
+             (int64_t)V * H, N, re_dev, im_dev);
   DGC_LAUNCHED(ctx, "stft_full_bins");
   return DGC_OK;
 }
@@ -616,8 +629,8 @@ DGC_EXPORT int32_t dgc_istft_ola(dgc_ctx *ctx, const float *re_dev, const float 
   if (N >= 64)
     return istft16_ola(ctx, N, re_dev, im_dev, V, H, T, hop, window_dev, gain, 0, accumulate, frames, out_dev, in_place);
   const int64_t rows = (int64_t)V * H;
-  full_to_half_kernel<<<dgc_div_up(rows * NB, 256), 256, 0, ctx->stream>>>(re_dev, im_dev, rows, N,
-                                                                          reinterpret_cast<float2 *>(scr));
+  dgc_launch(full_to_half_kernel, dgc_div_up(rows * NB, 256), 256, 0, ctx->stream, re_dev, im_dev, rows, N,
+             reinterpret_cast<float2 *>(scr));
   DGC_LAUNCHED(ctx, "istft_hermitian_part");
   return istft_ola(ctx, N, scr, V, H, T, hop, window_dev, gain, 0, accumulate, frames, out_dev);
 }
@@ -720,7 +733,7 @@ DGC_EXPORT int32_t dgc_partconv_bwd(dgc_ctx *ctx, const float *x_dev, int32_t V,
     if (rc != DGC_OK) return rc;
     rc = istft_frames(ctx, N, gs, K, gain, frames);
     if (rc != DGC_OK) return rc;
-    take_partitions_kernel<<<dgc_div_up(ir_len, 256), 256, 0, ctx->stream>>>(frames, ir_len, N, hop, g_ir_dev);
+    dgc_launch(take_partitions_kernel, dgc_div_up(ir_len, 256), 256, 0, ctx->stream, frames, ir_len, N, hop, g_ir_dev);
     DGC_LAUNCHED(ctx, "take_partitions");
   }
   return DGC_OK;

@@ -56,6 +56,7 @@ template <int N, int SRC>
 __global__ void __launch_bounds__(THREADS, 6)
 stft16_kernel(const float *__restrict__ x, int T, int hop, int H, const float *__restrict__ window,
               const float2 *__restrict__ tw, float2 *__restrict__ out) {
+  dgc_after_previous();
   constexpr int TT = Geo<N>::T, NF = THREADS / TT, PN = Lay::template size<N>(), NB = N / 2 + 1;
   __shared__ float2 sm[NF * PN];
   const int f = threadIdx.x / TT, lt = threadIdx.x % TT, v = blockIdx.y;
@@ -104,6 +105,7 @@ template <int N, bool FULL, int S>
 __global__ void __launch_bounds__(THREADS, 4)
 istft16_kernel(const float *__restrict__ Y, const float *__restrict__ Yim, int H, int T, const float *__restrict__ window,
                const float2 *__restrict__ tw, float gain, int offset, int accumulate, int run, float *__restrict__ out) {
+  dgc_after_previous();
   constexpr int TT = Geo<N>::T, NF = THREADS / TT, PN = Lay::template size<N>(), NB = N / 2 + 1, RL = Geo<N>::RL, NBL = Geo<N>::NBL;
   constexpr int WARM = S ? (16 / (S ? S : 1)) / 2 : 0;       // pairs whose frames reach past their own two hops
   __shared__ float2 sm[2][NF * PN];
@@ -243,6 +245,7 @@ __device__ __forceinline__ void hop_inverse(float2 (&z)[Geo<M>::PAIRS][2][Geo<M>
 template <int M>
 __global__ void __launch_bounds__(M)
 hop_spectrum_kernel(const float2 *__restrict__ Hs, int K, int NB, const float2 *__restrict__ tw, float2 *__restrict__ G) {
+  dgc_after_previous();
   extern __shared__ float2 sm[];
   constexpr int RL = Geo<M>::RL, TT = Geo<M>::T;
   const int bin = threadIdx.x % HOP_BINS, lt = threadIdx.x / HOP_BINS, k = blockIdx.x * HOP_BINS + bin;
@@ -270,6 +273,7 @@ template <int M, bool ADJ>
 __global__ void __launch_bounds__(M, M <= 256 ? 512 / M : 1)
 hop_convolve_kernel(const float2 *__restrict__ X, const float2 *__restrict__ Hs, const float2 *__restrict__ G, int H, int K, int NB,
                     const float2 *__restrict__ tw, float2 *__restrict__ Y) {
+  dgc_after_previous();
   extern __shared__ float2 sm[];
   __shared__ int lo[HOP_BINS], hi[HOP_BINS], direct[HOP_BINS];
   constexpr int RL = Geo<M>::RL, TT = Geo<M>::T;
@@ -342,6 +346,7 @@ template <int M>
 __global__ void __launch_bounds__(M)
 hop_correlate_kernel(const float2 *__restrict__ X, const float2 *__restrict__ U, int V, int H, int K, int NB, int segs,
                      const float2 *__restrict__ tw, float2 *__restrict__ P) {
+  dgc_after_previous();
   extern __shared__ float2 sm[];
   constexpr int RL = Geo<M>::RL, TT = Geo<M>::T;
   const int bin = threadIdx.x % HOP_BINS, lt = threadIdx.x / HOP_BINS, k = blockIdx.x * HOP_BINS + bin;
@@ -398,6 +403,7 @@ template <int M>
 __global__ void __launch_bounds__(M)
 hop_lags_kernel(const float2 *__restrict__ P, int parts, const float2 *__restrict__ X, const float2 *__restrict__ U, int V, int H, int K,
                 int NB, const float2 *__restrict__ tw, float2 *__restrict__ G) {
+  dgc_after_previous();
   extern __shared__ float2 sm[];
   __shared__ int direct[HOP_BINS];
   if (threadIdx.x < HOP_BINS) direct[threadIdx.x] = 0;      // (barriers of the transform before it is used)

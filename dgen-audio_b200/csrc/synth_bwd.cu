@@ -24,6 +24,7 @@ __device__ __forceinline__ float sigmoid(float x) { return 1.0f / (1.0f + expf(-
 
 __global__ void heads_fwd_kernel(const float *__restrict__ z, int M, int K, int NB, float *__restrict__ amps,
                                  float *__restrict__ bands) {
+  dgc_after_previous();
   int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (row >= M) return;
   const float *zr = z + (size_t)row * (K + NB);
@@ -39,6 +40,7 @@ __global__ void heads_fwd_kernel(const float *__restrict__ z, int M, int K, int 
 // amps_k = p_k / D, D = sum p + eps  =>  dL/dp_k = (g_k - sum_j g_j amps_j) / D ; dp/dz = sigmoid(z)
 __global__ void heads_bwd_kernel(const float *__restrict__ z, const float *__restrict__ g_amps,
                                  const float *__restrict__ g_bands, int M, int K, int NB, float *__restrict__ gz) {
+  dgc_after_previous();
   int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (row >= M) return;
   const float *zr = z + (size_t)row * (K + NB);
@@ -81,6 +83,7 @@ __global__ void __launch_bounds__(256)
 fir_bwd_kernel(dgc_fir_params prm, const float *__restrict__ play, const int *__restrict__ ranges,
                const float *__restrict__ noise, const float *__restrict__ ngain, const float *__restrict__ g_audio,
                float *__restrict__ part_lo, float *__restrict__ part_hi, int32_t *status) {
+  dgc_after_previous();
   extern __shared__ __align__(16) float sh[];
   const int B = prm.B, T = prm.T, F = prm.F, NT = prm.taps;
   const int r = blockIdx.x, b = blockIdx.y, nth = blockDim.x;
@@ -156,6 +159,7 @@ fir_bwd_kernel(dgc_fir_params prm, const float *__restrict__ play, const int *__
 // the same four elements at a time (row_elems a multiple of 4, 16-byte aligned buffers); row_elems4 = row_elems / 4
 __global__ void combine_rows4_kernel(const float4 *__restrict__ part_lo, const float4 *__restrict__ part_hi, int F,
                                      unsigned row_elems4, float4 *__restrict__ grad) {
+  dgc_after_previous();
   const unsigned e = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
   if (e >= row_elems4) return;
   const unsigned rp = r == 0 ? (unsigned)F - 1 : r - 1;
@@ -166,6 +170,7 @@ __global__ void combine_rows4_kernel(const float4 *__restrict__ part_lo, const f
 // grad[r] = part_lo[r] + part_hi[r-1]  (the ceil row of floor row F-1 is row 0)
 __global__ void combine_rows_kernel(const float *__restrict__ part_lo, const float *__restrict__ part_hi, int F,
                                     size_t row_elems, float *__restrict__ grad) {
+  dgc_after_previous();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)F * row_elems) return;
   size_t r = i / row_elems, e = i - r * row_elems;
@@ -186,6 +191,7 @@ harmonic_bwd_kernel(dgc_harmonic_params prm, float rsr, const float *__restrict_
                     const float *__restrict__ amps, const float *__restrict__ gain,
                     const float *__restrict__ anchors, const float *__restrict__ g_audio,
                     float *__restrict__ part_lo, float *__restrict__ part_hi) {
+  dgc_after_previous();
   constexpr int G = 128 / LPC;
   const int B = prm.B, T = prm.T, K = prm.K, F = prm.F;
   const int C = (T + CH - 1) / CH;
@@ -335,6 +341,7 @@ harmonic_bwd_q_kernel(dgc_harmonic_params prm, float rsr, const float2 *__restri
                       const unsigned long long *__restrict__ fund, const int2 *__restrict__ trk,
                       const float2 *__restrict__ sums, const float *__restrict__ g_audio, float *__restrict__ part_lo,
                       float *__restrict__ part_hi) {
+  dgc_after_previous();
   constexpr int G = 128 / LPC;
   constexpr int LOG_LPC = LPC == 8 ? 3 : LPC == 16 ? 4 : 5;
   constexpr float THREE_PI = 9.42477796076938f;
@@ -545,12 +552,12 @@ void launch_combine_rows(dgc_ctx *ctx, const float *pl, const float *ph, int F, 
                    ((((uintptr_t)pl) | ((uintptr_t)ph) | ((uintptr_t)grad)) & 15) == 0;
   if (vec) {
     const unsigned re4 = (unsigned)(row_elems / 4);
-    combine_rows4_kernel<<<dim3(dgc_div_up((int64_t)re4, 256), F), 256, 0, ctx->stream>>>(
-        reinterpret_cast<const float4 *>(pl), reinterpret_cast<const float4 *>(ph), F, re4,
-        reinterpret_cast<float4 *>(grad));
+    dgc_launch(combine_rows4_kernel, dim3(dgc_div_up((int64_t)re4, 256), F), 256, 0, ctx->stream,
+               reinterpret_cast<const float4 *>(pl), reinterpret_cast<const float4 *>(ph), F, re4,
+               reinterpret_cast<float4 *>(grad));
   } else {
     const size_t n = (size_t)F * row_elems;
-    combine_rows_kernel<<<dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream>>>(pl, ph, F, row_elems, grad);
+    dgc_launch(combine_rows_kernel, dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream, pl, ph, F, row_elems, grad);
   }
 }
 
@@ -561,14 +568,14 @@ void launch_hbwd_q(dgc_ctx *ctx, const dgc_harmonic_params &p, const float2 *row
   constexpr int G = 128 / LPC;
   const dim3 grid(dgc_div_up(p.F, G), p.B);
   if (x.fund && x.trk && have_sums && x.sums)
-    harmonic_bwd_q_kernel<LPC, P, true, true><<<grid, 128, 0, ctx->stream>>>(
-        p, 1.0f / p.sample_rate, rowtab, ranges, x.f0t, x.env, amps, x.anchors_q, x.fund, x.trk, x.sums, g_audio, pl, ph);
+    dgc_launch(harmonic_bwd_q_kernel<LPC, P, true, true>, grid, 128, 0, ctx->stream, p, 1.0f / p.sample_rate, rowtab, ranges,
+               x.f0t, x.env, amps, x.anchors_q, x.fund, x.trk, x.sums, g_audio, pl, ph);
   else if (x.fund && x.trk)
-    harmonic_bwd_q_kernel<LPC, P, true, false><<<grid, 128, 0, ctx->stream>>>(
-        p, 1.0f / p.sample_rate, rowtab, ranges, x.f0t, x.env, amps, x.anchors_q, x.fund, x.trk, nullptr, g_audio, pl, ph);
+    dgc_launch(harmonic_bwd_q_kernel<LPC, P, true, false>, grid, 128, 0, ctx->stream, p, 1.0f / p.sample_rate, rowtab, ranges,
+               x.f0t, x.env, amps, x.anchors_q, x.fund, x.trk, nullptr, g_audio, pl, ph);
   else
-    harmonic_bwd_q_kernel<LPC, P, false, false><<<grid, 128, 0, ctx->stream>>>(
-        p, 1.0f / p.sample_rate, rowtab, ranges, x.f0t, x.env, amps, x.anchors_q, x.fund, x.trk, nullptr, g_audio, pl, ph);
+    dgc_launch(harmonic_bwd_q_kernel<LPC, P, false, false>, grid, 128, 0, ctx->stream, p, 1.0f / p.sample_rate, rowtab, ranges,
+               x.f0t, x.env, amps, x.anchors_q, x.fund, x.trk, nullptr, g_audio, pl, ph);
 }
 
 template <int LPC, int P>
@@ -576,8 +583,8 @@ void launch_hbwd(dgc_ctx *ctx, const dgc_harmonic_params &p, const float *play, 
                  const float *uv, const float *amps, const float *gain, const float *anchors, const float *g_audio,
                  float *pl, float *ph) {
   constexpr int G = 128 / LPC;
-  harmonic_bwd_kernel<LPC, P><<<dim3(dgc_div_up(p.F, G), p.B), 128, 0, ctx->stream>>>(
-      p, 1.0f / p.sample_rate, play, ranges, f0, uv, amps, gain, anchors, g_audio, pl, ph);
+  dgc_launch(harmonic_bwd_kernel<LPC, P>, dim3(dgc_div_up(p.F, G), p.B), 128, 0, ctx->stream, p, 1.0f / p.sample_rate, play,
+             ranges, f0, uv, amps, gain, anchors, g_audio, pl, ph);
 }
 
 }  // namespace
@@ -587,7 +594,7 @@ DGC_EXPORT int32_t dgc_hn_heads_fwd(dgc_ctx *ctx, const float *z_dev, int32_t M,
   if (!ctx) return DGC_ERR_INVALID;
   DGC_REQUIRE(ctx, z_dev && amps_dev && bands_dev, "null pointer");
   DGC_REQUIRE(ctx, M > 0 && K > 0 && NB > 0, "size out of range");
-  heads_fwd_kernel<<<dgc_div_up((int64_t)M * 32, 256), 256, 0, ctx->stream>>>(z_dev, M, K, NB, amps_dev, bands_dev);
+  dgc_launch(heads_fwd_kernel, dgc_div_up((int64_t)M * 32, 256), 256, 0, ctx->stream, z_dev, M, K, NB, amps_dev, bands_dev);
   DGC_LAUNCHED(ctx, "heads_fwd");
   return DGC_OK;
 }
@@ -597,8 +604,8 @@ DGC_EXPORT int32_t dgc_hn_heads_bwd(dgc_ctx *ctx, const float *z_dev, const floa
   if (!ctx) return DGC_ERR_INVALID;
   DGC_REQUIRE(ctx, z_dev && g_amps_dev && g_bands_dev && gz_dev, "null pointer");
   DGC_REQUIRE(ctx, M > 0 && K > 0 && NB > 0, "size out of range");
-  heads_bwd_kernel<<<dgc_div_up((int64_t)M * 32, 256), 256, 0, ctx->stream>>>(z_dev, g_amps_dev, g_bands_dev, M, K,
-                                                                             NB, gz_dev);
+  dgc_launch(heads_bwd_kernel, dgc_div_up((int64_t)M * 32, 256), 256, 0, ctx->stream, z_dev, g_amps_dev, g_bands_dev, M, K, NB,
+             gz_dev);
   DGC_LAUNCHED(ctx, "heads_bwd");
   return DGC_OK;
 }
@@ -620,8 +627,8 @@ DGC_EXPORT int32_t dgc_fir_noise_bwd(dgc_ctx *ctx, const dgc_fir_params *p, cons
   // four taps per thread, whole warps
   const int nth = dgc_div_up(dgc_div_up(p->taps, 4), 32) * 32;
   size_t smem = (size_t)(3 * FB_MAXRUN + 4 * nth + 16) * sizeof(float);
-  fir_bwd_kernel<<<dim3(p->F, p->B), nth, smem, ctx->stream>>>(*p, play, ranges, noise_dev, noise_gain_dev,
-                                                                g_audio_dev, part, part + n, ctx->status_dev);
+  dgc_launch(fir_bwd_kernel, dim3(p->F, p->B), nth, smem, ctx->stream, *p, play, ranges, noise_dev, noise_gain_dev, g_audio_dev,
+             part, part + n, ctx->status_dev);
   DGC_LAUNCHED(ctx, "fir_bwd");
   launch_combine_rows(ctx, part, part + n, p->F, (size_t)p->B * p->taps, g_taps_dev);
   DGC_LAUNCHED(ctx, "combine_rows");

@@ -282,6 +282,7 @@ template <bool A_KMAJOR, bool B_KMAJOR, int EPI, int BM, int BN>
 __global__ void __launch_bounds__(THREADS + 32, 1)
 tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const float *__restrict__ bias, int M, int N,
                int K, int k_per_split, float *__restrict__ C, float *__restrict__ Ct, int32_t *status) {
+  dgc_after_previous();
   extern __shared__ __align__(128) char smem[];
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * STAGE_BYTES);      // two "stage multiplied" mbarriers
   uint64_t *ready = bars + 2;                                                 // two "stage written"
@@ -464,6 +465,7 @@ template <int EPI, int BK, bool SW, int BN = TBN, bool A4 = false>
 __global__ void __launch_bounds__(KK_THREADS, (BK == 16 && BN == TBN) ? 2 : 1)
 tc_gemm_kk_kernel(const float *__restrict__ A, const float *__restrict__ B, const float *__restrict__ bias, int M, int N,
                   int K, int k_per_split, float *__restrict__ C, float *__restrict__ Ct, int32_t *status) {
+  dgc_after_previous();
   using G = KK<BK, SW, BN>;
   KK_STAMP(0);
   extern __shared__ __align__(128) char smem_base[];
@@ -700,6 +702,7 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
 __global__ void __launch_bounds__(SK::THREADS_ALL, 1)
 tc_gemm_smallk_kernel(const float *__restrict__ A, const float *__restrict__ B, int M, int N, int K, int nblk,
                       int n_extra, int ctas_per_blk, float *__restrict__ C, int32_t *status) {
+  dgc_after_previous();
   extern __shared__ __align__(128) char smem[];
   char *b_hi = smem + SK::OFF_BHI, *b_lo = smem + SK::OFF_BLO, *a_hi = smem + SK::OFF_AHI, *a_lo = smem + SK::OFF_ALO;
   float *lin = reinterpret_cast<float *>(smem + SK::OFF_LIN);
