@@ -115,6 +115,10 @@ bool dgc_linear_bwd_reads_t(int64_t M, int64_t K, int64_t N);
 // true when dgc_gemm_nt() runs this shape on its persistent short-reduction tensor-core kernel
 bool dgc_gemm_nt_persistent(const dgc_ctx *ctx, const float *a, int M, int N, int K);
 const float2 *dgc_ctx_twiddles(dgc_ctx *ctx, int N);
+// dgc_harmonic_render; by_partial: in FUNDAMENTAL mode one sine per partial and frame instead of groups of eight (osc_bank.cu)
+int32_t dgc_harmonic_render_impl(dgc_ctx *ctx, const dgc_harmonic_params *p, const float *f0_dev, const float *uv_dev,
+                                 const float *amps_dev, const float *gain_dev, float *scratch_dev, float *audio_dev,
+                                 bool by_partial);
 // dgc_onepole_fwd as three launches (linrec.cu)
 int32_t dgc_onepole_in_passes(dgc_ctx *ctx, const float *x_dev, int32_t B, int32_t T, float a, float *y_dev);
 // dgc_mss_loss_fwd with the voices in groups, each after its own event (mss_loss.cu)

@@ -69,6 +69,7 @@ __device__ __forceinline__ float partial_number(float kf0, int step_times_i) { r
 // env[b][n] = lerp(gain) * lerp(uv) * harmonic_scale, and in SCAN mode the anchors as Q0.32 turns.
 // In FUNDAMENTAL mode no per-partial anchors exist (anchors_out is not written): extra->fund replaces them.
 struct dgc_harmonic_extra {
+  bool no_f0t = false;                 // asked of the FUNDAMENTAL mode: the track itself is read by nobody
   const float *f0t = nullptr;          // [B][T] per-sample fundamental
   const float *env = nullptr;          // [B][T] or nullptr
   const uint32_t *anchors_q = nullptr; // [B][C][K] (SCAN mode only) or nullptr

@@ -151,7 +151,9 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
         const uint64_t fb = (uint64_t)p.F * p.B, bt = (uint64_t)p.B * p.T;
         const float *f0 = R.at(a[0], fb), *uv = R.at(a[1], fb), *amps = R.at(a[2], fb * p.K), *gain = R.at(a[3], fb);
         float *scr = R.at(a[4], dgc_harmonic_scratch_floats(&p), true), *out = R.at(a[5], bt);
-        if (!R.bad) rc = dgc_harmonic_render(ctx, &p, f0, uv, amps, gain, scr, out);
+        // A step that keeps the scratch for its backward renders partial by partial, with the sines that the backward takes
+        // again: gradients of the log magnitudes hang on the audio's last bits (6e-8 of it moves a step's gradients by 3e-2).
+        if (!R.bad) rc = dgc_harmonic_render_impl(ctx, &p, f0, uv, amps, gain, scr, out, scr != nullptr);
       } break;
       case DGC_PLAN_BANDS_TO_TAPS: {
         const float *bands = R.at(a[0], (uint64_t)i[0] * i[1]), *w = R.at(a[1], (uint64_t)i[2] * i[1]);
