@@ -484,6 +484,7 @@ __device__ __forceinline__ bool biquad_stage(const float *__restrict__ xb, int T
   const int64_t i0 = (int64_t)blockIdx.x * blockDim.x, i = i0 + threadIdx.x, pairs = (int64_t)NC * L;
   const int c0 = (int)(i0 / L), c1 = (int)((min(i0 + blockDim.x, pairs) - 1) / L);
   const int span = (c1 - c0 + 1) * BQ_CHUNK + 2, t0 = c0 * BQ_CHUNK - 2;
+  sm += 2;                                      // a chunk's frames start at a multiple of 16 bytes
   for (int j = threadIdx.x; j < span; j += blockDim.x) sm[j] = t0 + j >= 0 && t0 + j < T ? xb[t0 + j] : 0.0f;
   __syncthreads();
   if (i >= pairs) return false;
@@ -507,7 +508,7 @@ biquad_fwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, i
                   float *__restrict__ state /* [B][NC][L][2] */, float *__restrict__ y,
                   const float *__restrict__ st0 = nullptr /* [B][4][L]: history cells before the call */) {
   dgc_after_previous();
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   const int b = blockIdx.y;
   int c, l;
   const float *xc;
@@ -526,13 +527,26 @@ biquad_fwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, i
     x2 = st0[((size_t)b * 4 + 3) * L + l];
   }
   float *yo = y + ((size_t)b * T + n0) * L + l;
-#pragma unroll 4
-  for (int n = 0; n < len; ++n) {
-    float x0 = xc[n];
-    float v = biquad_step(cf, x0, x1, x2, y1, y2);
-    if (PHASE == 1) yo[(size_t)n * L] = v;
+  auto step = [&](float x0) {
+    const float v = biquad_step(cf, x0, x1, x2, y1, y2);
+    if (PHASE == 1) {
+      *yo = v;
+      yo += L;
+    }
     x2 = x1; x1 = x0; y2 = y1; y1 = v;
+  };
+  int n = 0;
+  float4 next = *reinterpret_cast<const float4 *>(xc);   // four frames ahead of the recursion
+#pragma unroll 2
+  for (; n + 4 <= len; n += 4) {
+    const float4 now = next;
+    if (n + 8 <= len) next = *reinterpret_cast<const float4 *>(xc + n + 4);
+    step(now.x);
+    step(now.y);
+    step(now.z);
+    step(now.w);
   }
+  for (; n < len; ++n) step(xc[n]);
   if (PHASE == 0) {
     st[0] = y1;
     st[1] = y2;
@@ -552,7 +566,7 @@ biquad_fwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, i
 // Coefficients, the homogeneous transition M over one chunk, (y1, y2)_end = M (y1, y2)_start for zero input, and (G not null)
 // the table, in one launch: a warp per lane, whose first two threads walk the recursion from (1, 0) -- those are the hy[k]
 // -- and from (0, 1).  M's entries are large with cancelling signs where the poles are close to the unit circle: double.
-// Bound by the walk, 512 dependent steps: 11 us for 256 lanes; 54 us when a thread per lane did all of it in three kernels
+// Bound by the walk, 512 dependent steps: 10.5 us for 256 lanes; 54 us when a thread per lane did all of it in three kernels
 // and wrote its row of G value by value.
 __global__ void __launch_bounds__(128)
 biquad_tables_kernel(const float *__restrict__ cutoff, const float *__restrict__ q, int L, float gain, float mode,
@@ -568,6 +582,7 @@ biquad_tables_kernel(const float *__restrict__ cutoff, const float *__restrict__
   const double b0 = __ldcg(cp), b1 = __ldcg(cp + 1), b2 = __ldcg(cp + 2), a1 = __ldcg(cp + 3), a2 = __ldcg(cp + 4);
   double *hy = hys[warp] + 2;                  // hy[-2], hy[-1]: zero
   if (lane < 2) {
+    const double n1 = -a1, n2 = -a2;           // the sign ahead of the products: one step less in the chain, the same value
     double y1 = lane == 0 ? 1.0 : 0.0, y2 = lane == 0 ? 0.0 : 1.0;
     if (lane == 0) {
       hy[-2] = hy[-1] = 0.0;
@@ -576,7 +591,7 @@ biquad_tables_kernel(const float *__restrict__ cutoff, const float *__restrict__
     for (int n = 0; n < BQ_CHUNK; n += 4) {    // the order of rounding of four steps as it always was, see BiquadSweep
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const double v = j == 0 ? -__fma_rn(a1, y1, __dmul_rn(a2, y2)) : -__fma_rn(a2, y2, __dmul_rn(a1, y1));
+        const double v = j == 0 ? __fma_rn(n1, y1, __dmul_rn(n2, y2)) : __fma_rn(n2, y2, __dmul_rn(n1, y1));
         y2 = y1;
         y1 = v;
         if (lane == 0 && n + j + 1 < BQ_CHUNK) hy[n + j + 1] = v;
@@ -667,7 +682,8 @@ biquad_fwd4_kernel(const float *__restrict__ x, const float *__restrict__ coef, 
 // The next BQ_AHEAD chunks are in flight while the present ones are walked.  Not a scan by runs: a last-bit change of a
 // state is 140 times as much in the output of a low, sharp lane, and 10000 times in the gradient of its cutoff.
 // hist (optional): the end states come from the matrix product, which knows nothing of the x-history before a chunk: its
-// two terms are added here.  32 voices x 512 chunks x 256 lanes: 70 us, 110 us as two kernels with a load in every step.
+// two terms are added here.  Bound by the instructions of a lone warp: pointers that step and no tests in a whole run of chunks,
+// 32 voices x 512 chunks x 256 lanes 70 -> 25 us, 5 x 98 x 37 14 -> 6.
 constexpr int BQ_AHEAD = 16;
 __global__ void __launch_bounds__(32)
 biquad_carry_kernel(const double *__restrict__ trans, const float *__restrict__ x, const float *__restrict__ hist, int T, int L,
@@ -684,19 +700,20 @@ biquad_carry_kernel(const double *__restrict__ trans, const float *__restrict__ 
   // y[-1], y[-2]: the history cells before the call, else rest
   double s1 = st0 ? (double)st0[((size_t)b * 4 + 0) * L + l] : 0.0, s2 = st0 ? (double)st0[((size_t)b * 4 + 1) * L + l] : 0.0;
   float2 e[BQ_AHEAD], xx[BQ_AHEAD];
-  auto fetch = [&](int c0) {
+  const float2 *pe = st;                     // where the next chunks' end states lie, the last frames before them, their states
+  const float *px = xb - 2;
+  float2 *ps = st;
+  auto fetch = [&](int c0, auto whole) {
 #pragma unroll
-    for (int j = 0; j < BQ_AHEAD; ++j) {
-      const int c = c0 + j;
-      if (c < NC) {
-        e[j] = st[(size_t)c * L];
-        if (hist && c > 0) xx[j] = make_float2(__ldg(xb + (size_t)c * BQ_CHUNK - 1), __ldg(xb + (size_t)c * BQ_CHUNK - 2));
+    for (int j = 0; j < BQ_AHEAD; ++j, pe += L, px += BQ_CHUNK) {
+      if (decltype(whole)::value || c0 + j < NC) {
+        e[j] = *pe;
+        if (hist && c0 + j > 0) xx[j] = make_float2(__ldg(px + 1), __ldg(px));
       }
     }
     if (hist && c0 == 0 && st0) xx[0] = make_float2(st0[((size_t)b * 4 + 2) * L + l], st0[((size_t)b * 4 + 3) * L + l]);
   };
-  fetch(0);
-  for (int c0 = 0; c0 < NC; c0 += BQ_AHEAD) {
+  auto walk = [&](int c0, auto whole) {
     float2 v[BQ_AHEAD];
 #pragma unroll
     for (int j = 0; j < BQ_AHEAD; ++j) {
@@ -706,11 +723,12 @@ biquad_carry_kernel(const double *__restrict__ trans, const float *__restrict__ 
         v[j].y += h.y * xx[j].x + h.w * xx[j].y;
       }
     }
-    fetch(c0 + BQ_AHEAD);
+    if (c0 + 2 * BQ_AHEAD <= NC) fetch(c0 + BQ_AHEAD, std::true_type());
+    else fetch(c0 + BQ_AHEAD, std::false_type());
 #pragma unroll
-    for (int j = 0; j < BQ_AHEAD; ++j) {
-      if (c0 + j < NC) {
-        st[(size_t)(c0 + j) * L] = make_float2((float)s1, (float)s2);
+    for (int j = 0; j < BQ_AHEAD; ++j, ps += L) {
+      if (decltype(whole)::value || c0 + j < NC) {
+        *ps = make_float2((float)s1, (float)s2);
         // every chunk but possibly the last has full length; the state after the last chunk is unused
         const double e1 = v[j].x, e2 = v[j].y;
         const double n1 = m11 * s1 + m12 * s2 + e1, n2 = m21 * s1 + m22 * s2 + e2;
@@ -718,7 +736,11 @@ biquad_carry_kernel(const double *__restrict__ trans, const float *__restrict__ 
         s2 = n2;
       }
     }
-  }
+  };
+  fetch(0, std::false_type());
+  int c0 = 0;
+  for (; c0 + BQ_AHEAD <= NC; c0 += BQ_AHEAD) walk(c0, std::true_type());
+  if (c0 < NC) walk(c0, std::false_type());
 }
 
 // Backward sweep for loss = scale * sum (y - t)^2.  Adjoint recurrence (transposed filter, reverse time):
@@ -738,48 +760,77 @@ __device__ __forceinline__ float feedback(const Coef &c, float p, float q, bool 
   return a2_first ? __fmaf_rn(c.a1, p, __fmul_rn(c.a2, q)) : __fmaf_rn(c.a2, q, __fmul_rn(c.a1, p));
 }
 
-template <bool UP>
-struct BiquadSweep {
-  Coef cf;
-  float gscale, yc, ym1;                     // y[n], y[n-1]
-  float la1 = 0.f, la2 = 0.f;                // lam[n+1], lam[n+2] (local)
-  float h1a = 1.f, h1b = 0.f;                // homogeneous response to terminal (lam[n_end+1], lam[n_end+2]) = (1,0)
-  float h2a = 0.f, h2b = 1.f;                // ... = (0,1)
-  float S[15] = {}, sq = 0.f;
-
-  // frame n: x[n], x[n-1], x[n-2], y[n-2], target
-  __device__ __forceinline__ void step(float x0, float x1, float x2, float ym2, float tv, bool a2_first) {
-    const float fed = feedback(cf, la1, la2, true), d = UP ? 0.0f : __fsub_rn(yc, tv);
-    if (!UP) sq = fmaf(d, d, sq);
-    const float lam = UP ? __fsub_rn(tv, fed) : __fmaf_rn(gscale, d, -fed);
-    const float h1 = -feedback(cf, h1a, h1b, a2_first), h2 = -feedback(cf, h2a, h2b, a2_first);
-    S[0] = fmaf(lam, x0, S[0]); S[1] = fmaf(lam, x1, S[1]); S[2] = fmaf(lam, x2, S[2]);
-    S[3] = fmaf(lam, ym1, S[3]); S[4] = fmaf(lam, ym2, S[4]);
-    S[5] = fmaf(h1, x0, S[5]); S[6] = fmaf(h1, x1, S[6]); S[7] = fmaf(h1, x2, S[7]);
-    S[8] = fmaf(h1, ym1, S[8]); S[9] = fmaf(h1, ym2, S[9]);
-    S[10] = fmaf(h2, x0, S[10]); S[11] = fmaf(h2, x1, S[11]); S[12] = fmaf(h2, x2, S[12]);
-    S[13] = fmaf(h2, ym1, S[13]); S[14] = fmaf(h2, ym2, S[14]);
-    la2 = la1; la1 = lam;
-    h1b = h1a; h1a = h1;
-    h2b = h2a; h2a = h2;
-    yc = ym1; ym1 = ym2;
+// a response of the adjoint recurrence to a terminal state (lam[n_end+1], lam[n_end+2]) = (p, q), and its five sums
+struct BiquadResponse {
+  float p, q;
+  float S[5] = {};
+  __device__ __forceinline__ BiquadResponse(float p, float q) : p(p), q(q) {}
+  __device__ __forceinline__ void step(const Coef &cf, float x0, float x1, float x2, float ym1, float ym2, bool a2_first) {
+    const float h = -feedback(cf, p, q, a2_first);
+    S[0] = fmaf(h, x0, S[0]); S[1] = fmaf(h, x1, S[1]); S[2] = fmaf(h, x2, S[2]);
+    S[3] = fmaf(h, ym1, S[3]); S[4] = fmaf(h, ym2, S[4]);
+    q = p; p = h;
   }
   __device__ __forceinline__ void record(float *r, int L) const {
 #pragma unroll
-    for (int i = 0; i < 15; ++i) r[(size_t)i * L] = S[i];
+    for (int i = 0; i < 5; ++i) r[(size_t)i * L] = S[i];
+  }
+};
+
+// the local adjoint from rest, its sums, the squared error
+template <bool UP>
+struct BiquadAdjoint {
+  float la1 = 0.f, la2 = 0.f;                // lam[n+1], lam[n+2]
+  float S[5] = {}, sq = 0.f;
+  __device__ __forceinline__ void step(const Coef &cf, float gscale, float x0, float x1, float x2, float yc, float ym1, float ym2,
+                                       float tv) {
+    const float fed = feedback(cf, la1, la2, true), d = UP ? 0.0f : __fsub_rn(yc, tv);
+    if (!UP) sq = fmaf(d, d, sq);
+    const float lam = UP ? __fsub_rn(tv, fed) : __fmaf_rn(gscale, d, -fed);
+    S[0] = fmaf(lam, x0, S[0]); S[1] = fmaf(lam, x1, S[1]); S[2] = fmaf(lam, x2, S[2]);
+    S[3] = fmaf(lam, ym1, S[3]); S[4] = fmaf(lam, ym2, S[4]);
+    la2 = la1; la1 = lam;
+  }
+  __device__ __forceinline__ void record(float *r, int L) const {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) r[(size_t)i * L] = S[i];
     r[(size_t)15 * L] = la1;  // local adjoint at the first frame of the chunk: lam[n0]
     r[(size_t)16 * L] = la2;  // lam[n0+1]
     r[(size_t)17 * L] = sq;
   }
 };
 
+template <bool UP>
+struct BiquadSweep {
+  Coef cf;
+  float gscale, yc, ym1;                     // y[n], y[n-1]
+  BiquadAdjoint<UP> adj;
+  BiquadResponse h1{1.f, 0.f}, h2{0.f, 1.f};
+
+  // frame n: x[n], x[n-1], x[n-2], y[n-2], target
+  __device__ __forceinline__ void step(float x0, float x1, float x2, float ym2, float tv, bool a2_first) {
+    adj.step(cf, gscale, x0, x1, x2, yc, ym1, ym2, tv);
+    h1.step(cf, x0, x1, x2, ym1, ym2, a2_first);
+    h2.step(cf, x0, x1, x2, ym1, ym2, a2_first);
+    yc = ym1; ym1 = ym2;
+  }
+  __device__ __forceinline__ void record(float *r, int L) const {
+    adj.record(r, L);
+    h1.record(r + (size_t)5 * L, L);
+    h2.record(r + (size_t)10 * L, L);
+  }
+};
+
 // UP = false: g = gscale * (y - tgt) (the MSE loss, squared error summed on the way);  UP = true: `tgt` IS the
 // upstream gradient dL/dy [B][T][L] of an arbitrary loss.
 // A group of sixteen frames issues its 32 loads before the dependent recurrence steps: the sweep is bound by loads in
-// flight (32 voices x 262144 x 256 lanes: 17.2 GB in 3.20 ms, 82 % of the copy rate).  In the first and the last chunk frames
-// outside the chunk or the signal are zeros; with a load in every step those two took three times as long as the others,
-// and a bank of few lanes as long as they: 5 voices x 50001 x 37 lanes 124 us, now 76.  Asynchronous copies to a ring in
-// shared memory were measured: 6 % slower on the large bank, 66 us on this one but 80 for 61 with 64 lanes.
+// flight (32 voices x 262144 x 256 lanes: 17.2 GB in 3.12 ms, 84 % of the copy rate; 3.58 with 116 registers, a block less on an
+// SM, when the frames of x were read one by one).  In the first and the last chunk frames
+// outside the chunk or the signal are zeros.  A small bank takes as long as its slowest warp: only the groups that reach out of
+// the chunk test their frames, and a warp with lanes of an edge chunk and of others walks them together; testing every frame,
+// one kind after the other, 5 voices x 50001 x 37 lanes took 75 us, now 35.  A thread each for the adjoint and the two
+// responses there: 3 us less at 145 blocks, 20 % more at 384.  Asynchronous copies to a ring in
+// shared memory were measured: 6 % slower on the large bank.
 template <bool UP>
 __global__ void __launch_bounds__(BQ_THREADS)
 biquad_bwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, const float *__restrict__ y,
@@ -796,33 +847,41 @@ biquad_bwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, c
   const float *yb = y + ((size_t)b * T + n0) * L + l, *tb = tgt + ((size_t)b * T + n0) * L + l;
   auto y_at = [&](int n) { return n0 + n >= 0 ? yb[(ptrdiff_t)n * L] : 0.0f; };
   BiquadSweep<UP> w{load_coef(coef, l), gscale, y_at(len - 1), y_at(len - 2)};
-  if (len == BQ_CHUNK && n0 >= 2) {
-    auto group = [&](int nb, auto first) {
-      float yv[G], tv[G];
+  // edge chunks: the first, whose frames reach back before the signal, and a short last one
+  const bool edge = len < BQ_CHUNK || n0 < 2;
+  auto group = [&](int nb, auto whole, auto any_edge) {   // whole: no frame of it outside the chunk or before the signal
+    float yv[G], tv[G];
 #pragma unroll
-      for (int j = 0; j < G; ++j) {
-        yv[j] = __ldcs(yb + (ptrdiff_t)(nb + j - 2) * L);
-        tv[j] = __ldcs(tb + (ptrdiff_t)(nb + j) * L);
-      }
-#pragma unroll
-      for (int j = G - 1; j >= 0; --j)
-        w.step(xc[nb + j], xc[nb + j - 1], xc[nb + j - 2], yv[j], tv[j], j == G - 1 || (decltype(first)::value && j == G - 2));
-    };
-    group(BQ_CHUNK - G, std::true_type());
-    for (int nb = BQ_CHUNK - 2 * G; nb >= 0; nb -= G) group(nb, std::false_type());
-  } else {
-    for (int nb = (len - 1) / G * G; nb >= 0; nb -= G) {
-      float yv[G], tv[G];
-#pragma unroll
-      for (int j = 0; j < G; ++j) {
-        const int n = nb + j;
-        yv[j] = n < len && n0 + n >= 2 ? __ldcs(yb + (ptrdiff_t)(n - 2) * L) : 0.0f;
-        tv[j] = n < len ? __ldcs(tb + (ptrdiff_t)n * L) : 0.0f;
-      }
-#pragma unroll
-      for (int j = G - 1; j >= 0; --j)
-        if (nb + j < len) w.step(xc[nb + j], xc[nb + j - 1], xc[nb + j - 2], yv[j], tv[j], j & 1);
+    for (int j = 0; j < G; ++j) {
+      const int n = nb + j;
+      yv[j] = decltype(whole)::value || (n < len && n0 + n >= 2) ? __ldcs(yb + (ptrdiff_t)(n - 2) * L) : 0.0f;
+      tv[j] = decltype(whole)::value || n < len ? __ldcs(tb + (ptrdiff_t)n * L) : 0.0f;
     }
+    float xv[G + 2];                            // x[nb - 2 .. nb + G)
+    {
+      const float2 q = *reinterpret_cast<const float2 *>(xc + nb - 2);
+      xv[0] = q.x; xv[1] = q.y;
+    }
+#pragma unroll
+    for (int j = 0; j < G; j += 4) {
+      const float4 q = *reinterpret_cast<const float4 *>(xc + nb + j);
+      xv[j + 2] = q.x; xv[j + 3] = q.y; xv[j + 4] = q.z; xv[j + 5] = q.w;
+    }
+    const bool last = nb == BQ_CHUNK - G;
+#pragma unroll
+    for (int j = G - 1; j >= 0; --j) {
+      const bool a2_first = j == G - 1 || (decltype(any_edge)::value && edge ? (j & 1) != 0 : j == G - 2 && last);
+      if (decltype(whole)::value || nb + j < len) w.step(xv[j + 2], xv[j + 1], xv[j], yv[j], tv[j], a2_first);
+    }
+  };
+  if (__any_sync(__activemask(), edge)) {
+    for (int nb = BQ_CHUNK - G; nb >= 0; nb -= G) {
+      if (nb + G <= len && n0 + nb >= 2) group(nb, std::true_type(), std::true_type());
+      else if (nb < len) group(nb, std::false_type(), std::true_type());
+    }
+  } else {
+    group(BQ_CHUNK - G, std::true_type(), std::false_type());
+    for (int nb = BQ_CHUNK - 2 * G; nb >= 0; nb -= G) group(nb, std::true_type(), std::false_type());
   }
   w.record(rec + ((size_t)b * NC + c) * BW_REC * L + l, L);
 }
@@ -917,7 +976,8 @@ biquad_bwd_carry_kernel(const float *__restrict__ rec, const float *__restrict__
 // kernel), recomputes lam; the sum over the block's 128 lanes goes through a shared-memory tile of 32 frames, the
 // sum over lane blocks through per-block partial rows that a last kernel adds in a fixed order.
 // Bound by the walk's instructions: no tests in a whole group of frames, a pointer that steps, nothing to walk for a warp
-// without lanes: 5 voices x 50001 x 37 lanes 42 -> 27 us, 300 lanes 120 -> 80.  (The next group's loads sent ahead: 46 and 115.)
+// without lanes, a quarter of the lanes per warp in the sums: 5 voices x 50001 x 37 lanes 42 -> 24.5 us, 300 lanes 120 -> 80.
+// (The next group's loads sent ahead in registers: 46 and 115; by asynchronous copies: 22 us there, 7 % slower with 100 lanes.)
 constexpr int GX_FRAMES = 32;
 
 __global__ void __launch_bounds__(BQ_THREADS)
@@ -926,6 +986,8 @@ biquad_gx_kernel(const float *__restrict__ coef, const float *__restrict__ gy, c
                  float *__restrict__ part /* [gridDim.x][B][T] */) {
   dgc_after_previous();
   __shared__ float red[GX_FRAMES][BQ_THREADS + 1];
+  __shared__ float quarter[4][GX_FRAMES];
+  const int quarters = min(4, (L - (int)blockIdx.x * BQ_THREADS + 31) / 32);   // those with lanes
   const int tid = threadIdx.x, l = blockIdx.x * BQ_THREADS + tid, c = blockIdx.y, b = blockIdx.z;
   const int n0 = c * BQ_CHUNK, len = min(BQ_CHUNK, T - n0);
   const bool live = l < L;
@@ -966,17 +1028,19 @@ biquad_gx_kernel(const float *__restrict__ coef, const float *__restrict__ gy, c
       else walk(std::false_type());
     }
     __syncthreads();
-    // thread -> (frame j = tid / 4, quarter of the lanes): 32 adds, then the four quarters by shuffles
+    // warp -> quarter of the lanes, thread -> frame: 32 adds, then the four quarters
     {
-      const int j = tid >> 2, seg = tid & 3;
+      const int j = tid & 31, seg = tid >> 5;
       float sum = 0.f;
+      if (seg < quarters) {
 #pragma unroll 8
-      for (int k = 0; k < BQ_THREADS / 4; ++k) sum += red[j][seg * (BQ_THREADS / 4) + ((k + tid) & (BQ_THREADS / 4 - 1))];
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      if (seg == 0 && j < cnt) pb[n0 + lo + j] = sum;
+        for (int k = 0; k < BQ_THREADS / 4; ++k)
+          sum += red[j][seg * (BQ_THREADS / 4) + ((k + 4 * j + seg) & (BQ_THREADS / 4 - 1))];
+      }
+      quarter[seg][j] = sum;
     }
     __syncthreads();
+    if (tid < cnt) pb[n0 + lo + tid] = (quarter[0][tid] + quarter[1][tid]) + (quarter[2][tid] + quarter[3][tid]);
   }
 }
 
@@ -1183,9 +1247,9 @@ static int32_t biquad_backward(dgc_ctx *ctx, const dgc_biquad_params *p, const f
   dgc_launch(biquad_coef_kernel, dgc_div_up(L, 32), 32, 0, ctx->stream, cutoff, q, L, p->gain, p->mode, coef);
   DGC_LAUNCHED(ctx, "biquad_coef");
   const int nth = biquad_pairs(L), smem = biquad_stage_bytes(L);
+  const dim3 grid((unsigned)(((int64_t)NC * L + nth - 1) / nth), B);
   if (smem > 48 * 1024)
     DGC_CUDA(ctx, cudaFuncSetAttribute(biquad_bwd_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  const dim3 grid((unsigned)(((int64_t)NC * L + nth - 1) / nth), B);
   dgc_launch(biquad_bwd_kernel<UP>, grid, nth, smem, ctx->stream, x, coef, y, up, T, L, NC, gscale, rec);
   DGC_LAUNCHED(ctx, "biquad_bwd");
   dgc_launch(biquad_bwd_carry_kernel, dim3(dgc_div_up(L, 32), B), dim3(32, BQ_RUNS), 0, ctx->stream, rec, coef, L, NC, acc, term);
