@@ -142,22 +142,15 @@ int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *
                      float *Ct = nullptr, bool *ct_written = nullptr) {
   if (ct_written) *ct_written = false;
   const bool tc = use_tensor_cores() && (double)M * N * K >= (double)(1 << 21) && K >= 32;
-  static const int kk_bk = [] {   // DGC_GEMM_KK: 0 off; 16 (default) / 32: swizzled 16- / 32-wide k tiles; 17 / 33: the
-                                  // same without swizzle; 256: 16-wide k tiles with 128 x 256 output tiles where N >= 256
-    const char *e = getenv("DGC_GEMM_KK");
-    return e ? atoi(e) : 16;
-  }();
-  // the asynchronous pipeline needs both operands contiguous along k, K a multiple of 4 and aligned rows
-  const bool kk16 = tc && !TA && TB && kk_bk && (K & 3) == 0 && ((((uintptr_t)A) | ((uintptr_t)B)) & 15) == 0;
-  // rows that are not 16-byte aligned (K % 4 != 0, e.g. 65 band magnitudes): the same pipeline with 4-byte copies
-  const bool kk4 = tc && !TA && TB && kk_bk && !kk16 && EPI == 0;
-  const bool kk = kk16 || kk4;
-  // 128 x 256 tiles, one CTA per SM: 25 % less shared-memory traffic per flop, but prologue and epilogue are no
-  // longer hidden by a second resident CTA, so they only pay where a CTA runs a long reduction -- the split-K
-  // weight gradients (measured: training step 3.84 -> 3.78 ms; the forward layers get 4 % slower with them).
-  // DGC_GEMM_KK=256 forces them wherever N >= 256.
-  const bool long_reduction = EPI == 0 && K >= 2048 && dgc_div_up(N, dgtc::TBN) * dgc_div_up(M, dgtc::TBM) < ctx->sm_count;
-  const bool wide = kk16 && N >= 256 && (kk_bk == 256 || (kk_bk == 16 && long_reduction));
+  // both operands contiguous along k: rows of 16-byte units (A in tensor memory, 16-byte aligned rows), or any (4-byte copies,
+  // e.g. 165 outputs of the controller's heads)
+  const bool along_k = tc && !TA && TB;
+  const bool kk16 = along_k && (K & 3) == 0 && ((((uintptr_t)A) | ((uintptr_t)B)) & 15) == 0;
+  const bool kk = kk16 || (along_k && EPI == 0);
+  // 128 x 256 tiles: 12 % less shared-memory traffic per flop, but one accumulator and so an epilogue that nothing hides: where
+  // a CTA runs one long reduction, the split-K weight gradients
+  const bool wide = kk16 && N >= 256 && EPI == 0 && K >= 2048 &&
+                    dgc_div_up(N, dgtc::TBN) * dgc_div_up(M, dgtc::TBM) < ctx->sm_count;
   // short reductions (the band -> tap map): persistent CTAs that keep their block of B in shared memory
   if (!TA && TB && EPI == 0 && smallk_shape(ctx, A, M, N, K)) {
     const int rem = N % dgtc::TBN;
@@ -176,8 +169,8 @@ int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *
   const int tiles = dgc_div_up(N, bn) * dgc_div_up(M, bm);
   int splits = 1;
   if (EPI == 0 && tiles < ctx->sm_count && K >= 2048) {
-    // few output tiles and a long reduction (weight gradients): split the reduction over blocks -- two resident
-    // CTAs per SM for the narrow tiles, one (and never a second, nearly empty wave) for the wide ones
+    // few output tiles and a long reduction (weight gradients): split the reduction over blocks -- two per SM for the narrow
+    // tiles, one (and never a second, nearly empty wave) for the wide ones
     splits = wide ? ctx->sm_count / tiles : (2 * ctx->sm_count + tiles - 1) / tiles;
     if (splits > K / 256) splits = K / 256;
     if (splits < 1) splits = 1;
@@ -196,36 +189,26 @@ int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *
   const bool few = tc && splits == 1 && (int64_t)dgc_div_up(M, 64) * dgc_div_up(N, 64) <= ctx->sm_count;
   const bool piped = kk && !few && (splits == 1 || kps % 32 == 0);
   ctx->gemm_paths[piped ? (wide ? 3 : 2) : (tc ? 1 : 0)]++;
-  if (piped) {
-    // both operands contiguous along k: the cp.async pipeline
-#define DGC_KK_LAUNCH(BKV, SWV)                                                                                      \
-  do {                                                                                                              \
-    auto kern = dgtc::tc_gemm_kk_kernel<EPI, BKV, SWV, dgtc::TBN>;                                                  \
-    constexpr int SM = dgtc::KK<BKV, SWV, dgtc::TBN>::SMEM;                                                         \
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);                    \
-    if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));     \
-    dgc_launch(kern, grid, dgtc::KK_THREADS, SM, ctx->stream, A, B, bias, M, N, K, kps, dst, splits == 1 ? Ct : nullptr,    \
-                                                   ctx->status_dev);                                                \
-  } while (0)
-    if (kk4) {
-      auto kern = dgtc::tc_gemm_kk_kernel<0, 16, true, dgtc::TBN, true>;
-      constexpr int SM = dgtc::KK<16, true, dgtc::TBN>::SMEM;
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
-      if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));
-      dgc_launch(kern, grid, dgtc::KK_THREADS, SM, ctx->stream, A, B, nullptr, M, N, K, kps, dst, nullptr, ctx->status_dev);
-    } else if (wide) {
-      auto kern = dgtc::tc_gemm_kk_kernel<EPI, 16, true, 256>;
-      constexpr int SM = dgtc::KK<16, true, 256>::SMEM;
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
-      if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));
-      dgc_launch(kern, grid, dgtc::KK_THREADS, SM, ctx->stream, A, B, bias, M, N, K, kps, dst, splits == 1 ? Ct : nullptr,
-                 ctx->status_dev);
-    } else if (kk_bk == 16 || kk_bk == 256) DGC_KK_LAUNCH(16, true);
-    else if (kk_bk == 17) DGC_KK_LAUNCH(16, false);
-    else if (kk_bk == 33) DGC_KK_LAUNCH(32, false);
-    else DGC_KK_LAUNCH(32, true);
-#undef DGC_KK_LAUNCH
+  if (piped && kk16) {
+    auto kern = dgtc::tc_gemm_ts_kernel<EPI, dgtc::TBN>;
+    if constexpr (EPI == 0) {
+      if (wide) kern = dgtc::tc_gemm_ts_kernel<EPI, 256>;
+    }
+    const int smem = wide ? dgtc::TS<256>::SMEM : dgtc::TS<dgtc::TBN>::SMEM;
+    CUtensorMap map_a, map_b;
+    if (!dgtma::make_map_k16(&map_a, A, M, K, dgtc::TBM) || !dgtma::make_map_k16(&map_b, B, N, K, bn))
+      return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm: no tensor map for %d x %d x %d", M, N, K);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));
+    const int64_t items = (int64_t)grid.x * grid.y * grid.z;
+    dgc_launch(kern, (unsigned)std::min<int64_t>(items, ctx->sm_count), dgtc::TS<dgtc::TBN>::THREADS_ALL, smem, ctx->stream, map_a,
+               map_b, bias, M, N, K, kps, (int)items, dst, splits == 1 ? Ct : nullptr, ctx->status_dev);
     if (ct_written) *ct_written = Ct && splits == 1;
+  } else if (piped) {
+    auto kern = dgtc::tc_gemm_kk4_kernel;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dgtc::KK::SMEM);
+    if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));
+    dgc_launch(kern, grid, dgtc::KK_THREADS, dgtc::KK::SMEM, ctx->stream, A, B, M, N, K, kps, dst, ctx->status_dev);
   } else if (tc) {
     // tensor-core kernel: operand A is K-major in memory when it is NOT transposed ([M][K]);
     // operand B is K-major in memory when it IS given transposed ([N][K])
@@ -773,13 +756,3 @@ DGC_EXPORT int32_t dgc_gemm_path_counts(dgc_ctx *ctx, int64_t *out4) {
   return DGC_OK;
 }
 
-#ifdef DGC_KK_TIMING
-DGC_EXPORT int32_t dgc_debug_kk_times(unsigned long long *out8) {
-  cudaDeviceSynchronize();
-  return cudaMemcpyFromSymbol(out8, dgtc::dgc_kk_times, 8 * sizeof(unsigned long long)) == cudaSuccess ? 0 : -1;
-}
-DGC_EXPORT int32_t dgc_debug_sk_times(unsigned long long *out128) {
-  cudaDeviceSynchronize();
-  return cudaMemcpyFromSymbol(out128, dgtc::dgc_sk_times, 128 * sizeof(unsigned long long)) == cudaSuccess ? 0 : -1;
-}
-#endif

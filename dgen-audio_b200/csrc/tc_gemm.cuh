@@ -18,6 +18,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "tma.cuh"
+
 namespace dgtc {
 
 constexpr int TBM = 128, TBN = 128, TBK = 32, THREADS = 256;
@@ -392,91 +394,54 @@ tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const f
 
 
 // ---------------------------------------------------------------------------------------------------------
-// Both operands contiguous along k in memory (A [M][K], B [N][K]), K a multiple of 4, 16-byte aligned rows:
-// the asynchronous pipeline.  cp.async copies 16-byte chunks straight into the canonical K-major layout,
-// RAW raw stages deep, PF tiles ahead of the tensor core; the raw fp32 tile IS the "hi" operand (the tensor
-// core reads the top 19 bits of every 32-bit word and ignores the 13 low mantissa bits, i.e. it truncates
-// to TF32 itself), so the threads only compute lo = x - trunc(x), shared memory to shared memory, into one
-// of two lo buffers.  Tile t's MMAs commit to an mbarrier of their own raw stage; the only wait of
-// iteration t is on tile t-2 (it frees both the raw stage about to be refilled and the lo buffer about to
-// be rewritten), two iterations after its MMAs were issued.
+// Both operands contiguous along k in memory (A [M][K], B [N][K]), rows only 4-byte aligned (K not a multiple of 4): the
+// asynchronous pipeline by 4-byte copies.  cp.async copies floats straight into the 64-byte-swizzled K-major layout (8-row groups
+// of 512 bytes, 16-byte chunk c of row r at c ^ ((r / 2) % 4)), RAW raw stages deep, PF tiles ahead of the tensor core; the raw
+// fp32 tile IS the "hi" operand (the tensor core reads the top 19 bits of every 32-bit word and ignores the 13 low mantissa
+// bits, i.e. it truncates to TF32 itself), so the threads only compute lo = x - trunc(x), shared memory to shared memory, into
+// one of two lo buffers.  Tile t's MMAs commit to an mbarrier of their own raw stage; the only wait of iteration t is on tile
+// t-2 (it frees both the raw stage about to be refilled and the lo buffer about to be rewritten), two iterations after its
+// MMAs were issued.  97 KB per CTA: two share an SM, and one's epilogue runs under the other's main loop.
 // ---------------------------------------------------------------------------------------------------------
-// SW: the 128-byte-swizzle K-major layout (BK = 32: one row of a tile is exactly one 128-byte swizzle row;
-// 8-row groups of 1024 bytes, 16-byte chunk c of row r stored at chunk c ^ (r % 8)) instead of the
-// no-swizzle layout of 8 x 16-byte core matrices.
-// With BK = 16 a row is 64 bytes and the 64-byte swizzle applies (8-row groups of 512 bytes, chunk c of row r at
-// c ^ ((r / 2) % 4)); that variant needs 97 KB per CTA, so two CTAs share an SM and one's epilogue runs under
-// the other's main loop.
-// BN = 256 (swizzled layouts only): a 128 x 256 output tile per CTA.  Per flop the three MMAs of a k step then
-// fetch 25 % fewer operand bytes (A is shared by twice as many columns) and the copy / split traffic drops by
-// the same factor, which is what the kernel is bound by; 145 KB of shared memory, one CTA per SM.
-template <int BK, bool SW = false, int BN = TBN>
 struct KK {
-  static_assert(BN == TBN || SW, "the wide tile uses the swizzled layouts");
-  static constexpr int CHUNKS_K = BK / 4;
-  static constexpr int ROW_BYTES = BK * 4;                                  // 128 or 64
-  static constexpr int OPER = SW ? TBM * ROW_BYTES : CHUNKS_K * LBO_BYTES;  // operand A of one tile
-  static constexpr int OPER_B = SW ? BN * ROW_BYTES : CHUNKS_K * LBO_BYTES; // operand B of one tile
+  static constexpr int BK = 16, BN = TBN, CHUNKS_K = BK / 4, ROW_BYTES = BK * 4;
+  static constexpr int OPER = TBM * ROW_BYTES;            // one operand of one tile
   static constexpr int RAW = 4, PF = 2;
-  static constexpr int RAW_STAGE = OPER + OPER_B;         // A, B
-  static constexpr int SMEM = (RAW + 2) * RAW_STAGE + 128 + (SW ? 1024 : 0);   // + room to align to 1024
+  static constexpr int RAW_STAGE = 2 * OPER;              // A, B
+  static constexpr int SMEM = (RAW + 2) * RAW_STAGE + 128 + 1024;   // + room to align to 1024
   // byte offset of 16-byte chunk kc of row r inside one operand
   __device__ static __forceinline__ int unit_offset(int r, int kc) {
-    if (!SW) return kc * LBO_BYTES + r * 16;
-    return BK == 32 ? (r >> 3) * 1024 + (r & 7) * 128 + ((kc ^ (r & 7)) << 4)
-                    : (r >> 3) * 512 + (r & 7) * 64 + ((kc ^ ((r >> 1) & 3)) << 4);
+    return (r >> 3) * 512 + (r & 7) * 64 + ((kc ^ ((r >> 1) & 3)) << 4);
   }
-  static constexpr int UNITS = (TBM + BN) * CHUNKS_K;     // 16-byte units per tile (A and B)
 };
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, int src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
 // one float; src_bytes 0 = zero fill.  For operands whose rows are not 16-byte aligned (K not a multiple of 4).
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void *src, int src_bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
 
-// K-major, 128-byte swizzle: LBO unused (1), SBO = 1024 bytes between 8-row groups, layout type 2 at [61,64)
-// (64-byte swizzle: SBO = 512 bytes, layout type 4)
-template <int ROW_BYTES = 128>
-__device__ __forceinline__ uint64_t make_desc_sw128(uint32_t saddr) {
-  constexpr uint64_t sbo = ROW_BYTES * 8, type = ROW_BYTES == 128 ? 2 : 4;
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | ((sbo >> 4) << 32) | (1ull << 46) | (type << 61);
+// K-major, 64-byte swizzle: LBO unused (1), SBO = 512 bytes between 8-row groups, layout type 4 at [61,64)
+__device__ __forceinline__ uint64_t make_desc_sw64(uint32_t saddr) {
+  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | ((512ull >> 4) << 32) | (1ull << 46) | (4ull << 61);
 }
-
-#ifdef DGC_KK_TIMING
-// development aid: per-phase timestamps (ns) of CTA (0,0,0), read back with cudaMemcpyFromSymbol
-__device__ unsigned long long dgc_kk_times[8];
-__device__ __forceinline__ unsigned long long gtime() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-#define KK_STAMP(i) do { if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (threadIdx.x & 31) == 0 && (threadIdx.x == 0 || (i) == 3 || (i) == 4)) dgc_kk_times[i] = gtime(); } while (0)
-#else
-#define KK_STAMP(i) do {} while (0)
-#endif
 
 constexpr int KK_THREADS = THREADS + 32;   // 8 worker warps + 1 warp whose lane 0 issues the MMAs
 
-// A4: the operands' rows are only 4-byte aligned (K % 4 != 0): every 16-byte unit is fetched as four 4-byte copies.
-template <int EPI, int BK, bool SW, int BN = TBN, bool A4 = false>
-__global__ void __launch_bounds__(KK_THREADS, (BK == 16 && BN == TBN) ? 2 : 1)
-tc_gemm_kk_kernel(const float *__restrict__ A, const float *__restrict__ B, const float *__restrict__ bias, int M, int N,
-                  int K, int k_per_split, float *__restrict__ C, float *__restrict__ Ct, int32_t *status) {
+__global__ void __launch_bounds__(KK_THREADS, 2)
+tc_gemm_kk4_kernel(const float *__restrict__ A, const float *__restrict__ B, int M, int N, int K, int k_per_split,
+                   float *__restrict__ C, int32_t *status) {
   dgc_after_previous();
-  using G = KK<BK, SW, BN>;
-  KK_STAMP(0);
+  using G = KK;
+  constexpr int BK = G::BK;
   extern __shared__ __align__(128) char smem_base[];
   // the swizzle pattern is a function of the address: tiles start on 1024-byte boundaries
-  char *smem = SW ? smem_base + ((1024u - (smem_u32(smem_base) & 1023u)) & 1023u) : smem_base;
+  char *smem = smem_base + ((1024u - (smem_u32(smem_base) & 1023u)) & 1023u);
   char *raw = smem, *lob = smem + G::RAW * G::RAW_STAGE;
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (G::RAW + 2) * G::RAW_STAGE);  // RAW "tile consumed" mbarriers
   uint64_t *ready = bars + G::RAW;                                                    // 2 "lo buffer written" mbarriers
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + (G::RAW + 2) * G::RAW_STAGE + 64);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * TBM, n0 = blockIdx.x * BN;
+  const int m0 = blockIdx.y * TBM, n0 = blockIdx.x * TBN;
   const int k_begin = blockIdx.z * k_per_split, k_end = min(K, k_begin + k_per_split);
   C += (size_t)blockIdx.z * M * N;
   const int KT = (k_end - k_begin + BK - 1) / BK;
@@ -490,7 +455,7 @@ tc_gemm_kk_kernel(const float *__restrict__ A, const float *__restrict__ B, cons
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"((uint32_t)BN)
+                 "r"((uint32_t)TBN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -503,59 +468,31 @@ tc_gemm_kk_kernel(const float *__restrict__ A, const float *__restrict__ B, cons
   volatile int *failed = reinterpret_cast<volatile int *>(tmem_slot + 1);
   if (tid == 0) *failed = 0;
   __syncthreads();
-  KK_STAMP(1);
 
   if (warp < THREADS / 32) {
     // ---- worker warps: copy, split, publish -----------------------------------------------------------------
-    // This thread's share of every tile: units u = tid + 256 * i -> (operand, row, k-chunk), chunk fastest, so 8
-    // lanes fetch one 128-byte row.  Global pointers and shared offsets are fixed per thread, and the thread
-    // splits exactly the units it copied itself, so the only synchronisation of the loop is through mbarriers:
-    // "tile kt-2 consumed" before its raw stage and lo buffer are reused, "lo buffer written" towards the MMA warp.
-    constexpr int UPT = G::UNITS / THREADS;
-    const float *src0[UPT];
-    int soff[UPT], kc4[UPT];
-    bool rowok[UPT];
-#pragma unroll
-    for (int i = 0; i < UPT; ++i) {
-      const int u = tid + THREADS * i;
-      const int op = u >= TBM * G::CHUNKS_K, rem = u - op * (TBM * G::CHUNKS_K);   // A units first, then B
-      const int r = rem / G::CHUNKS_K, kc = rem % G::CHUNKS_K;
-      const int rows = op ? N : M, gr = (op ? n0 : m0) + r;
-      rowok[i] = gr < rows;
-      kc4[i] = 4 * kc;
-      src0[i] = (op ? B : A) + (rowok[i] ? (size_t)gr * K : 0) + k_begin + 4 * kc;
-      soff[i] = op * G::OPER + G::unit_offset(r, kc);
-    }
-    // A4 (rows only 4-byte aligned): the tile is copied float by float, element e = tid + 256 i -> (row e / BK,
-    // k = e % BK), so the lanes of a warp copy consecutive floats of two rows (a unit-wise assignment would
-    // make every instruction touch eight rows).  256 % BK == 0: k is the same for all of a thread's elements, its
-    // rows are 16 apart, and each element's place in shared memory moves by a constant from one to the next.
-    static_assert(!A4 || (BK == 16 && BN == TBN), "the 4-byte copy path is written for 16-wide k tiles and 128 columns");
-    constexpr int EPT4 = (TBM + BN) * BK / THREADS;          // 16 elements per thread: 8 of A, 8 of B
-    const int k4 = tid % BK, r4 = tid / BK;                  // A4: this thread's k and first row
+    // The tile is copied float by float, element e = tid + 256 i -> (row e / BK, k = e % BK), so the lanes of a warp copy
+    // consecutive floats of two rows (16-byte units would make every instruction touch eight rows).  256 % BK == 0: k is the
+    // same for all of a thread's elements, its rows are 16 apart, and each element's place in shared memory moves by a constant
+    // from one to the next.  The thread splits exactly the elements it copied itself, so the only synchronisation of the loop
+    // is through mbarriers: "tile kt-2 consumed" before its raw stage and lo buffer are reused, "lo buffer written" towards the
+    // MMA warp.
+    constexpr int EPT4 = 2 * TBM * BK / THREADS;             // 16 elements per thread: 8 of A, 8 of B
+    const int k4 = tid % BK, r4 = tid / BK;                  // this thread's k and first row
     const int soff4 = G::unit_offset(r4, k4 >> 2) + (k4 & 3) * 4;
     const int dsoff4 = G::unit_offset(r4 + THREADS / BK, k4 >> 2) - G::unit_offset(r4, k4 >> 2);
     auto issue_tile = [&](int kt) {
       if (kt < KT) {
         const int k0 = kt * BK;   // relative to k_begin
         const uint32_t st = smem_u32(raw + (kt % G::RAW) * G::RAW_STAGE);
-        if (A4) {
-          const bool kin = k_begin + k0 + k4 < k_end;
+        const bool kin = k_begin + k0 + k4 < k_end;
 #pragma unroll
-          for (int i = 0; i < EPT4; ++i) {
-            const int op = i >= EPT4 / 2, r = r4 + (THREADS / BK) * (i - op * (EPT4 / 2));
-            const int gr = (op ? n0 : m0) + r;
-            const bool in = kin && gr < (op ? N : M);
-            cp_async4(st + op * G::OPER + soff4 + (i - op * (EPT4 / 2)) * dsoff4,
-                      in ? (op ? B : A) + (size_t)gr * K + k_begin + k0 + k4 : A, in ? 4 : 0);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < UPT; ++i) {
-            int bytes = (k_end - k_begin - k0 - kc4[i]) * 4;
-            bytes = rowok[i] ? (bytes > 16 ? 16 : (bytes < 0 ? 0 : bytes)) : 0;
-            cp_async16(st + soff[i], bytes > 0 ? src0[i] + k0 : A, bytes);   // 0 bytes: zero fill, any valid address
-          }
+        for (int i = 0; i < EPT4; ++i) {
+          const int op = i >= EPT4 / 2, r = r4 + (THREADS / BK) * (i - op * (EPT4 / 2));
+          const int gr = (op ? n0 : m0) + r;
+          const bool in = kin && gr < (op ? N : M);
+          cp_async4(st + op * G::OPER + soff4 + (i - op * (EPT4 / 2)) * dsoff4,
+                    in ? (op ? B : A) + (size_t)gr * K + k_begin + k0 + k4 : A, in ? 4 : 0);
         }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");   // one group per call keeps the counting uniform
@@ -567,28 +504,17 @@ tc_gemm_kk_kernel(const float *__restrict__ A, const float *__restrict__ B, cons
         if (!mbar_wait(smem_u32(&bars[(kt - 2) % G::RAW]), (uint32_t)(((kt - 2) / G::RAW) & 1))) *failed = 1;
       }
       issue_tile(kt + G::PF);
-      asm volatile("cp.async.wait_group %0;" ::"n"(G::PF) : "memory");   // this thread's chunks of tile kt landed
-      if (kt == 0) KK_STAMP(2);
+      asm volatile("cp.async.wait_group %0;" ::"n"(G::PF) : "memory");   // this thread's floats of tile kt landed
       char *st = raw + (kt % G::RAW) * G::RAW_STAGE, *lo = lob + (kt & 1) * G::RAW_STAGE;
-      if (A4) {
-        float v[EPT4];
+      float v[EPT4];
 #pragma unroll
-        for (int i = 0; i < EPT4; ++i)
-          v[i] = *reinterpret_cast<const float *>(st + (i >= EPT4 / 2) * G::OPER + soff4 + (i % (EPT4 / 2)) * dsoff4);
+      for (int i = 0; i < EPT4; ++i)
+        v[i] = *reinterpret_cast<const float *>(st + (i >= EPT4 / 2) * G::OPER + soff4 + (i % (EPT4 / 2)) * dsoff4);
 #pragma unroll
-        for (int i = 0; i < EPT4; ++i) {
-          float h, l;
-          split_tf32(v[i], h, l);
-          *reinterpret_cast<float *>(lo + (i >= EPT4 / 2) * G::OPER + soff4 + (i % (EPT4 / 2)) * dsoff4) = l;
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < UPT; ++i) {
-          const float4 v = *reinterpret_cast<const float4 *>(st + soff[i]);
-          float4 h, l;
-          split_tf32(v.x, h.x, l.x); split_tf32(v.y, h.y, l.y); split_tf32(v.z, h.z, l.z); split_tf32(v.w, h.w, l.w);
-          *reinterpret_cast<float4 *>(lo + soff[i]) = l;
-        }
+      for (int i = 0; i < EPT4; ++i) {
+        float h, l;
+        split_tf32(v[i], h, l);
+        *reinterpret_cast<float *>(lo + (i >= EPT4 / 2) * G::OPER + soff4 + (i % (EPT4 / 2)) * dsoff4) = l;
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // this thread's writes -> tensor-core proxy
       __syncwarp();
@@ -597,24 +523,21 @@ tc_gemm_kk_kernel(const float *__restrict__ A, const float *__restrict__ B, cons
     asm volatile("cp.async.wait_group 0;" ::: "memory");
   } else if (lane == 0) {
     // ---- MMA issue: one thread, nothing else to do ----------------------------------------------------------
-    constexpr uint32_t ID = IDesc<true, true, BN>::value;
+    constexpr uint32_t ID = IDesc<true, true>::value;
     for (int kt = 0; kt < KT; ++kt) {
       if (*failed || !mbar_wait(smem_u32(&ready[kt & 1]), (uint32_t)((kt >> 1) & 1))) {
         *failed = 1;
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (kt == 0) KK_STAMP(3);
       const uint32_t a_hi = smem_u32(raw + (kt % G::RAW) * G::RAW_STAGE), b_hi = a_hi + G::OPER;
       const uint32_t a_lo = smem_u32(lob + (kt & 1) * G::RAW_STAGE), b_lo = a_lo + G::OPER;
 #pragma unroll
       for (int ks = 0; ks < BK / 8; ++ks) {
-        // 8 tf32 along k: two 16-byte chunks (no swizzle), or 32 bytes further inside the swizzled row
-        const uint32_t adv = SW ? ks * 32 : ks * 2 * LBO_BYTES;
-        const uint64_t dah = SW ? make_desc_sw128<G::ROW_BYTES>(a_hi + adv) : make_desc<true>(a_hi + adv);
-        const uint64_t dal = SW ? make_desc_sw128<G::ROW_BYTES>(a_lo + adv) : make_desc<true>(a_lo + adv);
-        const uint64_t dbh = SW ? make_desc_sw128<G::ROW_BYTES>(b_hi + adv) : make_desc<true>(b_hi + adv);
-        const uint64_t dbl = SW ? make_desc_sw128<G::ROW_BYTES>(b_lo + adv) : make_desc<true>(b_lo + adv);
+        // 8 tf32 along k: 32 bytes further inside the swizzled row
+        const uint32_t adv = ks * 32;
+        const uint64_t dah = make_desc_sw64(a_hi + adv), dal = make_desc_sw64(a_lo + adv);
+        const uint64_t dbh = make_desc_sw64(b_hi + adv), dbl = make_desc_sw64(b_lo + adv);
         mma_tf32(tmem_d, dal, dbh, ID, (kt | ks) ? 1u : 0u);
         mma_tf32(tmem_d, dah, dbl, ID, 1u);
         mma_tf32(tmem_d, dah, dbh, ID, 1u);
@@ -624,28 +547,290 @@ tc_gemm_kk_kernel(const float *__restrict__ A, const float *__restrict__ B, cons
     // the last commit covers every MMA issued before it
     if (KT > 0 && !*failed && !mbar_wait(smem_u32(&bars[(KT - 1) % G::RAW]), (uint32_t)(((KT - 1) / G::RAW) & 1)))
       *failed = 1;
-    KK_STAMP(4);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   ok = !*failed;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  KK_STAMP(5);
 
   if (ok && KT > 0) {
-    if (warp < THREADS / 32) epilogue<EPI, BN>(tmem_d, bias, M, N, m0, n0, C, warp, lane, Ct, reinterpret_cast<float *>(smem));
-    KK_STAMP(6);
+    if (warp < THREADS / 32) epilogue<0>(tmem_d, nullptr, M, N, m0, n0, C, warp, lane, nullptr, reinterpret_cast<float *>(smem));
   } else if (KT == 0) {
     const int gm = m0 + (warp & 3) * 32 + lane;
     if (gm < M && warp < 4)
-      for (int c = 0; c < BN; ++c)
+      for (int c = 0; c < TBN; ++c)
         if (n0 + c < N) C[(size_t)gm * N + n0 + c] = 0.0f;
   }
   if (!ok && tid == 0) atomicExch(status, 201);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"((uint32_t)BN) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"((uint32_t)TBN) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// Both operands contiguous along k, K a multiple of 4, 16-byte aligned rows: operand A in tensor memory, one persistent CTA per
+// SM.  Fetching both operands from shared memory for each of the three products, a pipeline like the one above carries 96 KB of
+// it per 16 k of a 128 x 128 tile, 768 cycles for 384 of multiplying, and a CTA's split, products and epilogue come one
+// after the other.  Here
+//   load      one thread has the copy engine bring 64-byte-swizzled tiles of both operands, RAW of them ahead
+//   split     eight warps in two groups, a tile each in turn: a group's lanes are the rows of A, whose hi and lo parts go to
+//             tensor memory side by side, a column per k; B's lo part goes to shared memory, its hi part is the raw tile
+//   multiply  one warp; the MMAs fetch only B from shared memory (64 KB in all) and fill one of two accumulators
+//   store     eight warps move the other accumulator, of the tile before, to global memory
+// The products and the order of their sums are those of a pipeline with both operands in shared memory: the same bits.
+// Bound by the shared memory, 512 cycles a tile (525 measured; the multiplying alone 393).  32000 x 512 over 512 k with
+// tanh, 16-byte copies and both operands in shared memory: 144 us; A in tensor memory, two CTAs per SM: 128, with two groups of
+// splitting warps (800 cycles from a tile's arrival to its split) 112; persistent with the epilogue apart 111, with the issuing
+// warp walking together 84.  Three or four groups: 88.  512 x 512 over 32000 k in 18 slices: 99 -> 80.
+// The 128 x 256 tiles of a long reduction have one accumulator: there is one tile for a CTA.
+// ---------------------------------------------------------------------------------------------------------
+template <int BN>
+struct TS {
+  static constexpr int BK = 16, ROW_BYTES = BK * 4, RAW = BN == 128 ? 8 : 4, ACCS = BN == 128 ? 2 : 1;
+  static constexpr int A_BYTES = TBM * ROW_BYTES, B_BYTES = BN * ROW_BYTES, STAGE = A_BYTES + B_BYTES;
+  static constexpr int GROUPS = 2, SPLITTERS = 4 * GROUPS, STORERS = 8;          // warps
+  static constexpr int THREADS_ALL = 32 * (SPLITTERS + STORERS + 2);
+  static constexpr int OFF_LO = RAW * STAGE, OFF_EPI = OFF_LO + RAW * B_BYTES, OFF_BARS = OFF_EPI + STORERS * EPI_STAGE_FLOATS * 4;
+  static constexpr int SMEM = OFF_BARS + 256 + 1024;             // + room to align to 1024
+  static constexpr int COLS = 512;                               // tensor memory: accumulators, split stages of A
+};
+static_assert(TS<128>::SMEM <= 227 * 1024 && TS<256>::SMEM <= 227 * 1024, "shared memory of one CTA");
+static_assert(2 * 128 + TS<128>::RAW * 32 <= 512 && 256 + TS<256>::RAW * 32 <= 512, "tensor memory");
+
+// the same wait for one of several that give up together: who runs out raises the flag, who sees it raised stops waiting
+__device__ __forceinline__ bool mbar_wait_or(uint32_t bar, uint32_t parity, volatile int *failed) {
+  for (uint32_t it = 0; it < SPIN_LIMIT; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if ((it & 255u) == 255u && *failed) return false;
+  }
+  *failed = 1;
+  return false;
+}
+
+// true in one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred q;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t"
+      "}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
+__device__ __forceinline__ void mma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t IDESC, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t"
+      "}\n" ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(IDESC), "r"(accumulate), "r"(0u)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_store8(uint32_t taddr, const float (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "f"(v[0]), "f"(v[1]),
+               "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+
+template <int EPI, int BN>
+__global__ void __launch_bounds__(TS<BN>::THREADS_ALL, 1)
+tc_gemm_ts_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                  const float *__restrict__ bias, int M, int N, int K, int k_per_split, int items, float *__restrict__ C,
+                  float *__restrict__ Ct, int32_t *status) {
+  dgc_after_previous();
+  using G = TS<BN>;
+  extern __shared__ __align__(128) char smem_base[];
+  char *smem = smem_base + ((1024u - (smem_u32(smem_base) & 1023u)) & 1023u);   // the swizzle is a function of the address
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem + G::OFF_BARS);   // raw tile landed
+  uint64_t *ready = full + G::RAW;                                     // split written
+  uint64_t *consumed = ready + G::RAW;                                 // multiplied
+  uint64_t *summed = consumed + G::RAW;                                // accumulator complete
+  uint64_t *stored = summed + G::ACCS;                                 // accumulator read
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(stored + G::ACCS);
+  volatile int *failed = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (tid == 0) {
+#pragma unroll
+    for (int i = 0; i < G::RAW; ++i) {
+      mbar_init(smem_u32(&full[i]), 1);
+      mbar_init(smem_u32(&ready[i]), 4);   // one arrival per warp of a group
+      mbar_init(smem_u32(&consumed[i]), 1);
+    }
+#pragma unroll
+    for (int i = 0; i < G::ACCS; ++i) {
+      mbar_init(smem_u32(&summed[i]), 1);
+      mbar_init(smem_u32(&stored[i]), G::STORERS);
+    }
+    *failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"((uint32_t)G::COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_d = *tmem_slot, tmem_a = tmem_d + G::ACCS * BN;
+
+  // item: (k slice, row tile, column tile), column tiles next to each other; this CTA takes every gridDim.x-th
+  const int nx = (N + BN - 1) / BN, ny = (M + TBM - 1) / TBM;
+  struct Item {
+    int m0, n0, k0, z, tiles;
+  };
+  auto item_at = [&](int i) {
+    Item t;
+    t.n0 = i % nx * BN;
+    t.m0 = i / nx % ny * TBM;
+    t.z = i / nx / ny;
+    t.k0 = t.z * k_per_split;
+    t.tiles = (min(K, t.k0 + k_per_split) - t.k0 + G::BK - 1) / G::BK;
+    return t;
+  };
+  // g: k tiles counted through all items; a: items of this CTA
+  auto wait = [&](uint64_t *bars, int g) {
+    return mbar_wait_or(smem_u32(&bars[g % G::RAW]), (uint32_t)((g / G::RAW) & 1), failed);
+  };
+  auto wait_acc = [&](uint64_t *bars, int a) {
+    return mbar_wait_or(smem_u32(&bars[a % G::ACCS]), (uint32_t)((a / G::ACCS) & 1), failed);
+  };
+  if (warp < G::SPLITTERS) {
+    // ---- split: row 32 (warp % 4) + lane of A, 16-byte units of B -------------------------------------------
+    const int gtid = tid & 127, r = gtid, row_off = (r >> 3) * 512 + (r & 7) * 64, swz = (r >> 1) & 3;
+    const uint32_t a_dst = tmem_a + ((uint32_t)((warp & 3) * 32) << 16);
+    constexpr int UPT = BN * G::BK / 4 / 128;
+    int total = 0;
+    for (int i = blockIdx.x; i < items; i += gridDim.x) total += item_at(i).tiles;
+    for (int g = warp >> 2; g < total; g += G::GROUPS) {
+      const int s = g % G::RAW;
+      // landed, and the split stage free (the loader waited for that, too); the whole warp goes on or gives up
+      const bool go = wait(full, g) && (g < G::RAW || wait(consumed, g - G::RAW));
+      if (!__all_sync(0xffffffffu, go)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const char *st = smem + s * G::STAGE;
+      float4 u[4], v[UPT];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) u[i] = *reinterpret_cast<const float4 *>(st + row_off + ((i ^ swz) << 4));
+#pragma unroll
+      for (int i = 0; i < UPT; ++i) v[i] = *reinterpret_cast<const float4 *>(st + G::A_BYTES + (gtid + 128 * i) * 16);
+#pragma unroll
+      for (int i = 0; i < 4; i += 2) {
+        const float x[8] = {u[i].x, u[i].y, u[i].z, u[i].w, u[i + 1].x, u[i + 1].y, u[i + 1].z, u[i + 1].w};
+        float h[8], l[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) split_tf32(x[j], h[j], l[j]);
+        tmem_store8(a_dst + s * 2 * G::BK + 4 * i, h);
+        tmem_store8(a_dst + s * 2 * G::BK + G::BK + 4 * i, l);
+      }
+      char *lo = smem + G::OFF_LO + s * G::B_BYTES;
+#pragma unroll
+      for (int i = 0; i < UPT; ++i) {
+        float4 hh, ll;
+        split_tf32(v[i].x, hh.x, ll.x); split_tf32(v[i].y, hh.y, ll.y); split_tf32(v[i].z, hh.z, ll.z); split_tf32(v[i].w, hh.w, ll.w);
+        *reinterpret_cast<float4 *>(lo + (gtid + 128 * i) * 16) = ll;   // the same place in the same swizzle
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // this thread's writes -> tensor-core proxy
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ready[s]));
+    }
+  } else if (warp < G::SPLITTERS + G::STORERS) {
+    // ---- store ----------------------------------------------------------------------------------------------
+    const int w = warp - G::SPLITTERS;
+    int a = 0;
+    for (int i = blockIdx.x; i < items; i += gridDim.x, ++a) {
+      if (!__all_sync(0xffffffffu, wait_acc(summed, a))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const Item t = item_at(i);
+      epilogue<EPI, BN>(tmem_d + a % G::ACCS * BN, bias, M, N, t.m0, t.n0, C + (size_t)t.z * M * N, w, lane, Ct,
+                        reinterpret_cast<float *>(smem + G::OFF_EPI));
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&stored[a % G::ACCS]));
+    }
+  } else if (warp == G::SPLITTERS + G::STORERS) {
+    // ---- multiply: the warp walks together, one lane issues ---------------------------------------------------
+    // (so that stages, addresses and descriptors are the same for the whole warp: worked out by the one lane alone, they and
+    // the six MMAs took 610 cycles a tile)
+    constexpr uint32_t ID = IDesc<true, true, BN>::value;
+    const bool leader = elect_one();
+    const uint32_t raw0 = smem_u32(smem), lo0 = raw0 + G::OFF_LO;
+    int a = 0, s = 0, phase = 0;
+    bool go = true;
+    for (int i = blockIdx.x; go && i < items; i += gridDim.x, ++a) {
+      go = __all_sync(0xffffffffu, a < G::ACCS || wait_acc(stored, a - G::ACCS));
+      const int tiles = item_at(i).tiles;
+      const uint32_t acc = tmem_d + a % G::ACCS * BN;
+      for (int k = 0; go && k < tiles; ++k) {
+        go = __all_sync(0xffffffffu, mbar_wait_or(smem_u32(&ready[s]), phase, failed));
+        if (!go) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (leader) {
+          const uint64_t bh = make_desc_sw64(raw0 + s * G::STAGE + G::A_BYTES);
+          const uint64_t bl = make_desc_sw64(lo0 + s * G::B_BYTES);
+          const uint32_t a_hi = tmem_a + s * 2 * G::BK, a_lo = a_hi + G::BK;
+#pragma unroll
+          for (int ks = 0; ks < G::BK / 8; ++ks) {   // 8 k: 32 bytes further inside the swizzled row, 8 columns
+            mma_tf32_ts(acc, a_lo + ks * 8, bh + ks * 2, ID, k | ks ? 1u : 0u);
+            mma_tf32_ts(acc, a_hi + ks * 8, bl + ks * 2, ID, 1u);
+            mma_tf32_ts(acc, a_hi + ks * 8, bh + ks * 2, ID, 1u);
+          }
+          commit_to(smem_u32(&consumed[s]));
+          if (k == tiles - 1) commit_to(smem_u32(&summed[a % G::ACCS]));   // covers every MMA issued before it
+        }
+        __syncwarp();
+        if (++s == G::RAW) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+    }
+    if (go && a > 0) wait_acc(summed, a - 1);
+  } else if (lane == 0) {
+    // ---- load -----------------------------------------------------------------------------------------------
+    int g = 0;
+    bool go = true;
+    for (int i = blockIdx.x; go && i < items; i += gridDim.x) {
+      const Item t = item_at(i);
+      for (int k = 0; k < t.tiles; ++k, ++g) {
+        go = g < G::RAW || wait(consumed, g - G::RAW);
+        if (!go) break;
+        char *st = smem + g % G::RAW * G::STAGE;
+        uint64_t *bar = &full[g % G::RAW];
+        dgtma::mbar_expect_tx(bar, G::STAGE);
+        dgtma::load_2d(st, &map_a, t.k0 + k * G::BK, t.m0, bar);
+        dgtma::load_2d(st + G::A_BYTES, &map_b, t.k0 + k * G::BK, t.n0, bar);
+      }
+    }
+    for (int i = max(0, g - G::RAW); i < g; ++i)   // nothing of this block's is in flight when it ends
+      if (!mbar_wait(smem_u32(&full[i % G::RAW]), (uint32_t)((i / G::RAW) & 1))) *failed = 1;
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (*failed && tid == 0) atomicExch(status, 201);
+  if (warp == 0) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"((uint32_t)G::COLS) : "memory");
   }
 }
 
@@ -667,12 +852,6 @@ tc_gemm_kk_kernel(const float *__restrict__ A, const float *__restrict__ B, cons
 // last column block, from the linear tile, instead of a third block of 127 empty columns.
 // Every wait is bounded; on expiry the kernel raises status 202, stops waiting everywhere and frees its TMEM.
 // ---------------------------------------------------------------------------------------------------------
-#ifdef DGC_KK_TIMING
-__device__ unsigned long long dgc_sk_times[128];
-#define SK_STAMP(i) do { if (tid == 0 && blockIdx.x == 0 && (i) < 128) dgc_sk_times[(i)] = gtime(); } while (0)
-#else
-#define SK_STAMP(i) do {} while (0)
-#endif
 struct SK {
   static constexpr int KP_MAX = 72;                          // largest K (nine k-steps of 8)
   static constexpr int WORKERS = 512, THREADS_ALL = WORKERS + 32;
@@ -739,7 +918,6 @@ tc_gemm_smallk_kernel(const float *__restrict__ A, const float *__restrict__ B, 
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_d = *tmem_slot;
-  SK_STAMP(0);
 
   if (warp < SK::WORKERS / 32) {
     // ---- worker warps ---------------------------------------------------------------------------------------
@@ -791,7 +969,6 @@ tc_gemm_smallk_kernel(const float *__restrict__ A, const float *__restrict__ B, 
               "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
             : "r"(taddr));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (h == 0) SK_STAMP(8 + 8 * (i + 1));
 #pragma unroll
         for (int q = 0; q < 4; ++q)
           *reinterpret_cast<uint4 *>(stage + lane * SK::EPI_ROW + 4 * q) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
@@ -803,26 +980,20 @@ tc_gemm_smallk_kernel(const float *__restrict__ A, const float *__restrict__ B, 
         float v[16];
 #pragma unroll
         for (int it = 0; it < 16; ++it) v[it] = stage[((it & 3) + 8 * (it >> 2) + 4 * rsub) * SK::EPI_ROW + col];
-        if (h == 0) SK_STAMP(9 + 8 * (i + 1));
 #pragma unroll
         for (int it = 0; it < 16; ++it) {
           const int grow = m0 + lane_base + (it & 3) + 8 * (it >> 2) + 4 * rsub;
           if (col_ok && grow < M) C[(size_t)grow * N + gn0 + col] = v[it];
         }
-        if (h == 0) SK_STAMP(10 + 8 * (i + 1));
         __syncwarp();
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      SK_STAMP(11 + 8 * (i + 1));
     };
-    SK_STAMP(1);
     for (int i = 0; i < nt; ++i) {
       // tile i has landed in the linear buffer; tile i-1 is multiplied: its accumulator is complete and the
       // operand parts of A may be overwritten
       if (!*failed && !mbar_wait(bar_load, (uint32_t)(i & 1))) *failed = 1;
-      SK_STAMP(4 + 8 * i);
       if (i >= 1 && !*failed && !mbar_wait(bar_done, (uint32_t)((i - 1) & 1))) *failed = 1;
-      SK_STAMP(5 + 8 * i);
       if (has_extra) {
         // four threads per row, every fourth k each (all loads first, then one chain of multiply-adds), combined in
         // a fixed order
@@ -845,7 +1016,6 @@ tc_gemm_smallk_kernel(const float *__restrict__ A, const float *__restrict__ B, 
           if (part == 0 && gm < M) C[(size_t)gm * N + nblk * TBN + x] = acc;
         }
       }
-      SK_STAMP(6 + 8 * i);
       {
         float v[SK::EPT];
 #pragma unroll
@@ -868,7 +1038,6 @@ tc_gemm_smallk_kernel(const float *__restrict__ A, const float *__restrict__ B, 
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_ready);
-      SK_STAMP(7 + 8 * i);
       if (i >= 1 && !*failed) store_tile(i - 1);   // while the tensor core multiplies tile i
     }
     if (nt > 0 && !*failed && !mbar_wait(bar_done, (uint32_t)((nt - 1) & 1))) *failed = 1;

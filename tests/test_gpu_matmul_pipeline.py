@@ -1,0 +1,65 @@
+"""The tensor-core matmul pipeline with A in tensor memory at the edges of its tiles and of its persistent walk: rows, columns and
+reductions that fill no tile, more tiles than CTAs, fewer k tiles than stages, split reductions in both tile widths."""
+import numpy as np
+import pytest
+import torch
+
+import dgen_b200
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = dgen_b200.Context(0)
+    yield c
+    c.close()
+
+
+def _tol(n):
+    """Three TF32 products leave out lo * lo and what lo loses by truncation, 2^-20 of a term; the accumulator is truncated at each
+    of 3 n / 8 steps, 2^-24 of the sum so far (a long reduction is cut into slices of 2048 or less, added in single precision)."""
+    return 2.0 ** -20 + 3 * min(n, 2048) / 8 * 2.0 ** -24
+
+
+def _rel(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+# (M, K, N): from 149 output tiles of 64 x 64 on and 2^21 products the pipeline takes the layer's three matmuls
+@pytest.mark.parametrize("M,K,N,act", [(1000, 32, 640, 0), (1537, 36, 513, 1), (5000, 100, 260, 1), (9600, 512, 128, 0),
+                                       (20001, 48, 128, 1), (19000, 68, 132, 0), (24004, 256, 300, 1)])
+def test_layers_that_fill_no_tile(ctx, M, K, N, act):
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    a = torch.randn(M, K, device="cuda", generator=g)
+    w = torch.randn(K, N, device="cuda", generator=g) * K ** -0.5
+    b = torch.randn(N, device="cuda", generator=g)
+    c, ct = ctx.linear_fwd(a, w, b, act=act, want_transposed=True)
+    z = a.double() @ w.double() + b.double()
+    want = torch.tanh(z) if act else z
+    assert _rel(c, want) < _tol(K) and torch.equal(ct.t(), c)
+    dc = torch.randn(M, N, device="cuda", generator=g)
+    dz = dc.double() * (1 - c.double() ** 2) if act else dc.double()
+    da, dw, db = ctx.linear_bwd(a, w, c, dc, act=act, a_t=a.t().contiguous())
+    assert _rel(da, dz @ w.double().t()) < _tol(N)
+    assert _rel(dw, a.double().t() @ dz) < _tol(M)
+    assert _rel(db, dz.sum(0)) < _tol(M)
+    again, _, _ = ctx.linear_bwd(a, w, c, dc, act=act, a_t=a.t().contiguous())
+    assert torch.equal(again, da)
+    ctx.sync()
+
+
+def test_rows_past_the_end_are_not_read(ctx):
+    """NaN behind the operand and in front of it: what the copy engine brings past the last row or column arrives as zeros."""
+    M, K, N = 4100, 132, 300
+    room = torch.full((M * K + 4096,), float("nan"), device="cuda")
+    room[2048:2048 + M * K] = torch.randn(M * K, device="cuda")
+    a = room[2048:2048 + M * K].view(M, K)
+    w = torch.randn(K, N, device="cuda") * K ** -0.5
+    c = ctx.linear_fwd(a, w)
+    assert torch.isfinite(c).all() and _rel(c, a.double() @ w.double()) < _tol(K)
+    # the operand's own values that are not finite stay in their rows
+    a[7, 3] = float("inf")
+    c2 = ctx.linear_fwd(a, w)
+    rows = torch.isfinite(c2).all(1)
+    assert not bool(rows[7]) and int(rows.sum()) == M - 1 and torch.equal(c2[rows], c[rows])
