@@ -67,6 +67,19 @@ __device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t da, uint64_t 
       : "memory");
 }
 
+// true in one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred q;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t"
+      "}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void commit_to(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -343,32 +356,38 @@ tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const f
       for (int j = 0; j < AHEAD; ++j)
         if (kt + j < KT) tile(kt + j, va[j], vb[j]);
     }
-  } else if (lane == 0) {
+  } else {
+    // The warp walks together and one lane issues: addresses and descriptors are then the same for the whole warp.  Worked out by
+    // the one lane alone they cost about as much as its twelve MMAs.
     constexpr uint32_t ID = IDesc<true, true, BN>::value;
-    for (int kt = 0; kt < KT; ++kt) {
+    const bool leader = elect_one();
+    bool go = true;
+    for (int kt = 0; go && kt < KT; ++kt) {
       const int s = kt & 1;
       // when the workers or the tensor core stop answering no further MMAs are issued, TMEM is still released below
-      if (*failed || !mbar_wait(smem_u32(&ready[s]), (uint32_t)((kt >> 1) & 1))) {
+      go = __all_sync(0xffffffffu, !*failed && mbar_wait(smem_u32(&ready[s]), (uint32_t)((kt >> 1) & 1)));
+      if (!go) {
         *failed = 1;
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a_hi = smem_u32(smem + s * STAGE_BYTES), a_lo = a_hi + OPER_BYTES, b_hi = a_hi + 2 * OPER_BYTES,
-                     b_lo = a_hi + 3 * OPER_BYTES;
+      if (leader) {
+        const uint32_t stage = smem_u32(smem) + s * STAGE_BYTES;
+        const uint64_t dah = make_desc<true>(stage), dal = make_desc<true>(stage + OPER_BYTES);
+        const uint64_t dbh = make_desc<true>(stage + 2 * OPER_BYTES), dbl = make_desc<true>(stage + 3 * OPER_BYTES);
 #pragma unroll
-      for (int ks = 0; ks < TBK / 8; ++ks) {
-        // 8 tf32 along k = two 16-byte k-chunks
-        const uint32_t adv = ks * 2 * LBO_BYTES;
-        const uint64_t dah = make_desc<true>(a_hi + adv), dal = make_desc<true>(a_lo + adv);
-        const uint64_t dbh = make_desc<true>(b_hi + adv), dbl = make_desc<true>(b_lo + adv);
-        mma_tf32(tmem_d, dal, dbh, ID, (kt | ks) ? 1u : 0u);   // small terms first
-        mma_tf32(tmem_d, dah, dbl, ID, 1u);
-        mma_tf32(tmem_d, dah, dbh, ID, 1u);
+        for (int ks = 0; ks < TBK / 8; ++ks) {
+          constexpr int STEP = 2 * LBO_BYTES / 16;   // 8 tf32 along k = two 16-byte k-chunks
+          mma_tf32(tmem_d, dal + ks * STEP, dbh + ks * STEP, ID, (kt | ks) ? 1u : 0u);   // small terms first
+          mma_tf32(tmem_d, dah + ks * STEP, dbl + ks * STEP, ID, 1u);
+          mma_tf32(tmem_d, dah + ks * STEP, dbh + ks * STEP, ID, 1u);
+        }
+        commit_to(smem_u32(&bars[s]));
       }
-      commit_to(smem_u32(&bars[s]));
+      __syncwarp();
     }
     // the last commit covers every MMA issued before it
-    if (KT > 0 && !*failed && !mbar_wait(smem_u32(&bars[(KT - 1) & 1]), (uint32_t)(((KT - 1) >> 1) & 1))) *failed = 1;
+    if (KT > 0 && go && !mbar_wait(smem_u32(&bars[(KT - 1) & 1]), (uint32_t)(((KT - 1) >> 1) & 1))) *failed = 1;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -521,32 +540,34 @@ tc_gemm_kk4_kernel(const float *__restrict__ A, const float *__restrict__ B, int
       if (lane == 0) mbar_arrive(smem_u32(&ready[kt & 1]));
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-  } else if (lane == 0) {
-    // ---- MMA issue: one thread, nothing else to do ----------------------------------------------------------
+  } else {
+    // ---- MMA issue: the warp walks together, one lane issues --------------------------------------------------
     constexpr uint32_t ID = IDesc<true, true>::value;
-    for (int kt = 0; kt < KT; ++kt) {
-      if (*failed || !mbar_wait(smem_u32(&ready[kt & 1]), (uint32_t)((kt >> 1) & 1))) {
+    const bool leader = elect_one();
+    bool go = true;
+    for (int kt = 0; go && kt < KT; ++kt) {
+      go = __all_sync(0xffffffffu, !*failed && mbar_wait(smem_u32(&ready[kt & 1]), (uint32_t)((kt >> 1) & 1)));
+      if (!go) {
         *failed = 1;
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a_hi = smem_u32(raw + (kt % G::RAW) * G::RAW_STAGE), b_hi = a_hi + G::OPER;
-      const uint32_t a_lo = smem_u32(lob + (kt & 1) * G::RAW_STAGE), b_lo = a_lo + G::OPER;
+      if (leader) {
+        const uint32_t hi = smem_u32(raw) + (kt % G::RAW) * G::RAW_STAGE, lo = smem_u32(lob) + (kt & 1) * G::RAW_STAGE;
+        const uint64_t dah = make_desc_sw64(hi), dbh = make_desc_sw64(hi + G::OPER);
+        const uint64_t dal = make_desc_sw64(lo), dbl = make_desc_sw64(lo + G::OPER);
 #pragma unroll
-      for (int ks = 0; ks < BK / 8; ++ks) {
-        // 8 tf32 along k: 32 bytes further inside the swizzled row
-        const uint32_t adv = ks * 32;
-        const uint64_t dah = make_desc_sw64(a_hi + adv), dal = make_desc_sw64(a_lo + adv);
-        const uint64_t dbh = make_desc_sw64(b_hi + adv), dbl = make_desc_sw64(b_lo + adv);
-        mma_tf32(tmem_d, dal, dbh, ID, (kt | ks) ? 1u : 0u);
-        mma_tf32(tmem_d, dah, dbl, ID, 1u);
-        mma_tf32(tmem_d, dah, dbh, ID, 1u);
+        for (int ks = 0; ks < BK / 8; ++ks) {   // 8 tf32 along k: 32 bytes further inside the swizzled row
+          mma_tf32(tmem_d, dal + ks * 2, dbh + ks * 2, ID, (kt | ks) ? 1u : 0u);
+          mma_tf32(tmem_d, dah + ks * 2, dbl + ks * 2, ID, 1u);
+          mma_tf32(tmem_d, dah + ks * 2, dbh + ks * 2, ID, 1u);
+        }
+        commit_to(smem_u32(&bars[kt % G::RAW]));
       }
-      commit_to(smem_u32(&bars[kt % G::RAW]));
+      __syncwarp();
     }
     // the last commit covers every MMA issued before it
-    if (KT > 0 && !*failed && !mbar_wait(smem_u32(&bars[(KT - 1) % G::RAW]), (uint32_t)(((KT - 1) / G::RAW) & 1)))
-      *failed = 1;
+    if (KT > 0 && go && !mbar_wait(smem_u32(&bars[(KT - 1) % G::RAW]), (uint32_t)(((KT - 1) / G::RAW) & 1))) *failed = 1;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -617,19 +638,6 @@ __device__ __forceinline__ bool mbar_wait_or(uint32_t bar, uint32_t parity, vola
   }
   *failed = 1;
   return false;
-}
-
-// true in one lane of a converged warp
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred q;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t"
-      "}\n"
-      : "=r"(p));
-  return p != 0;
 }
 
 __device__ __forceinline__ void mma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t IDESC, uint32_t accumulate) {
@@ -1042,9 +1050,10 @@ tc_gemm_smallk_kernel(const float *__restrict__ A, const float *__restrict__ B, 
     }
     if (nt > 0 && !*failed && !mbar_wait(bar_done, (uint32_t)((nt - 1) & 1))) *failed = 1;
     if (nt > 0 && !*failed) store_tile(nt - 1);
-  } else if (lane == 0) {
-    // ---- copy and MMA issue: one thread -------------------------------------------------------------------
+  } else {
+    // ---- copy and MMA issue: the warp walks together, one lane issues -----------------------------------------
     constexpr uint32_t ID = IDesc<true, true, TBN>::value;
+    const bool leader = elect_one();
     auto load_tile = [&](int i) {   // the CTA's i-th row tile -> linear buffer (rows past M keep stale values: never stored)
       const size_t a0 = (size_t)(slot + i * ctas_per_blk) * TBM * K, aend = (size_t)M * K;
       const size_t left = aend - a0;
@@ -1054,25 +1063,28 @@ tc_gemm_smallk_kernel(const float *__restrict__ A, const float *__restrict__ B, 
       mbar_expect_tx(bar_load, bulk);   // (release: the plain stores above are visible to whoever sees the phase)
       bulk_load(smem_u32(lin), A + a0, bulk, bar_load);
     };
-    if (nt > 0) load_tile(0);
+    if (nt > 0 && leader) load_tile(0);
     for (int i = 0; i < nt; ++i) {
-      if (*failed || !mbar_wait(bar_ready, (uint32_t)(i & 1))) {
+      if (!__all_sync(0xffffffffu, !*failed && mbar_wait(bar_ready, (uint32_t)(i & 1)))) {
         *failed = 1;
         break;
       }
-      if (i + 1 < nt) load_tile(i + 1);   // every worker has read tile i out of the linear buffer
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t d = tmem_d + (uint32_t)((i & 1) * TBN);
-      const uint32_t ah = smem_u32(a_hi), al = smem_u32(a_lo), bh = smem_u32(b_hi), bl = smem_u32(b_lo);
-      for (int ks = 0; ks < ksteps; ++ks) {
-        const uint32_t adv = ks * 2 * LBO_BYTES;   // 8 tf32 along k: two 16-byte chunks
-        const uint64_t dah = make_desc<true>(ah + adv), dal = make_desc<true>(al + adv);
-        const uint64_t dbh = make_desc<true>(bh + adv), dbl = make_desc<true>(bl + adv);
-        mma_tf32(d, dal, dbh, ID, ks ? 1u : 0u);
-        mma_tf32(d, dah, dbl, ID, 1u);
-        mma_tf32(d, dah, dbh, ID, 1u);
+      if (leader) {
+        if (i + 1 < nt) load_tile(i + 1);   // every worker has read tile i out of the linear buffer
+        const uint32_t d = tmem_d + (uint32_t)((i & 1) * TBN), s0 = smem_u32(smem);
+        uint64_t dah = make_desc<true>(s0 + SK::OFF_AHI), dal = make_desc<true>(s0 + SK::OFF_ALO);
+        uint64_t dbh = make_desc<true>(s0 + SK::OFF_BHI), dbl = make_desc<true>(s0 + SK::OFF_BLO);
+        for (int ks = 0; ks < ksteps; ++ks) {
+          mma_tf32(d, dal, dbh, ID, ks ? 1u : 0u);
+          mma_tf32(d, dah, dbl, ID, 1u);
+          mma_tf32(d, dah, dbh, ID, 1u);
+          constexpr int STEP = 2 * LBO_BYTES / 16;   // 8 tf32 along k: two 16-byte chunks
+          dah += STEP, dal += STEP, dbh += STEP, dbl += STEP;
+        }
+        commit_to(bar_done);
       }
-      commit_to(bar_done);
+      __syncwarp();
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
