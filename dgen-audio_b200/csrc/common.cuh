@@ -104,6 +104,7 @@ unsigned long long *dgc_ctx_chain(dgc_ctx *ctx, uint64_t n);
 const int *dgc_ctx_row_ranges(dgc_ctx *ctx, int F, int T);
 // [T] float2: x = bits of the floor control row (int), y = lerp fraction of sampleRow at the cached clock
 const float2 *dgc_ctx_row_table(dgc_ctx *ctx, int F, int T);
+// N values, then the same N turned by one place (the last one first)
 const float *dgc_ctx_hann_sym(dgc_ctx *ctx, int N);
 const float *dgc_ctx_hann_per(dgc_ctx *ctx, int N);
 // C[M][N] = A[M][K] * B[N][K]^T on the matmul path of gemm.cu

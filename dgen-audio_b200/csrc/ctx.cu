@@ -101,8 +101,11 @@ static T *upload_table(dgc_ctx *ctx, const std::vector<T> &h) {
 const float *dgc_ctx_hann_sym(dgc_ctx *ctx, int N) {
   auto it = ctx->hann_sym.find(N);
   if (it != ctx->hann_sym.end()) return it->second;
-  std::vector<float> h(N);
-  for (int i = 0; i < N; ++i) h[i] = (float)(0.5 * (1.0 - cos(2.0 * M_PI * (double)i / (double)(N - 1))));
+  std::vector<float> h(2 * N);   // then the same turned by one place, the last value first
+  for (int i = 0; i < N; ++i) {
+    h[i] = (float)(0.5 * (1.0 - cos(2.0 * M_PI * (double)i / (double)(N - 1))));
+    h[N + (i + 1) % N] = h[i];
+  }
   float *d = upload_table(ctx, h);
   if (d) ctx->hann_sym[N] = d;
   return d;

@@ -224,21 +224,26 @@ __device__ __forceinline__ void mss_fwd16_body(float2 *sm, float *red, int bx, i
     }
     __syncthreads();   // every warp has read its samples before any transform writes into that buffer
   } else
-  // a window ends at frame h * hop <= T - 1, so only its start can fall outside the signal
+  // A window ends at frame h hop, a multiple of 32 for N >= 128: it starts one place after a 128-byte line of the signal, and
+  // every coalesced load of it would touch two.  Magnitudes do not change when the windowed frames are turned by one place, so
+  // the transform takes the last frame first and the others from there on, whole lines.  (Only its start can fall outside the
+  // signal.)
   if (valid && t_base >= 0) {
-    const float *p1 = x1 + t_base + lt, *p2 = x2 + t_base + lt, *wp = window + lt;
+    const float *p1 = x1 + (t_base - 1 + lt), *p2 = x2 + (t_base - 1 + lt), *wp = window + N + lt;
+    const int first = lt == 0 ? N : 0;
 #pragma unroll
     for (int m = 0; m < 16; ++m) {
       const float w = __ldg(wp + m * TT);
-      x[m] = make_float2(p1[m * TT] * w, p2[m * TT] * w);
+      const int o = m == 0 ? first : m * TT;
+      x[m] = make_float2(p1[o] * w, p2[o] * w);
     }
   } else {
 #pragma unroll
     for (int m = 0; m < 16; ++m) {
-      const int i = lt + m * TT, t = t_base + i;
+      const int i = lt + m * TT, t = t_base + (i == 0 ? N - 1 : i - 1);
       float2 v = make_float2(0.0f, 0.0f);
       if (valid && t >= 0) {
-        const float w = __ldg(&window[i]);
+        const float w = __ldg(&window[N + i]);
         v = make_float2(x1[t] * w, x2[t] * w);
       }
       x[m] = v;
