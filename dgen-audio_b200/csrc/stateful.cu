@@ -605,12 +605,46 @@ __device__ __forceinline__ float principal_arg(float v) {
 }
 
 // The same for the running phase of the synthesis, where a step's latency counts and a multiple of tau more or less is the
-// same phase: turns counted by a multiplication and rounded to the nearest even.
+// same phase: turns counted by a multiplication and rounded to the nearest even by an addition (below 2^22 turns; a single-
+// precision phase beyond has no fraction left).
 __device__ __forceinline__ float wrapped(float v) {
+  const float tau = 6.28318530717958647692f, big = 12582912.0f;
+  return fmaf(-tau, fmaf(v, 0.15915494309189533577f, big) - big, v);
+}
+// as it is handed on: within half a turn
+__device__ __forceinline__ float settled(float w) {
   const float tau = 6.28318530717958647692f, half = 3.14159265358979323846f;
-  const float w = fmaf(-tau, rintf(v * 0.15915494309189533577f), v);
   const float wh = w > half ? w - tau : w;
   return w < -half ? wh + tau : wh;
+}
+
+// Sine and cosine of a wrapped phase, each to 1.2e-7: folded about a quarter turn, then both polynomials in x^2 (minimax on that
+// range, 1e-11 and 2e-10) as the halves of packed multiply-adds: 16 instructions, the library's pair takes three times as many.
+// A phase that is not wrapped (a state handed in, nothing finite) goes to the library.
+__device__ __noinline__ float2 sincos_any(float p) {
+  float2 r;
+  sincosf(p, &r.y, &r.x);
+  return r;
+}
+__device__ __forceinline__ void sincos_wrapped(float p, float &s, float &c) {
+  if (!(fabsf(p) <= 3.2f)) {
+    const float2 r = sincos_any(p);
+    s = r.y;
+    c = r.x;
+    return;
+  }
+  const bool far = fabsf(p) > 1.57079632679489661923f;
+  const float x = far ? (copysignf(3.1415927410125732422f, p) - p) - copysignf(8.7422776573475857731e-8f, p) : p;
+  const float z = x * x;
+  const float2 zz = make_float2(z, z);
+  float2 q = make_float2(-2.3794711816e-8f, -2.6051493821e-7f);
+  q = __ffma2_rn(q, zz, make_float2(2.7518855533e-6f, 2.4760161284e-5f));
+  q = __ffma2_rn(q, zz, make_float2(-1.9840702860e-4f, -1.3888361399e-3f));
+  q = __ffma2_rn(q, zz, make_float2(8.3333292644e-3f, 4.1666636258e-2f));
+  q = __ffma2_rn(q, zz, make_float2(-1.6666666541e-1f, -4.9999999359e-1f));
+  q = __ffma2_rn(q, zz, make_float2(1.0f, 1.0f));
+  s = q.x * x;
+  c = far ? -q.y : q.y;
 }
 
 __device__ __forceinline__ float mixf(float a, float b, float t) { return fmaf(b, t, a * (1.0f - t)); }
@@ -618,8 +652,9 @@ __device__ __forceinline__ float mixf(float a, float b, float t) { return fmaf(b
 // Analysis (Emit+PhaseVocoder.swift:57-71), parallel over (voice, bin, runs of hops): the "previous analysis phase" of hop h
 // is the phase of hop h - 1 of the INPUT (the state cell only for the first hop of the call), so nothing here is a
 // recurrence.  A thread takes PV_RUN hops of a bin and so evaluates one arc tangent per element (and one for the hop before
-// the run): 35 us, 70 us with two per element.  Magnitude and frequency go out side by side: the synthesis gathers both at the same places.
-constexpr int PV_RUN = 8;
+// the run), four hops in flight (eight at once outgrew the instruction cache): 33 us, 35 with eight, 70 with two arc tangents per
+// element.  Magnitude and frequency go out side by side: the synthesis gathers both at the same places.
+constexpr int PV_RUN = 8, PV_AHEAD = 4;
 __global__ void __launch_bounds__(128)
 pv_analysis_kernel(const float *__restrict__ re, const float *__restrict__ im, int64_t H, int N, float omega_scale,
                    const float *__restrict__ state, float2 *__restrict__ mag_omega) {
@@ -629,121 +664,157 @@ pv_analysis_kernel(const float *__restrict__ re, const float *__restrict__ im, i
   if (i >= N) return;
   const size_t at = ((size_t)v * H + h0) * N + i;
   const int cnt = (int)min((int64_t)PV_RUN, H - h0);
-  float r[PV_RUN], q[PV_RUN];
-#pragma unroll
-  for (int j = 0; j < PV_RUN; ++j) {
-    r[j] = j < cnt ? re[at + (size_t)j * N] : 0.0f;
-    q[j] = j < cnt ? im[at + (size_t)j * N] : 0.0f;
-  }
+  const float *pr = re + at, *pq = im + at;
+  float2 *out = mag_omega + at;
   float prev = h0 > 0 ? atan2f(im[at - N], re[at - N]) : (state ? state[(size_t)v * (2 * N + 1) + i] : 0.0f);
   const float target = (float)i * omega_scale;
+#pragma unroll 1
+  for (int j0 = 0; j0 < cnt; j0 += PV_AHEAD) {
+    float r[PV_AHEAD], q[PV_AHEAD];
 #pragma unroll
-  for (int j = 0; j < PV_RUN; ++j)
-    if (j < cnt) {
-      const float phase = atan2f(q[j], r[j]);
-      mag_omega[at + (size_t)j * N] = make_float2(sqrtf(r[j] * r[j] + q[j] * q[j]), target + principal_arg(phase - prev - target));
-      prev = phase;
+    for (int j = 0; j < PV_AHEAD; ++j) {
+      const bool in = j0 + j < cnt;
+      r[j] = in ? pr[(ptrdiff_t)j * N] : 0.0f;
+      q[j] = in ? pq[(ptrdiff_t)j * N] : 0.0f;
     }
+#pragma unroll
+    for (int j = 0; j < PV_AHEAD; ++j)
+      if (j0 + j < cnt) {
+        const float phase = atan2f(q[j], r[j]);
+        out[(ptrdiff_t)j * N] = make_float2(sqrtf(r[j] * r[j] + q[j] * q[j]), target + principal_arg(phase - prev - target));
+        prev = phase;
+      }
+    pr += (size_t)PV_AHEAD * N;
+    pq += (size_t)PV_AHEAD * N;
+    out += (size_t)PV_AHEAD * N;
+  }
 }
 
 // Resynthesis (Emit+PhaseVocoder.swift:73-108): the synthesis phase of an output bin is the one value carried from hop to
 // hop, one addition and one wrap.  Everything else about a hop -- where its bin comes from, the gathered pairs of
-// (magnitude, frequency), sine and cosine -- is independent of it.  A block takes 32 bins of a voice; its eight warps share
-// the hops of a tile of 32, four each, and leave the frequencies in shared memory, where one warp (not the same one in every
-// block) adds them up in hop order while the others already turn the tile before into spectra.  Bound by issue (a
-// division, a gather and a sincosf per element) and by the additions of a tile, 32 wraps one after the other.  8 voices x 469
-// hops x 2048 bins: 80 us, 522 us for a thread per bin that did everything in hop order.
+// (magnitude, frequency), sine and cosine -- is independent of it.  A block takes 32 bins of a voice, tile after tile of 32
+// hops; eight warps share a tile's hops, four each.  While a ninth warp adds up one tile's frequencies in hop order, the eight
+// leave the next tile's in shared memory, turn the tile before into spectra and send for the one after the next: one barrier a
+// tile, three tiles of shared memory.  Bound by issue (a division, a gather and a sine and cosine per element).  8 voices x 469
+// hops x 2048 bins: 522 us for a thread per bin that did everything in hop order, 82 with the library's sine and one of the
+// eight warps adding between two barriers, 71 with the sine above, 63 like this.
 // ratio_mode 0: one value, 1: [H], 2: [V][H].
-constexpr int PV_BINS = 32, PV_WARPS = 8, PV_PER = 4, PV_TILE = PV_WARPS * PV_PER;
-__global__ void __launch_bounds__(PV_BINS * PV_WARPS)
+constexpr int PV_BINS = 32, PV_WARPS = 8, PV_PER = 4, PV_TILE = PV_WARPS * PV_PER, PV_THREADS = PV_BINS * (PV_WARPS + 1);
+__global__ void __launch_bounds__(PV_THREADS, 4)
 pv_synthesis_kernel(const float *__restrict__ re, const float *__restrict__ im, const float2 *__restrict__ mag_omega,
                     const float *__restrict__ ratio, int ratio_mode, int64_t H, int N, float *__restrict__ state,
                     float *__restrict__ out_re, float *__restrict__ out_im) {
   dgc_after_previous();
-  __shared__ float phase[2][PV_TILE][PV_BINS];      // a tile's unscaled frequencies, then, in place, its phases
-  __shared__ float ratios[2][PV_TILE];
+  __shared__ float phase[3][PV_TILE][PV_BINS];      // a tile's unscaled frequencies, then, in place, its phases
+  __shared__ float ratios[3][PV_TILE];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, v = blockIdx.y;
   const int k = blockIdx.x * PV_BINS + lane;
-  const bool live = k < N, adds = warp == (int)((blockIdx.x + blockIdx.y) % PV_WARPS);
+  const bool live = k < N;
   float *st = state ? state + (size_t)v * (2 * N + 1) : nullptr;
-  float synth = st && live ? st[N + k] : 0.0f;
   const bool started = st ? st[2 * N] != 0.0f : false;
-  const float nm1 = (float)(N - 1), kf = (float)k;
   const size_t base = (size_t)v * H * N;
-  float mag[PV_PER], frac[PV_PER], r[PV_PER];
+  const int tiles = (int)((H + PV_TILE - 1) / PV_TILE);
+  if (warp == PV_WARPS) {                            // the one that adds
+    float synth = st && live ? st[N + k] : 0.0f;
+    __syncthreads();
+    for (int t = 0, slot = 0; t <= tiles; ++t, slot = slot == 2 ? 0 : slot + 1) {
+      if (t < tiles) {
+        const int cnt = (int)min((int64_t)PV_TILE, H - (int64_t)t * PV_TILE);
+#pragma unroll 8
+        for (int j = 0; j < cnt; ++j) {
+          const float om = phase[slot][j][lane];
+          synth = t + j == 0 && !started ? om : wrapped(fmaf(om, ratios[slot][j], synth));
+          phase[slot][j][lane] = synth;
+        }
+      }
+      __syncthreads();
+    }
+    if (st && live) {
+      const size_t last = base + (size_t)(H - 1) * N + k;
+      // the "started" flag is shared by all bins of a voice and other blocks may still have to read it: a launch of
+      // its own sets it afterwards
+      st[N + k] = settled(synth);
+      st[k] = atan2f(im[last], re[last]);
+    }
+    return;
+  }
+  const float nm1 = (float)(N - 1), kf = (float)k;
+  const int w0 = warp * PV_PER;                      // this thread's first hop of a tile
+  const float *ratio_v = ratio_mode == 2 ? ratio + (size_t)v * H : ratio;
+  const float2 *rows = mag_omega + base + (size_t)w0 * N;        // of the tile that is fetched
+  float *o_re = out_re + base + (size_t)w0 * N + k, *o_im = out_im + base + (size_t)w0 * N + k;   // of the tile that goes out
+  float mag[2][PV_PER], frac[PV_PER], r[PV_PER];     // magnitudes of the tile that is added up and of the next one
   float2 lo[PV_PER], hi[PV_PER];
   unsigned in_range = 0;
-  // this thread's hops of the tile at h0: where their bin comes from, and the loads of the two pairs there
-  auto fetch = [&](int64_t h0) {
+  // this thread's hops of tile t: where their bin comes from, and the loads of the two pairs there
+  auto fetch = [&](int t) {
     in_range = 0;
+    const int64_t h0 = (int64_t)t * PV_TILE;
+    const int last = (int)min((int64_t)PV_TILE, H - h0) - 1 - w0;   // the last hop of them there is (below zero: none)
 #pragma unroll
     for (int j = 0; j < PV_PER; ++j) {
-      const int64_t h = min(h0 + warp * PV_PER + j, H - 1);
-      r[j] = fmaxf(ratio_mode == 0 ? ratio[0] : ratio_mode == 1 ? ratio[h] : ratio[(size_t)v * H + h], 1e-4f);
+      const int jj = min(j, last);                   // a hop past the end reads the last one's
+      r[j] = fmaxf(ratio_mode == 0 ? ratio[0] : ratio_v[h0 + w0 + jj], 1e-4f);
       const float src = kf / r[j];
       const bool in = src <= nm1;
       if (in) in_range |= 1u << j;
       const float srcc = in ? src : nm1, fl = floorf(srcc);
       frac[j] = srcc - fl;
       const int i0 = (int)fl, i1 = i0 < N - 1 ? i0 + 1 : i0;
-      const float2 *row = mag_omega + base + (size_t)h * N;
+      const float2 *row = rows + (ptrdiff_t)jj * N;
       lo[j] = __ldg(row + i0);
       hi[j] = __ldg(row + i1);
-      if (h == 0 && !started) {
+      if (t == 0 && w0 + j == 0 && !started) {
         // first hop of the stream: start from the interpolated analysis phase of this hop
         const float p0 = atan2f(im[base + i0], re[base + i0]), p1 = atan2f(im[base + i1], re[base + i1]);
         phase[0][0][lane] = principal_arg(mixf(p0, p1, frac[j]));
       }
     }
+    rows += (size_t)PV_TILE * N;
   };
-  if (live) fetch(0);
-  for (int64_t h0 = 0; h0 < H + PV_TILE; h0 += PV_TILE) {
-    const int par = (int)(h0 / PV_TILE) & 1;
-    float before[PV_PER];
+  // what was fetched: the magnitudes kept, the frequencies for the one that adds
+  auto leave = [&](int t, int slot) {
 #pragma unroll
-    for (int j = 0; j < PV_PER; ++j) before[j] = mag[j];
-    if (live && h0 < H) {
-#pragma unroll
-      for (int j = 0; j < PV_PER; ++j) {
-        mag[j] = in_range & (1u << j) ? mixf(lo[j].x, hi[j].x, frac[j]) : 0.0f;
-        const int64_t h = h0 + warp * PV_PER + j;
-        if (h > 0 || started) phase[par][warp * PV_PER + j][lane] = mixf(lo[j].y, hi[j].y, frac[j]);
-        if (lane == 0) ratios[par][warp * PV_PER + j] = r[j];
-      }
-      if (h0 + PV_TILE < H) fetch(h0 + PV_TILE);      // in flight while this tile's phases are added up
+    for (int j = 0; j < PV_PER; ++j) {
+      mag[0][j] = mag[1][j];
+      mag[1][j] = in_range & (1u << j) ? mixf(lo[j].x, hi[j].x, frac[j]) : 0.0f;
+      if (t > 0 || w0 + j > 0 || started) phase[slot][w0 + j][lane] = mixf(lo[j].y, hi[j].y, frac[j]);
+      if (lane == 0) ratios[slot][w0 + j] = r[j];
     }
-    __syncthreads();
-    if (adds && h0 < H) {
-      const int cnt = (int)min((int64_t)PV_TILE, H - h0);
-#pragma unroll 8
-      for (int j = 0; j < cnt; ++j) {
-        const float om = phase[par][j][lane];
-        synth = h0 + j == 0 && !started ? om : wrapped(fmaf(om, ratios[par][j], synth));
-        phase[par][j][lane] = synth;
-      }
-    }
-    if (live && h0 > 0) {
-#pragma unroll
-      for (int j = 0; j < PV_PER; ++j) {
-        const int64_t h = h0 - PV_TILE + warp * PV_PER + j;
-        if (h < H) {
-          float sn, cs;
-          sincosf(phase[par ^ 1][warp * PV_PER + j][lane], &sn, &cs);
-          const size_t o = base + (size_t)h * N + k;
-          out_re[o] = before[j] * cs;
-          out_im[o] = before[j] * sn;
-        }
-      }
-    }
-    __syncthreads();
+  };
+  if (live) {
+    fetch(0);
+    leave(0, 0);
+    if (tiles > 1) fetch(1);
   }
-  if (st && live && adds) {
-    const size_t last = base + (size_t)(H - 1) * N + k;
-    const float ph = atan2f(im[last], re[last]);
-    // the "started" flag is shared by all bins of a voice and other blocks may still have to read it: a launch of
-    // its own sets it afterwards
-    st[N + k] = synth;
-    st[k] = ph;
+  __syncthreads();
+  for (int t = 0, slot = 0; t <= tiles; ++t, slot = slot == 2 ? 0 : slot + 1) {   // tile t is added up
+    if (live) {
+      float before[PV_PER];
+#pragma unroll
+      for (int j = 0; j < PV_PER; ++j) before[j] = mag[0][j];
+      if (t + 1 < tiles) {
+        leave(t + 1, slot == 2 ? 0 : slot + 1);
+        if (t + 2 < tiles) fetch(t + 2);
+      } else {
+#pragma unroll
+        for (int j = 0; j < PV_PER; ++j) mag[0][j] = mag[1][j];
+      }
+      if (t > 0) {
+        const int cnt = (int)min((int64_t)PV_PER, H - (int64_t)(t - 1) * PV_TILE - w0);
+#pragma unroll
+        for (int j = 0; j < PV_PER; ++j)
+          if (j < cnt) {
+            float sn, cs;
+            sincos_wrapped(phase[slot == 0 ? 2 : slot - 1][w0 + j][lane], sn, cs);
+            o_re[(ptrdiff_t)j * N] = before[j] * cs;
+            o_im[(ptrdiff_t)j * N] = before[j] * sn;
+          }
+        o_re += (size_t)PV_TILE * N;
+        o_im += (size_t)PV_TILE * N;
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -919,7 +990,7 @@ DGC_EXPORT int32_t dgc_phase_vocoder(dgc_ctx *ctx, const float *re_dev, const fl
   dgc_launch(pv_analysis_kernel, dim3((unsigned)runs, dgc_div_up(N, 128), V), 128, 0, ctx->stream, re_dev, im_dev, H, N,
              omega_scale, state_dev, mag_omega);
   DGC_LAUNCHED(ctx, "phase_vocoder_analysis");
-  dgc_launch(pv_synthesis_kernel, dim3(dgc_div_up(N, PV_BINS), V), PV_BINS * PV_WARPS, 0, ctx->stream, re_dev, im_dev, mag_omega,
+  dgc_launch(pv_synthesis_kernel, dim3(dgc_div_up(N, PV_BINS), V), PV_THREADS, 0, ctx->stream, re_dev, im_dev, mag_omega,
              ratio_dev, ratio_mode, H, N, state_dev, out_re_dev, out_im_dev);
   DGC_LAUNCHED(ctx, "phase_vocoder_synthesis");
   if (state_dev) {
