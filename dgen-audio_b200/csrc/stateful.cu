@@ -295,9 +295,11 @@ __global__ void latch_out_kernel(const float *__restrict__ value, const float *_
 
 // The output pass with FOUR lanes per thread (W a multiple of 4): a warp reads 512 contiguous bytes of a frame, the
 // block = (W / 4 lane groups) x (chunks) covers whole rows, results leave as 128-bit streaming stores.
+// Bound by the loads in flight of the few threads that a chunk of 128 frames leaves: SHARED, one condition per frame, keeps
+// sixteen frames of values on their way.  262144 frames of 64 lanes: 30 us with eight, 22.6 with sixteen.
+template <bool SHARED>
 __global__ void __launch_bounds__(256)
-latch_out4_kernel(const float *__restrict__ value, const float *__restrict__ cond, int cond_mode, int64_t T, int W,
-                  int NC, const int *__restrict__ src_off, const int *__restrict__ src_chunk,
+latch_out4_kernel(const float *__restrict__ value, const float *__restrict__ cond, int64_t T, int W, int NC, const int *__restrict__ src_off, const int *__restrict__ src_chunk,
                   const float *__restrict__ state, float *__restrict__ y) {
   dgc_after_previous();
   const int e = (blockIdx.x * blockDim.x + threadIdx.x) * 4, c = blockIdx.y * blockDim.y + threadIdx.y;
@@ -310,27 +312,27 @@ latch_out4_kernel(const float *__restrict__ value, const float *__restrict__ con
                       : (state ? state[e + k] : 0.0f);
   }
   const int64_t n0 = (int64_t)c * LATCH_CHUNK, n1 = min(n0 + (int64_t)LATCH_CHUNK, T);
-  constexpr int G = 8;
+  constexpr int G = SHARED ? 16 : 8;
   for (int64_t n = n0; n < n1; n += G) {
-    float4 v[G], cc[G];
+    float4 v[G], cc[SHARED ? 1 : G];
+    float shared_cond[SHARED ? G : 1];
 #pragma unroll
     for (int j = 0; j < G; ++j) {
       const int64_t m = min(n + j, n1 - 1);
       v[j] = __ldcs(reinterpret_cast<const float4 *>(value + m * W + e));
-      if (cond_mode == 1) {
-        const float t = cond[m];
-        cc[j] = make_float4(t, t, t, t);
-      } else {
-        cc[j] = __ldcs(reinterpret_cast<const float4 *>(cond + m * W + e));
-      }
+      if constexpr (SHARED) shared_cond[j] = cond[m];
+      else cc[j] = __ldcs(reinterpret_cast<const float4 *>(cond + m * W + e));
     }
 #pragma unroll
     for (int j = 0; j < G; ++j)
       if (n + j < n1) {
-        if (cc[j].x > 0.0f) held[0] = v[j].x;
-        if (cc[j].y > 0.0f) held[1] = v[j].y;
-        if (cc[j].z > 0.0f) held[2] = v[j].z;
-        if (cc[j].w > 0.0f) held[3] = v[j].w;
+        float4 c4;
+        if constexpr (SHARED) c4 = make_float4(shared_cond[j], shared_cond[j], shared_cond[j], shared_cond[j]);
+        else c4 = cc[j];
+        if (c4.x > 0.0f) held[0] = v[j].x;
+        if (c4.y > 0.0f) held[1] = v[j].y;
+        if (c4.z > 0.0f) held[2] = v[j].z;
+        if (c4.w > 0.0f) held[3] = v[j].w;
         __stcs(reinterpret_cast<float4 *>(y + (n + j) * W + e), make_float4(held[0], held[1], held[2], held[3]));
       }
   }
@@ -907,8 +909,9 @@ DGC_EXPORT int32_t dgc_latch(dgc_ctx *ctx, const float *value_dev, const float *
                     ((((uintptr_t)value_dev) | ((uintptr_t)y_dev) | (cond_mode == 2 ? (uintptr_t)cond_dev : 0)) & 15) == 0;
   if (quad) {
     const int bx = lanes / 4 >= 64 ? 64 : lanes / 4, by = 256 / bx >= 1 ? (256 / bx > 8 ? 8 : 256 / bx) : 1;
-    dgc_launch(latch_out4_kernel, dim3(dgc_div_up(lanes / 4, bx), dgc_div_up(NC, by)), dim3(bx, by), 0, ctx->stream, value_dev,
-               cond_dev, cond_mode, T, lanes, NC, last, src_chunk, state_dev, y_dev);
+    auto kern = cond_mode == 1 ? latch_out4_kernel<true> : latch_out4_kernel<false>;
+    dgc_launch(kern, dim3(dgc_div_up(lanes / 4, bx), dgc_div_up(NC, by)), dim3(bx, by), 0, ctx->stream, value_dev, cond_dev, T,
+               lanes, NC, last, src_chunk, state_dev, y_dev);
   } else {
     dgc_launch(latch_out_kernel, grid, 128, 0, ctx->stream, value_dev, cond_dev, cond_mode, T, lanes, NC, last, src_chunk,
                state_dev, y_dev);
