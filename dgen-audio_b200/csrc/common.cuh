@@ -113,6 +113,10 @@ int32_t dgc_gemm_nt(dgc_ctx *ctx, const float *a, const float *b, int M, int N, 
 unsigned int *dgc_ctx_ticket(dgc_ctx *ctx);
 // whether dgc_linear_bwd has a use for a transposed copy of the layer's input
 bool dgc_linear_bwd_reads_t(int64_t M, int64_t K, int64_t N);
+// dgc_linear_bwd, its weight gradients on the side stream where that helps (gemm.cu)
+int32_t dgc_linear_bwd_beside(dgc_ctx *ctx, const float *a_dev, const float *w_dev, const float *c_dev, const float *dc_dev,
+                              int32_t M, int32_t K, int32_t N, int32_t act, float *dz_dev, float *da_dev, float *dw_dev,
+                              float *dbias_dev, const float *at_dev, bool *beside);
 // true when dgc_gemm_nt() runs this shape on its persistent short-reduction tensor-core kernel
 bool dgc_gemm_nt_persistent(const dgc_ctx *ctx, const float *a, int M, int N, int K);
 const float2 *dgc_ctx_twiddles(dgc_ctx *ctx, int N);

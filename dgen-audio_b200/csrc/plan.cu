@@ -13,10 +13,15 @@
 
 namespace {
 
-__global__ void plan_add_kernel(const float *a, const float *__restrict__ b, size_t n, float *out) {
+// copy (optional): the sum goes there too
+__global__ void plan_add_kernel(const float *a, const float *b, size_t n, float *out, float *copy) {
   dgc_after_previous();
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = __fadd_rn(a[i], b[i]);
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) {
+    const float v = __fadd_rn(a[i], b[i]);
+    out[i] = v;
+    if (copy) copy[i] = v;
+  }
 }
 
 // A step's inputs to their places, one launch for all of them: blockIdx.y picks the pair (eight copies of their own took 20
@@ -118,9 +123,29 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
       forked = false;
     }
   };
+  // Weight gradients left on the side stream by the layers' backward steps (dgc_linear_bwd_beside): the steps right after them
+  // that are such too go on, as long as they keep off the buffers that are read and written there; anything else joins first.
+  struct Range {
+    uint64_t off, n;
+  };
+  std::vector<Range> side_reads, side_writes;
+  auto join_side = [&]() {
+    if (side_writes.empty()) return;
+    cudaEventRecord(ctx->join_ev, ctx->aux_stream);
+    cudaStreamWaitEvent(main_stream, ctx->join_ev, 0);
+    side_reads.clear();
+    side_writes.clear();
+  };
+  auto meets = [](const std::vector<Range> &x, const std::vector<Range> &y) {
+    for (const Range &p : x)
+      for (const Range &q : y)
+        if (p.off != DGC_PLAN_NONE && q.off != DGC_PLAN_NONE && p.off < q.off + q.n && q.off < p.off + p.n) return true;
+    return false;
+  };
   for (int k = first; k < last && rc == DGC_OK; ++k) {
     const dgc_plan_step &s = plan->steps[k];
     R.step = k;
+    if (s.op != DGC_PLAN_LINEAR_BWD) join_side();
     if (s.stream == 1 && !forked && s.op != DGC_PLAN_FORK) {
       rc = dgc_fail(ctx, DGC_ERR_INVALID, "dgc_plan_run: step %d runs on the side stream before a FORK", k);
       break;
@@ -171,8 +196,16 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
         const uint64_t n = a[3];
         const float *x = R.at(a[0], n), *y = R.at(a[1], n);
         float *out = R.at(a[2], n);
+        // a copy of the sum, the next step, goes out with it (unless it lands on what the sum reads or writes)
+        float *copy = nullptr;
+        if (!R.bad && n > 0 && k + 1 < last && plan->steps[k + 1].op == DGC_PLAN_COPY && plan->steps[k + 1].stream == s.stream &&
+            plan->steps[k + 1].a[0] == a[2] && plan->steps[k + 1].a[2] == n &&
+            !meets({{plan->steps[k + 1].a[1], n}}, {{a[0], n}, {a[1], n}, {a[2], n}})) {
+          R.step = ++k;
+          copy = R.at(plan->steps[k].a[1], n);
+        }
         if (!R.bad && n > 0) {
-          dgc_launch(plan_add_kernel, dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream, x, y, n, out);
+          dgc_launch(plan_add_kernel, dgc_div_up((int64_t)n, 256), 256, 0, ctx->stream, x, y, n, out, copy);
           ctx->launches++;
           rc = dgc_check_launch(ctx, "plan_add");
         }
@@ -256,7 +289,20 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
         const float *A = R.at(a[0], M * K), *W = R.at(a[1], K * N), *Cm = R.at(a[2], M * N), *dC = R.at(a[3], M * N);
         float *dZ = R.at(a[4], M * N), *dA = R.at(a[5], M * K, true), *dW = R.at(a[6], K * N), *db = R.at(a[7], N, true);
         const float *At = R.at(a[8], M * K, true);
-        if (!R.bad) rc = dgc_linear_bwd(ctx, A, W, Cm, dC, i[0], i[1], i[2], i[3], dZ, dA, dW, db, At);
+        if (!R.bad) {
+          const std::vector<Range> reads = {{a[0], M * K}, {a[1], K * N}, {a[2], M * N}, {a[3], M * N}, {a[8], M * K}};
+          const std::vector<Range> writes = {{a[4], M * N}, {a[5], M * K}, {a[6], K * N}, {a[7], N}};
+          if (meets(writes, side_reads) || meets(writes, side_writes) || meets(reads, side_writes)) join_side();
+          // what the step itself hands on (dZ is read beside, the gradients are written there) must not be one buffer
+          const bool own = meets({writes[1]}, {{a[0], M * K}, writes[0], writes[2], writes[3]}) || meets({writes[2], writes[3]}, reads);
+          bool beside = false;
+          rc = dgc_linear_bwd_beside(ctx, A, W, Cm, dC, i[0], i[1], i[2], i[3], dZ, dA, dW, db, At,
+                                     s.stream == 0 && !forked && !own ? &beside : nullptr);
+          if (beside) {
+            side_reads.insert(side_reads.end(), {{a[0], M * K}, {a[4], M * N}});
+            side_writes.insert(side_writes.end(), {writes[2], writes[3]});
+          }
+        }
       } break;
       case DGC_PLAN_HEADS_FWD: {
         const uint64_t M = i[0], K = i[1], NB = i[2];
@@ -330,6 +376,7 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
     }
   }
   ctx->stream = main_stream;
+  join_side();
   join();
   return rc;
 }
@@ -481,7 +528,8 @@ DGC_EXPORT int32_t dgc_hn_train_plan(const dgc_hn_train_config *c, dgc_hn_train_
     s.i[0] = B; s.i[1] = T; s.i[2] = c->ir_len; s.i[3] = c->conv_n; s.i[4] = c->conv_hop; s.i[5] = 1;
     s.f[0] = 1.0f;
     S.push_back(s);
-    s = mk(DGC_PLAN_MSS_LOSS_FWD);
+    S.push_back(mk(DGC_PLAN_FORK));
+    s = mk(DGC_PLAN_MSS_LOSS_FWD, 1);   // nothing waits for the loss's value: beside the spectral and reverb gradients
     s.a[0] = lay->audio; s.a[1] = lay->target; s.a[3] = lay->loss;
     put_mss(s, c->mss, B, T);
     S.push_back(s);
@@ -499,6 +547,7 @@ DGC_EXPORT int32_t dgc_hn_train_plan(const dgc_hn_train_config *c, dgc_hn_train_
     s.f[0] = 1.0f;
     S.push_back(s);
   }
+  S.push_back(mk(DGC_PLAN_JOIN));
   S.push_back(mk(DGC_PLAN_FORK));
   {
     dgc_plan_step s = mk(DGC_PLAN_FIR_BWD, 1);

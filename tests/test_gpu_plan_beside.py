@@ -1,0 +1,91 @@
+"""Steps of a plan that the library runs beside each other or in one launch: weight gradients of a layer beside the backward of
+the next, a sum and its copy.  What they read and write decides, so the buffers here meet in every way they can."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+import dgen_b200
+from dgen_b200 import PLAN_ADD, PLAN_COPY, PLAN_LINEAR_BWD, Plan, PlanStep, plan_step
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = dgen_b200.Context(0)
+    yield c
+    c.close()
+
+
+def _run(ctx, arena, steps):
+    arr = (PlanStep * len(steps))(*steps)
+    plan = Plan(arr, len(steps), None, None, 0)
+    h = C.c_void_p()
+    ctx.check(ctx.lib.dgc_arena_wrap(ctx.h, arena.data_ptr(), arena.numel(), C.byref(h)))
+    ctx.check(ctx.lib.dgc_plan_run(ctx.h, h, C.byref(plan), 0, -1))
+    ctx.sync()
+    ctx.lib.dgc_arena_destroy(h)
+
+
+# shared: which buffers the layers have in common ("" none; dz: one dZ for all; act: the second layer's dA lands on the first
+# layer's input, which its weight gradient reads; grads: one weight gradient buffer, the last one written stays)
+@pytest.mark.parametrize("shared", ["", "dz", "act", "grads"])
+@pytest.mark.parametrize("M,H", [(300, 64), (750, 128), (2100, 64)])
+def test_layers_backward_as_a_plan(ctx, M, H, shared):
+    g = torch.Generator(device="cuda").manual_seed(M + H)
+    used = 0
+
+    def take(n):
+        nonlocal used
+        used += (n + 63) // 64 * 64
+        return used - (n + 63) // 64 * 64
+
+    L = 3
+    x = [take(M * H) for _ in range(L + 1)]            # inputs of the layers, the last layer's output
+    w = [take(H * H) for _ in range(L)]
+    d = [take(M * H) for _ in range(L + 1)]            # gradients of x
+    dz = [take(M * H) for _ in range(L)]
+    dw, db = [take(H * H) for _ in range(L)], [take(H) for _ in range(L)]
+    if shared == "dz":
+        dz = [dz[0]] * L
+    if shared == "act":
+        d[1] = x[2]                                    # layer 1's dA on the input of layer 2, whose gradient may still be read
+    if shared == "grads":
+        dw, db = [dw[0]] * L, [db[0]] * L
+    arena = torch.randn(used, device="cuda", generator=g) * 0.3
+    for o in x[1:]:
+        arena[o:o + M * H].tanh_()
+    want = arena.clone()
+    view = lambda t, o, *s: t[o:o + int(np.prod(s))].view(*s)
+    steps = []
+    for l in reversed(range(L)):
+        steps.append(plan_step(PLAN_LINEAR_BWD, a=(x[l], w[l], x[l + 1], d[l + 1], dz[l], d[l], dw[l], db[l], None), i=(M, H, H, 1)))
+        ctx.check(ctx.lib.dgc_linear_bwd(ctx.h, *[want.data_ptr() + 4 * o for o in (x[l], w[l], x[l + 1], d[l + 1])], M, H, H, 1,
+                                         *[want.data_ptr() + 4 * o for o in (dz[l], d[l], dw[l], db[l])], None))
+    ctx.sync()
+    for _ in range(3):
+        got = arena.clone()
+        _run(ctx, got, steps)
+        assert torch.equal(got, want)
+    if not shared:
+        z = view(arena, d[L], M, H).double() * (1 - view(arena, x[L], M, H).double() ** 2)
+        ref = view(arena, x[L - 1], M, H).double().t() @ z
+        assert float((view(want, dw[L - 1], H, H).double() - ref).norm() / ref.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("n", [1, 255, 1000])
+def test_sum_and_its_copy(ctx, n):
+    base = torch.randn(4 * 1024, device="cuda")
+    for src, dst, copy_n in ((2048, 3072, n), (2048, 0, n), (2048, 1024, n), (2048, 2048 + n // 2, n), (0, 3072, n), (2048, 3072, 1)):
+        # the sum of [0, n) and [1024, ..) at 2048 (or over its first term), then a copy of it elsewhere, on a term, on itself
+        want = base.clone()
+        want[src:src + n] = want[0:n] + want[1024:1024 + n]
+        want[dst:dst + copy_n] = want[src:src + copy_n].clone()
+        got = base.clone()
+        steps = [plan_step(PLAN_ADD, a=(0, 1024, src, n)), plan_step(PLAN_COPY, a=(src, dst, copy_n))]
+        if dst < src + n and src < dst + copy_n:
+            continue       # a copy onto itself is left to the device's copy, whose overlap is not defined
+        _run(ctx, got, steps)
+        assert torch.equal(got, want), (src, dst)
