@@ -357,6 +357,7 @@ class Context:
         self.lib = load()
         self.torch = torch
         self.device = device
+        self._device = self.torch.device("cuda", device)
         torch.cuda.set_device(device)
         h = _vp()
         rc = self.lib.dgc_ctx_create(device, C.byref(h))
@@ -408,7 +409,7 @@ class Context:
         return tuple(out)
 
     def _empty(self, *shape, dtype=None):
-        return self.torch.empty(*shape, dtype=dtype or self.torch.float32, device="cuda:%d" % self.device)
+        return self.torch.empty(*shape, dtype=dtype or self.torch.float32, device=self._device)
 
     # ---- clocks -----------------------------------------------------------------------------
     def clock_accum(self, incr, mn, mx, T, state0=0.0):
