@@ -294,7 +294,8 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
           const std::vector<Range> writes = {{a[4], M * N}, {a[5], M * K}, {a[6], K * N}, {a[7], N}};
           if (meets(writes, side_reads) || meets(writes, side_writes) || meets(reads, side_writes)) join_side();
           // what the step itself hands on (dZ is read beside, the gradients are written there) must not be one buffer
-          const bool own = meets({writes[1]}, {{a[0], M * K}, writes[0], writes[2], writes[3]}) || meets({writes[2], writes[3]}, reads);
+          const bool own = meets({writes[1]}, {{a[0], M * K}, writes[0], writes[2], writes[3]}) ||
+                           meets({writes[2], writes[3]}, reads);
           bool beside = false;
           rc = dgc_linear_bwd_beside(ctx, A, W, Cm, dC, i[0], i[1], i[2], i[3], dZ, dA, dW, db, At,
                                      s.stream == 0 && !forked && !own ? &beside : nullptr);

@@ -299,8 +299,9 @@ __global__ void latch_out_kernel(const float *__restrict__ value, const float *_
 // sixteen frames of values on their way.  262144 frames of 64 lanes: 30 us with eight, 22.6 with sixteen.
 template <bool SHARED>
 __global__ void __launch_bounds__(256)
-latch_out4_kernel(const float *__restrict__ value, const float *__restrict__ cond, int64_t T, int W, int NC, const int *__restrict__ src_off, const int *__restrict__ src_chunk,
-                  const float *__restrict__ state, float *__restrict__ y) {
+latch_out4_kernel(const float *__restrict__ value, const float *__restrict__ cond, int64_t T, int W, int NC,
+                  const int *__restrict__ src_off, const int *__restrict__ src_chunk, const float *__restrict__ state,
+                  float *__restrict__ y) {
   dgc_after_previous();
   const int e = (blockIdx.x * blockDim.x + threadIdx.x) * 4, c = blockIdx.y * blockDim.y + threadIdx.y;
   if (e >= W || c >= NC) return;
