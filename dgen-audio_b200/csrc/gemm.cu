@@ -137,13 +137,24 @@ bool smallk_shape(const dgc_ctx *ctx, const float *A, int M, int N, int K) {
   return nblk <= ctx->sm_count;
 }
 
+// 64 x 64 tiles of the output that the chip takes at once
+bool few_tiles(const dgc_ctx *ctx, int M, int N) {
+  return (int64_t)dgc_div_up(M, 64) * dgc_div_up(N, 64) <= ctx->sm_count;
+}
+
+// copies of both operands' rows, laid 16-byte aligned ld floats apart
+struct AlignedRows {
+  const float *A = nullptr, *B = nullptr;
+  int ld = 0;
+};
+
 template <bool TA, bool TB, int EPI>
 int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *bias, int M, int N, int K, float *C,
-                     float *Ct = nullptr, bool *ct_written = nullptr) {
+                     float *Ct = nullptr, bool *ct_written = nullptr, AlignedRows rows = {}) {
   if (ct_written) *ct_written = false;
   const bool tc = use_tensor_cores() && (double)M * N * K >= (double)(1 << 21) && K >= 32;
-  // both operands contiguous along k: rows of 16-byte units (A in tensor memory, 16-byte aligned rows), or any (4-byte copies,
-  // e.g. 165 outputs of the controller's heads)
+  // both operands contiguous along k: rows of 16-byte units (A in tensor memory), or any (4-byte copies, where no pass before
+  // has left copies of the rows that are aligned)
   const bool along_k = tc && !TA && TB;
   const bool kk16 = along_k && (K & 3) == 0 && ((((uintptr_t)A) | ((uintptr_t)B)) & 15) == 0;
   const bool kk = kk16 || (along_k && EPI == 0);
@@ -186,17 +197,22 @@ int32_t launch_sgemm(dgc_ctx *ctx, const float *A, const float *B, const float *
   dim3 grid(dgc_div_up(N, bn), dgc_div_up(M, bm), splits);
   // a whole reduction whose 64 x 64 tiles the chip takes at once: smaller tiles beat the pipeline (750 x 128 over 128 k: 10 -> 7 us,
   // 750 x 512 over 512 k: 30 -> 17 us)
-  const bool few = tc && splits == 1 && (int64_t)dgc_div_up(M, 64) * dgc_div_up(N, 64) <= ctx->sm_count;
+  const bool few = tc && splits == 1 && few_tiles(ctx, M, N);
   const bool piped = kk && !few && (splits == 1 || kps % 32 == 0);
   ctx->gemm_paths[piped ? (wide ? 3 : 2) : (tc ? 1 : 0)]++;
-  if (piped && kk16) {
+  if (piped && !kk16 && rows.A) {
+    A = rows.A;
+    B = rows.B;
+  }
+  if (piped && (kk16 || rows.A)) {
+    const int ld = kk16 ? K : rows.ld;
     auto kern = dgtc::tc_gemm_ts_kernel<EPI, dgtc::TBN>;
     if constexpr (EPI == 0) {
       if (wide) kern = dgtc::tc_gemm_ts_kernel<EPI, 256>;
     }
     const int smem = wide ? dgtc::TS<256>::SMEM : dgtc::TS<dgtc::TBN>::SMEM;
     CUtensorMap map_a, map_b;
-    if (!dgtma::make_map_k16(&map_a, A, M, K, dgtc::TBM) || !dgtma::make_map_k16(&map_b, B, N, K, bn))
+    if (!dgtma::make_map_k16(&map_a, A, M, K, ld, dgtc::TBM) || !dgtma::make_map_k16(&map_b, B, N, K, ld, bn))
       return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm: no tensor map for %d x %d x %d", M, N, K);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return dgc_fail(ctx, DGC_ERR_CUDA, "tc_gemm smem opt-in: %s", cudaGetErrorString(e));
@@ -269,13 +285,22 @@ __device__ __forceinline__ void store_tile_t(const float (*t)[TT + 1], int m0, i
 // memory), so that the weight-gradient product can read both of its operands along the reduction index.  Four passes
 // over the layer and nothing else: 32000 x 512 in 39 us (6.6 TB/s; 61 us in 32 x 32 tiles of single loads).  M a
 // multiple of 4; VEC: N too, and every buffer on 16 bytes.
-template <bool VEC>
+// Rows that are not (165 outputs of the heads) the copy engine cannot fetch: ALIGN (without VEC) lays them ld floats apart in
+// dZ_ld for the input gradient, and the blocks past the last tile of dZ do the same for the K rows of W.
+template <bool VEC, bool ALIGN>
 __global__ void __launch_bounds__(256)
 act_bwd_t_kernel(const float *__restrict__ dC, const float *__restrict__ Cv, int M, int N, int act,
-                 float *__restrict__ dZ, float *__restrict__ dZt) {
+                 float *__restrict__ dZ, float *__restrict__ dZt, int ld, float *__restrict__ dZ_ld,
+                 const float *__restrict__ W, int K, float *__restrict__ W_ld) {
   dgc_after_previous();
   __shared__ float t[TT][TT + 1];
   const int n0 = blockIdx.x * TT, m0 = blockIdx.y * TT;
+  if (ALIGN && m0 >= M) {
+    const int n = n0 + (threadIdx.x & 63), k0 = (blockIdx.y - (M + TT - 1) / TT) * TT;
+    for (int k = k0 + (threadIdx.x >> 6); k < min(K, k0 + TT); k += 4)
+      if (n < N) W_ld[(size_t)k * ld + n] = W[(size_t)k * N + n];
+    return;
+  }
   if (VEC) {
     const int n = (threadIdx.x & 15) * 4, mr = threadIdx.x >> 4;
     float4 g[4], c[4];
@@ -315,6 +340,7 @@ act_bwd_t_kernel(const float *__restrict__ dC, const float *__restrict__ Cv, int
           g *= (1.0f - c * c);
         }
         dZ[idx] = g;
+        if (ALIGN) dZ_ld[(size_t)(m0 + m) * ld + n0 + n] = g;
       }
       t[m][n] = g;
     }
@@ -655,21 +681,32 @@ int32_t dgc_linear_bwd_beside(dgc_ctx *ctx, const float *a_dev, const float *w_d
   // With a transposed copy of the layer input at hand, the weight gradient reads both operands along the
   // reduction index m (the asynchronous K-major pipeline): dZ is then written in both orientations.
   const bool dw_kmajor = at_dev && dgc_linear_bwd_reads_t(M, K, N) && (((uintptr_t)at_dev) & 15) == 0;
+  AlignedRows rows;
   if (dw_kmajor) {
-    if (!ctx->dzt_buf || ctx->dzt_floats < n) {
+    // The input gradient dZ W^T reads rows of N floats, too: where they are not on 16 bytes, copies of dZ and W that are (of no
+    // use to a few tiles or a short reduction).  N = 165, K = 512, the layer's whole backward with 4-byte copies for this product
+    // and with aligned rows: 2000 rows 100 -> 94 us, 8000 rows 85 -> 72, 32000 rows 176 -> 134, 64000 rows 300 -> 224; K = 128:
+    // 68.7 -> 60 (8000 rows), 102 -> 93 (32000).  A pass of its own over dZ for the copies: 146 us at 32000 rows, and slower than
+    // 4-byte copies at 16000 rows and K = 128 (71 -> 77).
+    const bool align = da_dev && (N & 3) && N >= 32 && !few_tiles(ctx, M, K) && !smallk_shape(ctx, dz_dev, M, K, N);
+    const int ld = (N + 3) & ~3;
+    const size_t need = n + (align ? (size_t)(M + (int64_t)K) * ld : 0);   // M, so n, is a multiple of 4
+    if (!ctx->dzt_buf || ctx->dzt_floats < need) {
       if (ctx->dzt_buf) {
         cudaStreamSynchronize(ctx->stream);
         cudaFree(ctx->dzt_buf);
         ctx->buffer_generation++;
         ctx->dzt_buf = nullptr;
       }
-      DGC_CUDA(ctx, cudaMalloc(&ctx->dzt_buf, n * sizeof(float)));
-      ctx->dzt_floats = n;
+      DGC_CUDA(ctx, cudaMalloc(&ctx->dzt_buf, need * sizeof(float)));
+      ctx->dzt_floats = need;
     }
+    float *dz_ld = align ? ctx->dzt_buf + n : nullptr, *w_ld = align ? dz_ld + (size_t)M * ld : nullptr;
+    if (align) rows = {dz_ld, w_ld, ld};
     const bool vec = (N & 3) == 0 && ((((uintptr_t)dc_dev) | ((uintptr_t)dz_dev) | (act == 1 ? (uintptr_t)c_dev : 0)) & 15) == 0;
-    auto kern = vec ? act_bwd_t_kernel<true> : act_bwd_t_kernel<false>;
-    dgc_launch(kern, dim3(dgc_div_up(N, TT), dgc_div_up(M, TT)), 256, 0, ctx->stream, dc_dev, c_dev, M, N, act, dz_dev,
-               ctx->dzt_buf);
+    auto kern = vec ? act_bwd_t_kernel<true, false> : align ? act_bwd_t_kernel<false, true> : act_bwd_t_kernel<false, false>;
+    dgc_launch(kern, dim3(dgc_div_up(N, TT), dgc_div_up(M, TT) + (align ? dgc_div_up(K, TT) : 0)), 256, 0, ctx->stream, dc_dev,
+               c_dev, M, N, act, dz_dev, ctx->dzt_buf, ld, dz_ld, w_dev, K, w_ld);
   } else {
     const bool vec = (n & 3) == 0 && ((((uintptr_t)dc_dev) | ((uintptr_t)dz_dev) | (act == 1 ? (uintptr_t)c_dev : 0)) & 15) == 0;
     if (vec)
@@ -697,7 +734,7 @@ int32_t dgc_linear_bwd_beside(dgc_ctx *ctx, const float *a_dev, const float *w_d
   if (rc != DGC_OK) return rc;
   if (da_dev) {
     // dA[M][K] = dZ[M][N] * W^T[N][K]
-    rc = launch_sgemm<false, true, 0>(ctx, dz_dev, w_dev, nullptr, M, K, N, da_dev);
+    rc = launch_sgemm<false, true, 0>(ctx, dz_dev, w_dev, nullptr, M, K, N, da_dev, nullptr, nullptr, rows);
     if (rc != DGC_OK) return rc;
     DGC_LAUNCHED(ctx, "linear_bwd_da");
   }

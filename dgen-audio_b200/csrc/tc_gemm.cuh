@@ -413,8 +413,8 @@ tc_gemm_kernel(const float *__restrict__ A, const float *__restrict__ B, const f
 
 
 // ---------------------------------------------------------------------------------------------------------
-// Both operands contiguous along k in memory (A [M][K], B [N][K]), rows only 4-byte aligned (K not a multiple of 4): the
-// asynchronous pipeline by 4-byte copies.  cp.async copies floats straight into the 64-byte-swizzled K-major layout (8-row groups
+// Both operands contiguous along k in memory (A [M][K], B [N][K]), rows only 4-byte aligned (K not a multiple of 4, and no pass
+// before that could leave aligned copies of them): the asynchronous pipeline by 4-byte copies.  cp.async copies floats straight into the 64-byte-swizzled K-major layout (8-row groups
 // of 512 bytes, 16-byte chunk c of row r at c ^ ((r / 2) % 4)), RAW raw stages deep, PF tiles ahead of the tensor core; the raw
 // fp32 tile IS the "hi" operand (the tensor core reads the top 19 bits of every 32-bit word and ignores the 13 low mantissa
 // bits, i.e. it truncates to TF32 itself), so the threads only compute lo = x - trunc(x), shared memory to shared memory, into
@@ -591,7 +591,7 @@ tc_gemm_kk4_kernel(const float *__restrict__ A, const float *__restrict__ B, int
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Both operands contiguous along k, K a multiple of 4, 16-byte aligned rows: operand A in tensor memory, one persistent CTA per
+// Both operands contiguous along k, 16-byte aligned rows: operand A in tensor memory, one persistent CTA per
 // SM.  Fetching both operands from shared memory for each of the three products, a pipeline like the one above carries 96 KB of
 // it per 16 k of a 128 x 128 tile, 768 cycles for 384 of multiplying, and a CTA's split, products and epilogue come one
 // after the other.  Here

@@ -45,12 +45,12 @@ inline bool make_map_2d(CUtensorMap *map, const float *base, uint64_t rows, uint
 }
 
 // boxes of box_rows rows of 16 floats (64 bytes), each row of 16-byte chunks permuted by the 64-byte swizzle (chunk c of row r at
-// c ^ ((r / 2) % 4)): a tile of a matmul operand that is contiguous along k
-inline bool make_map_k16(CUtensorMap *map, const float *base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+// c ^ ((r / 2) % 4)): a tile of a matmul operand that is contiguous along k, its rows ld floats apart (past cols it reads zeros)
+inline bool make_map_k16(CUtensorMap *map, const float *base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
   EncodeTiledFn fn = encode_fn();
-  if (!fn || (((uintptr_t)base) & 15) != 0 || (cols & 3) != 0 || box_rows == 0 || box_rows > 256) return false;
+  if (!fn || (((uintptr_t)base) & 15) != 0 || (ld & 3) != 0 || ld < cols || box_rows == 0 || box_rows > 256) return false;
   const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {cols * sizeof(float)};
+  const cuuint64_t strides[1] = {ld * sizeof(float)};
   const cuuint32_t box[2] = {16, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box, estr,

@@ -49,6 +49,26 @@ def test_layers_that_fill_no_tile(ctx, M, K, N, act):
     ctx.sync()
 
 
+# N not a multiple of 4: the input gradient reads copies of dZ and W in aligned rows (but for few tiles, the second case, and
+# a short reduction over 128 columns, the third)
+@pytest.mark.parametrize("M,K,N,act", [(4000, 512, 165, 0), (1024, 300, 61, 1), (8000, 130, 70, 0), (9604, 65, 33, 1),
+                                       (20000, 100, 35, 0), (5000, 257, 127, 1), (32000, 36, 18, 0)])
+def test_input_gradient_of_unaligned_rows(ctx, M, K, N, act):
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    a = torch.randn(M, K, device="cuda", generator=g)
+    w = torch.randn(K, N, device="cuda", generator=g) * K ** -0.5
+    b = torch.randn(N, device="cuda", generator=g)
+    c = ctx.linear_fwd(a, w, b, act=act)
+    dc = torch.randn(M, N, device="cuda", generator=g)
+    dz = dc.double() * (1 - c.double() ** 2) if act else dc.double()
+    at = a.t().contiguous()
+    ctx.linear_bwd(a, w, c, torch.full_like(dc, float("nan")), act=act, a_t=at)   # what an earlier call leaves between the rows
+    da, dw, db = ctx.linear_bwd(a, w, c, dc, act=act, a_t=at)
+    assert _rel(da, dz @ w.double().t()) < _tol(N)
+    assert _rel(dw, a.double().t() @ dz) < _tol(M)
+    assert _rel(db, dz.sum(0)) < _tol(M)
+
+
 def test_rows_past_the_end_are_not_read(ctx):
     """NaN behind the operand and in front of it: what the copy engine brings past the last row or column arrives as zeros."""
     M, K, N = 4100, 132, 300
