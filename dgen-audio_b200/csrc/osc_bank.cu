@@ -806,9 +806,10 @@ harmonic_render_frame_kernel(dgc_harmonic_params prm, const float2 *__restrict__
   *dst = prm.accumulate ? *dst + val : val;
 }
 
-// sin and cos of 2 pi p, p in Q0.32, to 1.2e-7: the angle is taken from the nearest half turn, x in [-1/2, 1/2) half turns (an
-// exact integer, converted with 24 bits), and both polynomials in x^2 (minimax on that range: 3e-9 and 5e-8) are walked as the
-// two halves of packed multiply-adds.  Twelve instructions for the two of them, where the fast ones are good to 3.6e-7 each.
+// sin and cos of 2 pi p, p in Q0.32, to 2.0e-7 (5e-8 root mean square): the angle is taken from the nearest half turn, x in
+// [-1/2, 1/2) half turns (an exact integer, converted with 24 bits), and both polynomials in x^2 (minimax on that range: 3e-9 and
+// 5e-8) are walked as the two halves of packed multiply-adds.  Twelve instructions for the two of them, where the fast ones are
+// good to 3.6e-7 each.
 __device__ __forceinline__ void sincos_q32(uint32_t q, float &s, float &c) {
   const float x = __int2float_rn((int)(q << 1)) * 0x1p-32f;
   const float z = x * x;
@@ -823,17 +824,41 @@ __device__ __forceinline__ void sincos_q32(uint32_t q, float &s, float &c) {
   c = __uint_as_float(__float_as_uint(p.y) ^ flip);
 }
 
+// The same to 1.0e-7 (2.1e-8 root mean square), for a turn that is applied again and again: from the nearest QUARTER turn, where
+// the rounding inside the polynomials is small (minimax for x^2 <= 1/16: 1e-10 and 2e-10); behind odd ones the two change places.
+__device__ __forceinline__ void sincos_turn_q32(uint32_t q, float &s, float &c) {
+  const uint32_t j = (q + 0x20000000u) >> 30;
+  const float x = __int2float_rn((int)(q - (j << 30))) * 0x1p-31f;
+  const float z = x * x;
+  const float2 zz = make_float2(z, z);
+  float2 p = make_float2(0.0812296873f, 0.2321258803f);
+  p = __ffma2_rn(p, zz, make_float2(-0.5992288066f, -1.3351378576f));
+  p = __ffma2_rn(p, zz, make_float2(2.5501635938f, 4.0587105667f));
+  p = __ffma2_rn(p, zz, make_float2(-5.1677127792f, -4.9348021975f));
+  const float sx = fmaf(x * z, p.x, x * 3.14159265358979f), cx = fmaf(p.y, z, 1.0f);
+  s = __uint_as_float(__float_as_uint(j & 1 ? cx : sx) ^ ((j & 2) << 30));
+  c = __uint_as_float(__float_as_uint(j & 1 ? sx : cx) ^ (((j + 1) & 2) << 30));
+}
+
 // The same frames with the partials in groups of eight around a centre: partials k0 + 1 .. k0 + 8 lie at half-integer
 // distances d = 1/2, 3/2, 5/2, 7/2 on both sides of k0 + 9/2, so with U = sum_d (a_+ + a_-) cos d, V = sum_d (a_+ - a_-) sin d
 //   sum_k a_k sin(2 pi k P) = Im e^(2 pi i (k0 + 9/2) P) (U + i V),
 // the distances being the same in every group.  The groups are a polynomial in e^(2 pi i 8 P), taken by Horner from the last,
 // partly audible one down, each amplitude entering by two multiply-adds, two partials at a time: six angles per frame in all
 // instead of one per partial, a third fewer instructions.  Bound by the loads of the amplitudes that a warp broadcasts (52 % of
-// the L1's data rate) and by issue: 419 -> 368 us at 256 voices x 64000 frames, 35 -> 29 at 16.  Against double precision on the
-// same track the render is off by 2.0e-7 of its norm, partial by partial by 5.8e-7 (23 bits of phase and the fast sine).
+// the L1's data rate) and by issue: 419 -> 368 us at 256 voices x 64000 frames, 35 -> 29 at 16.
 // Several tiles of frames per block, the next one's lookups in flight, gave 4 % at 256 voices and cost 4 % at 16; fewer
 // registers (48, 40) cost 2 and 23 %.
-template <bool VEC>
+//
+// The turn from a group to the next is one rounded value, and what it is off by adds up in one direction, group after group.
+// Against double on the same phases, with amplitudes that are uniform, or zero but for the last eight (relative 2-norm; partial by
+// partial it is 6e-7 at any count: 23 bits of phase and the fast sine):
+//   16 partials 1.3e-7 | 1.4e-7, 64: 1.9e-7 | 2.4e-7, 104: 2.4e-7 | 3.7e-7, 128: 2.7e-7 | 4.5e-7, 512: 1.0e-6 | 1.9e-6
+// so a row of more than RENDER_ROW partials (SEGMENTS) is taken in polynomials of RENDER_SEGMENT, each turned to its place by an
+// angle of its own, 512 partials 2.0e-7 | 2.4e-7.  The other rows, which need none, are spared the registers and the time: 474 us
+// for the whole render of 256 voices with 100 partials, 499 with segments.
+constexpr int RENDER_ROW = 104, RENDER_SEGMENT = 64;
+template <bool VEC, bool SEGMENTS>
 __global__ void __launch_bounds__(128)
 harmonic_render_group_kernel(dgc_harmonic_params prm, const float2 *__restrict__ rowtab, const float *__restrict__ env,
                              const float *__restrict__ amps, const unsigned long long *__restrict__ fund,
@@ -865,7 +890,7 @@ harmonic_render_group_kernel(dgc_harmonic_params prm, const float2 *__restrict__
   sincos_q32((uint32_t)((half_r + (step << 1)) >> 32), S2, C2);
   sincos_q32((uint32_t)((half_r + (step << 1) + step) >> 32), S3, C3);
   sincos_q32((uint32_t)((half_r + (step << 2)) >> 32), s0, c0);                 // the first group's centre
-  sincos_q32((uint32_t)(((step << 3) + (1ull << 31)) >> 32), s8, c8);           // from a group to the next
+  sincos_turn_q32((uint32_t)(((step << 3) + (1ull << 31)) >> 32), s8, c8);      // from a group to the next
   const float2 C01 = make_float2(C0, C1), C23 = make_float2(C2, C3), C10 = make_float2(C1, C0), C32 = make_float2(C3, C2);
   const float2 S01 = make_float2(S0, S1), S23 = make_float2(S2, S3), S10 = make_float2(-S1, -S0), S32 = make_float2(-S3, -S2);
   const float2 W = make_float2(c8, c8), X = make_float2(s8, s8), Y = make_float2(-s8, -s8);
@@ -905,15 +930,28 @@ harmonic_render_group_kernel(dgc_harmonic_params prm, const float2 *__restrict__
     }
     group(make_float2(a[0], a[1]), make_float2(a[2], a[3]), make_float2(a[4], a[5]), make_float2(a[6], a[7]));
   }
+  auto down = [&](int end) {
 #pragma unroll 2
-  for (; k > 0; k -= 8) {
-    pl -= 8;
-    ph -= 8;
-    const float4 l0 = four(pl), l1 = four(pl + 4), h0 = four(ph), h1 = four(ph + 4);
-    group(mix(l0.x, l0.y, h0.x, h0.y), mix(l0.z, l0.w, h0.z, h0.w), mix(l1.x, l1.y, h1.x, h1.y), mix(l1.z, l1.w, h1.z, h1.w));
+    for (; k > end; k -= 8) {
+      pl -= 8;
+      ph -= 8;
+      const float4 l0 = four(pl), l1 = four(pl + 4), h0 = four(ph), h1 = four(ph + 4);
+      group(mix(l0.x, l0.y, h0.x, h0.y), mix(l0.z, l0.w, h0.z, h0.w), mix(l1.x, l1.y, h1.x, h1.y), mix(l1.z, l1.w, h1.z, h1.w));
+    }
+  };
+  float im = 0.0f;
+  if (SEGMENTS) {
+    for (int k0 = (max(count, 1) - 1) & -RENDER_SEGMENT; k0 > 0; k0 -= RENDER_SEGMENT) {
+      down(k0);
+      float sk, ck;   // the first centre of the segment
+      sincos_q32((uint32_t)((half_r + step * (uint32_t)(k0 + 4)) >> 32), sk, ck);
+      im = fmaf(sk, U.x + U.y, fmaf(ck, V.x + V.y, im));
+      U = V = make_float2(0.0f, 0.0f);
+    }
   }
+  down(0);
   const float inv = 1.0f / (sum.x + sum.y + 1e-8f);
-  const float ratio = fmaf(s0, U.x + U.y, c0 * (V.x + V.y)) * inv;
+  const float ratio = fmaf(s0, U.x + U.y, fmaf(c0, V.x + V.y, im)) * inv;
   if (sums) sums[(size_t)b * T + n] = make_float2(ratio, inv);   // for the backward: it then reduces nothing per frame
   const float val = ratio * env[(size_t)b * T + n];
   float *dst = audio + (size_t)b * T + n;
@@ -968,8 +1006,10 @@ void launch_render_q(dgc_ctx *ctx, const dgc_harmonic_params &p, const float2 *r
     const dim3 fgrid(dgc_div_up(p.T, 128), p.B);
     const bool vec = (p.K & 3) == 0 && (((uintptr_t)amps) & 15) == 0;
     float2 *keep = keep_sums ? x.sums : nullptr;
+    const bool segments = p.K > RENDER_ROW;
     auto kern = by_partial ? (vec ? harmonic_render_frame_kernel<true> : harmonic_render_frame_kernel<false>)
-                           : (vec ? harmonic_render_group_kernel<true> : harmonic_render_group_kernel<false>);
+              : segments   ? (vec ? harmonic_render_group_kernel<true, true> : harmonic_render_group_kernel<false, true>)
+                           : (vec ? harmonic_render_group_kernel<true, false> : harmonic_render_group_kernel<false, false>);
     dgc_launch(kern, fgrid, 128, 0, ctx->stream, p, rowtab, x.env, amps, x.fund, x.trk, keep, out);
   } else
     dgc_launch(harmonic_render_q_kernel<LPC, P, MODE>, grid, 128, 0, ctx->stream, p, 1.0f / p.sample_rate, rowtab, x.f0t, x.env,
