@@ -854,11 +854,18 @@ __device__ __forceinline__ void sincos_turn_q32(uint32_t q, float &s, float &c) 
 // Against double on the same phases, with amplitudes that are uniform, or zero but for the last eight (relative 2-norm; partial by
 // partial it is 6e-7 at any count: 23 bits of phase and the fast sine):
 //   16 partials 1.3e-7 | 1.4e-7, 64: 1.9e-7 | 2.4e-7, 104: 2.4e-7 | 3.7e-7, 128: 2.7e-7 | 4.5e-7, 512: 1.0e-6 | 1.9e-6
-// so a row of more than RENDER_ROW partials (SEGMENTS) is taken in polynomials of RENDER_SEGMENT, each turned to its place by an
+// so a row of more than RENDER_ROW partials (ROW_SEGMENTS) is taken in polynomials of RENDER_SEGMENT, each turned to its place by an
 // angle of its own, 512 partials 2.0e-7 | 2.4e-7.  The other rows, which need none, are spared the registers and the time: 474 us
 // for the whole render of 256 voices with 100 partials, 499 with segments.
-constexpr int RENDER_ROW = 104, RENDER_SEGMENT = 64;
-template <bool VEC, bool SEGMENTS>
+//
+// Few partials do not pay for six angles.  Where no frame of a warp has more than RENDER_FEW the polynomial is one in e^(2 pi i P),
+// partial by partial, from one angle: 4 of 100 partials audible, 256 voices: 314 -> 292 us, 8: 314 -> 310 (longer walks there are
+// slower than groups).  A row that never has many (ROW_FEW) leaves the groups' code out, 50 -> 32 registers, and takes eights of them
+// as a polynomial in e^(2 pi i 8 P): rows of 1, 4, 8, 12, 16, 20 partials 282, 298, 296, 331, 320, 359 -> 212, 206, 224, 282, 306,
+// 337 us (224, 251, 271, 292, 315, 335 with a fast sine each); 24: 355 -> 363, and rows without 16-byte loads 13: 320 -> 333.
+constexpr int RENDER_FEW = 8, RENDER_FEW_ROW = 20, RENDER_FEW_ROW_ODD = 12, RENDER_ROW = 104, RENDER_SEGMENT = 64;
+enum RenderRow { ROW_FEW, ROW_GROUPS, ROW_SEGMENTS };
+template <bool VEC, RenderRow ROW>
 __global__ void __launch_bounds__(128)
 harmonic_render_group_kernel(dgc_harmonic_params prm, const float2 *__restrict__ rowtab, const float *__restrict__ env,
                              const float *__restrict__ amps, const unsigned long long *__restrict__ fund,
@@ -875,87 +882,139 @@ harmonic_render_group_kernel(dgc_harmonic_params prm, const float2 *__restrict__
   const unsigned long long step = fund[(size_t)b * C + n / CH] + ((unsigned long long)(uint32_t)tk.x << 32);
   const int count = min(tk.y, K);
   const float *rl = amps + ((size_t)lo * B + b) * K, *rh = amps + ((size_t)hi * B + b) * K;
-  {   // as above: the lines of both rows are on their way before the walk comes to them
+  if (ROW != ROW_FEW) {   // as above: the lines of both rows are on their way before the walk comes to them
     const int l = threadIdx.x & 31, k0 = l * 32;
     if (k0 < count) {
       asm volatile("prefetch.global.L1 [%0];" ::"l"(rl + min(k0, K - 1)));
       asm volatile("prefetch.global.L1 [%0];" ::"l"(rh + min(k0, K - 1)));
     }
   }
-  // angles as the rounded high words of the exact products
-  const unsigned long long half = step >> 1, half_r = half + (1ull << 31);
-  float C0, C1, C2, C3, S0, S1, S2, S3, c8, s8, c0, s0;
-  sincos_q32((uint32_t)(half_r >> 32), S0, C0);
-  sincos_q32((uint32_t)((half_r + step) >> 32), S1, C1);
-  sincos_q32((uint32_t)((half_r + (step << 1)) >> 32), S2, C2);
-  sincos_q32((uint32_t)((half_r + (step << 1) + step) >> 32), S3, C3);
-  sincos_q32((uint32_t)((half_r + (step << 2)) >> 32), s0, c0);                 // the first group's centre
-  sincos_turn_q32((uint32_t)(((step << 3) + (1ull << 31)) >> 32), s8, c8);      // from a group to the next
-  const float2 C01 = make_float2(C0, C1), C23 = make_float2(C2, C3), C10 = make_float2(C1, C0), C32 = make_float2(C3, C2);
-  const float2 S01 = make_float2(S0, S1), S23 = make_float2(S2, S3), S10 = make_float2(-S1, -S0), S32 = make_float2(-S3, -S2);
-  const float2 W = make_float2(c8, c8), X = make_float2(s8, s8), Y = make_float2(-s8, -s8);
-  const float2 fr2 = make_float2(fr, fr), neg = make_float2(-1.0f, -1.0f);
-  float2 U = make_float2(0.0f, 0.0f), V = U, sum = U;   // two interleaved polynomials each, added up at the end
-  // partials k + 1, 2 | 3, 4 | 5, 6 | 7, 8 of a group: distances -7/2, -5/2 | -3/2, -1/2 | 1/2, 3/2 | 5/2, 7/2
-  auto group = [&](float2 a01, float2 a23, float2 a45, float2 a67) {
-    sum = __fadd2_rn(sum, __fadd2_rn(__fadd2_rn(a01, a23), __fadd2_rn(a45, a67)));
-    float2 u = __fmul2_rn(U, W), v = __fmul2_rn(U, X);
-    u = __ffma2_rn(V, Y, u);
-    v = __ffma2_rn(V, W, v);
-    u = __ffma2_rn(a45, C01, u);
-    v = __ffma2_rn(a45, S01, v);
-    u = __ffma2_rn(a67, C23, u);
-    v = __ffma2_rn(a67, S23, v);
-    u = __ffma2_rn(a23, C10, u);
-    v = __ffma2_rn(a23, S10, v);
-    U = __ffma2_rn(a01, C32, u);
-    V = __ffma2_rn(a01, S32, v);
+  auto done = [&](float part, float total) {
+    const float inv = 1.0f / (total + 1e-8f);
+    const float ratio = part * inv;
+    if (sums) sums[(size_t)b * T + n] = make_float2(ratio, inv);   // for the backward: it then reduces nothing per frame
+    const float val = ratio * env[(size_t)b * T + n];
+    float *dst = audio + (size_t)b * T + n;
+    *dst = prm.accumulate ? *dst + val : val;
   };
-  auto mix = [&](float lx, float ly, float hx, float hy) {
-    const float2 l = make_float2(lx, ly);
-    return __ffma2_rn(fr2, __ffma2_rn(l, neg, make_float2(hx, hy)), l);
-  };
-  auto four = [&](const float *p) {
-    return VEC ? __ldg(reinterpret_cast<const float4 *>(p)) : make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
-  };
-  int k = count & ~7;
-  const float *pl = rl + k, *ph = rh + k;
-  if (k < count) {   // the last group: what is not audible counts nothing and is not read past the row
-    const int m = count - k;
-    float a[8];
+  const int most = __reduce_max_sync(__activemask(), count);   // of the frames of this warp
+  if (ROW == ROW_FEW || most <= RENDER_FEW) {
+    float c, s, u = 0.0f, v = 0.0f, total = 0.0f;
+    sincos_turn_q32((uint32_t)((step + (1ull << 31)) >> 32), s, c);
+    auto four_down = [&](int k) {   // partials k + 4 .. k + 1, those that are audible
+      auto at = [&](const float *row, int i) { return k + i < K ? __ldg(row + k + i) : 0.0f; };
+      float4 l, h;
+      if (VEC) {
+        l = __ldg(reinterpret_cast<const float4 *>(rl + k));
+        h = __ldg(reinterpret_cast<const float4 *>(rh + k));
+      } else {
+        l = make_float4(at(rl, 0), at(rl, 1), at(rl, 2), at(rl, 3));
+        h = make_float4(at(rh, 0), at(rh, 1), at(rh, 2), at(rh, 3));
+      }
+      const float a[4] = {fmaf(fr, h.x - l.x, l.x), fmaf(fr, h.y - l.y, l.y), fmaf(fr, h.z - l.z, l.z), fmaf(fr, h.w - l.w, l.w)};
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float l = i < m ? __ldg(pl + i) : 0.0f, h = i < m ? __ldg(ph + i) : 0.0f;
-      a[i] = fmaf(fr, h - l, l);
+      for (int i = 3; i >= 0; --i) {
+        const float x = k + i < count ? a[i] : 0.0f;
+        total += x;
+        u += x;
+        const float w = fmaf(-v, s, u * c);
+        v = fmaf(v, c, u * s);
+        u = w;
+      }
+    };
+    auto eight_down = [&](int k) {
+      u = v = 0.0f;
+      if (most > k + 4) four_down(k + 4);
+      if (most > k) four_down(k);
+    };
+    if (ROW == ROW_FEW && most > RENDER_FEW) {   // eights are a polynomial in e^(2 pi i 8 P)
+      float c8, s8, U = 0.0f, V = 0.0f;
+      sincos_turn_q32((uint32_t)(((step << 3) + (1ull << 31)) >> 32), s8, c8);
+      for (int k = (most - 1) & -8; k >= 0; k -= 8) {
+        eight_down(k);
+        const float w = fmaf(-V, s8, fmaf(U, c8, u));
+        V = fmaf(V, c8, fmaf(U, s8, v));
+        U = w;
+      }
+      done(V, total);
+    } else {
+      static_assert(RENDER_FEW == 8, "one eight");
+      eight_down(0);
+      done(v, total);
     }
-    group(make_float2(a[0], a[1]), make_float2(a[2], a[3]), make_float2(a[4], a[5]), make_float2(a[6], a[7]));
+    return;
   }
-  auto down = [&](int end) {
+  if constexpr (ROW != ROW_FEW) {
+    // angles as the rounded high words of the exact products
+    const unsigned long long half = step >> 1, half_r = half + (1ull << 31);
+    float C0, C1, C2, C3, S0, S1, S2, S3, c8, s8, c0, s0;
+    sincos_q32((uint32_t)(half_r >> 32), S0, C0);
+    sincos_q32((uint32_t)((half_r + step) >> 32), S1, C1);
+    sincos_q32((uint32_t)((half_r + (step << 1)) >> 32), S2, C2);
+    sincos_q32((uint32_t)((half_r + (step << 1) + step) >> 32), S3, C3);
+    sincos_q32((uint32_t)((half_r + (step << 2)) >> 32), s0, c0);                 // the first group's centre
+    sincos_turn_q32((uint32_t)(((step << 3) + (1ull << 31)) >> 32), s8, c8);      // from a group to the next
+    const float2 C01 = make_float2(C0, C1), C23 = make_float2(C2, C3), C10 = make_float2(C1, C0), C32 = make_float2(C3, C2);
+    const float2 S01 = make_float2(S0, S1), S23 = make_float2(S2, S3), S10 = make_float2(-S1, -S0), S32 = make_float2(-S3, -S2);
+    const float2 W = make_float2(c8, c8), X = make_float2(s8, s8), Y = make_float2(-s8, -s8);
+    const float2 fr2 = make_float2(fr, fr), neg = make_float2(-1.0f, -1.0f);
+    float2 U = make_float2(0.0f, 0.0f), V = U, sum = U;   // two interleaved polynomials each, added up at the end
+    // partials k + 1, 2 | 3, 4 | 5, 6 | 7, 8 of a group: distances -7/2, -5/2 | -3/2, -1/2 | 1/2, 3/2 | 5/2, 7/2
+    auto group = [&](float2 a01, float2 a23, float2 a45, float2 a67) {
+      sum = __fadd2_rn(sum, __fadd2_rn(__fadd2_rn(a01, a23), __fadd2_rn(a45, a67)));
+      float2 u = __fmul2_rn(U, W), v = __fmul2_rn(U, X);
+      u = __ffma2_rn(V, Y, u);
+      v = __ffma2_rn(V, W, v);
+      u = __ffma2_rn(a45, C01, u);
+      v = __ffma2_rn(a45, S01, v);
+      u = __ffma2_rn(a67, C23, u);
+      v = __ffma2_rn(a67, S23, v);
+      u = __ffma2_rn(a23, C10, u);
+      v = __ffma2_rn(a23, S10, v);
+      U = __ffma2_rn(a01, C32, u);
+      V = __ffma2_rn(a01, S32, v);
+    };
+    auto mix = [&](float lx, float ly, float hx, float hy) {
+      const float2 l = make_float2(lx, ly);
+      return __ffma2_rn(fr2, __ffma2_rn(l, neg, make_float2(hx, hy)), l);
+    };
+    auto four = [&](const float *p) {
+      return VEC ? __ldg(reinterpret_cast<const float4 *>(p)) : make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+    };
+    int k = count & ~7;
+    const float *pl = rl + k, *ph = rh + k;
+    if (k < count) {   // the last group: what is not audible counts nothing and is not read past the row
+      const int m = count - k;
+      float a[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float l = i < m ? __ldg(pl + i) : 0.0f, h = i < m ? __ldg(ph + i) : 0.0f;
+        a[i] = fmaf(fr, h - l, l);
+      }
+      group(make_float2(a[0], a[1]), make_float2(a[2], a[3]), make_float2(a[4], a[5]), make_float2(a[6], a[7]));
+    }
+    auto down = [&](int end) {
 #pragma unroll 2
-    for (; k > end; k -= 8) {
-      pl -= 8;
-      ph -= 8;
-      const float4 l0 = four(pl), l1 = four(pl + 4), h0 = four(ph), h1 = four(ph + 4);
-      group(mix(l0.x, l0.y, h0.x, h0.y), mix(l0.z, l0.w, h0.z, h0.w), mix(l1.x, l1.y, h1.x, h1.y), mix(l1.z, l1.w, h1.z, h1.w));
+      for (; k > end; k -= 8) {
+        pl -= 8;
+        ph -= 8;
+        const float4 l0 = four(pl), l1 = four(pl + 4), h0 = four(ph), h1 = four(ph + 4);
+        group(mix(l0.x, l0.y, h0.x, h0.y), mix(l0.z, l0.w, h0.z, h0.w), mix(l1.x, l1.y, h1.x, h1.y), mix(l1.z, l1.w, h1.z, h1.w));
+      }
+    };
+    float im = 0.0f;
+    if constexpr (ROW == ROW_SEGMENTS) {
+      for (int k0 = (max(count, 1) - 1) & -RENDER_SEGMENT; k0 > 0; k0 -= RENDER_SEGMENT) {
+        down(k0);
+        float sk, ck;   // the first centre of the segment
+        sincos_q32((uint32_t)((half_r + step * (uint32_t)(k0 + 4)) >> 32), sk, ck);
+        im = fmaf(sk, U.x + U.y, fmaf(ck, V.x + V.y, im));
+        U = V = make_float2(0.0f, 0.0f);
+      }
     }
-  };
-  float im = 0.0f;
-  if (SEGMENTS) {
-    for (int k0 = (max(count, 1) - 1) & -RENDER_SEGMENT; k0 > 0; k0 -= RENDER_SEGMENT) {
-      down(k0);
-      float sk, ck;   // the first centre of the segment
-      sincos_q32((uint32_t)((half_r + step * (uint32_t)(k0 + 4)) >> 32), sk, ck);
-      im = fmaf(sk, U.x + U.y, fmaf(ck, V.x + V.y, im));
-      U = V = make_float2(0.0f, 0.0f);
-    }
+    down(0);
+    done(fmaf(s0, U.x + U.y, fmaf(c0, V.x + V.y, im)), sum.x + sum.y);
   }
-  down(0);
-  const float inv = 1.0f / (sum.x + sum.y + 1e-8f);
-  const float ratio = fmaf(s0, U.x + U.y, fmaf(c0, V.x + V.y, im)) * inv;
-  if (sums) sums[(size_t)b * T + n] = make_float2(ratio, inv);   // for the backward: it then reduces nothing per frame
-  const float val = ratio * env[(size_t)b * T + n];
-  float *dst = audio + (size_t)b * T + n;
-  *dst = prm.accumulate ? *dst + val : val;
 }
 
 template <int LPC, int P>
@@ -1006,10 +1065,12 @@ void launch_render_q(dgc_ctx *ctx, const dgc_harmonic_params &p, const float2 *r
     const dim3 fgrid(dgc_div_up(p.T, 128), p.B);
     const bool vec = (p.K & 3) == 0 && (((uintptr_t)amps) & 15) == 0;
     float2 *keep = keep_sums ? x.sums : nullptr;
-    const bool segments = p.K > RENDER_ROW;
     auto kern = by_partial ? (vec ? harmonic_render_frame_kernel<true> : harmonic_render_frame_kernel<false>)
-              : segments   ? (vec ? harmonic_render_group_kernel<true, true> : harmonic_render_group_kernel<false, true>)
-                           : (vec ? harmonic_render_group_kernel<true, false> : harmonic_render_group_kernel<false, false>);
+              : p.K <= (vec ? RENDER_FEW_ROW : RENDER_FEW_ROW_ODD)
+                  ? (vec ? harmonic_render_group_kernel<true, ROW_FEW> : harmonic_render_group_kernel<false, ROW_FEW>)
+              : p.K <= RENDER_ROW
+                  ? (vec ? harmonic_render_group_kernel<true, ROW_GROUPS> : harmonic_render_group_kernel<false, ROW_GROUPS>)
+                  : (vec ? harmonic_render_group_kernel<true, ROW_SEGMENTS> : harmonic_render_group_kernel<false, ROW_SEGMENTS>);
     dgc_launch(kern, fgrid, 128, 0, ctx->stream, p, rowtab, x.env, amps, x.fund, x.trk, keep, out);
   } else
     dgc_launch(harmonic_render_q_kernel<LPC, P, MODE>, grid, 128, 0, ctx->stream, p, 1.0f / p.sample_rate, rowtab, x.f0t, x.env,

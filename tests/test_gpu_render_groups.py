@@ -1,5 +1,7 @@
 """The harmonic render in groups of eight partials, where its grouping can go wrong: fewer partials than a group, one more or
 one less than whole groups, rows that no 16-byte load fits, counts that change inside a warp, phases at zero and half turns."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -123,3 +125,66 @@ def test_error_does_not_grow_with_the_partials(ctx, K, spectrum):
     err = [_norm_error(got[b].cpu().double().numpy(), want[b]) for b in range(4)]
     print("K %d %s: %s" % (K, spectrum, " ".join("%.2e" % e for e in err)))
     assert max(err) < PER_PARTIAL
+
+
+@pytest.mark.parametrize("K", [1, 2, 3, 4, 5, 7, 8, 9, 11, 12, 13, 16, 17, 20, 21, 24, 28, 100, 128])
+def test_few_audible_partials(ctx, K):
+    """Rows of few partials and rows of many of which few are heard: at the edges of fours, eights, of the count that a warp takes
+    partial by partial and of the row lengths that always are."""
+    counts = [c for c in (1, 2, 3, 4, 5, 7, 8, 9, 12, 13, 16, 17, 20, 24) if c < K] + [K, K]
+    f0, amps, want, sr = _exact_phases(K, counts, "flat", len(counts), 4097, 100 + K)
+    for b, c in enumerate(counts):
+        amps[0, b, c:] = float("nan")           # what is not audible is not to come in
+    one = torch.ones(1, len(counts), device="cuda")
+    got = ctx.harmonic_render(f0.cuda(), one, amps.cuda(), one, 4097, sr, phase_mode=dgen_b200.PHASE_FUNDAMENTAL).cpu().double()
+    for b, c in enumerate(counts):
+        assert _norm_error(got[b].numpy(), want[b]) < PER_PARTIAL, c
+
+
+def test_counts_that_change_inside_a_warp(ctx):
+    """f0 sweeps the audible count of 100 partials from 100 to 1 and back within a few hundred frames: warps on both sides of the
+    rule and across it."""
+    g = torch.Generator().manual_seed(3)
+    f0 = torch.tensor([79.0, 8000.0 / 6, 7000.0, 900.0, 1000.0, 8000.0 / 9])[:, None].repeat(1, 2)
+    amps = torch.rand(6, 2, 100, generator=g)
+    got = _render(ctx, f0, amps, 640).cpu().double()
+    assert (got - _double(f0, amps, 640)).abs().max() < 1e-6 + 2 * np.pi * 100 * 640 * 2.0 ** -33
+
+
+@pytest.mark.parametrize("K", [1, 4, 12])
+def test_few_partials_are_no_slower_than_a_sine_each(ctx, K):
+    """The render of a plan step that keeps its scratch takes a fast sine per partial; fewer partials than a group must not take longer
+    than that (it also stores the track and its sums, a few per cent)."""
+    B, T, F = 256, 64000, 1000
+    f0, one = torch.full((F, B), 100.0, device="cuda"), torch.ones(F, B, device="cuda")
+    hp = dgen_b200.HarmonicParams(B, T, K, F, SR, 1.0, dgen_b200.PHASE_FUNDAMENTAL, 0)
+    n = [F * B, F * B, F * B * K, F * B, int(ctx.lib.dgc_harmonic_scratch_floats(C.byref(hp))), B * T]
+    off = np.concatenate([[0], np.cumsum([(v + 63) // 64 * 64 for v in n])])
+    arena = torch.zeros(int(off[-1]), device="cuda")
+    arena[:n[0]] = 100.0
+    for i in (1, 3):
+        arena[off[i]:off[i] + n[i]] = 1.0
+    amps = arena[off[2]:off[2] + n[2]].uniform_()
+    steps = (dgen_b200.PlanStep * 1)(dgen_b200.plan_step(dgen_b200.PLAN_HARMONIC_RENDER, a=[int(o) for o in off[:6]],
+                                                         i=(B, T, K, F, dgen_b200.PHASE_FUNDAMENTAL, 0), f=(SR, 1.0)))
+    plan = dgen_b200.Plan(steps, 1, None, None, 0)
+    h = C.c_void_p()
+    ctx.check(ctx.lib.dgc_arena_wrap(ctx.h, arena.data_ptr(), arena.numel(), C.byref(h)))
+    out = torch.empty(B, T, device="cuda")
+    calls = (lambda: ctx.harmonic_render(f0, one, amps.view(F, B, K), one, T, SR, phase_mode=dgen_b200.PHASE_FUNDAMENTAL, out=out),
+             lambda: ctx.check(ctx.lib.dgc_plan_run(ctx.h, h, C.byref(plan), 0, -1)))
+    times = ([], [])
+    for rep in range(13):
+        for call, ts in zip(calls, times):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            call()
+            b.record()
+            torch.cuda.synchronize()
+            if rep >= 3:
+                ts.append(a.elapsed_time(b))
+    ctx.lib.dgc_arena_destroy(h)
+    groups, sines = (sorted(ts)[len(ts) // 2] for ts in times)
+    print("K %d: %.1f us, a sine each %.1f us" % (K, 1e3 * groups, 1e3 * sines))
+    assert torch.allclose(out, arena[off[5]:off[5] + n[5]].view(B, T), atol=2e-6)
+    assert groups < 1.02 * sines
