@@ -688,7 +688,9 @@ int32_t dgc_linear_bwd_beside(dgc_ctx *ctx, const float *a_dev, const float *w_d
     // and with aligned rows: 2000 rows 100 -> 94 us, 8000 rows 85 -> 72, 32000 rows 176 -> 134, 64000 rows 300 -> 224; K = 128:
     // 68.7 -> 60 (8000 rows), 102 -> 93 (32000).  A pass of its own over dZ for the copies: 146 us at 32000 rows, and slower than
     // 4-byte copies at 16000 rows and K = 128 (71 -> 77).
-    const bool align = da_dev && (N & 3) && N >= 32 && !few_tiles(ctx, M, K) && !smallk_shape(ctx, dz_dev, M, K, N);
+    // The blocks that copy W stand behind dZ's in the grid's second dimension, which ends at 65535.
+    const bool align = da_dev && (N & 3) && N >= 32 && !few_tiles(ctx, M, K) && !smallk_shape(ctx, dz_dev, M, K, N) &&
+                       (int64_t)dgc_div_up(M, TT) + dgc_div_up(K, TT) <= 65535;
     const int ld = (N + 3) & ~3;
     const size_t need = n + (align ? (size_t)(M + (int64_t)K) * ld : 0);   // M, so n, is a multiple of 4
     if (!ctx->dzt_buf || ctx->dzt_floats < need) {

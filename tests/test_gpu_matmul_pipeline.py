@@ -83,3 +83,24 @@ def test_rows_past_the_end_are_not_read(ctx):
     c2 = ctx.linear_fwd(a, w)
     rows = torch.isfinite(c2).all(1)
     assert not bool(rows[7]) and int(rows.sum()) == M - 1 and torch.equal(c2[rows], c[rows])
+
+
+@pytest.mark.parametrize("M", [65535 * 64 - 64, 65535 * 64])
+def test_input_gradient_of_unaligned_rows_at_the_edge_of_the_grid(ctx, M):
+    """The blocks that copy dZ and those that copy W together are one more than a grid's second dimension holds (the second case)."""
+    K, N = 64, 33
+    if torch.cuda.mem_get_info()[0] < 12 << 30:
+        pytest.skip("12 GB of device memory")
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    a = torch.randn(M, K, device="cuda", generator=g)
+    w = torch.randn(K, N, device="cuda", generator=g) * K ** -0.5
+    dc = torch.randn(M, N, device="cuda", generator=g)
+    da, dw, db = ctx.linear_bwd(a, w, None, dc, act=0, a_t=a.t().contiguous())
+    for lo in (0, M // 2, M - 1000):
+        assert _rel(da[lo:lo + 1000], dc[lo:lo + 1000].double() @ w.double().t()) < _tol(N)
+    # one output tile, so as many slices of the rows as two blocks an SM: M / 296 rows each (more, on fewer SMs)
+    slices = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert _rel(dw, a.double().t() @ dc.double()) < 2.0 ** -20 + 3 * (M / slices) / 8 * 2.0 ** -24
+    # sums of 1024 rows by eight threads, then 4096 of those one after the other
+    assert _rel(db, dc.double().sum(0)) < (128 + 4096) * 2.0 ** -24
+    ctx.sync()
