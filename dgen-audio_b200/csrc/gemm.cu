@@ -689,10 +689,12 @@ int32_t dgc_linear_bwd_beside(dgc_ctx *ctx, const float *a_dev, const float *w_d
     // 68.7 -> 60 (8000 rows), 102 -> 93 (32000).  A pass of its own over dZ for the copies: 146 us at 32000 rows, and slower than
     // 4-byte copies at 16000 rows and K = 128 (71 -> 77).
     // The blocks that copy W stand behind dZ's in the grid's second dimension, which ends at 65535.
-    const bool align = da_dev && (N & 3) && N >= 32 && !few_tiles(ctx, M, K) && !smallk_shape(ctx, dz_dev, M, K, N) &&
+    bool align = da_dev && (N & 3) && N >= 32 && !few_tiles(ctx, M, K) && !smallk_shape(ctx, dz_dev, M, K, N) &&
                        (int64_t)dgc_div_up(M, TT) + dgc_div_up(K, TT) <= 65535;
     const int ld = (N + 3) & ~3;
-    const size_t need = n + (align ? (size_t)(M + (int64_t)K) * ld : 0);   // M, so n, is a multiple of 4
+    size_t need = n + (size_t)(M + (int64_t)K) * ld;   // M, so n, is a multiple of 4
+    align = align && need < ctx->dzt_refused;
+    if (!align) need = n;
     if (!ctx->dzt_buf || ctx->dzt_floats < need) {
       if (ctx->dzt_buf) {
         cudaStreamSynchronize(ctx->stream);
@@ -700,7 +702,14 @@ int32_t dgc_linear_bwd_beside(dgc_ctx *ctx, const float *a_dev, const float *w_d
         ctx->buffer_generation++;
         ctx->dzt_buf = nullptr;
       }
-      DGC_CUDA(ctx, cudaMalloc(&ctx->dzt_buf, need * sizeof(float)));
+      ctx->dzt_floats = 0;
+      if (align && cudaMalloc(&ctx->dzt_buf, need * sizeof(float)) != cudaSuccess) {   // no room for the copies: do without
+        cudaGetLastError();
+        ctx->dzt_refused = need;
+        align = false;
+        need = n;
+      }
+      if (!ctx->dzt_buf) DGC_CUDA(ctx, cudaMalloc(&ctx->dzt_buf, need * sizeof(float)));
       ctx->dzt_floats = need;
     }
     float *dz_ld = align ? ctx->dzt_buf + n : nullptr, *w_ld = align ? dz_ld + (size_t)M * ld : nullptr;

@@ -104,3 +104,43 @@ def test_input_gradient_of_unaligned_rows_at_the_edge_of_the_grid(ctx, M):
     # sums of 1024 rows by eight threads, then 4096 of those one after the other
     assert _rel(db, dc.double().sum(0)) < (128 + 4096) * 2.0 ** -24
     ctx.sync()
+
+
+def test_input_gradient_of_unaligned_rows_without_room_for_the_copies():
+    """Device memory that holds dZ transposed but not the aligned copies beside it: the layer goes on without them."""
+    M, K, N = 400000, 64, 165
+    ctx = dgen_b200.Context(0)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a = torch.randn(M, K, device="cuda", generator=g)
+    w = torch.randn(K, N, device="cuda", generator=g) * K ** -0.5
+    dc = torch.randn(M, N, device="cuda", generator=g)
+    at = a.t().contiguous()
+    dz, da, dw, db = dc.clone(), torch.empty_like(a), torch.empty_like(w), torch.empty(N, device="cuda")
+    call = lambda da_ptr: ctx.check(ctx.lib.dgc_linear_bwd(ctx.h, a.data_ptr(), w.data_ptr(), None, dc.data_ptr(), M, K, N, 0, dz.data_ptr(),
+                                                           da_ptr, dw.data_ptr(), db.data_ptr(), at.data_ptr()))
+    call(None)                      # dZ transposed, and the scratch of everything else
+    ctx.sync()
+    torch.cuda.empty_cache()
+    spare, blocks = M * N * 2, []   # half of dZ; with dZ itself given back, one and a half: the call with copies wants two
+    while True:
+        free = torch.cuda.mem_get_info()[0] - spare
+        if free < 4 << 20:
+            break
+        blocks.append(torch.empty(min(free // (2 << 20) * (2 << 20), 8 << 30), dtype=torch.uint8, device="cuda"))
+    try:
+        call(da.data_ptr())
+        ctx.sync()
+        left = torch.cuda.mem_get_info()[0]
+        call(da.data_ptr())         # and does not ask again
+        assert torch.cuda.mem_get_info()[0] == left
+        ctx.sync()
+    finally:
+        del blocks
+        torch.cuda.empty_cache()
+    for lo in (0, M // 2, M - 1000):
+        assert _rel(da[lo:lo + 1000], dc[lo:lo + 1000].double() @ w.double().t()) < _tol(N)
+    ctx.close()
+    ctx = dgen_b200.Context(0)
+    da2, _, _ = ctx.linear_bwd(a, w, None, dc, act=0, a_t=at)
+    assert torch.equal(da2, da)     # with them the same bits
+    ctx.close()
