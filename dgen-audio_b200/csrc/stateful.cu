@@ -609,16 +609,13 @@ __device__ __forceinline__ float principal_arg(float v) {
 
 // The same for the running phase of the synthesis, where a step's latency counts and a multiple of tau more or less is the
 // same phase: turns counted by a multiplication and rounded to the nearest even by an addition (below 2^22 turns; a single-
-// precision phase beyond has no fraction left).
+// precision phase beyond has no fraction left).  A count that its rounding makes one too many or too few leaves the phase just
+// outside half a turn; it is folded at every step, so that a stream cut in two calls goes on with what one call has.
 __device__ __forceinline__ float wrapped(float v) {
-  const float tau = 6.28318530717958647692f, big = 12582912.0f;
-  return fmaf(-tau, fmaf(v, 0.15915494309189533577f, big) - big, v);
-}
-// as it is handed on: within half a turn
-__device__ __forceinline__ float settled(float w) {
-  const float tau = 6.28318530717958647692f, half = 3.14159265358979323846f;
-  const float wh = w > half ? w - tau : w;
-  return w < -half ? wh + tau : wh;
+  const float tau = 6.28318530717958647692f, half = 3.14159265358979323846f, big = 12582912.0f;
+  const float w = fmaf(-tau, fmaf(v, 0.15915494309189533577f, big) - big, v);
+  const float folded = w - copysignf(tau, w);
+  return fabsf(w) > half ? folded : w;
 }
 
 // Sine and cosine of a wrapped phase, each to 1.2e-7: folded about a quarter turn, then both polynomials in x^2 (minimax on that
@@ -736,7 +733,7 @@ pv_synthesis_kernel(const float *__restrict__ re, const float *__restrict__ im, 
       const size_t last = base + (size_t)(H - 1) * N + k;
       // the "started" flag is shared by all bins of a voice and other blocks may still have to read it: a launch of
       // its own sets it afterwards
-      st[N + k] = settled(synth);
+      st[N + k] = synth;
       st[k] = atan2f(im[last], re[last]);
     }
     return;

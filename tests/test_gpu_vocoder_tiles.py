@@ -43,3 +43,22 @@ def test_tiles_of_hops_and_bins(ctx, H, N, hop):
             cut = torch.cat([p[i] for p in parts], 1)[v].cpu().numpy()
             assert np.abs(cut - want).max() < tol
     assert bool((state[:, N:2 * N].abs() <= np.pi + 1e-6).all())
+
+
+@pytest.mark.parametrize("N,hop", [(2048, 2048), (1024, 512)])
+def test_a_stream_in_parts_is_the_same_bits_as_in_one(ctx, N, hop):
+    """High bins advance by hundreds of turns a hop, and counting them is now and then one off: the phase that a call hands on has
+    to be the one that the next hop would have gone on from."""
+    rng = np.random.default_rng(N)
+    V, H, cuts = 8, 13, (0, 1, 3, 4, 6, 9, 12, 13)
+    re, im = (torch.from_numpy(rng.standard_normal((V, H, N)).astype(f32)).cuda() for _ in range(2))
+    ratio = torch.from_numpy(rng.uniform(0.7, 1.4, (V, H)).astype(f32)).cuda()
+    whole = torch.zeros(V, 2 * N + 1, device="cuda")
+    want = ctx.phase_vocoder(re, im, ratio, hop, state=whole)
+    state = torch.zeros(V, 2 * N + 1, device="cuda")
+    parts = [ctx.phase_vocoder(re[:, a:b].contiguous(), im[:, a:b].contiguous(), ratio[:, a:b].contiguous(), hop, state=state)
+             for a, b in zip(cuts, cuts[1:])]
+    for i in range(2):
+        assert torch.equal(torch.cat([p[i] for p in parts], 1), want[i])
+    assert torch.equal(state, whole)
+    assert bool((state[:, N:2 * N].abs() <= float(f32(np.pi))).all())
