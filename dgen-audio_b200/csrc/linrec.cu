@@ -837,7 +837,7 @@ biquad_bwd_kernel(const float *__restrict__ x, const float *__restrict__ coef, c
                   const float *__restrict__ tgt, int T, int L, int NC, float gscale,
                   float *__restrict__ rec /* [B][NC][BW_REC][L] */) {
   dgc_after_previous();
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];   // staged frames are read four at a time
   constexpr int G = 16;
   const int b = blockIdx.y;
   int c, l;
