@@ -123,8 +123,9 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
       forked = false;
     }
   };
-  // Weight gradients left on the side stream by the layers' backward steps (dgc_linear_bwd_beside): the steps right after them
-  // that are such too go on, as long as they keep off the buffers that are read and written there; anything else joins first.
+  // Steps of the main stream that nothing right after them waits for are left on the side stream: layers' weight gradients
+  // (dgc_linear_bwd_beside) and the loss's value ahead of its gradient.  Backward steps go on beside them as long as they keep off
+  // the buffers that are read and written there; anything else joins first.
   struct Range {
     uint64_t off, n;
   };
@@ -142,10 +143,13 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
         if (p.off != DGC_PLAN_NONE && q.off != DGC_PLAN_NONE && p.off < q.off + q.n && q.off < p.off + p.n) return true;
     return false;
   };
+  auto keep_off_side = [&](const std::vector<Range> &reads, const std::vector<Range> &writes) {
+    if (meets(writes, side_reads) || meets(writes, side_writes) || meets(reads, side_writes)) join_side();
+  };
   for (int k = first; k < last && rc == DGC_OK; ++k) {
     const dgc_plan_step &s = plan->steps[k];
     R.step = k;
-    if (s.op != DGC_PLAN_LINEAR_BWD) join_side();
+    if (s.op != DGC_PLAN_LINEAR_BWD && s.op != DGC_PLAN_MSS_LOSS_BWD && s.op != DGC_PLAN_PARTCONV_BWD) join_side();
     if (s.stream == 1 && !forked && s.op != DGC_PLAN_FORK) {
       rc = dgc_fail(ctx, DGC_ERR_INVALID, "dgc_plan_run: step %d runs on the side stream before a FORK", k);
       break;
@@ -261,6 +265,9 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
         const float *x = R.at(a[0], (uint64_t)V * T), *ir = R.at(a[1], irl), *go = R.at(a[2], (uint64_t)V * T);
         float *scr = R.at(a[3], dgc_partconv_bwd_scratch_floats(V, T, irl, N, hop), true);
         float *gx = R.at(a[4], (uint64_t)V * T, true), *gir = R.at(a[5], irl, true);
+        const uint64_t vt = (uint64_t)V * T;
+        keep_off_side({{a[0], vt}, {a[1], (uint64_t)irl}, {a[2], vt}, {a[4], vt}},
+                      {{a[3], dgc_partconv_bwd_scratch_floats(V, T, irl, N, hop)}, {a[4], vt}, {a[5], (uint64_t)irl}});
         if (!R.bad) rc = dgc_partconv_bwd(ctx, x, V, T, ir, irl, N, hop, f[0], go, scr, i[5], gx, gir);
       } break;
       case DGC_PLAN_MSS_LOSS_FWD: {
@@ -269,13 +276,29 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
         const float *pred = R.at(a[0], bt), *tg = R.at(a[1], bt);
         float *part = R.at(a[2], dgc_mss_partial_floats(&m), true), *loss = R.at(a[3], 2);
         if (!R.bad && (a[3] & 1)) R.fail("a double must sit at an even offset");
-        if (!R.bad) rc = dgc_mss_loss_fwd(ctx, &m, pred, tg, part, reinterpret_cast<double *>(loss));
+        if (R.bad) break;
+        // nothing waits for the value, so where the loss's gradient comes next the two run beside each other (3 x 16001 frames: a
+        // training step 15 us shorter)
+        const bool beside = s.stream == 0 && !forked && k + 1 < last && plan->steps[k + 1].op == DGC_PLAN_MSS_LOSS_BWD &&
+                            plan->steps[k + 1].stream == 0;
+        if (beside) {
+          if (cudaEventRecord(ctx->fork_ev, main_stream) != cudaSuccess ||
+              cudaStreamWaitEvent(ctx->aux_stream, ctx->fork_ev, 0) != cudaSuccess) {
+            rc = dgc_fail(ctx, DGC_ERR_CUDA, "the side stream does not follow");
+            break;
+          }
+          ctx->stream = ctx->aux_stream;
+          side_reads.insert(side_reads.end(), {{a[0], bt}, {a[1], bt}});
+          side_writes.insert(side_writes.end(), {{a[2], dgc_mss_partial_floats(&m)}, {a[3], 2}});
+        }
+        rc = dgc_mss_loss_fwd(ctx, &m, pred, tg, part, reinterpret_cast<double *>(loss));
       } break;
       case DGC_PLAN_MSS_LOSS_BWD: {
         const dgc_mss_params m = mss_of(s);
         const uint64_t bt = (uint64_t)m.B * m.T;
         const float *pred = R.at(a[0], bt), *tg = R.at(a[1], bt);
         float *g = R.at(a[2], bt);
+        keep_off_side({{a[0], bt}, {a[1], bt}}, {{a[2], bt}});
         if (!R.bad) rc = dgc_mss_loss_bwd(ctx, &m, pred, tg, f[2], g);
       } break;
       case DGC_PLAN_LINEAR_FWD: {
@@ -292,7 +315,7 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
         if (!R.bad) {
           const std::vector<Range> reads = {{a[0], M * K}, {a[1], K * N}, {a[2], M * N}, {a[3], M * N}, {a[8], M * K}};
           const std::vector<Range> writes = {{a[4], M * N}, {a[5], M * K}, {a[6], K * N}, {a[7], N}};
-          if (meets(writes, side_reads) || meets(writes, side_writes) || meets(reads, side_writes)) join_side();
+          keep_off_side(reads, writes);
           // what the step itself hands on (dZ is read beside, the gradients are written there) must not be one buffer
           const bool own = meets({writes[1]}, {{a[0], M * K}, writes[0], writes[2], writes[3]}) ||
                            meets({writes[2], writes[3]}, reads);
@@ -529,8 +552,7 @@ DGC_EXPORT int32_t dgc_hn_train_plan(const dgc_hn_train_config *c, dgc_hn_train_
     s.i[0] = B; s.i[1] = T; s.i[2] = c->ir_len; s.i[3] = c->conv_n; s.i[4] = c->conv_hop; s.i[5] = 1;
     s.f[0] = 1.0f;
     S.push_back(s);
-    S.push_back(mk(DGC_PLAN_FORK));
-    s = mk(DGC_PLAN_MSS_LOSS_FWD, 1);   // nothing waits for the loss's value: beside the spectral and reverb gradients
+    s = mk(DGC_PLAN_MSS_LOSS_FWD);
     s.a[0] = lay->audio; s.a[1] = lay->target; s.a[3] = lay->loss;
     put_mss(s, c->mss, B, T);
     S.push_back(s);
@@ -548,7 +570,6 @@ DGC_EXPORT int32_t dgc_hn_train_plan(const dgc_hn_train_config *c, dgc_hn_train_
     s.f[0] = 1.0f;
     S.push_back(s);
   }
-  S.push_back(mk(DGC_PLAN_JOIN));
   S.push_back(mk(DGC_PLAN_FORK));
   {
     dgc_plan_step s = mk(DGC_PLAN_FIR_BWD, 1);

@@ -1,13 +1,15 @@
 """Steps of a plan that the library runs beside each other or in one launch: weight gradients of a layer beside the backward of
 the next, a sum and its copy.  What they read and write decides, so the buffers here meet in every way they can."""
 import ctypes as C
+import re
 
 import numpy as np
 import pytest
 import torch
 
 import dgen_b200
-from dgen_b200 import PLAN_ADD, PLAN_COPY, PLAN_LINEAR_BWD, Plan, PlanStep, plan_step
+from dgen_b200 import (PLAN_ADD, PLAN_COPY, PLAN_LINEAR_BWD, PLAN_MSS_LOSS_BWD, PLAN_MSS_LOSS_FWD, PLAN_PARTCONV_BWD, Plan, PlanStep,
+                       plan_step, trainer)
 
 pytestmark = pytest.mark.gpu
 
@@ -27,6 +29,26 @@ def _run(ctx, arena, steps):
     ctx.check(ctx.lib.dgc_plan_run(ctx.h, h, C.byref(plan), 0, -1))
     ctx.sync()
     ctx.lib.dgc_arena_destroy(h)
+
+
+def _recorded(ctx, arena, steps, path):
+    """The number of nodes of the plan's recording, and whether any work lies beside other work: two first nodes, or two that
+    follow one."""
+    arr = (PlanStep * len(steps))(*steps)
+    plan = Plan(arr, len(steps), None, None, 0)
+    h = C.c_void_p()
+    ctx.check(ctx.lib.dgc_arena_wrap(ctx.h, arena.data_ptr(), arena.numel(), C.byref(h)))
+    s, g = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
+    g.enable_debug_mode()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=s), ctx.on_stream(s):
+        ctx.check(ctx.lib.dgc_plan_run(ctx.h, h, C.byref(plan), 0, -1))
+    g.debug_dump(str(path))
+    ctx.lib.dgc_arena_destroy(h)
+    edges = re.findall(r'"(\w+)"\s*->\s*"(\w+)"', path.read_text())
+    nodes = set(re.findall(r'"(graph_\w+_node_\d+)"', path.read_text()))
+    before = [a for a, _ in edges]
+    return len(nodes), len(nodes - {b for _, b in edges}) > 1 or any(before.count(a) > 1 for a in set(before))
 
 
 # shared: which buffers the layers have in common ("" none; dz: one dZ for all; act: the second layer's dA lands on the first
@@ -89,3 +111,60 @@ def test_sum_and_its_copy(ctx, n):
             continue       # a copy onto itself is left to the device's copy, whose overlap is not defined
         _run(ctx, got, steps)
         assert torch.equal(got, want), (src, dst)
+
+
+# meet: where the loss's buffers meet those of the steps after it ("" nowhere; partial: its sums lie in the gradient; pred: the
+# convolution's gradient lands on the signal; cell: the loss's value lies in the impulse response's gradient)
+@pytest.mark.parametrize("meet", ["", "partial", "pred", "cell"])
+def test_loss_beside_its_gradient(ctx, meet, tmp_path):
+    B, T, N, ir = 6, 30000, 256, 1000
+    sizes = (512, 128, 64)
+    mp = dgen_b200.mss_params(B, T, sizes)
+    n_part, bt = int(ctx.lib.dgc_mss_partial_floats(C.byref(mp))), B * T
+    off = {}
+    used = 0
+    for name, n in (("pred", bt), ("target", bt), ("grad", max(bt, n_part)), ("part", n_part), ("loss", 64), ("x", bt), ("ir", ir),
+                    ("g_ir", ir), ("gx", bt)):
+        off[name] = used
+        used += (n + 63) // 64 * 64
+    if meet == "partial":
+        off["part"] = off["grad"]
+    if meet == "pred":
+        off["gx"] = off["pred"]
+    if meet == "cell":
+        off["loss"] = off["g_ir"] + 2
+    arena = torch.randn(used, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)) * 0.3
+    want = arena.clone()
+    p = lambda name: want.data_ptr() + 4 * off[name]
+    ctx.check(ctx.lib.dgc_mss_loss_fwd(ctx.h, C.byref(mp), p("pred"), p("target"), p("part"), p("loss")))
+    ctx.check(ctx.lib.dgc_mss_loss_bwd(ctx.h, C.byref(mp), p("pred"), p("target"), 1.0, p("grad")))
+    ctx.check(ctx.lib.dgc_partconv_bwd(ctx.h, p("x"), B, T, p("ir"), ir, N, N // 2, 1.0, p("grad"), None, 0, p("gx"), p("g_ir")))
+    ctx.sync()
+    shape = (B, T, len(sizes), mp.hop_div) + sizes
+    steps = [plan_step(PLAN_MSS_LOSS_FWD, a=(off["pred"], off["target"], off["part"], off["loss"]), i=shape, f=(mp.w_lin, mp.w_log)),
+             plan_step(PLAN_MSS_LOSS_BWD, a=(off["pred"], off["target"], off["grad"]), i=shape, f=(mp.w_lin, mp.w_log, 1.0)),
+             plan_step(PLAN_PARTCONV_BWD, a=(off["x"], off["ir"], off["grad"], None, off["gx"], off["g_ir"]),
+                       i=(B, T, ir, N, N // 2, 0), f=(1.0,))]
+    for _ in range(3):
+        got = arena.clone()
+        _run(ctx, got, steps)
+        assert torch.equal(got, want)
+    assert _recorded(ctx, arena.clone(), steps, tmp_path / "loss.dot")[1] == (meet != "partial")
+    assert not _recorded(ctx, arena.clone(), steps[:1], tmp_path / "loss.dot")[1]
+
+
+def test_the_loss_step_of_a_training_plan_runs_by_itself(ctx):
+    """A host that changes the audio, or times the steps one by one, runs the loss's step alone."""
+    m = trainer.HarmonicModel(ctx, 2, 4000, K=12, F=50, nbands=9, taps=33, hidden=32, ir_len=300, conv_n=256, conv_hop=128, sizes=(512, 128))
+    g = torch.Generator(device="cuda").manual_seed(2)
+    for v in m.input_views():
+        v.copy_(torch.rand(v.shape, device="cuda", generator=g))
+    m.forward(*m.input_views())
+    ctx.sync()
+    want = m.loss.clone()
+    assert float(want[0]) > 0.0
+    m.loss.zero_()
+    m._run(m.i_backward - 1, 1)
+    ctx.sync()
+    assert torch.equal(m.loss, want)
+    m.close()
