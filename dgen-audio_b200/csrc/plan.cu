@@ -204,6 +204,7 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
         float *copy = nullptr;
         if (!R.bad && n > 0 && k + 1 < last && plan->steps[k + 1].op == DGC_PLAN_COPY && plan->steps[k + 1].stream == s.stream &&
             plan->steps[k + 1].a[0] == a[2] && plan->steps[k + 1].a[2] == n &&
+            plan->steps[k + 1].a[1] <= arena->n && n <= arena->n - plan->steps[k + 1].a[1] &&
             !meets({{plan->steps[k + 1].a[1], n}}, {{a[0], n}, {a[1], n}, {a[2], n}})) {
           R.step = ++k;
           copy = R.at(plan->steps[k].a[1], n);

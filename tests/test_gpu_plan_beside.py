@@ -113,6 +113,16 @@ def test_sum_and_its_copy(ctx, n):
         assert torch.equal(got, want), (src, dst)
 
 
+def test_a_copy_beyond_the_arena_leaves_the_sum_before_it(ctx):
+    """The step that fails is the copy; the sum before it is enqueued as it would be alone."""
+    arena = torch.randn(1024, device="cuda")
+    want = arena[0:64] + arena[64:128]
+    with pytest.raises(dgen_b200.DgenCudaError, match="step 1.*beyond the arena"):
+        _run(ctx, arena, [plan_step(PLAN_ADD, a=(0, 64, 128, 64)), plan_step(PLAN_COPY, a=(128, 1000, 64))])
+    ctx.sync()
+    assert torch.equal(arena[128:192], want)
+
+
 # meet: where the loss's buffers meet those of the steps after it ("" nowhere; partial: its sums lie in the gradient; pred: the
 # convolution's gradient lands on the signal; cell: the loss's value lies in the impulse response's gradient)
 @pytest.mark.parametrize("meet", ["", "partial", "pred", "cell"])
