@@ -55,7 +55,7 @@ def _recorded(ctx, arena, steps, path):
 # layer's input, which its weight gradient reads; grads: one weight gradient buffer, the last one written stays)
 @pytest.mark.parametrize("shared", ["", "dz", "act", "grads"])
 @pytest.mark.parametrize("M,H", [(300, 64), (750, 128), (2100, 64)])
-def test_layers_backward_as_a_plan(ctx, M, H, shared):
+def test_layers_backward_as_a_plan(ctx, M, H, shared, tmp_path):
     g = torch.Generator(device="cuda").manual_seed(M + H)
     used = 0
 
@@ -91,6 +91,8 @@ def test_layers_backward_as_a_plan(ctx, M, H, shared):
         got = arena.clone()
         _run(ctx, got, steps)
         assert torch.equal(got, want)
+    # all gradients of these sizes run beside the next layer's backward; where they meet its buffers it waits for them
+    assert _recorded(ctx, arena.clone(), steps, tmp_path / "layers.dot")[1]
     if not shared:
         z = view(arena, d[L], M, H).double() * (1 - view(arena, x[L], M, H).double() ** 2)
         ref = view(arena, x[L - 1], M, H).double().t() @ z
@@ -98,19 +100,25 @@ def test_layers_backward_as_a_plan(ctx, M, H, shared):
 
 
 @pytest.mark.parametrize("n", [1, 255, 1000])
-def test_sum_and_its_copy(ctx, n):
+def test_sum_and_its_copy(ctx, n, tmp_path):
     base = torch.randn(4 * 1024, device="cuda")
-    for src, dst, copy_n in ((2048, 3072, n), (2048, 0, n), (2048, 1024, n), (2048, 2048 + n // 2, n), (0, 3072, n), (2048, 3072, 1)):
-        # the sum of [0, n) and [1024, ..) at 2048 (or over its first term), then a copy of it elsewhere, on a term, on itself
+    # the sum of [0, n) and [1024, ..) at 2048 (or over its first term), then a copy of it elsewhere, on a term, on the upper half of
+    # itself, of a part of it; one launch only where it lands apart and is whole
+    for src, dst, copy_n, one in ((2048, 3072, n, True), (2048, 0, n, False), (2048, 1024, n, False), (2048, 2048 + n // 2, n, False),
+                                  (0, 3072, n, True), (2048, 3072, 1, n == 1)):
         want = base.clone()
         want[src:src + n] = want[0:n] + want[1024:1024 + n]
-        want[dst:dst + copy_n] = want[src:src + copy_n].clone()
-        got = base.clone()
+        defined = torch.ones(base.numel(), dtype=torch.bool, device="cuda")
+        if dst < src + copy_n and src < dst + copy_n:
+            defined[dst:dst + copy_n] = False      # what a copy leaves where its two ranges meet is not defined
+        else:
+            want[dst:dst + copy_n] = want[src:src + copy_n].clone()
         steps = [plan_step(PLAN_ADD, a=(0, 1024, src, n)), plan_step(PLAN_COPY, a=(src, dst, copy_n))]
-        if dst < src + n and src < dst + copy_n:
-            continue       # a copy onto itself is left to the device's copy, whose overlap is not defined
+        got = base.clone()
         _run(ctx, got, steps)
-        assert torch.equal(got, want), (src, dst)
+        assert torch.equal(got[defined], want[defined]), (src, dst)
+        nodes, _ = _recorded(ctx, base.clone(), steps, tmp_path / "sum.dot")
+        assert nodes == (1 if one else 2), (src, dst, nodes)
 
 
 def test_a_copy_beyond_the_arena_leaves_the_sum_before_it(ctx):
