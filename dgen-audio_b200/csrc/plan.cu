@@ -180,8 +180,10 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
         const uint64_t fb = (uint64_t)p.F * p.B, bt = (uint64_t)p.B * p.T;
         const float *f0 = R.at(a[0], fb), *uv = R.at(a[1], fb), *amps = R.at(a[2], fb * p.K), *gain = R.at(a[3], fb);
         float *scr = R.at(a[4], dgc_harmonic_scratch_floats(&p), true), *out = R.at(a[5], bt);
-        // A step that keeps the scratch for its backward renders partial by partial, with the sines that the backward takes
-        // again: gradients of the log magnitudes hang on the audio's last bits (6e-8 of it moves a step's gradients by 3e-2).
+        // A step that keeps the scratch for its backward is a training step's and renders partial by partial: gradients of the log
+        // magnitudes hang on the audio's last bits (6e-8 of it moves a step's gradients by 3e-2), so a run that goes on from saved
+        // parameters would go on differently.  dgc_harmonic_render sums in groups with a scratch, too: its audio is the same with and
+        // without one, and the sums it leaves there are the more exact ones.
         if (!R.bad) rc = dgc_harmonic_render_impl(ctx, &p, f0, uv, amps, gain, scr, out, scr != nullptr);
       } break;
       case DGC_PLAN_BANDS_TO_TAPS: {

@@ -145,7 +145,12 @@ typedef struct dgc_harmonic_params {
  * Nyquist mask + renormalise (Synth.swift:161-170), stateful phasor of k*f0, sin, weighted sum over
  * partials, times gain*uv*scale.  audio is [B][T].
  * scratch: needs dgc_harmonic_scratch_floats(p) floats of device memory (phase anchors and the
- * per-sample fundamental); pass NULL to let the context keep a buffer of its own. */
+ * per-sample fundamental); pass NULL to let the context keep a buffer of its own.  The audio is the same bits
+ * with and without.
+ * DGC_PHASE_FUNDAMENTAL: the partials of a frame are summed as polynomials in its rotation, to 4e-7 of the
+ * audio's norm whatever K.  A DGC_PLAN_HARMONIC_RENDER step that is given a scratch differs by up to 6e-7 of it:
+ * that is a training step's, whose plan keeps one fast sine per partial from step to step and version to version
+ * (6e-8 of the audio moves the gradients of log magnitudes by 3e-2); without a scratch the step is this call. */
 uint64_t dgc_harmonic_scratch_floats(const dgc_harmonic_params *p);
 int32_t dgc_harmonic_render(dgc_ctx *ctx, const dgc_harmonic_params *p, const float *f0_dev, const float *uv_dev,
                             const float *amps_dev, const float *gain_dev, float *scratch_dev, float *audio_dev);

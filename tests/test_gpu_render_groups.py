@@ -151,6 +151,53 @@ def test_counts_that_change_inside_a_warp(ctx):
     assert (got - _double(f0, amps, 640)).abs().max() < 1e-6 + 2 * np.pi * 100 * 640 * 2.0 ** -33
 
 
+@pytest.mark.parametrize("K", [5, 12, 60, 130])
+def test_a_plan_step_and_the_direct_call(ctx, K):
+    """The step without a scratch is the direct call, bit for bit, whether that is given one or not; with one, a training step's, it
+    takes a fast sine per partial: the same audio, and the same gradient from the sums left there, to that sine's error."""
+    B, T, F = 2, 3000, 40
+    hp = dgen_b200.HarmonicParams(B, T, K, F, SR, 1.0, dgen_b200.PHASE_FUNDAMENTAL, 0)
+    g = torch.Generator(device="cuda").manual_seed(K)
+    draw = lambda lo, hi, *s: torch.rand(*s, generator=g, device="cuda") * (hi - lo) + lo
+    ins = [draw(60.0, 400.0, F, B), draw(0.5, 1.0, F, B), draw(0.0, 1.0, F, B, K), draw(0.5, 1.0, F, B)]
+    n_scr = int(ctx.lib.dgc_harmonic_bwd_scratch_floats(C.byref(hp)))
+    n = [t.numel() for t in ins] + [n_scr, B * T]
+    off = [int(o) for o in np.concatenate([[0], np.cumsum([(v + 63) // 64 * 64 for v in n])])]
+    arena = torch.zeros(off[-1], device="cuda")
+    for o, t in zip(off, ins):
+        arena[o:o + t.numel()] = t.reshape(-1)
+    h = C.c_void_p()
+    ctx.check(ctx.lib.dgc_arena_wrap(ctx.h, arena.data_ptr(), arena.numel(), C.byref(h)))
+
+    def step(scratch):
+        a = off[:4] + [off[4] if scratch else None, off[5]]
+        steps = (dgen_b200.PlanStep * 1)(dgen_b200.plan_step(dgen_b200.PLAN_HARMONIC_RENDER, a=a,
+                                                             i=(B, T, K, F, dgen_b200.PHASE_FUNDAMENTAL, 0), f=(SR, 1.0)))
+        plan = dgen_b200.Plan(steps, 1, None, None, 0)
+        ctx.check(ctx.lib.dgc_plan_run(ctx.h, h, C.byref(plan), 0, -1))
+        ctx.sync()
+        return arena[off[5]:off[5] + B * T].view(B, T).clone()
+
+    ga = torch.randn(B, T, generator=g, device="cuda")
+
+    def gradient(scratch_ptr):
+        out = torch.empty(F, B, K, device="cuda")
+        ctx.check(ctx.lib.dgc_harmonic_render_bwd_prepared(ctx.h, C.byref(hp), *[t.data_ptr() for t in ins], ga.data_ptr(), scratch_ptr,
+                                                           out.data_ptr()))
+        ctx.sync()
+        return out.double()
+
+    scratch = torch.empty(n_scr, device="cuda")
+    kw = dict(phase_mode=dgen_b200.PHASE_FUNDAMENTAL)
+    direct, kept = ctx.harmonic_render(*ins, T, SR, **kw), ctx.harmonic_render(*ins, T, SR, scratch=scratch, **kw)
+    assert torch.equal(direct, kept) and torch.equal(step(False), direct)
+    training = step(True)
+    assert float((training - direct).double().norm() / direct.double().norm()) < 1e-6
+    a, b = gradient(scratch.data_ptr()), gradient(arena.data_ptr() + 4 * off[4])
+    assert float((a - b).norm() / b.norm()) < 1e-6
+    ctx.lib.dgc_arena_destroy(h)
+
+
 @pytest.mark.parametrize("K", [1, 4, 12])
 def test_few_partials_are_no_slower_than_a_sine_each(ctx, K):
     """The render of a plan step that keeps its scratch takes a fast sine per partial; fewer partials than a group must not take longer
