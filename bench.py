@@ -12,8 +12,8 @@ the timed region).  Multi-GPU: one process per GPU (torchrun), voices sharded, n
 collective (forward-only render): weak scaling.
 
 The same JSON line carries, beside the headline:
-  stages       per-stage time with the roofline that bounds that stage (SFU for the oscillator bank, FP32 for the
-               FIR and the loss transforms, HBM for the band -> tap map), and the HBM figure beside it;
+  stages       per-stage time with the roofline that bounds that stage (FP32 for the oscillator bank, the FIR and the
+               loss transforms, HBM for the band -> tap map), and the HBM figure beside it;
   sustained    the step replayed for >= 2 s over rotating input sets (working set > L2) with the SM clock sampled;
   target_b256  (one GPU only) the same step at 256 voices on this one GPU: the configuration the path's
                throughput target is stated on;
@@ -183,6 +183,22 @@ def measured_peaks():
         return {}
 
 
+def host_link_rate(pinned, copies=8):
+    """GB/s of a plain copy from pinned host memory to the device, best of `copies`."""
+    import torch
+    there = torch.empty(pinned.shape, dtype=pinned.dtype, device="cuda")
+    best = 0.0
+    for _ in range(copies):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        a.record()
+        there.copy_(pinned, non_blocking=True)
+        b.record()
+        torch.cuda.synchronize()
+        best = max(best, pinned.numel() * pinned.element_size() / (a.elapsed_time(b) * 1e6))
+    return best
+
+
 def audible_fraction(f0):
     """Share of the (control row, voice, partial) triples whose partial lies below Nyquist: fl(k f0) < sr / 2, the
     reference's mask.  The render evaluates a sine only for those; the rest contribute an exact zero."""
@@ -194,9 +210,11 @@ def audible_fraction(f0):
 def stage_rooflines(B, T, stage_ms, sm_mhz, sm_count, hbm_peak, audible=1.0):
     """Per stage: the bound that applies to it and the fraction reached, the HBM figure beside it.
     Algorithmic work per launch (fp32 = 4 bytes; B voices, T frames, K partials, F control rows):
-      harmonic_render  one sine per (voice, frame, partial BELOW NYQUIST) on the special-function lanes (`audible` =
-                       that share of the B T K partial-frames; the reference evaluates all K and multiplies the
-                       others by a zero mask); bytes 4 (B F (K+2) + B T)
+      harmonic_render  `audible`: share of the B T K partial-frames below Nyquist (the reference evaluates all K and
+                       multiplies the others by a zero mask).  Fundamental mode: 9 flops per audible partial-frame
+                       (interpolation 3, two multiply-adds 4, the amplitude sum 1, an eighth of a complex turn 1) and
+                       140 per frame (six sine-cosine pairs of 23); the other modes one sine per audible partial-frame
+                       on the special-function lanes; bytes 4 (B F (K+2) + B T)
       fir_noise        2 x taps multiply-adds per sample for the two control rows a sample is interpolated between
                        (4 taps flops per sample); bytes 4 (B T + B F nbands + B T): noise in, band magnitudes in, out
       mss_loss_fwd     one complex transform of N points per window carries both signals: 5 N log2 N flops per
@@ -216,7 +234,11 @@ def stage_rooflines(B, T, stage_ms, sm_mhz, sm_count, hbm_peak, audible=1.0):
             continue
         hop = max(1, n // 4)
         fft_flops += 5.0 * n * np.log2(n) * ((T + hop - 1) // hop) * B
-    work = {"harmonic_render": ("sfu", B * T * K * audible / 1e9, sfu_peak, "G sin/s"),
+    if PHASE["mode"] == "fundamental":
+        render = ("fp32", (9.0 * K * audible + 140.0) * B * T / 1e12, fp32_peak, "TFLOP/s")
+    else:
+        render = ("sfu", B * T * K * audible / 1e9, sfu_peak, "G sin/s")
+    work = {"harmonic_render": render,
             "fir_noise": ("fp32", 4.0 * taps * B * T / 1e12, fp32_peak, "TFLOP/s"),
             "mss_loss_fwd": ("fp32", fft_flops / 1e12, fp32_peak, "TFLOP/s"),
             "bands_to_taps": ("hbm", alg_bytes["bands_to_taps"] / 1e9, hbm_peak, "GB/s")}
@@ -229,7 +251,6 @@ def stage_rooflines(B, T, stage_ms, sm_mhz, sm_count, hbm_peak, audible=1.0):
                      "hbm": {"algorithmic_bytes": alg_bytes[name], "achieved_gbs": gbs, "frac": gbs / hbm_peak}}
         bound_time_ms += amount / peak * 1e3
     out["harmonic_render"]["audible_share_of_partials"] = audible
-    out["harmonic_render"]["masked_form_sines_per_s"] = B * T * K / (stage_ms["harmonic_render"] * 1e-3) / 1e9
     return out, alg_bytes, bound_time_ms
 
 
@@ -541,6 +562,7 @@ def run_ours(args, rank, world, local_rank):
     lean_ms = a.elapsed_time(b)
     barrier()
     clocks = sampler.stop() if rank == 0 else None
+    link_gbs = host_link_rate(P["noise"])
     h2d_lean = 4 * sum(int(P[k].numel()) for k in ("f0", "uv", "amps", "gain", "noise_gain", "bands", "W"))
     h2d = 4 * sum(int(P[k].numel()) for k in ("f0", "uv", "amps", "gain", "noise_gain", "bands", "W", "noise")) \
         + 4 * int(target_host.numel())
@@ -592,6 +614,9 @@ def run_ours(args, rank, world, local_rank):
                 # _wait); "blocking" is the one-call-at-a-time form of the same API (dgc_hn_forward_loss_host)
                 "e2e": {"value": samples_per_step * args.steps / (lean_ms * 1e-3), "unit": UNIT,
                         "h2d_bytes_per_step": h2d_lean, "d2h_bytes_per_step": 8, "ms_per_step": lean_ms / args.steps,
+                        # what the link of this box gives one plain copy from the same kind of memory, and the time
+                        # that the step's bytes take at that rate: a slow link reads differently from a slow path
+                        "link_h2d_gbs": link_gbs, "link_ms": h2d_lean / link_gbs / 1e6,
                         "mode": "two steps in flight: step i+1 uploads while step i computes; every step's control-rate "
                                 "inputs (f0, voicing, harmonic amplitudes, gains, band magnitudes, band->tap matrix) come "
                                 "from pinned host memory and its loss returns to the host inside the timed region; the "
@@ -618,8 +643,8 @@ def run_ours(args, rank, world, local_rank):
                                        "peak": hbm_peak, "peak_source": "measured" if peaks else "fallback"},
                                "bound_ms": bound_ms, "frac_of_bound": bound_ms / step_ms,
                                "what": "bound_ms = sum over the stages of (stage work / the peak that bounds it): "
-                                       "special-function lanes for the oscillator bank, FP32 lanes for the FIR "
-                                       "and the loss transforms, measured copy bandwidth for the band -> tap map"},
+                                       "FP32 lanes for the oscillator bank, the FIR and the loss transforms, "
+                                       "measured copy bandwidth for the band -> tap map"},
                 "loss": loss_val, "e2e_loss": e2e_loss}
         if sustained:
             line["sustained"] = sustained
