@@ -46,7 +46,7 @@ STEP_MODE = {"mode": "replay"}
 
 
 def config_json(n_gpus):
-    return {"workload": "harmonic+noise synthesis fwd + multi-scale spectral loss (BASELINE.json configs[1])",
+    return {"workload": "harmonic+noise synthesis fwd + multi-scale spectral loss",
             "voices_per_gpu": CFG["B"], "frames": CFG["T"], "harmonics": CFG["K"], "control_frames": CFG["F"],
             "sample_rate": CFG["sr"], "noise_bands": CFG["nbands"], "fir_taps": CFG["taps"],
             "fft_sizes": list(SIZES), "overlap": 0.75, "global_voices": CFG["B"] * n_gpus,
@@ -717,7 +717,7 @@ def run_target(ctx, args, flush, sm_count, local_rank):
 
 
 # --------------------------------------------------------------------------------------------------
-# training-step workload (BASELINE.json configs[4]): 32 voices per GPU, controller MLP 2-512-512-512-165,
+# training-step workload: 32 voices per GPU, controller MLP 2-512-512-512-165,
 # harmonic+noise synthesis, 1 s learnable IR reverb, multi-scale spectral loss, backward, gradient
 # all-reduce (NCCL) and one Adam step
 # --------------------------------------------------------------------------------------------------
@@ -860,7 +860,7 @@ def train_measure(ctx, args, rank, world, local_rank, steps, voices=32, want_e2e
                          "via": "dgc_allreduce_sum" if used_ctx_comm else
                                 ("torch.distributed" if world > 1 else "none (one rank)"),
                          "what": "CUDA events around the NCCL all-reduce between the two recordings, max over ranks"},
-           "config": {"workload": "full training step (BASELINE.json configs[4])", "frames": T, "harmonics": K,
+           "config": {"workload": "full training step", "frames": T, "harmonics": K,
                       "control_frames": F, "controller": "MLP 2-512-512-512-165 fp32", "ir_taps": 16000,
                       "fft_sizes": list(SIZES), "optimizer": "Adam lr 1e-3", "phase_mode": PHASE["mode"],
                       "l2": "working set (>1 GB per step) exceeds L2"},
@@ -897,7 +897,7 @@ def run_train(args, rank, world, local_rank):
 
 
 # --------------------------------------------------------------------------------------------------
-# the other configurations of the path (BASELINE.json configs[2], configs[3]) and the streaming kernels: one JSON
+# the other configurations of the path and the streaming kernels: one JSON
 # line per kernel family with its own roofline (algorithmic bytes / CUDA-event time against the measured copy
 # bandwidth).  Single GPU; these are replicas-only workloads (no exchange between voices).
 # --------------------------------------------------------------------------------------------------
@@ -920,8 +920,8 @@ def run_filters(args, local_rank):
 
 
 def filters_measure(ctx, args, quick):
-    """One dict per kernel family (the JSON lines of --workload filters).  quick: the configurations BASELINE.json
-    names only (oscillator -> filter -> FFT, biquad bank forward / BPTT, partitioned convolution), fewer steps."""
+    """One dict per kernel family (the JSON lines of --workload filters).  quick: the headline's companions
+    only (oscillator -> filter -> FFT, biquad bank forward / BPTT, partitioned convolution), fewer steps."""
     import ctypes as C
     import torch
     import dgen_b200
@@ -956,7 +956,7 @@ def filters_measure(ctx, args, quick):
         lines.append(line)
 
     scale = args.voices if args.voices > 0 else 0
-    # the reference's own small case (BASELINE.json configs[0]): 64 partials -> one-pole -> buffer(1024, hop 256) -> FFT
+    # the reference's own small case: 64 partials -> one-pole -> buffer(1024, hop 256) -> FFT
     # magnitudes, 65536 frames.  Three launches' worth of work: launch latency, not a roofline, bounds it.
     c1 = wl.osc_filter_fft_inputs()
     fq, am = dev(c1["freq"]), dev(c1["amp"])
@@ -966,7 +966,7 @@ def filters_measure(ctx, args, quick):
         return ctx.stft_mag(ctx.onepole_fwd(osc.view(1, -1), c1["pole"]), c1["N"], c1["hop"])
 
     ms = timed(c1_chain)
-    emit("oscillator bank -> one-pole -> FFT", "64 partials, 65536 frames at 44.1 kHz, FFT 1024 hop 256 (BASELINE.json configs[0])",
+    emit("oscillator bank -> one-pole -> FFT", "64 partials, 65536 frames at 44.1 kHz, FFT 1024 hop 256",
          ms, 4.0 * (2 * 64 + c1["T"] + 256 * 513),
          {"samples_per_s": c1["T"] / (ms * 1e-3), "partial_samples_per_s": 64 * c1["T"] / (ms * 1e-3),
           "roofline_note": "launch bound at this size: three small launches and their allocations"},
@@ -979,7 +979,7 @@ def filters_measure(ctx, args, quick):
     p = dgen_b200.BiquadParams(B, T, L, 1.0, 0.0)
     ms = timed(lambda: ctx.check(ctx.lib.dgc_biquad_fwd(ctx.h, C.byref(p), x.data_ptr(), cut.data_ptr(), q.data_ptr(),
                                                         None, y.data_ptr())))
-    emit("biquad bank forward", "biquad bank %d lanes x %d voices x %d frames (BASELINE.json configs[2])" % (L, B, T),
+    emit("biquad bank forward", "biquad bank %d lanes x %d voices x %d frames" % (L, B, T),
          ms, 4.0 * T * (B + B * L), {"lane_samples_per_s": B * L * T / (ms * 1e-3)})
     target = ctx.biquad_fwd(x, cut * 1.05, q)
     gc, gq = torch.empty(L, device="cuda"), torch.empty(L, device="cuda")
@@ -1000,22 +1000,18 @@ def filters_measure(ctx, args, quick):
     po = torch.empty_like(px)
     ms = timed(lambda: ctx.partconv(px, ir, dd["N"], dd["hop"], out=po))
     K, H, N = (dd["ir"].size + dd["hop"] - 1) // dd["hop"], (px.shape[1] + dd["hop"] - 1) // dd["hop"], dd["N"]
-    emit("partitioned convolution", "partitioned convolution %d voices x %d frames, %d-tap IR (BASELINE.json configs[3])"
+    emit("partitioned convolution", "partitioned convolution %d voices x %d frames, %d-tap IR"
          % (V, px.shape[1], dd["ir"].size), ms, 4.0 * 2 * px.numel() + 8.0 * K * N,
-         {"mac_gflops": 8.0 * K * N * H * V / (ms * 1e6),
-          "roofline_fp32": {"bound": "fp32", "achieved": 8.0 * K * N * H * V / (ms * 1e9), "unit": "TFLOP/s",
-                            "peak": 148 * FP32_LANES_PER_SM * 2 * 1.965e-3,
-                            "frac": 8.0 * K * N * H * V / (ms * 1e9) / (148 * FP32_LANES_PER_SM * 2 * 1.965e-3),
-                            "what": "complex multiply-accumulates of the partitions alone against 148 SMs x 128 "
-                                    "lanes x 2 flops at the maximum SM clock"},
-          "roofline_note": "compute bound: the partitioned multiply-accumulate does 8 K N flops per hop and voice"})
+         {"direct_form_gflops": 8.0 * K * N * H * V / (ms * 1e6),
+          "roofline_note": "bound by the transforms' exchanges through shared memory; the partitions are convolved along the hops by "
+                           "transforms, so the 8 K N flops per hop and voice of the direct form (direct_form_gflops) are not done"})
     del px, ir, po
     torch.cuda.empty_cache()
     return lines
 
 
 def filters_streams(ctx, args, scale, timed, emit):
-    """The streaming kernels and the ring / hold ops on long signals (not BASELINE.json configurations)."""
+    """The streaming kernels and the ring / hold ops on long signals (beside the configurations)."""
     import ctypes as C
     import torch
     import dgen_b200

@@ -280,8 +280,8 @@ DGC_EXPORT int32_t dgc_plan_run(dgc_ctx *ctx, dgc_arena *arena, const dgc_plan *
         float *part = R.at(a[2], dgc_mss_partial_floats(&m), true), *loss = R.at(a[3], 2);
         if (!R.bad && (a[3] & 1)) R.fail("a double must sit at an even offset");
         if (R.bad) break;
-        // nothing waits for the value, so where the loss's gradient comes next the two run beside each other (3 x 16001 frames: a
-        // training step 15 us shorter)
+        // nothing waits for the value, so where the loss's gradient comes next the two run beside each other: a training step of
+        // 32 x 64000 frames 1996 -> 1970 us, one of 3 x 16001 the same 248
         const bool beside = s.stream == 0 && !forked && k + 1 < last && plan->steps[k + 1].op == DGC_PLAN_MSS_LOSS_BWD &&
                             plan->steps[k + 1].stream == 0;
         if (beside) {

@@ -618,7 +618,7 @@ __device__ __forceinline__ float wrapped(float v) {
   return fabsf(w) > half ? folded : w;
 }
 
-// Sine and cosine of a wrapped phase, each to 1.2e-7: folded about a quarter turn, then both polynomials in x^2 (minimax on that
+// Sine and cosine of a wrapped phase, each to 1.5e-7: folded about a quarter turn, then both polynomials in x^2 (minimax on that
 // range, 1e-11 and 2e-10) as the halves of packed multiply-adds: 16 instructions, the library's pair takes three times as many.
 // A phase that is not wrapped (a state handed in, nothing finite) goes to the library.
 __device__ __noinline__ float2 sincos_any(float p) {
