@@ -175,6 +175,7 @@ def test_the_loss_step_of_a_training_plan_runs_by_itself(ctx):
     """A host that changes the audio, or times the steps one by one, runs the loss's step alone."""
     m = trainer.HarmonicModel(ctx, 2, 4000, K=12, F=50, nbands=9, taps=33, hidden=32, ir_len=300, conv_n=256, conv_hop=128, sizes=(512, 128))
     g = torch.Generator(device="cuda").manual_seed(2)
+    assert m.lay.n_steps == 28
     for v in m.input_views():
         v.copy_(torch.rand(v.shape, device="cuda", generator=g))
     m.forward(*m.input_views())
