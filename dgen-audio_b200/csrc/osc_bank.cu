@@ -845,7 +845,7 @@ __device__ __forceinline__ void sincos_turn_q32(uint32_t q, float &s, float &c) 
 //   sum_k a_k sin(2 pi k P) = Im e^(2 pi i (k0 + 9/2) P) (U + i V),
 // the distances being the same in every group.  The groups are a polynomial in e^(2 pi i 8 P), taken by Horner from the last,
 // partly audible one down, each amplitude entering by two multiply-adds, two partials at a time: six angles per frame in all
-// instead of one per partial, a third fewer instructions.  Bound by the loads of the amplitudes that a warp broadcasts (52 % of
+// instead of one per partial, a third fewer instructions.  Bound by the loads of the amplitudes that a warp broadcasts (60 % of
 // the L1's data rate) and by issue: 419 -> 368 us at 256 voices x 64000 frames, 35 -> 29 at 16.
 // Several tiles of frames per block, the next one's lookups in flight, gave 4 % at 256 voices and cost 4 % at 16; fewer
 // registers (48, 40) cost 2 and 23 %.
@@ -874,6 +874,7 @@ harmonic_render_group_kernel(dgc_harmonic_params prm, const float2 *__restrict__
   const int B = prm.B, T = prm.T, K = prm.K, F = prm.F;
   const int C = (T + CH - 1) / CH;
   const int n = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;
+  const unsigned lanes = __ballot_sync(0xffffffffu, n < T);   // of this warp that have a frame
   if (n >= T) return;
   const float2 rt = rowtab[n];
   const int lo = __float_as_int(rt.x), hi = lo + 1 >= F ? 0 : lo + 1;
@@ -897,7 +898,7 @@ harmonic_render_group_kernel(dgc_harmonic_params prm, const float2 *__restrict__
     float *dst = audio + (size_t)b * T + n;
     *dst = prm.accumulate ? *dst + val : val;
   };
-  const int most = __reduce_max_sync(__activemask(), count);   // of the frames of this warp
+  const int most = __reduce_max_sync(lanes, count);   // of the frames of this warp
   if (ROW == ROW_FEW || most <= RENDER_FEW) {
     float c, s, u = 0.0f, v = 0.0f, total = 0.0f;
     sincos_turn_q32((uint32_t)((step + (1ull << 31)) >> 32), s, c);
